@@ -366,25 +366,35 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1) adj_kernel(const AdjA
   }
 }
 
-__global__ void grad_finalize_kernel(const double2 *__restrict__ partial, int n_spans, int E,
-                                     const int32_t *__restrict__ exprs, int n_exprs,
-                                     const int64_t *__restrict__ const_off,
-                                     const int32_t *__restrict__ const_cnt,
-                                     const double *__restrict__ grad_acc, float *__restrict__ mse,
-                                     float *__restrict__ grad, double2 *__restrict__ sums) {
-  const int q_ = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q_ >= n_exprs) return;
+// One warp per expression, its lanes the spans (see finalize_dd_kernel).
+__global__ void __launch_bounds__(256)
+    grad_finalize_kernel(const double2 *__restrict__ partial, int n_spans, int E,
+                         const int32_t *__restrict__ exprs, int n_exprs,
+                         const int64_t *__restrict__ const_off,
+                         const int32_t *__restrict__ const_cnt,
+                         const double *__restrict__ grad_acc, float *__restrict__ mse,
+                         float *__restrict__ grad, double2 *__restrict__ sums) {
+  const int q_ = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (q_ >= n_exprs) return;  // warp-uniform
   const int e = exprs[q_];
   double s = 0.0, c = 0.0;
-  for (int k = 0; k < n_spans; ++k) {
+  for (int k = lane; k < n_spans; k += 32) {
     const double2 q = partial[static_cast<int64_t>(k) * E + e];
     s += q.x;
     c += q.y;
   }
-  if (mse) mse[e] = (c > 0.0) ? static_cast<float>(s / c) : qnan();
-  if (sums) sums[e] = make_double2(s, c);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    c += __shfl_xor_sync(0xffffffffu, c, o);
+  }
+  if (lane == 0) {
+    if (mse) mse[e] = (c > 0.0) ? static_cast<float>(s / c) : qnan();
+    if (sums) sums[e] = make_double2(s, c);
+  }
   const int64_t o = const_off[e];
-  for (int k = 0; k < const_cnt[e]; ++k)
+  for (int k = lane; k < const_cnt[e]; k += 32)
     grad[o + k] = (c > 0.0) ? static_cast<float>(grad_acc[o + k] / c) : qnan();
 }
 
@@ -462,7 +472,7 @@ cudaError_t launch_grad_finalize(const double2 *partial, int n_spans, int E,
                                  const int32_t *const_cnt, const double *grad_acc, float *mse,
                                  float *grad, double2 *sums, cudaStream_t stream) {
   if (n_exprs <= 0) return cudaSuccess;
-  grad_finalize_kernel<<<(n_exprs + 255) / 256, 256, 0, stream>>>(
+  grad_finalize_kernel<<<(n_exprs + 7) / 8, 256, 0, stream>>>(
       partial, n_spans, E, exprs, n_exprs, const_off, const_cnt, grad_acc, mse, grad, sums);
   return cudaGetLastError();
 }

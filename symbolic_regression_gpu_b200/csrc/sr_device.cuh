@@ -734,6 +734,19 @@ __device__ __forceinline__ void dd_add(double &hi, double &lo, double x) {
   hi = s;
 }
 
+// Double-double sums and counts of a warp's lanes added over the warp in a
+// fixed order (lane 0 holds the result).
+__device__ __forceinline__ void dd_warp_sum(double &hi, double &lo, double &cnt) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double h2 = __shfl_down_sync(0xffffffffu, hi, o);
+    const double l2 = __shfl_down_sync(0xffffffffu, lo, o);
+    cnt += __shfl_down_sync(0xffffffffu, cnt, o);
+    dd_add(hi, lo, h2);
+    dd_add(hi, lo, l2);
+  }
+}
+
 // What the producer of an MSE launch folds: the span slots, its accumulators
 // and where a finished item's sums go ([span group][E] entries of two
 // double2: (hi, lo) and (count, 0)).  n_valid: expressions in the launch's

@@ -532,38 +532,56 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) tan_kernel(const TanArg
   }
 }
 
-// mse and grad of the expressions of one tangent launch: the span groups'
-// double-double MSE sums and FP64 gradient sums added in span-group order;
-// the FP64 sums themselves go to sums ((sum, count) per expression) and gsum
-// (per constant).
-__global__ void tan_finalize_kernel(const double2 *__restrict__ partial,
-                                    const double *__restrict__ gout, int n_groups, int E,
-                                    int64_t C, const int32_t *__restrict__ exprs, int n_exprs,
-                                    const int64_t *__restrict__ const_off,
-                                    const int32_t *__restrict__ const_cnt, int K,
-                                    float *__restrict__ mse, float *__restrict__ grad,
-                                    double *__restrict__ gsum, double2 *__restrict__ sums) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n_exprs) return;
+// mse and grad of the expressions of one tangent launch: one warp per
+// expression, the span groups over its lanes (see finalize_dd_kernel), their
+// double-double MSE sums and FP64 gradient sums added over the warp in a fixed
+// order; the FP64 sums themselves go to sums ((sum, count) per expression) and
+// gsum (per constant).  Up to kMaxTangentConsts constants are summed together
+// so that their loads overlap.
+__global__ void __launch_bounds__(256)
+    tan_finalize_kernel(const double2 *__restrict__ partial, const double *__restrict__ gout,
+                        int n_groups, int E, int64_t C, const int32_t *__restrict__ exprs,
+                        int n_exprs, const int64_t *__restrict__ const_off,
+                        const int32_t *__restrict__ const_cnt, int K, float *__restrict__ mse,
+                        float *__restrict__ grad, double *__restrict__ gsum,
+                        double2 *__restrict__ sums) {
+  const int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (q >= n_exprs) return;  // warp-uniform
   const int e = exprs[q];
+  const int nc = min(const_cnt[e], K);
+  const int64_t o = const_off[e];
   double hi = 0.0, lo = 0.0, cnt = 0.0;
-  for (int k = 0; k < n_groups; ++k) {
+  double g[kMaxTangentConsts];
+#pragma unroll
+  for (int c = 0; c < kMaxTangentConsts; ++c) g[c] = 0.0;
+  for (int k = lane; k < n_groups; k += 32) {
     const double2 *pp = partial + 2 * (static_cast<int64_t>(k) * E + e);
     const double2 v = pp[0];
     dd_add(hi, lo, v.x);
     dd_add(hi, lo, v.y);
     cnt += pp[1].x;
+    const double *gk = gout + static_cast<int64_t>(k) * C + o;
+#pragma unroll
+    for (int c = 0; c < kMaxTangentConsts; ++c)
+      if (c < nc) g[c] += gk[c];
   }
-  const double s = isfinite(hi) ? __dadd_rn(hi, lo) : hi;
-  mse[e] = (cnt > 0.0) ? static_cast<float>(s / cnt) : qnan();
-  sums[e] = make_double2(s, cnt);
-  const int nc = min(const_cnt[e], K);
-  const int64_t o = const_off[e];
-  for (int c = 0; c < nc; ++c) {
-    double g = 0.0;
-    for (int k = 0; k < n_groups; ++k) g += gout[static_cast<int64_t>(k) * C + o + c];
-    gsum[o + c] = g;
-    grad[o + c] = (cnt > 0.0) ? static_cast<float>(g / cnt) : qnan();
+  dd_warp_sum(hi, lo, cnt);
+  cnt = __shfl_sync(0xffffffffu, cnt, 0);
+#pragma unroll
+  for (int c = 0; c < kMaxTangentConsts; ++c) {
+    if (c >= nc) break;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) g[c] += __shfl_xor_sync(0xffffffffu, g[c], d);
+    if (lane == 0) {
+      gsum[o + c] = g[c];
+      grad[o + c] = (cnt > 0.0) ? static_cast<float>(g[c] / cnt) : qnan();
+    }
+  }
+  if (lane == 0) {
+    const double s = isfinite(hi) ? __dadd_rn(hi, lo) : hi;
+    mse[e] = (cnt > 0.0) ? static_cast<float>(s / cnt) : qnan();
+    sums[e] = make_double2(s, cnt);
   }
 }
 
@@ -625,7 +643,7 @@ cudaError_t launch_tan_finalize(const double2 *partial, const double *gout, int 
                                 float *mse, float *grad, double *gsum, double2 *sums,
                                 cudaStream_t stream) {
   if (n_exprs <= 0) return cudaSuccess;
-  tan_finalize_kernel<<<(n_exprs + 127) / 128, 128, 0, stream>>>(
+  tan_finalize_kernel<<<(n_exprs + 7) / 8, 256, 0, stream>>>(
       partial, gout, n_groups, E, C, exprs, n_exprs, const_off, const_cnt, K, mse, grad, gsum,
       sums);
   return cudaGetLastError();
