@@ -175,7 +175,7 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1) adj_kernel(const AdjA
   if (warp == W) {
     if (lane == 0)
       run_producer<false>(p.n_groups, n_items, 1, p.n_spans, p.work_counter, p.error, p.X,
-                          p.ldx, rows, span, xbuf, desc, full, empty, FoldArgs{});
+                          p.ldx, rows, span, span, xbuf, desc, full, empty, FoldArgs{});
     return;
   }
 
@@ -266,34 +266,16 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1) adj_kernel(const AdjA
           float y[DPT];
           lds_vec<DPT>(xs + p.V * span, lane, y);
           const bool full_tile = dp0 + TILE <= p.N;
-          float s = 0.0f, c = 0.0f;
-          int nv = 0;
+          float dsq[DPT];
 #pragma unroll
           for (int k = 0; k < DPT; ++k) {
             const bool valid =
                 (full_tile || dp0 + (k / 4) * 128 + lane * 4 + (k % 4) < p.N) && isfinite(T[k]);
             const float df = __fsub_rn(T[k], y[k]);
-            const float sq = valid ? __fmul_rn(df, df) : 0.0f;
-            nv += valid ? 1 : 0;
-            const float yk = __fsub_rn(sq, c);
-            const float tt = __fadd_rn(s, yk);
-            c = __fsub_rn(__fsub_rn(tt, s), yk);
-            s = tt;
+            dsq[k] = __fmul_rn(df, df);
             gT[k] = valid ? 2.0f * df : 0.0f;
           }
-          double tile_sum = static_cast<double>(s) - static_cast<double>(c);
-          if (!isfinite(tile_sum)) {
-            tile_sum = 0.0;
-#pragma unroll
-            for (int k = 0; k < DPT; ++k) {
-              const bool valid = (full_tile || dp0 + (k / 4) * 128 + lane * 4 + (k % 4) < p.N) &&
-                                 isfinite(T[k]);
-              const float df = __fsub_rn(T[k], y[k]);
-              tile_sum += valid ? static_cast<double>(__fmul_rn(df, df)) : 0.0;
-            }
-          }
-          acc += tile_sum;
-          cnt += nv;
+          add_squares<DPT>(T, dsq, full_tile, dp0, lane, p.N, acc, cnt);
         }
         // ---- backward sweep ----
         if (!RECOMP) {

@@ -123,6 +123,7 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
           return;
         }
       }
+      for (Instr &in : code) in.w = sr::with_dispatch(in.w);
     }
   });
   for (int c = 0; c < nt; ++c)
@@ -189,9 +190,9 @@ sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, i
   p.dpt = dpt;
   p.W = W;
   p.ops = (!pred && protected_profile(ps)) ? sr::kOpsProtected : sr::kOpsAll;
-  p.cache = !pred && ps.cache_refs;
   p.smax = std::max(ps.smax, 0);
   p.s_smem = std::min(p.smax, split < 0 ? sr::smem_spill_slots(dpt) : split);
+  p.general = !pred && (ps.cache_refs || p.s_smem < p.smax);
   const int64_t tile = 32 * dpt;
   const int E = ps.E;
   p.G = std::max(1, W * per_warp);
@@ -210,14 +211,14 @@ sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, i
   // (9 variables, 8 datapoints x 8 warps: 2 -> 3 blocks per SM at 512).
   if (span_target > 0) {
     int bps_now = 0;
-    SR_TRY_CUDA(ctx, sr::interp_configure(dpt, pred, p.ops, p.cache,
+    SR_TRY_CUDA(ctx, sr::interp_configure(dpt, pred, p.ops, p.general,
                                           sr::interp_smem_bytes(dpt, W, ctx->V, p.s_smem,
                                                                 static_cast<int>(span), p.G,
                                                                 pred),
                                           W, &bps_now));
     while (span / 2 >= std::max<int64_t>(tile, kMinSpan) && (span / 2) % tile == 0) {
       int bps_half = 0;
-      SR_TRY_CUDA(ctx, sr::interp_configure(dpt, pred, p.ops, p.cache,
+      SR_TRY_CUDA(ctx, sr::interp_configure(dpt, pred, p.ops, p.general,
                                             sr::interp_smem_bytes(dpt, W, ctx->V, p.s_smem,
                                                                   static_cast<int>(span / 2),
                                                                   p.G, pred),
@@ -260,7 +261,7 @@ sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, i
                            "datapoints");
   }
   int bps = 0;
-  SR_TRY_CUDA(ctx, sr::interp_configure(dpt, pred, p.ops, p.cache, p.smem, W, &bps));
+  SR_TRY_CUDA(ctx, sr::interp_configure(dpt, pred, p.ops, p.general, p.smem, W, &bps));
   if (bps <= 0) return ctx->fail(SR_ERR_UNSUPPORTED, "launch shape does not fit on an SM");
   const int64_t resident = static_cast<int64_t>(bps) * ctx->num_sms;
   // Few single-span items per resident block (a small population over few
@@ -357,7 +358,7 @@ sr_status launch_set(sr_context *ctx, ProgramSet &ps, bool pred, int32_t *counte
   a.ldp = ldp;
   a.pred_row = pred_row;
   SR_TRY_CUDA(ctx, cudaMemsetAsync(counter, 0, sizeof(int32_t), ctx->stream));
-  SR_TRY_CUDA(ctx, sr::launch_interp(ps.plan.dpt, pred, ps.plan.ops, ps.plan.cache, a,
+  SR_TRY_CUDA(ctx, sr::launch_interp(ps.plan.dpt, pred, ps.plan.ops, ps.plan.general, a,
                                      ps.plan.blocks, ps.plan.smem,
                                      ctx->stream));
   return SR_OK;

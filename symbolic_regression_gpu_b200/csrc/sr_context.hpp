@@ -97,7 +97,9 @@ struct Plan {
   int dpt = 8;
   int W = 8;           // evaluating warps per block
   int ops = 0;         // operator profile dispatched inline (kOpsAll / kOpsProtected)
-  bool cache = false;  // programs read cached subtrees (cached-operand paths compiled in)
+  // programs read cached subtrees, or spill slots in global scratch (the
+  // interpreter's general operand paths compiled in)
+  bool general = false;
   int smax = 0;        // spill slots per warp
   int s_smem = 0;      // of which in shared memory
   int G = 0;           // expressions per group

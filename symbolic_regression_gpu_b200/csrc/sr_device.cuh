@@ -509,12 +509,12 @@ constexpr int kInlineMaxDpt = 8;  // wider launches call them (16 copies overflo
       CALLED                                                                   \
     }                                                                          \
     break;
-#define SR_C_EXPC_INL                                                          \
-  SR_C_INL_OR(32, T[k] = expf(fminf(T[k], 80.0f)),                             \
+#define SR_EXPC_INL(CASE)                                                      \
+  SR_C_INL_OR(CASE, T[k] = expf(fminf(T[k], 80.0f)),                             \
               _Pragma("unroll") for (int k = 0; k < DPT; ++k) T[k] = fminf(T[k], 80.0f); \
               SR_MAP1(v_exp, T, T))
-#define SR_C_LSQRT_INL                                                         \
-  SR_C_INL_OR(27, T[k] = __fsqrt_rn(fabsf(T[k])),                              \
+#define SR_LSQRT_INL(CASE)                                                     \
+  SR_C_INL_OR(CASE, T[k] = __fsqrt_rn(fabsf(T[k])),                              \
               _Pragma("unroll") for (int k = 0; k < DPT; ++k) T[k] = fabsf(T[k]); \
               SR_MAP1(v_sqrt, T, T))
 #define SR_C_LDIV_INL                                                          \
@@ -559,10 +559,8 @@ __device__ __noinline__ void sincos_cold(float *T, int q_offset) {
       SR_MAP1(NAME, T, T)                                                      \
     }                                                                          \
     break;
-#define SR_C_SIN_INL SR_C_SINCOS_INL(10, 0, v_sin)
-#define SR_C_COS_INL SR_C_SINCOS_INL(11, 1, v_cos)
-#define SR_C_LLOG_INL                                                          \
-  SR_C_INL_OR(22, if ((k & 1) == 0) {                                          \
+#define SR_LLOG_INL(CASE)                                                      \
+  SR_C_INL_OR(CASE, if ((k & 1) == 0) {                                          \
                 const float2 l_ = sr_log_nonneg2(fabsf(T[k]), fabsf(T[k + 1])); \
                 T[k] = T[k] == 0.0f ? -1e9f : l_.x;                            \
                 T[k + 1] = T[k + 1] == 0.0f ? -1e9f : l_.y;                    \
@@ -589,10 +587,12 @@ __device__ __noinline__ void sincos_cold(float *T, int q_offset) {
 // a population that uses every operator (the reference generator's) runs
 // faster with all of them inline.
 
+// Every operator but 0 and + - *, which the dispatch codes cover for every
+// kind of operand.
 template <int DPT>
 __device__ __forceinline__ void apply_op_any(uint32_t op, float (&T)[DPT], float (&b)[DPT]) {
   switch (op) {
-    SR_C_NONE SR_C_ADD SR_C_SUB SR_C_RSUB SR_C_MUL SR_C_DIV SR_C_RDIV SR_C_POW SR_C_RPOW
+    SR_C_DIV SR_C_RDIV SR_C_POW SR_C_RPOW
     SR_C_MIN SR_C_RMIN SR_C_MAX SR_C_RMAX SR_C_LDIV SR_C_RLDIV SR_C_LPOW SR_C_RLPOW
     SR_C_SIN SR_C_COS SR_C_TAN SR_C_SINH SR_C_COSH SR_C_TANH SR_C_EXP SR_C_LOG SR_C_INV
     SR_C_ASIN SR_C_ACOS SR_C_ATAN SR_C_LLOG SR_C_LINV SR_C_ABS SR_C_NEG SR_C_SQRT SR_C_LSQRT
@@ -613,8 +613,8 @@ __device__ __forceinline__ void apply_op_cold_switch(uint32_t op, float (&T)[DPT
     SR_C_NONE SR_C_ADD SR_C_SUB SR_C_RSUB SR_C_MUL SR_C_DIV SR_C_RDIV SR_C_POW SR_C_RPOW
     SR_C_MIN SR_C_RMIN SR_C_MAX SR_C_RMAX SR_C_LDIV_INL SR_C_RLDIV_INL SR_C_LPOW SR_C_RLPOW
     SR_C_SIN SR_C_COS SR_C_TAN SR_C_SINH SR_C_COSH SR_C_TANH SR_C_EXP SR_C_LOG SR_C_INV
-    SR_C_ASIN SR_C_ACOS SR_C_ATAN SR_C_LLOG SR_C_LINV SR_C_ABS SR_C_NEG SR_C_SQRT SR_C_LSQRT_INL
-    SR_C_EXPC_INL
+    SR_C_ASIN SR_C_ACOS SR_C_ATAN SR_C_LLOG SR_C_LINV SR_C_ABS SR_C_NEG SR_C_SQRT SR_LSQRT_INL(27)
+    SR_EXPC_INL(32)
     default: SR_EACH(T[k] = 0.0f)
   }
 }
@@ -632,44 +632,28 @@ __device__ __noinline__ void apply_op_cold(uint32_t op, float *T, float *b) {
   for (int k = 0; k < DPT; ++k) T[k] = t[k];
 }
 
-#define SR_C_COLD                                                              \
-  default: {                                                                   \
-    float t_[DPT], b_[DPT];                                                    \
-    _Pragma("unroll") for (int k = 0; k < DPT; ++k) {                          \
-      t_[k] = T[k];                                                            \
-      b_[k] = b[k];                                                            \
-    }                                                                          \
-    apply_op_cold<DPT>(op, t_, b_);                                            \
-    _Pragma("unroll") for (int k = 0; k < DPT; ++k) T[k] = t_[k];              \
-  } break;
-
-template <int DPT, int OPS>
-__device__ __forceinline__ void apply_op(uint32_t op, float (&T)[DPT], float (&b)[DPT]) {
-  if constexpr (OPS == kOpsProtected) {
-    switch (op) {
-      SR_C_NONE SR_C_ADD SR_C_SUB SR_C_RSUB SR_C_MUL SR_C_LDIV_INL SR_C_RLDIV_INL SR_C_SIN_INL
-      SR_C_COS_INL SR_C_EXPC_INL SR_C_LLOG_INL SR_C_LSQRT_INL
-      SR_C_COLD
-    }
-  } else {
-    apply_op_any<DPT>(op, T, b);
-  }
-}
-
-#undef SR_EACH
-#undef SR_CALL1
-#undef SR_CALL2
-#undef SR_C_COLD
 
 // Run one compiled program over the warp's DPT x 32 datapoints of a tile.
-// xs points at the tile's first datapoint of X row 0; rows are xrs floats
-// apart.
-template <int DPT, int OPS, bool CACHE>
-__device__ __forceinline__ void run_program(const Instr *__restrict__ code,
-                                            int len, const float *xs, int xrs,
-                                            const SpillStack &st, int lane,
+// xs points at the tile's X rows [rows][TILE] in shared memory.  GEN = false
+// leaves out cached-subtree operands and spill slots beyond the shared-memory
+// ones, for launches whose programs have none (dispatch stays short).
+//
+// Issue-bound: the schedulers issue on nearly every cycle, so time is the
+// number of instructions.  Each bytecode instruction costs one test of the
+// load / spill flags, one operand address and one indirect branch on its
+// dispatch code, whose case loads the operand where the operator takes it
+// (+ - * straight into the paired operations; a constant is not spread over
+// DPT registers first).  Batched population (10,000 x 1M) 55.1 -> 49.2 ms,
+// 8,000 long programs x 4M 326 -> 287 ms against separate branches for the
+// operand's kind and the opcode.
+template <int DPT, int OPS, bool GEN>
+__device__ __forceinline__ void run_program(const Instr *__restrict__ code, int len,
+                                            const float *xs, const SpillStack &st, int lane,
                                             const float *cache, int64_t ldc, int64_t dp0,
                                             float (&T)[DPT]) {
+  constexpr int TILE = 32 * DPT;
+  const float *xl = xs + lane * 4;
+  float *sl = st.ss + lane * 4;
   // Every program starts with an instruction that loads T.
   uint4 ins = ldg_instr(code);
   for (int i = 0; i < len; ++i) {
@@ -678,33 +662,202 @@ __device__ __forceinline__ void run_program(const Instr *__restrict__ code,
     const uint4 nxt = ldg_instr(code + i + 1);
     const uint32_t w = ins.x;
     if (w & (kLoadBit | kSpillBit)) {
-      if (instr_spill(w)) spill_store<DPT>(st, instr_spill_slot(w), lane, T);
-      if (instr_load(w))
-        load_leaf<DPT, CACHE>(instr_leaf_kind(w), ins.y, T, xs, xrs, lane, cache, ldc, dp0);
+      if (GEN) {
+        if (instr_spill(w)) spill_store<DPT>(st, instr_spill_slot(w), lane, T);
+      } else if (instr_spill(w)) {
+        sts_vec<DPT>(sl + instr_spill_slot(w) * TILE, 0, T);
+      }
+      if (instr_load(w)) {
+        if (instr_leaf_kind(w) == kLeafX) {
+          lds_vec<DPT>(xl + ins.y * TILE, 0, T);
+        } else if (!GEN || instr_leaf_kind(w) == kLeafC) {
+          const float c = __uint_as_float(ins.y);
+#pragma unroll
+          for (int k = 0; k < DPT; ++k) T[k] = c;
+        } else {
+          ldg_vec<DPT>(cache + static_cast<int64_t>(ins.y) * ldc + dp0, lane, T);
+        }
+      }
     }
-    float b[DPT];
-    const uint32_t bk = instr_b_kind(w);
-    if (bk != kBNone) load_operand<DPT, CACHE>(bk, ins.z, b, xs, xrs, st, lane, cache, ldc, dp0);
-    apply_op<DPT, OPS>(instr_op(w), T, b);
+    const uint32_t d = instr_dispatch(w);
+    const float cb = __uint_as_float(ins.z);
+    const float2 c2 = make_float2(cb, cb);
+    // Operand b in shared memory: a spill slot (kind 1) or a variable row (2).
+    const float *bp = ((w & (2u << 9)) ? xl : sl) + ins.z * TILE;
+    // General launches read a memory operand into registers by its kind.
+    float bg[GEN ? DPT : 1];
+    if constexpr (GEN) {
+      const uint32_t bk = instr_b_kind(w);
+      if (bk == kBR)
+        ldg_vec<DPT>(cache + static_cast<int64_t>(ins.z) * ldc + dp0, lane, bg);
+      else if (bk == kBS)
+        spill_load<DPT>(st, ins.z, lane, bg);
+      else if (bk == kBX)
+        lds_vec<DPT>(bp, 0, bg);
+    }
+    auto quad_b = [&](int h) {
+      if constexpr (GEN)
+        return make_float4(bg[4 * h], bg[4 * h + 1], bg[4 * h + 2], bg[4 * h + 3]);
+      else
+        return *reinterpret_cast<const float4 *>(bp + h * 128);
+    };
+#define SR_F_MEM(EXPR)                                                         \
+  {                                                                            \
+    _Pragma("unroll") for (int h = 0; h < DPT / 4; ++h) {                      \
+      const float4 q = quad_b(h);                                              \
+      {                                                                        \
+        const float2 t_ = make_float2(T[4 * h], T[4 * h + 1]);                 \
+        const float2 u_ = make_float2(q.x, q.y);                               \
+        const float2 r_ = (EXPR);                                              \
+        T[4 * h] = r_.x;                                                       \
+        T[4 * h + 1] = r_.y;                                                   \
+      }                                                                        \
+      {                                                                        \
+        const float2 t_ = make_float2(T[4 * h + 2], T[4 * h + 3]);             \
+        const float2 u_ = make_float2(q.z, q.w);                               \
+        const float2 r_ = (EXPR);                                              \
+        T[4 * h + 2] = r_.x;                                                   \
+        T[4 * h + 3] = r_.y;                                                   \
+      }                                                                        \
+    }                                                                          \
+  }                                                                            \
+  break;
+#define SR_F_CONST(EXPR)                                                       \
+  {                                                                            \
+    _Pragma("unroll") for (int k = 0; k < DPT; k += 2) {                       \
+      const float2 t_ = make_float2(T[k], T[k + 1]);                           \
+      const float2 u_ = c2;                                                    \
+      const float2 r_ = (EXPR);                                                \
+      T[k] = r_.x;                                                             \
+      T[k + 1] = r_.y;                                                         \
+    }                                                                          \
+  }                                                                            \
+  break;
+#define SR_F_CHEAP                                                             \
+  case kDNone: break;                                                          \
+  case kDAddM: SR_F_MEM(__fadd2_rn(t_, u_))                                    \
+  case kDSubM: SR_F_MEM(__fadd2_rn(t_, make_float2(-u_.x, -u_.y)))             \
+  case kDRSubM: SR_F_MEM(__fadd2_rn(u_, make_float2(-t_.x, -t_.y)))            \
+  case kDMulM: SR_F_MEM(__fmul2_rn(t_, u_))                                    \
+  case kDAddC: SR_F_CONST(__fadd2_rn(t_, u_))                                  \
+  case kDSubC: SR_F_CONST(__fadd2_rn(t_, make_float2(-u_.x, -u_.y)))           \
+  case kDRSubC: SR_F_CONST(__fadd2_rn(u_, make_float2(-t_.x, -t_.y)))          \
+  case kDMulC: SR_F_CONST(__fmul2_rn(t_, u_))
+    auto memory_b = [&](float (&b)[DPT]) {
+#pragma unroll
+      for (int h = 0; h < DPT / 4; ++h) unquad<DPT>(b, h, quad_b(h));
+    };
+    auto operand = [&](float (&b)[DPT]) {
+      const uint32_t bk = instr_b_kind(w);
+      if (bk == kBC) {
+#pragma unroll
+        for (int k = 0; k < DPT; ++k) b[k] = cb;
+      } else if (bk != kBNone) {
+        memory_b(b);
+      }
+    };
+    if constexpr (OPS == kOpsProtected) {
+      switch (d) {
+        SR_F_CHEAP
+        case kDLDivM:
+        case kDRLDivM:
+        case kDLDivC:
+        case kDRLDivC: {  // T / protected(b), b / protected(T): one division
+          float b[DPT];
+          if ((d - kDLDivM) & 2u) {
+#pragma unroll
+            for (int k = 0; k < DPT; ++k) b[k] = cb;
+          } else {
+            memory_b(b);
+          }
+          if ((d - kDLDivM) & 1u) {
+#pragma unroll
+            for (int k = 0; k < DPT; ++k) {
+              const float t = T[k];
+              T[k] = b[k];
+              b[k] = t;
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < DPT; ++k) b[k] = loose_denom(b[k]);
+          if constexpr (DPT <= kInlineMaxDpt) {
+#pragma unroll
+            for (int k = 0; k < DPT; ++k) T[k] = __fdiv_rn(T[k], b[k]);
+          } else {
+            SR_MAP2(v_div, T, T, b)
+          }
+        } break;
+        SR_C_SINCOS_INL(kDSin, 0, v_sin)
+        SR_C_SINCOS_INL(kDCos, 1, v_cos)
+        SR_EXPC_INL(kDExpC)
+        SR_LLOG_INL(kDLLog)
+        SR_LSQRT_INL(kDLSqrt)
+        default: {
+          float t_[DPT], b_[DPT];
+          operand(b_);
+#pragma unroll
+          for (int k = 0; k < DPT; ++k) t_[k] = T[k];
+          apply_op_cold<DPT>(instr_op(w), t_, b_);
+#pragma unroll
+          for (int k = 0; k < DPT; ++k) T[k] = t_[k];
+        }
+      }
+    } else {
+      switch (d) {
+        SR_F_CHEAP
+        default: {
+          float b[DPT];
+          operand(b);
+          apply_op_any<DPT>(instr_op(w), T, b);
+        }
+      }
+    }
+#undef SR_F_CHEAP
+#undef SR_F_MEM
+#undef SR_F_CONST
     ins = nxt;
   }
 }
+#undef SR_EACH
+#undef SR_CALL1
+#undef SR_CALL2
 
-// Sum of the valid squared errors of a lane's DPT datapoints in FP64: the
-// fallback when the FP32 Kahan sum overflowed (or a square is infinite); exact
-// for DPT finite squares and +Inf when one is infinite, like the reference's
-// double sum.  Out of line: it almost never runs.
+// Adds a lane's DPT squared errors (FP32 products, dsq) to its running FP64
+// sum and counts the valid datapoints (finite predictions, inside the dataset;
+// reference cl_cpu_eval.cpp:147-150).  A full tile whose FP64 sum is finite
+// holds no invalid prediction (a NaN or infinite one makes its square NaN or
+// infinite) and, DPT finite floats never overflowing a double, no infinite
+// square: its sum and count stand.  Any other lane goes over its datapoints one
+// by one; an infinite square of a finite prediction gives +Inf like the
+// reference's double sum.  Conversions and FP64 adds replace an FP32 Kahan
+// chain with a validity test, a select and a count per datapoint: about half
+// the instructions, and the sum is that of the products without its own
+// rounding (batched population 56.7 -> 55.1 ms).
 template <int DPT>
-__device__ __noinline__ double tile_sum_fp64(const float *T, const float *y, bool full,
-                                             int64_t dp0, int lane, int64_t N) {
-  double sum = 0.0;
+__device__ __forceinline__ void add_squares(const float (&T)[DPT], const float (&dsq)[DPT],
+                                            bool full, int64_t dp0, int lane, int64_t N,
+                                            double &acc, int &cnt) {
+  double s0 = static_cast<double>(dsq[0]), s1 = static_cast<double>(dsq[1]);
 #pragma unroll
-  for (int k = 0; k < DPT; ++k) {
-    const bool valid = (full || dp0 + (k / 4) * 128 + lane * 4 + (k % 4) < N) && isfinite(T[k]);
-    const float df = __fsub_rn(T[k], y[k]);
-    sum += valid ? static_cast<double>(__fmul_rn(df, df)) : 0.0;
+  for (int k = 2; k < DPT; k += 2) {
+    s0 += static_cast<double>(dsq[k]);
+    s1 += static_cast<double>(dsq[k + 1]);
   }
-  return sum;
+  double s = s0 + s1;
+  int n = DPT;
+  if (!full || !isfinite(s)) {
+    s = 0.0;
+    n = 0;
+#pragma unroll
+    for (int k = 0; k < DPT; ++k) {
+      const bool valid =
+          (full || dp0 + (k / 4) * 128 + lane * 4 + (k % 4) < N) && isfinite(T[k]);
+      s += static_cast<double>(valid ? dsq[k] : 0.0f);
+      n += valid ? 1 : 0;
+    }
+  }
+  acc += s;
+  cnt += n;
 }
 
 // Per-span result of one expression of a work item, written by the warp that
@@ -776,14 +929,17 @@ struct FoldArgs {
 // cheapest), and copies each of the item's spans
 // (k_spans consecutive spans, the last group shorter) with every row of X
 // into one of kBufs shared-memory buffers with the bulk-copy engine;
-// publishes item -1 when the work runs out.  With FOLD (MSE launches) it also
+// publishes item -1 when the work runs out.  A span lies in its buffer as
+// [span / chunk][rows][chunk] (`chunk` divides the span and is a multiple of 4
+// floats): with chunk = the tile of a warp, variable rows and spill slots have
+// the same stride, so one address computation serves both.  With FOLD (MSE launches) it also
 // folds, once the warps have released a buffer, the span slots written for it
 // into the item's accumulators (in span order) and writes each finished
 // item's sums out.  Every wait is bounded.
 template <bool FOLD>
 __device__ __noinline__ void run_producer(int n_groups, int n_items, int k_spans, int n_spans,
                                           int32_t *work_counter, int32_t *error, const float *X,
-                                          int64_t ldx, int rows, int span, float *xbuf,
+                                          int64_t ldx, int rows, int span, int chunk, float *xbuf,
                                           ItemDesc *desc, uint64_t *full, uint64_t *empty,
                                           FoldArgs fa) {
   uint32_t buf = 0, phase = 0;
@@ -793,6 +949,7 @@ __device__ __noinline__ void run_producer(int n_groups, int n_items, int k_spans
   int held_item[kBufs] = {0, 0}, held_group[kBufs] = {0, 0};
   int acc_item = -1, acc_sg = 0, acc_n = 0;
   const uint32_t row_bytes = static_cast<uint32_t>(span) * sizeof(float);
+  const uint32_t chunk_bytes = static_cast<uint32_t>(chunk) * sizeof(float);
 
   auto flush = [&]() {
     if constexpr (FOLD) {
@@ -880,8 +1037,10 @@ __device__ __noinline__ void run_producer(int n_groups, int n_items, int k_spans
       mbar_arrive_expect_tx(&full[buf], row_bytes * rows);
       const float *src = X + static_cast<int64_t>(sp) * span;
       float *dst = xbuf + static_cast<size_t>(buf) * rows * span;
-      for (int v = 0; v < rows; ++v)
-        bulk_g2s(dst + static_cast<size_t>(v) * span, src + v * ldx, row_bytes, &full[buf]);
+      for (int c = 0; c < span; c += chunk)
+        for (int v = 0; v < rows; ++v)
+          bulk_g2s(dst + static_cast<size_t>(c) * rows + static_cast<size_t>(v) * chunk,
+                   src + v * ldx + c, chunk_bytes, &full[buf]);
       armed |= 1u << buf;
       fill_phase[buf] = phase;
       held[buf] = FOLD;

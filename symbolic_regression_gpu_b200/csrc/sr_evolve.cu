@@ -552,7 +552,11 @@ __global__ void compile_kernel(const int32_t *__restrict__ tok, const float *__r
   }
   code_len[i] = count;
   int prot = 0;
-  for (int k = 0; k < count; ++k) prot += in_protected_profile(instr_op(code[base + k].w)) ? 1 : 0;
+  for (int k = 0; k < count; ++k) {
+    const uint32_t w = with_dispatch(code[base + k].w);
+    code[base + k].w = w;
+    prot += in_protected_profile(instr_op(w)) ? 1 : 0;
+  }
   if (prot) atomicAdd(&summary[6], prot);
   atomicMax(&summary[0], need);
   atomicAdd(reinterpret_cast<unsigned long long *>(summary + 2), static_cast<unsigned long long>(n));

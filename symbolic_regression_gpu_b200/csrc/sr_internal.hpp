@@ -29,6 +29,10 @@
 //                        2 = variable row, 3 = constant, 4 = cached subtree
 //            bit  12     spill: store T into S[spill slot] first
 //            bits 13..17 spill slot
+//            bits 18..22 dispatch code (kD*): what the interpreter's switch
+//                        branches on, a function of opcode and operand kind
+//                        (with_dispatch), filled in when programs are laid
+//                        out for the device; no other kernel reads it
 //   Instr.a  payload of leaf A, Instr.b payload of operand b: spill slot /
 //            variable row / float bits of the constant / cache slot
 //   Instr.c  bits 0..9 / 10..19: constant index (token order) of leaf A /
@@ -94,6 +98,39 @@ SR_HD bool in_protected_profile(uint32_t op) {
   return op == 0 || op == 1 || op == 2 || op == kOpReversed + 2 || op == 3 || op == 8 ||
          op == kOpReversed + 8 || op == 10 || op == 11 || op == kOpExpClamp || op == 22 ||
          op == 27;
+}
+
+// Dispatch codes: the frequent operators with the place of operand b folded
+// in (M: memory, a variable row, a spill slot or a cached subtree; C: a
+// constant), so that one branch reaches code that loads the operand and
+// applies the operator.  kDAny: every other combination (operand by kind, then a switch
+// over the opcodes).
+enum : uint32_t {
+  kDAny = 0, kDNone, kDAddM, kDSubM, kDRSubM, kDMulM, kDAddC, kDSubC, kDRSubC, kDMulC,
+  kDLDivM, kDRLDivM, kDLDivC, kDRLDivC, kDSin, kDCos, kDExpC, kDLLog, kDLSqrt
+};
+constexpr int kDShift = 18;
+SR_HD uint32_t instr_dispatch(uint32_t w) { return (w >> kDShift) & 31u; }
+SR_HD uint32_t with_dispatch(uint32_t w) {
+  const uint32_t bk = instr_b_kind(w);
+  const bool m = bk == kBS || bk == kBX || bk == kBR, c = bk == kBC;
+  uint32_t d = kDAny;
+  switch (instr_op(w)) {
+    case 0: d = kDNone; break;
+    case 1: d = m ? kDAddM : (c ? kDAddC : kDAny); break;
+    case 2: d = m ? kDSubM : (c ? kDSubC : kDAny); break;
+    case kOpReversed + 2: d = m ? kDRSubM : (c ? kDRSubC : kDAny); break;
+    case 3: d = m ? kDMulM : (c ? kDMulC : kDAny); break;
+    case 8: d = m ? kDLDivM : (c ? kDLDivC : kDAny); break;
+    case kOpReversed + 8: d = m ? kDRLDivM : (c ? kDRLDivC : kDAny); break;
+    case 10: d = kDSin; break;
+    case 11: d = kDCos; break;
+    case kOpExpClamp: d = kDExpC; break;
+    case 22: d = kDLLog; break;
+    case 27: d = kDLSqrt; break;
+    default: break;
+  }
+  return (w & ~(31u << kDShift)) | (d << kDShift);
 }
 
 // Device-side error word bits.

@@ -15,8 +15,8 @@
 //                             32 lanes x DPT datapoints per instruction fetch,
 //                             accumulator in registers, spilled values in a
 //                             per-warp shared stack.  The epilogue either
-//                             accumulates the squared error (FP32 Kahan over a
-//                             lane's DPT values, FP64 across tiles and lanes)
+//                             accumulates the squared error (FP32 squares, FP64
+//                             sums)
 //                             or stores the predictions.
 //  finalize_kernel            per-expression combination of span partials in
 //                             a fixed order: mse = sum / count.
@@ -49,7 +49,7 @@ namespace {
 
 // MAXW / MINB: launch bounds of the instantiation (at most MAXW evaluating
 // warps, at least MINB resident blocks per SM), which set the register budget.
-template <int DPT, bool PRED, int MAXW, int MINB, int OPS, bool CACHE>
+template <int DPT, bool PRED, int MAXW, int MINB, int OPS, bool GEN>
 __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) interp_kernel(const EvalArgs p) {
   constexpr int TILE = 32 * DPT;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) interp_kernel(const Eva
   if (warp == W) {
     if (lane == 0)
       run_producer<!PRED>(p.n_groups, n_items, k_spans, p.n_spans, p.work_counter, p.error, p.X,
-                          p.ldx, rows, span, xbuf, desc, full, empty,
+                          p.ldx, rows, span, TILE, xbuf, desc, full, empty,
                           FoldArgs{part, gacc, p.partial, p.G, p.E, p.E, 0, nullptr, nullptr, nullptr,
                                    nullptr, nullptr, 0});
     return;
@@ -116,17 +116,15 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) interp_kernel(const Eva
       for (int t = 0; t < tiles; ++t) {
         const int64_t dp0 = dp_span + static_cast<int64_t>(t) * TILE;
         if (dp0 >= p.N) break;  // tail of the last span
-        const float *xs = xb + t * TILE;
+        const float *xs = xb + static_cast<size_t>(t) * rows * TILE;
         float T[DPT];
-        run_program<DPT, OPS, CACHE>(code, len, xs, span, st, lane, p.cache, p.ldc, dp0, T);
+        run_program<DPT, OPS, GEN>(code, len, xs, st, lane, p.cache, p.ldc, dp0, T);
         if constexpr (PRED) {
           stg_vec<DPT>(p.pred + static_cast<int64_t>(p.pred_row[e]) * p.ldp + dp0, lane, T);
         } else {
           float y[DPT];
-          lds_vec<DPT>(xs + p.V * span, lane, y);
+          lds_vec<DPT>(xs + p.V * TILE, lane, y);
           const bool full = dp0 + TILE <= p.N;  // warp-uniform
-          float s = 0.0f, c = 0.0f;  // Kahan over the lane's DPT values
-          int nv = 0;
           float dsq[DPT];  // squared residuals, two datapoints per paired operation
 #pragma unroll
           for (int k = 0; k < DPT; k += 2) {
@@ -136,29 +134,7 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) interp_kernel(const Eva
             dsq[k] = sq2.x;
             dsq[k + 1] = sq2.y;
           }
-#pragma unroll
-          for (int k = 0; k < DPT; ++k) {
-            const bool valid =
-                (full || dp0 + (k / 4) * 128 + lane * 4 + (k % 4) < p.N) && isfinite(T[k]);
-            const float sq = valid ? dsq[k] : 0.0f;
-            nv += valid ? 1 : 0;
-            const float yk = __fsub_rn(sq, c);
-            const float tt = __fadd_rn(s, yk);
-            c = __fsub_rn(__fsub_rn(tt, s), yk);
-            s = tt;
-          }
-          double tile_sum = static_cast<double>(s) - static_cast<double>(c);
-          if (!isfinite(tile_sum)) {
-            float tc[DPT], yc[DPT];
-#pragma unroll
-            for (int k = 0; k < DPT; ++k) {
-              tc[k] = T[k];
-              yc[k] = y[k];
-            }
-            tile_sum = tile_sum_fp64<DPT>(tc, yc, full, dp0, lane, p.N);
-          }
-          acc += tile_sum;
-          cnt += nv;
+          add_squares<DPT>(T, dsq, full, dp0, lane, p.N, acc, cnt);
         }
       }
       if constexpr (!PRED) {
@@ -487,14 +463,14 @@ size_t interp_smem_bytes(int dpt, int W, int V, int s_smem, int span, int G, boo
          (pred ? 0 : static_cast<size_t>(G) * (kBufs * sizeof(SpanPart) + sizeof(GroupAcc)));
 }
 
-template <int DPT, bool PRED, int MAXW, int MINB, int OPS = kOpsAll, bool CACHE = false>
+template <int DPT, bool PRED, int MAXW, int MINB, int OPS = kOpsAll, bool GEN = true>
 static const void *interp_fn() {
-  return reinterpret_cast<const void *>(&interp_kernel<DPT, PRED, MAXW, MINB, OPS, CACHE>);
+  return reinterpret_cast<const void *>(&interp_kernel<DPT, PRED, MAXW, MINB, OPS, GEN>);
 }
 
 template <int DPT, int MAXW, int MINB>
-static const void *interp_mse(int ops, bool cache) {
-  if (cache)
+static const void *interp_mse(int ops, bool general) {
+  if (general)
     return ops == kOpsProtected ? interp_fn<DPT, false, MAXW, MINB, kOpsProtected, true>()
                                 : interp_fn<DPT, false, MAXW, MINB, kOpsAll, true>();
   return ops == kOpsProtected ? interp_fn<DPT, false, MAXW, MINB, kOpsProtected, false>()
@@ -507,23 +483,24 @@ static const void *interp_mse(int ops, bool cache) {
 // block of up to 31 + 1 warps, both at 64 registers: on the batched
 // population the interpreter is latency-bound, and 30 or 31 evaluating warps
 // per SM beat 24 at 72 registers: 65.2 -> 60.1 and 58.8 ms).  MSE launches
-// come in both operator profiles, with and without cached-subtree operands;
-// prediction launches (cache fills, predictions) in kOpsAll without.
-static const void *select_interp(int dpt, bool pred, int ops, bool cache, int W) {
+// come in both operator profiles, with and without the general operand paths
+// (cached subtrees, spill slots in global scratch); prediction launches (cache
+// fills, predictions) in kOpsAll with them.
+static const void *select_interp(int dpt, bool pred, int ops, bool general, int W) {
   if (W > kMaxWarps && (pred || dpt != 8)) return nullptr;
   const bool narrow = W <= 8;
   if (dpt == 16) {
-    if (narrow) return pred ? interp_fn<16, true, 8, 2>() : interp_mse<16, 8, 2>(ops, cache);
-    return pred ? interp_fn<16, true, 16, 1>() : interp_mse<16, 16, 1>(ops, cache);
+    if (narrow) return pred ? interp_fn<16, true, 8, 2>() : interp_mse<16, 8, 2>(ops, general);
+    return pred ? interp_fn<16, true, 16, 1>() : interp_mse<16, 16, 1>(ops, general);
   }
   if (dpt == 8) {
-    if (narrow) return pred ? interp_fn<8, true, 8, 3>() : interp_mse<8, 8, 3>(ops, cache);
+    if (narrow) return pred ? interp_fn<8, true, 8, 3>() : interp_mse<8, 8, 3>(ops, general);
     if (pred) return interp_fn<8, true, 16, 1>();
-    return W <= 15 ? interp_mse<8, 15, 2>(ops, cache) : interp_mse<8, 31, 1>(ops, cache);
+    return W <= 15 ? interp_mse<8, 15, 2>(ops, general) : interp_mse<8, 31, 1>(ops, general);
   }
   if (dpt == 4) {
-    if (narrow) return pred ? interp_fn<4, true, 8, 4>() : interp_mse<4, 8, 4>(ops, cache);
-    return pred ? interp_fn<4, true, 16, 2>() : interp_mse<4, 16, 2>(ops, cache);
+    if (narrow) return pred ? interp_fn<4, true, 8, 4>() : interp_mse<4, 8, 4>(ops, general);
+    return pred ? interp_fn<4, true, 16, 2>() : interp_mse<4, 16, 2>(ops, general);
   }
   return nullptr;
 }
@@ -537,9 +514,9 @@ cudaError_t raise_smem_limit(const void *fn, size_t smem) {
                               static_cast<int>(smem));
 }
 
-cudaError_t interp_configure(int dpt, bool pred, int ops, bool cache, size_t smem, int W,
+cudaError_t interp_configure(int dpt, bool pred, int ops, bool general, size_t smem, int W,
                              int *blocks_per_sm) {
-  const void *fn = select_interp(dpt, pred, ops, cache, W);
+  const void *fn = select_interp(dpt, pred, ops, general, W);
   if (!fn || W < 1 || W > kMaxInterpWarps) return cudaErrorInvalidValue;
   const cudaError_t err = raise_smem_limit(fn, smem);
   if (err != cudaSuccess) return err;
@@ -547,9 +524,9 @@ cudaError_t interp_configure(int dpt, bool pred, int ops, bool cache, size_t sme
                                                        (W + 1) * 32, smem);
 }
 
-cudaError_t launch_interp(int dpt, bool pred, int ops, bool cache, const EvalArgs &args,
+cudaError_t launch_interp(int dpt, bool pred, int ops, bool general, const EvalArgs &args,
                           int blocks, size_t smem, cudaStream_t stream) {
-  const void *fn = select_interp(dpt, pred, ops, cache, args.W);
+  const void *fn = select_interp(dpt, pred, ops, general, args.W);
   if (!fn || args.W < 1 || args.W > kMaxInterpWarps) return cudaErrorInvalidValue;
   // Plans of one instantiation can differ in shared-memory size (main and
   // cache-fill sets, autotune candidates); the attribute belongs to the

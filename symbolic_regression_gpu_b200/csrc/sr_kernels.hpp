@@ -28,12 +28,12 @@ inline int smem_spill_slots(int dpt) { return dpt >= 16 ? 2 : (dpt == 8 ? 4 : 8)
 // captured, however they are replayed.
 cudaError_t raise_smem_limit(const void *fn, size_t smem);
 // Sets the dynamic-smem attribute and returns resident blocks per SM.
-// `ops` is the operator profile (kOpsAll / kOpsProtected) and `cache` whether
-// the programs read cached subtrees (MSE mode only; prediction launches use
-// kOpsAll without cached operands).
-cudaError_t interp_configure(int dpt, bool pred, int ops, bool cache, size_t smem, int W,
+// `ops` is the operator profile (kOpsAll / kOpsProtected) and `general`
+// whether the programs read cached subtrees or spill slots in global scratch
+// (MSE mode only; prediction launches use kOpsAll and always admit both).
+cudaError_t interp_configure(int dpt, bool pred, int ops, bool general, size_t smem, int W,
                              int *blocks_per_sm);
-cudaError_t launch_interp(int dpt, bool pred, int ops, bool cache, const EvalArgs &args,
+cudaError_t launch_interp(int dpt, bool pred, int ops, bool general, const EvalArgs &args,
                           int blocks, size_t smem, cudaStream_t stream);
 cudaError_t launch_finalize(const double2 *partial, int n_spans, int E,
                             float *mse, cudaStream_t stream);

@@ -410,7 +410,7 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) tan_kernel(const TanArg
   if (warp == W) {
     if (lane == 0)
       run_producer<true>(p.n_groups, n_items, k_spans, p.n_spans, p.work_counter, p.error, p.X,
-                         p.ldx, rows, span, xbuf, desc, full, empty,
+                         p.ldx, rows, span, span, xbuf, desc, full, empty,
                          FoldArgs{part, gacc, p.partial, p.G, p.E, a.n_valid, K, gpart, ggacc,
                                   a.gout, a.const_off, a.const_cnt, a.C});
     return;
@@ -454,8 +454,6 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) tan_kernel(const TanArg
         float y[DPT], sd[DPT];
         lds_vec<DPT>(xs + p.V * span, lane, y);
         const bool full_tile = dp0 + TILE <= p.N;  // warp-uniform
-        float s = 0.0f, c = 0.0f;  // Kahan over the lane's DPT values
-        int nv = 0;
         float dfs[DPT], dsq[DPT];
 #pragma unroll
         for (int k = 0; k < DPT; k += 2) {
@@ -466,31 +464,13 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) tan_kernel(const TanArg
           dsq[k] = sq2.x;
           dsq[k + 1] = sq2.y;
         }
+        add_squares<DPT>(T, dsq, full_tile, dp0, lane, p.N, acc, cnt);
 #pragma unroll
         for (int k = 0; k < DPT; ++k) {
           const bool valid =
               (full_tile || dp0 + (k / 4) * 128 + lane * 4 + (k % 4) < p.N) && isfinite(T[k]);
-          const float df = dfs[k];
-          const float sq = valid ? dsq[k] : 0.0f;
-          nv += valid ? 1 : 0;
-          const float yk = __fsub_rn(sq, c);
-          const float tt = __fadd_rn(s, yk);
-          c = __fsub_rn(__fsub_rn(tt, s), yk);
-          s = tt;
-          sd[k] = valid ? 2.0f * df : 0.0f;
+          sd[k] = valid ? 2.0f * dfs[k] : 0.0f;
         }
-        double tile_sum = static_cast<double>(s) - static_cast<double>(c);
-        if (!isfinite(tile_sum)) {
-          float tc[DPT], yc[DPT];
-#pragma unroll
-          for (int k = 0; k < DPT; ++k) {
-            tc[k] = T[k];
-            yc[k] = y[k];
-          }
-          tile_sum = tile_sum_fp64<DPT>(tc, yc, full_tile, dp0, lane, p.N);
-        }
-        acc += tile_sum;
-        cnt += nv;
         // d MSE / d c (times the count): seed * t_c, zero where the seed is;
         // each lane adds its DPT products in order in FP32, FP64 from there
         // on (an FP32 lane sum overflows only for products beyond ~4e37).

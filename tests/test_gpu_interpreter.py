@@ -1,0 +1,100 @@
+"""The MSE interpreter against the prediction launches of the same programs:
+the two are different instantiations (operator profile, general or direct
+operand paths, datapoints per thread), so each dispatch code, tile remainder
+and span-group count of the MSE kernel is checked against predictions that
+went another way.
+
+Tolerance, derived: both sides square the same FP32 residual (bit-identical
+predictions) and sum the squares in FP64, N <= 1.1e5 terms of relative error
+2^-53 each in any order (below 2^-35), then round once to FP32: at most one
+unit in the last place apart."""
+import numpy as np
+import pytest
+
+import symbolic_regression_gpu_b200 as sg
+from symbolic_regression_gpu_b200 import opcodes as op
+
+pytestmark = pytest.mark.gpu
+
+V = 3
+
+
+def _forms():
+    """Every binary operator of the protected set with each kind and side of
+    operand (variable, constant, spilled subtree), every unary one on a leaf
+    and on a subtree, single leaves, constants only, invalid predictions."""
+    x = lambda i: ([-1], [float(i)])  # noqa: E731
+    c = lambda v: ([0], [v])  # noqa: E731
+
+    def un(o, a):
+        return [o] + a[0], [0.0] + a[1]
+
+    def bi(o, a, b):
+        return [o] + a[0] + b[0], [0.0] + a[1] + b[1]
+
+    s1 = bi(op.ADD, x(0), un(op.SIN, x(1)))
+    s2 = bi(op.MUL, x(2), un(op.COS, x(0)))
+    es = [x(0), x(2), c(1.5), x(7), bi(op.SUB, c(2.0), c(0.5))]
+    for o in op.WORKLOAD_BINARY:
+        for a in (x(0), c(0.75), s1):
+            for b in (x(1), c(-1.25), s2):
+                es.append(bi(o, a, b))
+    for o in op.WORKLOAD_UNARY:
+        es += [un(o, x(1)), un(o, c(2.0)), un(o, s1)]
+    deep = s1
+    for k in range(6):  # needs several spill slots
+        deep = bi(op.SUB if k % 2 else op.ADD, bi(op.MUL, s1, s2) if k == 0 else deep,
+                  bi(op.LOOSE_DIV, deep, s2))
+        if len(deep[0]) > 400:
+            break
+    es.append(deep)
+    big = un(op.EXP_CLAMP, bi(op.MUL, c(40.0), x(0)))
+    es.append(bi(op.SUB, bi(op.MUL, big, big), bi(op.MUL, big, big)))  # inf - inf: NaN rows
+    es.append(bi(op.MUL, big, c(3e4)))  # finite predictions, infinite squares
+    return sg.Population.from_lists(es)
+
+
+def _data(n, seed):
+    r = np.random.default_rng(seed)
+    X = r.uniform(-3.0, 3.0, (V + 1, n)).astype(np.float32)
+    X[0, : min(n, 5)] = [0.0, -0.0, 1e-10, 40000.0, -2.5][: min(n, 5)]
+    return X
+
+
+def _from_predictions(pred, y):
+    with np.errstate(all="ignore"):
+        d = (pred - y[None, :]).astype(np.float32)
+        sq = (d * d).astype(np.float32).astype(np.float64)
+    ok = np.isfinite(pred)
+    n = ok.sum(axis=1)
+    s = np.where(ok, sq, 0.0).sum(axis=1)
+    with np.errstate(all="ignore"):
+        return np.where(n > 0, s / n, np.nan).astype(np.float32)
+
+
+def _agree(a, b):
+    assert np.array_equal(np.isnan(a), np.isnan(b))
+    assert np.array_equal(np.isinf(a), np.isinf(b))
+    f = np.isfinite(a)
+    ulp = np.abs(a[f].view(np.int32).astype(np.int64) - b[f].view(np.int32).astype(np.int64))
+    assert ulp.max(initial=0) <= 1
+
+
+@pytest.mark.parametrize("n", [1, 31, 255, 256, 257, 1023, 1025, 8191, 33_001, 110_007])
+@pytest.mark.parametrize("opts", [{}, {"smem_spill_slots": 0}, {"smem_spill_slots": 1},
+                                  {"dpt": 4, "warps_per_block": 16},
+                                  {"dpt": 16, "warps_per_block": 8}])
+def test_mse_is_the_mean_of_the_predictions_squares(n, opts):
+    pop = _forms()
+    X = _data(n, n)
+    with sg.Evaluator(device=0) as ev:
+        ev.set_data(X)
+        want = _from_predictions(ev.predictions(pop), X[V])
+    with sg.Evaluator(device=0, **opts) as ev:
+        ev.set_data(X)
+        _agree(ev.eval_mse(pop), want)
+        s, cnt = ev.read_sums()
+        with np.errstate(all="ignore"):
+            _agree(np.where(cnt > 0, s / cnt, np.nan).astype(np.float32), want)
+        _agree(ev.eval_mse(pop, cache=True, clear_cache=True), want)
+        _agree(ev.eval_grad(pop)[0], want)
