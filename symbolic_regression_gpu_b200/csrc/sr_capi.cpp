@@ -179,11 +179,46 @@ bool protected_profile(const ProgramSet &ps) {
          static_cast<double>(ps.n_instr_protected) >= sr::kProtectedShare * ps.n_instr;
 }
 
+// Size class of a launch, from its 256-datapoint tiles of expressions per SM:
+// 0 below 120, 1 below 600, 2 below 6,000, 3 above.  A small launch wants every
+// warp of every SM at work on one expression and one tile: groups of one
+// expression per warp and 256-datapoint spans, in blocks of 8 warps at first,
+// then in the wide ones (500 expressions x 1,000 datapoints 86 -> 34 us, 1,000 x
+// 10,000 186 -> 112 us against groups of 124).  A middle one takes groups of two
+// expressions per warp, so that the last groups balance over the SMs (1,000 x
+// 100,000 720 -> 517 us, 4,000 x 30,000 853 -> 638 us); a large one reuses each
+// staged span for four (1,531 x 250,007: 2,172 us with two, 2,165 us).  Timed on
+// expressions of 2 to 7 variables around each line.
+int launch_size(const sr_context *ctx, int E) {
+  const double tiles = static_cast<double>(E) * static_cast<double>((ctx->N + 255) / 256);
+  const double per_sm = tiles / std::max(ctx->num_sms, 1);
+  return per_sm < 120.0 ? 0 : (per_sm < 600.0 ? 1 : (per_sm < 6000.0 ? 2 : 3));
+}
+
+// interp_configure with its answer kept (the shared-memory limit it raises is
+// raised again by the launch).
+static cudaError_t resident_blocks(sr_context *ctx, int dpt, bool pred, int ops, bool general,
+                                   size_t smem, int W, int *bps) {
+  const std::array<int64_t, 6> key{dpt, pred, ops, general, static_cast<int64_t>(smem), W};
+  const auto it = ctx->occupancy.find(key);
+  if (it != ctx->occupancy.end()) {
+    *bps = it->second;
+    return cudaSuccess;
+  }
+  const cudaError_t e = sr::interp_configure(dpt, pred, ops, general, smem, W, bps);
+  if (e == cudaSuccess) {
+    if (ctx->occupancy.size() >= 1024) ctx->occupancy.clear();
+    ctx->occupancy.emplace(key, *bps);
+  }
+  return e;
+}
+
 // Launch shape: groups of G cost-sorted expressions x spans of datapoints.
 // `split`: spill slots per warp kept in shared memory (-1 = the default for
 // the dpt); the deeper slots live in per-warp global scratch.  `per_warp`:
 // expressions per group and evaluating warp (a group of G = W x per_warp
-// expressions shares each staged X span).
+// expressions shares each staged X span), 0 to choose it, and the span, by the
+// launch's size.
 sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, int split,
                    int per_warp, int span_target) {
   sr::Plan p;
@@ -195,44 +230,40 @@ sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, i
   p.general = !pred && (ps.cache_refs || p.s_smem < p.smax);
   const int64_t tile = 32 * dpt;
   const int E = ps.E;
+  const bool by_size = per_warp <= 0;
+  if (by_size) {
+    const int size = launch_size(ctx, E);
+    per_warp = size <= 1 ? 1 : (size == 2 ? 2 : 4);
+    if (size <= 1) span_target = static_cast<int>(std::max<int64_t>(tile, kMinSpan));
+  }
   p.G = std::max(1, W * per_warp);
   p.n_groups = (E + p.G - 1) / p.G;
-  int dev_max_smem = 0;
-  cudaDeviceGetAttribute(&dev_max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
+  const size_t max_smem = static_cast<size_t>(ctx->max_smem);
   // Span: the target, shrunk to the data and to the shared-memory budget.
   int64_t span = std::min<int64_t>(span_target, std::max<int64_t>(tile, round_up(ctx->N, tile)));
-  while (span > tile &&
-         sr::interp_smem_bytes(dpt, W, ctx->V, p.s_smem, static_cast<int>(span), p.G, pred) >
-             static_cast<size_t>(dev_max_smem))
-    span = std::max<int64_t>(tile, (span / 2) / tile * tile);
+  auto smem_at = [&](int64_t sp) {
+    return sr::interp_smem_bytes(dpt, W, ctx->V, p.s_smem, static_cast<int>(sp), p.G, pred);
+  };
+  while (span > tile && smem_at(span) > max_smem) span = std::max<int64_t>(tile, (span / 2) / tile * tile);
   // Then, while the span's shared memory (the X buffers grow with the
   // variable count) rather than the registers limits the resident blocks,
   // halve it: more resident warps pay for more, shorter work items
   // (9 variables, 8 datapoints x 8 warps: 2 -> 3 blocks per SM at 512).
-  if (span_target > 0) {
-    int bps_now = 0;
-    SR_TRY_CUDA(ctx, sr::interp_configure(dpt, pred, p.ops, p.general,
-                                          sr::interp_smem_bytes(dpt, W, ctx->V, p.s_smem,
-                                                                static_cast<int>(span), p.G,
-                                                                pred),
-                                          W, &bps_now));
-    while (span / 2 >= std::max<int64_t>(tile, kMinSpan) && (span / 2) % tile == 0) {
-      int bps_half = 0;
-      SR_TRY_CUDA(ctx, sr::interp_configure(dpt, pred, p.ops, p.general,
-                                            sr::interp_smem_bytes(dpt, W, ctx->V, p.s_smem,
-                                                                  static_cast<int>(span / 2),
-                                                                  p.G, pred),
-                                            W, &bps_half));
-      if (bps_half <= bps_now) break;
-      span /= 2;
-      bps_now = bps_half;
-    }
+  int bps = 0;
+  SR_TRY_CUDA(ctx, resident_blocks(ctx, dpt, pred, p.ops, p.general, smem_at(span), W, &bps));
+  while (span / 2 >= std::max<int64_t>(tile, kMinSpan) && (span / 2) % tile == 0) {
+    int bps_half = 0;
+    SR_TRY_CUDA(ctx, resident_blocks(ctx, dpt, pred, p.ops, p.general, smem_at(span / 2), W,
+                                     &bps_half));
+    if (bps_half <= bps) break;
+    span /= 2;
+    bps = bps_half;
   }
   // The kernel walks a span tile by tile: it must hold whole tiles.
   if (span % tile != 0) return ctx->fail(SR_ERR_UNSUPPORTED, "span is not a multiple of the tile");
   p.span = static_cast<int>(span);
-  p.smem = sr::interp_smem_bytes(dpt, W, ctx->V, p.s_smem, p.span, p.G, pred);
-  if (p.smem > static_cast<size_t>(dev_max_smem))
+  p.smem = smem_at(p.span);
+  if (p.smem > max_smem)
     return ctx->fail(SR_ERR_UNSUPPORTED, "launch shape needs " + std::to_string(p.smem) +
                                              " bytes of shared memory");
   p.n_spans = (ctx->N == 0 || E == 0) ? 0 : static_cast<int>((ctx->N + span - 1) / span);
@@ -260,19 +291,17 @@ sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, i
                            " bytes) exceeds the device memory; split the population or the "
                            "datapoints");
   }
-  int bps = 0;
-  SR_TRY_CUDA(ctx, sr::interp_configure(dpt, pred, p.ops, p.general, p.smem, W, &bps));
   if (bps <= 0) return ctx->fail(SR_ERR_UNSUPPORTED, "launch shape does not fit on an SM");
   const int64_t resident = static_cast<int64_t>(bps) * ctx->num_sms;
-  // Few single-span items per resident block (a small population over few
-  // datapoints): shorter spans give more, smaller items and a shorter tail.
-  if (!pred && p.k_spans == 1) {
+  // Few single-span items per resident block in a shape given from outside:
+  // shorter spans give more, smaller items and a shorter tail.
+  if (!pred && !by_size && p.k_spans == 1) {
     while (p.items() < 16 * resident && p.span / 2 >= std::max<int64_t>(tile, 256) &&
            (p.span / 2) % tile == 0) {
       p.span /= 2;
       p.n_spans = static_cast<int>((ctx->N + p.span - 1) / p.span);
     }
-    p.smem = sr::interp_smem_bytes(dpt, W, ctx->V, p.s_smem, p.span, p.G, pred);
+    p.smem = smem_at(p.span);
   }
   p.blocks = static_cast<int>(std::min<int64_t>(resident, std::max<int64_t>(p.items(), 1)));
   // Global scratch for the spill slots that do not fit in shared memory.
@@ -494,7 +523,7 @@ sr_status autotune_main(sr_context *ctx, const std::string &key) {
 
 sr_status prepare_main_shape(sr_context *ctx, bool allow_tune) {
   ProgramSet &ps = ctx->main;
-  int dpt = ctx->opts.dpt, W = ctx->opts.warps_per_block, split = -1, per_warp = 4;
+  int dpt = ctx->opts.dpt, W = ctx->opts.warps_per_block, split = -1, per_warp = 0;
   if (dpt == 0 || W == 0) {
     if (!ctx->tune_loaded) load_tune_cache(ctx);
     const std::string key = tune_key(ctx, ps);
@@ -508,21 +537,21 @@ sr_status prepare_main_shape(sr_context *ctx, bool allow_tune) {
     // block's shared memory would not fit even at the shortest span (many
     // variables); 4 x 16 for populations over every operator, whose larger
     // dispatch switch fits the instruction cache better at 4 datapoints
-    // (150 -> 82 ms on 4,000 all-operator expressions x 1M datapoints).
+    // (150 -> 82 ms on 4,000 all-operator expressions x 1M datapoints); 8
+    // warps for small launches (launch_size).
     const bool prot = protected_profile(ps);
     const bool have = it != ctx->tuned.end();
     int wide = 8;
     if (prot) {
-      int dev_max_smem = 0;
-      cudaDeviceGetAttribute(&dev_max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
       const int s_smem = std::min(std::max(ps.smax, 0), sr::smem_spill_slots(8));
       const int W = sr::kMaxInterpWarps;
-      if (sr::interp_smem_bytes(8, W, ctx->V, s_smem, 32 * 8 * 2, W * per_warp, false) <=
-          static_cast<size_t>(dev_max_smem))
+      if (sr::interp_smem_bytes(8, W, ctx->V, s_smem, 32 * 8 * 2, W * 4, false) <=
+          static_cast<size_t>(ctx->max_smem))
         wide = W;
     }
     const int tdpt = have ? it->second.dpt : (prot ? 8 : 4);
-    const int tw = have ? it->second.W : (prot ? wide : 16);
+    const bool small = launch_size(ctx, ps.E) == 0;
+    const int tw = have ? it->second.W : (small ? 8 : (prot ? wide : 16));
     // the tuned split belongs to the tuned shape only
     if (have && (dpt == 0 || dpt == tdpt) && (W == 0 || W == tw)) {
       split = it->second.split;
@@ -656,6 +685,7 @@ sr_status sr_create(const sr_options *opts, sr_context **out) {
   }
   ctx->num_sms = prop.multiProcessorCount;
   ctx->device_memory = prop.totalGlobalMem;
+  ctx->max_smem = static_cast<int>(prop.sharedMemPerBlockOptin);
   ctx->device_name = prop.name;
   ctx->cache.capacity = o.cache_capacity;
   cudaError_t e = cudaSuccess;

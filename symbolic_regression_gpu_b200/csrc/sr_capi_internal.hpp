@@ -43,9 +43,10 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
 bool protected_profile(const ProgramSet &ps);
 // Launch shape: groups of G cost-sorted expressions x spans of datapoints.
 // `split`: spill slots per warp kept in shared memory (-1 = the default for
-// the dpt); `per_warp`: expressions per group and evaluating warp.
+// the dpt); `per_warp`: expressions per group and evaluating warp (0: by the
+// launch's size, launch_size).
 sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, int split = -1,
-                   int per_warp = 4, int span_target = 1024);
+                   int per_warp = 0, int span_target = 1024);
 sr_status upload_groups(sr_context *ctx, ProgramSet &ps);
 sr_status upload_code(sr_context *ctx, ProgramSet &ps);
 EvalArgs make_args(sr_context *ctx, ProgramSet &ps, int32_t *counter);

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cstdint>
 #include <map>
@@ -237,6 +238,7 @@ struct sr_context {
   sr_options opts{};
   int device = 0;
   int num_sms = 0;
+  int max_smem = 0;          // opt-in shared memory per block
   size_t device_memory = 0;  // bytes of device memory (cudaDeviceProp::totalGlobalMem)
   std::string device_name;
   cudaStream_t stream = nullptr;
@@ -303,6 +305,10 @@ struct sr_context {
 
   // statistics of the prepared population
   sr_stats prep_stats{};
+
+  // resident blocks per SM of the interpreter shapes planned so far (the
+  // occupancy query costs microseconds, a small call plans three shapes)
+  std::map<std::array<int64_t, 6>, int> occupancy;
 
   // tuned launch shapes: key -> (dpt, W, spill slots in shared memory (-1 =
   // the default for the dpt), expressions per group and warp)
