@@ -355,7 +355,9 @@ __global__ void __launch_bounds__(256)
                          const int64_t *__restrict__ const_off,
                          const int32_t *__restrict__ const_cnt,
                          const double *__restrict__ grad_acc, float *__restrict__ mse,
-                         float *__restrict__ grad, double2 *__restrict__ sums) {
+                         float *__restrict__ grad, double2 *__restrict__ sums,
+                         SequenceEnd end) {
+  end_sequence(end);
   const int q_ = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (q_ >= n_exprs) return;  // warp-uniform
@@ -452,10 +454,11 @@ int adj_segment() { return kSeg; }
 cudaError_t launch_grad_finalize(const double2 *partial, int n_spans, int E,
                                  const int32_t *exprs, int n_exprs, const int64_t *const_off,
                                  const int32_t *const_cnt, const double *grad_acc, float *mse,
-                                 float *grad, double2 *sums, cudaStream_t stream) {
+                                 float *grad, double2 *sums, SequenceEnd end,
+                                 cudaStream_t stream) {
   if (n_exprs <= 0) return cudaSuccess;
   grad_finalize_kernel<<<(n_exprs + 7) / 8, 256, 0, stream>>>(
-      partial, n_spans, E, exprs, n_exprs, const_off, const_cnt, grad_acc, mse, grad, sums);
+      partial, n_spans, E, exprs, n_exprs, const_off, const_cnt, grad_acc, mse, grad, sums, end);
   return cudaGetLastError();
 }
 

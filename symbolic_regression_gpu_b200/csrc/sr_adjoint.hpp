@@ -57,7 +57,7 @@ cudaError_t launch_tan_finalize(const double2 *partial, const double *gout, int 
                                 int64_t C, const int32_t *exprs, int n_exprs,
                                 const int64_t *const_off, const int32_t *const_cnt, int K,
                                 float *mse, float *grad, double *gsum, double2 *sums,
-                                cudaStream_t stream);
+                                SequenceEnd end, cudaStream_t stream);
 
 // Datapoints per thread of the adjoint kernel.
 int adj_dpt();
@@ -75,7 +75,8 @@ cudaError_t launch_adjoint(const AdjArgs &args, bool recompute, int blocks, size
 cudaError_t launch_grad_finalize(const double2 *partial, int n_spans, int E,
                                  const int32_t *exprs, int n_exprs, const int64_t *const_off,
                                  const int32_t *const_cnt, const double *grad_acc, float *mse,
-                                 float *grad, double2 *sums, cudaStream_t stream);
+                                 float *grad, double2 *sums, SequenceEnd end,
+                                 cudaStream_t stream);
 cudaError_t launch_adam(int64_t C, const float *grad, float *m, float *v, float *consts,
                         const int64_t *loc, Instr *code, int step, float lr, float beta1,
                         float beta2, float eps, cudaStream_t stream);

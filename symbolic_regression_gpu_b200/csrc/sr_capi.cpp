@@ -133,9 +133,7 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
                            msg[static_cast<size_t>(c)]);
   int64_t total = 0;
   for (auto &c : codes) total += static_cast<int64_t>(c.size());
-  SR_TRY_CUDA(ctx, ps.h_code.ensure(static_cast<size_t>(total + 1)));
-  SR_TRY_CUDA(ctx, ps.h_off.ensure(static_cast<size_t>(std::max(E, 1))));
-  SR_TRY_CUDA(ctx, ps.h_len.ensure(static_cast<size_t>(std::max(E, 1))));
+  SR_TRY_CUDA(ctx, ps.layout_host(static_cast<size_t>(total + 1), static_cast<size_t>(E)));
   int64_t pos = 0;
   for (auto &c : codes) {
     std::memcpy(ps.h_code.p + pos, c.data(), c.size() * sizeof(Instr));
@@ -310,7 +308,7 @@ sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, i
   if (spill_floats > 0) SR_TRY_CUDA(ctx, ctx->spill.ensure(spill_floats));
   // Group table: expressions in decreasing modelled cost, G per group, so
   // every group holds similar work and hands out its largest first.
-  SR_TRY_CUDA(ctx, ps.h_group.ensure(static_cast<size_t>(std::max(p.n_groups * p.G, 1))));
+  if (p.G > sr::kMaxGroup) return ctx->fail(SR_ERR_UNSUPPORTED, "expression group too large");
   std::vector<int32_t> order(static_cast<size_t>(E));
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
@@ -326,29 +324,38 @@ sr_status upload_groups(sr_context *ctx, ProgramSet &ps) {
   SR_TRACE("sr: upload groups");
   const size_t ng = static_cast<size_t>(std::max(ps.plan.n_groups * ps.plan.G, 1));
   ctx->prep_stats.h2d_bytes += static_cast<int64_t>(ng * sizeof(int32_t));
-  SR_TRY_CUDA(ctx, ps.group.ensure(ng));
   SR_TRY_CUDA(ctx, cudaMemcpyAsync(ps.group.p, ps.h_group.p, ng * sizeof(int32_t),
                                    cudaMemcpyHostToDevice, ctx->stream));
   return SR_OK;
 }
 
-sr_status upload_code(sr_context *ctx, ProgramSet &ps) {
-  SR_TRACE("sr: upload code");
-  const int E = ps.E;
-  SR_TRY_CUDA(ctx, ps.code.ensure(static_cast<size_t>(ps.n_instr + 1)));
-  SR_TRY_CUDA(ctx, ps.off.ensure(static_cast<size_t>(std::max(E, 1))));
-  SR_TRY_CUDA(ctx, ps.len.ensure(static_cast<size_t>(std::max(E, 1))));
-  SR_TRY_CUDA(ctx, cudaMemcpyAsync(ps.code.p, ps.h_code.p, (ps.n_instr + 1) * sizeof(Instr),
-                                   cudaMemcpyHostToDevice, ctx->stream));
-  ctx->prep_stats.h2d_bytes += static_cast<int64_t>((ps.n_instr + 1) * sizeof(Instr)) +
-                               static_cast<int64_t>(E) * (sizeof(int64_t) + sizeof(int32_t));
-  if (E > 0) {
-    SR_TRY_CUDA(ctx, cudaMemcpyAsync(ps.off.p, ps.h_off.p, E * sizeof(int64_t),
-                                     cudaMemcpyHostToDevice, ctx->stream));
-    SR_TRY_CUDA(ctx, cudaMemcpyAsync(ps.len.p, ps.h_len.p, E * sizeof(int32_t),
-                                     cudaMemcpyHostToDevice, ctx->stream));
-  }
+sr_status upload_set(sr_context *ctx, ProgramSet &ps, bool groups) {
+  SR_TRACE("sr: upload");
+  SR_TRY_CUDA(ctx, ps.layout_device(static_cast<size_t>(ps.n_instr + 1), static_cast<size_t>(ps.E)));
+  const size_t ng = groups ? static_cast<size_t>(ps.plan.n_groups) * ps.plan.G : 0;
+  const size_t bytes = static_cast<size_t>(
+      reinterpret_cast<unsigned char *>(ps.h_group.p + ng) - ps.h_pack.p);
+  ctx->prep_stats.h2d_bytes += static_cast<int64_t>(bytes);
+  SR_TRY_CUDA(ctx, cudaMemcpyAsync(ps.pack.p, ps.h_pack.p, bytes, cudaMemcpyHostToDevice,
+                                   ctx->stream));
   return SR_OK;
+}
+
+sr_status begin_sequence(sr_context *ctx) {
+  if (ctx->counters_used)
+    SR_TRY_CUDA(ctx, cudaMemsetAsync(ctx->d_counter, 0, sr::kCounters * sizeof(int32_t),
+                                     ctx->stream));
+  ctx->counters_used = true;
+  return SR_OK;
+}
+
+sr::SequenceEnd sequence_end(sr_context *ctx) {
+  sr::SequenceEnd e;
+  e.counters = ctx->d_counter;
+  e.n_counters = sr::kCounters;
+  e.error = ctx->d_error;
+  e.error_out = reinterpret_cast<int32_t *>(ctx->mse.p) + ctx->E;
+  return e;
 }
 
 sr::EvalArgs make_args(sr_context *ctx, ProgramSet &ps, int32_t *counter) {
@@ -386,7 +393,6 @@ sr_status launch_set(sr_context *ctx, ProgramSet &ps, bool pred, int32_t *counte
   a.pred = pred_out;
   a.ldp = ldp;
   a.pred_row = pred_row;
-  SR_TRY_CUDA(ctx, cudaMemsetAsync(counter, 0, sizeof(int32_t), ctx->stream));
   SR_TRY_CUDA(ctx, sr::launch_interp(ps.plan.dpt, pred, ps.plan.ops, ps.plan.general, a,
                                      ps.plan.blocks, ps.plan.smem,
                                      ctx->stream));
@@ -460,6 +466,7 @@ static sr_status time_shape(sr_context *ctx, int dpt, int W, int split, int per_
   cudaEvent_t a = ctx->ev[4], b = ctx->ev[5];
   float t_sum = 0.f;
   for (int rep = 0; rep < 3; ++rep) {
+    SR_TRY(begin_sequence(ctx));
     SR_TRY_CUDA(ctx, cudaEventRecord(a, ctx->stream));
     SR_TRY(launch_set(ctx, ctx->main, false, ctx->d_counter, nullptr, 0, nullptr));
     SR_TRY_CUDA(ctx, cudaEventRecord(b, ctx->stream));
@@ -521,7 +528,7 @@ sr_status autotune_main(sr_context *ctx, const std::string &key) {
   return SR_OK;
 }
 
-sr_status prepare_main_shape(sr_context *ctx, bool allow_tune) {
+sr_status prepare_main_shape(sr_context *ctx, bool allow_tune, bool on_device) {
   ProgramSet &ps = ctx->main;
   int dpt = ctx->opts.dpt, W = ctx->opts.warps_per_block, split = -1, per_warp = 0;
   if (dpt == 0 || W == 0) {
@@ -529,6 +536,8 @@ sr_status prepare_main_shape(sr_context *ctx, bool allow_tune) {
     const std::string key = tune_key(ctx, ps);
     auto it = ctx->tuned.find(key);
     if (it == ctx->tuned.end() && allow_tune && ctx->opts.autotune && ps.E > 0 && ctx->N > 0) {
+      if (!on_device) SR_TRY(upload_set(ctx, ps, false));
+      on_device = true;
       SR_TRY(autotune_main(ctx, key));
       it = ctx->tuned.find(key);
     }
@@ -562,7 +571,10 @@ sr_status prepare_main_shape(sr_context *ctx, bool allow_tune) {
   }
   if (ctx->opts.smem_spill_slots >= 0) split = ctx->opts.smem_spill_slots;
   SR_TRY(plan_set(ctx, ps, false, dpt, W, split, per_warp));
-  SR_TRY(upload_groups(ctx, ps));
+  if (on_device)
+    SR_TRY(upload_groups(ctx, ps));
+  else
+    SR_TRY(upload_set(ctx, ps, true));
   SR_TRY_CUDA(ctx, ctx->partial.ensure(static_cast<size_t>(std::max<int64_t>(
                        2 * static_cast<int64_t>(ps.plan.n_span_groups()) * ps.E, 1))));
   return SR_OK;
@@ -585,6 +597,7 @@ cudaError_t sr::capi::record_event(sr_context *ctx, int k) {
 // point into buffers that the next prepare / set_data may move).
 void sr::capi::reset_prepared(sr_context *ctx) {
   ctx->mode = sr::Mode::kNone;
+  ctx->launched = false;
   ctx->cache.rollback();  // subtrees of a launch that never ran hold no values
   if (ctx->graph_exec) {
     cudaGraphExecDestroy(ctx->graph_exec);
@@ -695,9 +708,11 @@ sr_status sr_create(const sr_options *opts, sr_context **out) {
     e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     ctx->own_stream = (e == cudaSuccess);
   }
-  if (e == cudaSuccess) e = cudaMalloc(&ctx->d_counter, 2 * sizeof(int32_t));
+  if (e == cudaSuccess) e = cudaMalloc(&ctx->d_counter, sr::kCounters * sizeof(int32_t));
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(ctx->d_counter, 0, sr::kCounters * sizeof(int32_t), ctx->stream);
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_error, sizeof(int32_t));
-  if (e == cudaSuccess) e = cudaMemset(ctx->d_error, 0, sizeof(int32_t));
+  if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_error, 0, sizeof(int32_t), ctx->stream);
   if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_error, sizeof(int32_t));
   for (int i = 0; i < 6 && e == cudaSuccess; ++i) e = cudaEventCreate(&ctx->ev[i]);
   if (e != cudaSuccess) {
@@ -1060,16 +1075,10 @@ sr_status prepare_cached(sr_context *ctx, const sr_population *pop, uint32_t fla
   // Subtrees to evaluate into the cache this call.
   const double tc0 = now_ms();
   SR_TRY(compile_set(ctx, n_new, sub_tok.data(), sub_val.data(), sub_off.data(), nullptr, ctx->sub));
-  SR_TRY_CUDA(ctx, ctx->sub.h_row.ensure(static_cast<size_t>(std::max(n_new, 1))));
   for (int k = 0; k < n_new; ++k) ctx->sub.h_row.p[k] = sub_slot[static_cast<size_t>(k)];
   if (n_new > 0) {
     SR_TRY(plan_set(ctx, ctx->sub, true, 8, sr::kMaxWarps));
-    SR_TRY(upload_code(ctx, ctx->sub));
-    SR_TRY(upload_groups(ctx, ctx->sub));
-    SR_TRY_CUDA(ctx, ctx->sub.row.ensure(static_cast<size_t>(n_new)));
-    SR_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->sub.row.p, ctx->sub.h_row.p, n_new * sizeof(int32_t),
-                                     cudaMemcpyHostToDevice, ctx->stream));
-    ctx->prep_stats.h2d_bytes += static_cast<int64_t>(n_new) * sizeof(int32_t);
+    SR_TRY(upload_set(ctx, ctx->sub, true));
   } else {
     ctx->sub.plan = sr::Plan{};
   }
@@ -1081,8 +1090,7 @@ sr_status prepare_cached(sr_context *ctx, const sr_population *pop, uint32_t fla
                                                    ctx->cache, threads, ctx->hints.data());
   SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, ctx->hints.data(), ctx->main));
   ctx->prep_stats.host_compile_time_ms = now_ms() - tc0;
-  SR_TRY(upload_code(ctx, ctx->main));
-  SR_TRY(prepare_main_shape(ctx, false));
+  SR_TRY(prepare_main_shape(ctx, false, false));
   ctx->prep_stats.node_evals = T * ctx->N;
   ctx->prep_stats.node_evals_executed = (T - removed + static_cast<int64_t>(sub_tok.size())) * ctx->N;
   return SR_OK;
@@ -1106,8 +1114,10 @@ sr_status sr_prepare(sr_context *ctx, const sr_population *pop, uint32_t flags) 
   const int E = pop->num_exprs;
   ctx->E = E;
   if (E == 0) return SR_OK;
-  SR_TRY_CUDA(ctx, ctx->mse.ensure(static_cast<size_t>(E)));
-  SR_TRY_CUDA(ctx, ctx->h_mse.ensure(static_cast<size_t>(E)));
+  // One entry more than expressions: the device error word travels behind the
+  // results (SequenceEnd).
+  SR_TRY_CUDA(ctx, ctx->mse.ensure(static_cast<size_t>(E) + 1));
+  SR_TRY_CUDA(ctx, ctx->h_mse.ensure(static_cast<size_t>(E) + 1));
   SR_TRY_CUDA(ctx, cudaEventRecord(ctx->ev[4], ctx->stream));
   if (flags & SR_EVAL_GRADIENT) {
     SR_TRY(prepare_grad(ctx, pop, (flags & SR_EVAL_GRAD_RECOMPUTE) != 0,
@@ -1123,8 +1133,7 @@ sr_status sr_prepare(sr_context *ctx, const sr_population *pop, uint32_t flags) 
     const double tc0 = now_ms();
     SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, nullptr, ctx->main));
     ctx->prep_stats.host_compile_time_ms = now_ms() - tc0;
-    SR_TRY(upload_code(ctx, ctx->main));
-    SR_TRY(prepare_main_shape(ctx, true));
+    SR_TRY(prepare_main_shape(ctx, true, false));
     ctx->prep_stats.node_evals = ctx->main.n_tokens * ctx->N;
     ctx->prep_stats.node_evals_executed = ctx->prep_stats.node_evals;
     ctx->mode = sr::Mode::kBatched;
@@ -1152,6 +1161,7 @@ static sr_status enqueue_launch(sr_context *ctx, int *launches_out) {
                                          ctx->E, ctx->mse.p, s));
     ++launches;
   } else {
+    SR_TRY(begin_sequence(ctx));
     if (ctx->mode == sr::Mode::kCached && ctx->sub.plan.items() > 0) {
       SR_TRY(launch_set(ctx, ctx->sub, true, ctx->d_counter + 1, ctx->cache_vals.p, ctx->ldx,
                         ctx->sub.row.p));
@@ -1164,7 +1174,9 @@ static sr_status enqueue_launch(sr_context *ctx, int *launches_out) {
     }
     SR_TRY_CUDA(ctx, record_event(ctx, 2));
     SR_TRY_CUDA(ctx, sr::launch_finalize_groups(ctx->partial.p, ctx->main.plan.n_span_groups(),
-                                                ctx->E, ctx->mse.p, nullptr, s));
+                                                ctx->E, ctx->mse.p, nullptr, sequence_end(ctx),
+                                                s));
+    ctx->counters_used = false;
     ++launches;
   }
   SR_TRY_CUDA(ctx, record_event(ctx, 3));
@@ -1213,6 +1225,7 @@ static sr_status launch_prepared(sr_context *ctx, bool allow_graph) {
   }
   ctx->cache.commit();  // the subtree launch that writes the new cached values is enqueued
   ctx->timing_valid = true;
+  ctx->launched = true;
   ctx->prep_stats.kernel_launches = launches;
   return SR_OK;
 }
@@ -1267,12 +1280,16 @@ sr_status sr_read_mse(sr_context *ctx, float *mse_out, sr_stats *stats) {
   if (ctx->mode == sr::Mode::kNone) return ctx->fail(SR_ERR_INVALID_ARGUMENT, "nothing launched");
   if (!mse_out) return ctx->fail(SR_ERR_INVALID_ARGUMENT, "mse_out is NULL");
   DeviceScope scope(ctx->device);
-  SR_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->h_mse.p, ctx->mse.p, ctx->E * sizeof(float),
-                                   cudaMemcpyDeviceToHost, ctx->stream));
-  SR_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->h_error, ctx->d_error, sizeof(int32_t),
+  // The error word comes with the results of a launch (the plain path raises none).
+  const bool with_error = ctx->launched && ctx->mode != sr::Mode::kPlain;
+  SR_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->h_mse.p, ctx->mse.p,
+                                   (ctx->E + (with_error ? 1 : 0)) * sizeof(float),
                                    cudaMemcpyDeviceToHost, ctx->stream));
   SR_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  SR_TRY(check_device_error(ctx));
+  if (with_error) {
+    std::memcpy(ctx->h_error, ctx->h_mse.p + ctx->E, sizeof(int32_t));
+    SR_TRY(check_device_error(ctx));
+  }
   std::memcpy(mse_out, ctx->h_mse.p, ctx->E * sizeof(float));
   fill_stats(ctx, stats);
   return SR_OK;
@@ -1302,7 +1319,7 @@ sr_status sr_read_sums(sr_context *ctx, double *sum_out, double *count_out) {
     ;  // the gradient finalize kernels wrote ctx->sums
   else
     SR_TRY_CUDA(ctx, sr::launch_finalize_groups(ctx->partial.p, n_spans, E, nullptr,
-                                                ctx->sums.p, ctx->stream));
+                                                ctx->sums.p, sr::SequenceEnd{}, ctx->stream));
   SR_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->h_sums.p, ctx->sums.p, E * sizeof(double2),
                                    cudaMemcpyDeviceToHost, ctx->stream));
   SR_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->h_error, ctx->d_error, sizeof(int32_t),
@@ -1404,18 +1421,14 @@ sr_status sr_eval_predictions(sr_context *ctx, const sr_population *pop, int64_t
   SR_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   reset_prepared(ctx);
   SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, nullptr, ctx->main));
-  SR_TRY_CUDA(ctx, ctx->main.h_row.ensure(static_cast<size_t>(E)));
   for (int x = 0; x < E; ++x) ctx->main.h_row.p[x] = x;
   int dpt = ctx->opts.dpt ? ctx->opts.dpt : 8;
   int W = ctx->opts.warps_per_block ? std::min(ctx->opts.warps_per_block, sr::kMaxWarps)
                                      : sr::kMaxWarps;
   SR_TRY(plan_set(ctx, ctx->main, true, dpt, W));
-  SR_TRY(upload_code(ctx, ctx->main));
-  SR_TRY(upload_groups(ctx, ctx->main));
-  SR_TRY_CUDA(ctx, ctx->main.row.ensure(static_cast<size_t>(E)));
-  SR_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->main.row.p, ctx->main.h_row.p, E * sizeof(int32_t),
-                                   cudaMemcpyHostToDevice, ctx->stream));
+  SR_TRY(upload_set(ctx, ctx->main, true));
   SR_TRY_CUDA(ctx, ctx->pred.ensure(static_cast<size_t>(E) * ctx->ldx));
+  SR_TRY(begin_sequence(ctx));
   SR_TRY(launch_set(ctx, ctx->main, true, ctx->d_counter, ctx->pred.p, ctx->ldx, ctx->main.row.p));
   SR_TRY_CUDA(ctx, cudaMemcpy2DAsync(pred_out, dp_count * sizeof(float), ctx->pred.p + dp_begin,
                                      ctx->ldx * sizeof(float), dp_count * sizeof(float), E,

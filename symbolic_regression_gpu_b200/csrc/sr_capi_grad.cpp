@@ -78,7 +78,7 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
   ProgramSet &ps = ctx->main;
   const int E = pop->num_exprs;
   SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, nullptr, ps));
-  SR_TRY(upload_code(ctx, ps));
+  SR_TRY(upload_set(ctx, ps, false));
   // Constants: CSR offsets and the bytecode word that holds each one.
   SR_TRY_CUDA(ctx, g.h_const_off.ensure(static_cast<size_t>(E) + 1));
   SR_TRY_CUDA(ctx, g.h_const_cnt.ensure(static_cast<size_t>(std::max(E, 1))));
@@ -376,8 +376,8 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
     std::memcpy(g.h_exprs.p, expr_list.data(), expr_list.size() * sizeof(int32_t));
   SR_TRY_CUDA(ctx, g.exprs.ensure(std::max<size_t>(expr_list.size(), 1)));
   SR_TRY_CUDA(ctx, ctx->sums.ensure(static_cast<size_t>(E)));
-  SR_TRY_CUDA(ctx, ctx->mse.ensure(static_cast<size_t>(E)));
-  SR_TRY_CUDA(ctx, ctx->h_mse.ensure(static_cast<size_t>(E)));
+  SR_TRY_CUDA(ctx, ctx->mse.ensure(static_cast<size_t>(E) + 1));
+  SR_TRY_CUDA(ctx, ctx->h_mse.ensure(static_cast<size_t>(E) + 1));
   cudaStream_t s = ctx->stream;
   SR_TRY_CUDA(ctx, cudaMemcpyAsync(g.tmask.p, g.h_tmask.p,
                                    (static_cast<size_t>(ps.n_instr) + 1) * sizeof(uint32_t),
@@ -434,10 +434,12 @@ sr_status launch_grad(sr_context *ctx) {
         SR_TRY_CUDA(ctx, sr::adj_set_smem_limit(gt == 1, g.recompute, adj_max[gt]));
   }
   SR_TRY_CUDA(ctx, record_event(ctx, 1));
+  SR_TRY(begin_sequence(ctx));
+  int32_t *counter = ctx->d_counter + 2;  // one per launch of the sequence
   for (const sr::TanSet &ts : g.tsets) {
     if (ts.plan.items() == 0) continue;
     sr::TanArgs a{};
-    a.e = make_args(ctx, ps, ctx->d_counter);
+    a.e = make_args(ctx, ps, counter++);
     a.e.W = ts.plan.W;
     a.e.smax = ts.plan.smax;
     a.e.s_smem = ts.plan.s_smem;
@@ -455,13 +457,12 @@ sr_status launch_grad(sr_context *ctx) {
     a.C = g.C;
     a.n_valid = ts.n_exprs;
     a.K = ts.K;
-    SR_TRY_CUDA(ctx, cudaMemsetAsync(ctx->d_counter, 0, sizeof(int32_t), s));
     SR_TRY_CUDA(ctx, sr::launch_tangent(a, ts.plan.blocks, ts.plan.smem, s));
   }
   for (const sr::AdjClass &cl : g.classes) {
     if (cl.plan.items() == 0) continue;
     sr::AdjArgs a{};
-    a.e = make_args(ctx, ps, ctx->d_counter);
+    a.e = make_args(ctx, ps, counter++);
     a.e.W = cl.plan.W;
     a.e.smax = cl.plan.smax;
     a.e.s_smem = cl.plan.s_smem;
@@ -478,21 +479,22 @@ sr_status launch_grad(sr_context *ctx) {
     a.tape_len = cl.tape_len;
     a.seg_cap = cl.seg_cap;
     a.gmax = cl.gmax;
-    SR_TRY_CUDA(ctx, cudaMemsetAsync(ctx->d_counter, 0, sizeof(int32_t), s));
     SR_TRY_CUDA(ctx, sr::launch_adjoint(a, g.recompute, cl.plan.blocks, cl.plan.smem, s));
   }
   SR_TRY_CUDA(ctx, record_event(ctx, 2));
+  const sr::SequenceEnd end = sequence_end(ctx);
   for (const sr::TanSet &ts : g.tsets)
     SR_TRY_CUDA(ctx, sr::launch_tan_finalize(
                          g.tan_partial.p + ts.part_off, g.tan_gout.p + ts.gout_off,
                          ts.plan.n_span_groups(), ps.E, g.C, g.exprs.p + ts.expr_off, ts.n_exprs,
                          g.const_off.p, g.const_cnt.p, ts.K, ctx->mse.p, g.grad.p, g.grad_acc.p,
-                         ctx->sums.p, s));
+                         ctx->sums.p, end, s));
   if (g.n_rev > 0)
     SR_TRY_CUDA(ctx, sr::launch_grad_finalize(ctx->partial.p, g.n_spans, ps.E,
                                               g.exprs.p + g.rev_expr_off, g.n_rev, g.const_off.p,
                                               g.const_cnt.p, g.grad_acc.p, ctx->mse.p, g.grad.p,
-                                              ctx->sums.p, s));
+                                              ctx->sums.p, end, s));
+  if (!g.tsets.empty() || g.n_rev > 0) ctx->counters_used = false;
   return SR_OK;
 }
 
@@ -571,14 +573,13 @@ sr_status sr_optimize_constants(sr_context *ctx, const sr_population *pop,
   SR_TRY_CUDA(ctx, cudaEventRecord(ctx->ev[3], s));
   ctx->timing_valid = true;
   const int E = pop->num_exprs;
-  SR_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->h_mse.p, ctx->mse.p, E * sizeof(float),
+  SR_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->h_mse.p, ctx->mse.p, (E + 1) * sizeof(float),
                                    cudaMemcpyDeviceToHost, s));
   if (g.C > 0 && const_out)
     SR_TRY_CUDA(ctx, cudaMemcpyAsync(const_out, g.consts.p, g.C * sizeof(float),
                                      cudaMemcpyDeviceToHost, s));
-  SR_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->h_error, ctx->d_error, sizeof(int32_t),
-                                   cudaMemcpyDeviceToHost, s));
   SR_TRY_CUDA(ctx, cudaStreamSynchronize(s));
+  std::memcpy(ctx->h_error, ctx->h_mse.p + E, sizeof(int32_t));
   SR_TRY(check_device_error(ctx));
   std::memcpy(mse_out, ctx->h_mse.p, E * sizeof(float));
   ctx->prep_stats.kernel_launches = launches;

@@ -48,11 +48,17 @@ bool protected_profile(const ProgramSet &ps);
 sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, int split = -1,
                    int per_warp = 0, int span_target = 1024);
 sr_status upload_groups(sr_context *ctx, ProgramSet &ps);
-sr_status upload_code(sr_context *ctx, ProgramSet &ps);
+// The set's packed buffer, with or without its group table, in one copy.
+sr_status upload_set(sr_context *ctx, ProgramSet &ps, bool groups);
+// Work counters at zero before a launch sequence, and what its last kernel
+// does for the next one.
+sr_status begin_sequence(sr_context *ctx);
+sr::SequenceEnd sequence_end(sr_context *ctx);
 EvalArgs make_args(sr_context *ctx, ProgramSet &ps, int32_t *counter);
 sr_status launch_set(sr_context *ctx, ProgramSet &ps, bool pred, int32_t *counter,
                      float *pred_out, int64_t ldp, const int32_t *pred_row);
-sr_status prepare_main_shape(sr_context *ctx, bool allow_tune);
+// `on_device`: the programs are on the device already (device populations).
+sr_status prepare_main_shape(sr_context *ctx, bool allow_tune, bool on_device);
 cudaError_t record_event(sr_context *ctx, int k);
 void reset_prepared(sr_context *ctx);
 void invalidate_data(sr_context *ctx);

@@ -223,13 +223,12 @@ sr_status sr_prepare_device_population(sr_context *ctx, const int32_t *tokens,
   ProgramSet &ps = ctx->main;
   ps.E = E;
   const size_t n_code = static_cast<size_t>(E) * (static_cast<size_t>(stride) + 1) + 1;
-  SR_TRY_CUDA(ctx, ps.code.ensure(n_code));
-  SR_TRY_CUDA(ctx, ps.off.ensure(static_cast<size_t>(E)));
-  SR_TRY_CUDA(ctx, ps.len.ensure(static_cast<size_t>(E)));
+  SR_TRY_CUDA(ctx, ps.layout_device(n_code, static_cast<size_t>(E)));
+  SR_TRY_CUDA(ctx, ps.layout_host(0, static_cast<size_t>(E)));  // the group table only
   SR_TRY_CUDA(ctx, ctx->evo_summary.ensure(8));
   SR_TRY_CUDA(ctx, ctx->h_evo_summary.ensure(8));
-  SR_TRY_CUDA(ctx, ctx->mse.ensure(static_cast<size_t>(E)));
-  SR_TRY_CUDA(ctx, ctx->h_mse.ensure(static_cast<size_t>(E)));
+  SR_TRY_CUDA(ctx, ctx->mse.ensure(static_cast<size_t>(E) + 1));
+  SR_TRY_CUDA(ctx, ctx->h_mse.ensure(static_cast<size_t>(E) + 1));
   // The interpreter prefetches one instruction past a program: keep the
   // padding word defined.
   SR_TRY_CUDA(ctx, cudaMemsetAsync(ps.code.p + (n_code - 1), 0, sizeof(Instr), ctx->stream));
@@ -260,7 +259,7 @@ sr_status sr_prepare_device_population(sr_context *ctx, const int32_t *tokens,
   // No timing here: a generation loop would re-tune whenever its populations
   // move to another shape class; the tuned shape of a class is used when the
   // context has one, else the profile's default.
-  SR_TRY(prepare_main_shape(ctx, false));
+  SR_TRY(prepare_main_shape(ctx, false, true));
   ctx->prep_stats.node_evals = n_tok * ctx->N;
   ctx->prep_stats.node_evals_executed = ctx->prep_stats.node_evals;
   ctx->mode = sr::Mode::kBatched;

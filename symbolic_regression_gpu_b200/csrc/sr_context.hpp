@@ -114,18 +114,50 @@ struct Plan {
   int64_t items() const { return static_cast<int64_t>(n_groups) * n_span_groups(); }
 };
 
-// A compiled population resident on the device.
+// A typed region of a packed buffer.
+template <class T>
+struct Region {
+  T *p = nullptr;
+};
+
+// Largest group (warps x expressions per warp): the padding of a group table.
+constexpr int kMaxGroup = 512;
+
+// A compiled population resident on the device.  Programs, offsets, lengths,
+// output rows and the group table lie in one buffer (on the host in one pinned
+// buffer of the same layout), so that one copy brings all of it to the device.
 struct ProgramSet {
-  DevBuf<Instr> code;
-  DevBuf<int64_t> off;
-  DevBuf<int32_t> len;
-  DevBuf<int32_t> group;
-  DevBuf<int32_t> row;
-  PinnedBuf<Instr> h_code;
-  PinnedBuf<int64_t> h_off;
-  PinnedBuf<int32_t> h_len;
-  PinnedBuf<int32_t> h_group;
-  PinnedBuf<int32_t> h_row;
+  DevBuf<unsigned char> pack;
+  PinnedBuf<unsigned char> h_pack;
+  Region<Instr> code, h_code;
+  Region<int64_t> off, h_off;
+  Region<int32_t> len, h_len;
+  Region<int32_t> row, h_row;
+  Region<int32_t> group, h_group;  // the last region: E + kMaxGroup entries
+  template <class B>
+  static void place(unsigned char *base, size_t n_code, size_t E, Region<Instr> &c,
+                    Region<int64_t> &o, Region<int32_t> &l, Region<int32_t> &r, B &g) {
+    c.p = reinterpret_cast<Instr *>(base);
+    o.p = reinterpret_cast<int64_t *>(base + n_code * sizeof(Instr));
+    l.p = reinterpret_cast<int32_t *>(o.p + E);
+    r.p = l.p + E;
+    g.p = r.p + E;
+  }
+  static size_t pack_bytes(size_t n_code, size_t E) {
+    return n_code * sizeof(Instr) + E * (sizeof(int64_t) + 3 * sizeof(int32_t)) +
+           kMaxGroup * sizeof(int32_t);
+  }
+  // Room for n_code instructions (the padding one included) and n expressions.
+  cudaError_t layout_host(size_t n_code, size_t n) {
+    const cudaError_t e = h_pack.ensure(pack_bytes(n_code, n));
+    if (e == cudaSuccess) place(h_pack.p, n_code, n, h_code, h_off, h_len, h_row, h_group);
+    return e;
+  }
+  cudaError_t layout_device(size_t n_code, size_t n) {
+    const cudaError_t e = pack.ensure(pack_bytes(n_code, n));
+    if (e == cudaSuccess) place(pack.p, n_code, n, code, off, len, row, group);
+    return e;
+  }
   std::vector<float> cost;  // per expression
   std::vector<int32_t> n_const;  // constants per expression
   int E = 0;
@@ -230,6 +262,8 @@ struct GradSet {
   bool recompute = false;
 };
 
+constexpr int kCounters = 16;
+
 enum class Mode { kNone, kBatched, kCached, kPlain, kGrad };
 
 }  // namespace sr
@@ -262,7 +296,11 @@ struct sr_context {
   sr::DevBuf<double2> partial;
   sr::DevBuf<float> mse;
   sr::PinnedBuf<float> h_mse;
-  int32_t *d_counter = nullptr;   // [2]: main and subtree launches
+  // Work counters: [0] main, [1] subtree launches, [2..] gradient launches.
+  // They are zero before a launch sequence: its last kernel (a finalize)
+  // zeroes them for the next one; counters_used marks sequences that had none.
+  int32_t *d_counter = nullptr;
+  bool counters_used = false;
   int32_t *d_error = nullptr;
   int32_t *h_error = nullptr;     // pinned
 
@@ -302,6 +340,7 @@ struct sr_context {
   int graph_launches = 0;
   bool capturing = false;  // sr_launch is capturing graph_exec
   bool timing_valid = false;
+  bool launched = false;   // the prepared launch has been enqueued
 
   // statistics of the prepared population
   sr_stats prep_stats{};

@@ -9,6 +9,7 @@
 
 #include "sr_eval.h"
 #include "sr_internal.hpp"
+#include "sr_kernels.hpp"
 #include "sr_ops.cuh"
 
 namespace sr {
@@ -898,6 +899,12 @@ __device__ __forceinline__ void dd_warp_sum(double &hi, double &lo, double &cnt)
     dd_add(hi, lo, h2);
     dd_add(hi, lo, l2);
   }
+}
+
+__device__ __forceinline__ void end_sequence(const SequenceEnd &end) {
+  if (blockIdx.x != 0) return;
+  if (static_cast<int>(threadIdx.x) < end.n_counters) end.counters[threadIdx.x] = 0;
+  if (threadIdx.x == 0 && end.error_out) *end.error_out = *end.error;
 }
 
 // What the producer of an MSE launch folds: the span slots, its accumulators

@@ -163,7 +163,8 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) interp_kernel(const Eva
 // the other (1,000 expressions x 391 span groups: 100 -> 6 us).
 __global__ void __launch_bounds__(256)
     finalize_dd_kernel(const double2 *__restrict__ partial, int n_groups, int E,
-                       float *__restrict__ mse, double2 *__restrict__ sums) {
+                       float *__restrict__ mse, double2 *__restrict__ sums, SequenceEnd end) {
+  end_sequence(end);
   const int e = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (e >= E) return;  // warp-uniform
@@ -545,9 +546,9 @@ cudaError_t launch_finalize(const double2 *partial, int n_spans, int E,
 }
 
 cudaError_t launch_finalize_groups(const double2 *partial, int n_groups, int E, float *mse,
-                                   double2 *sums, cudaStream_t stream) {
+                                   double2 *sums, SequenceEnd end, cudaStream_t stream) {
   if (E <= 0) return cudaSuccess;
-  finalize_dd_kernel<<<(E + 7) / 8, 256, 0, stream>>>(partial, n_groups, E, mse, sums);
+  finalize_dd_kernel<<<(E + 7) / 8, 256, 0, stream>>>(partial, n_groups, E, mse, sums, end);
   return cudaGetLastError();
 }
 

@@ -17,6 +17,17 @@ constexpr int64_t kDataAlign = 4096;               // X / cache row stride multi
 constexpr int kPlainStack = 128;                    // plain kernel stack depth
 constexpr int kFp64Stack = 96;                      // FP64 reference kernel stack depth
 
+// What the last kernel of a launch sequence does besides its own work: it
+// zeroes the sequence's work counters for the next one and copies the device
+// error word behind the results, so that neither costs a memset or a copy of
+// its own.  Null pointers: nothing.
+struct SequenceEnd {
+  int32_t *counters = nullptr;
+  int32_t n_counters = 0;
+  const int32_t *error = nullptr;
+  int32_t *error_out = nullptr;
+};
+
 // Dynamic shared memory of interp_kernel for a launch shape.
 size_t interp_smem_bytes(int dpt, int W, int V, int s_smem, int span, int G, bool pred);
 // Spill slots per warp kept in shared memory for a datapoints-per-thread
@@ -41,7 +52,7 @@ cudaError_t launch_finalize(const double2 *partial, int n_spans, int E,
 // see EvalArgs::span_per_item): mse = sum / count (NaN without a valid
 // datapoint) into `mse`, and (sum, count) into `sums`; either may be NULL.
 cudaError_t launch_finalize_groups(const double2 *partial, int n_groups, int E, float *mse,
-                                   double2 *sums, cudaStream_t stream);
+                                   double2 *sums, SequenceEnd end, cudaStream_t stream);
 // (sum of valid squared errors, valid count) per expression, combined over
 // the span partials in the order launch_finalize uses (plain and gradient
 // launches).

@@ -524,7 +524,8 @@ __global__ void __launch_bounds__(256)
                         int n_exprs, const int64_t *__restrict__ const_off,
                         const int32_t *__restrict__ const_cnt, int K, float *__restrict__ mse,
                         float *__restrict__ grad, double *__restrict__ gsum,
-                        double2 *__restrict__ sums) {
+                        double2 *__restrict__ sums, SequenceEnd end) {
+  end_sequence(end);
   const int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (q >= n_exprs) return;  // warp-uniform
@@ -621,11 +622,11 @@ cudaError_t launch_tan_finalize(const double2 *partial, const double *gout, int 
                                 int64_t C, const int32_t *exprs, int n_exprs,
                                 const int64_t *const_off, const int32_t *const_cnt, int K,
                                 float *mse, float *grad, double *gsum, double2 *sums,
-                                cudaStream_t stream) {
+                                SequenceEnd end, cudaStream_t stream) {
   if (n_exprs <= 0) return cudaSuccess;
   tan_finalize_kernel<<<(n_exprs + 7) / 8, 256, 0, stream>>>(
       partial, gout, n_groups, E, C, exprs, n_exprs, const_off, const_cnt, K, mse, grad, gsum,
-      sums);
+      sums, end);
   return cudaGetLastError();
 }
 
