@@ -100,32 +100,47 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
   ps.n_instr = 0;
   ps.n_tokens = 0;
   ps.sfu_per_dp = ps.fp32_per_dp = 0.0;
-  const int nt = std::max(1, std::min(host_threads(ctx), std::max(1, E / 32)));
+  // About 20 ns a token, and tens of microseconds to wake the workers: chunks
+  // of 2,500 tokens or more, one thread below two of them.
+  const int64_t n_tok = E > 0 ? off[E] - off[0] : 0;
+  const int nt = static_cast<int>(
+      std::max<int64_t>(1, std::min<int64_t>({host_threads(ctx), E, n_tok / 2500})));
   std::vector<std::vector<Instr>> codes(static_cast<size_t>(nt));
   std::vector<sr::ExprInfo> infos(static_cast<size_t>(E));
   std::vector<sr_status> st(static_cast<size_t>(nt), SR_OK);
   std::vector<std::string> msg(static_cast<size_t>(nt));
   std::vector<int64_t> bad(static_cast<size_t>(nt), -1);
-  sr::parallel_for(nt, nt, [&](int64_t b, int64_t e) {
-    for (int64_t c = b; c < e; ++c) {
-      const int64_t x0 = static_cast<int64_t>(E) * c / nt, x1 = static_cast<int64_t>(E) * (c + 1) / nt;
-      auto &code = codes[static_cast<size_t>(c)];
-      code.reserve(static_cast<size_t>((off[x1] - off[x0]) / 2 + 8));
-      for (int64_t x = x0; x < x1; ++x) {
-        std::string err;
-        const sr_status s = sr::compile_expression(
-            tok + off[x], val + off[x], static_cast<int>(off[x + 1] - off[x]), ctx->V,
-            hints ? hints + off[x] : nullptr, code, infos[static_cast<size_t>(x)], &err);
-        if (s != SR_OK) {
-          st[static_cast<size_t>(c)] = s;
-          msg[static_cast<size_t>(c)] = err;
-          bad[static_cast<size_t>(c)] = x;
-          return;
-        }
+  std::vector<int64_t> in_profile(static_cast<size_t>(nt), 0);
+  std::vector<char> refs(static_cast<size_t>(nt), 0);
+  const auto compile_chunk = [&](int ci) {
+    const size_t c = static_cast<size_t>(ci);
+    const int64_t x0 = static_cast<int64_t>(E) * ci / nt, x1 = static_cast<int64_t>(E) * (ci + 1) / nt;
+    auto &code = codes[c];
+    code.reserve(static_cast<size_t>((off[x1] - off[x0]) * 2 / 3 + 8));
+    std::string err;
+    for (int64_t x = x0; x < x1; ++x) {
+      const sr_status s = sr::compile_expression(
+          tok + off[x], val + off[x], static_cast<int>(off[x + 1] - off[x]), ctx->V,
+          hints ? hints + off[x] : nullptr, code, infos[static_cast<size_t>(x)], &err);
+      if (s != SR_OK) {
+        st[c] = s;
+        msg[c] = err;
+        bad[c] = x;
+        return;
       }
-      for (Instr &in : code) in.w = sr::with_dispatch(in.w);
     }
-  });
+    int64_t n_prot = 0;
+    bool cached = false;
+    for (Instr &in : code) {
+      in.w = sr::with_dispatch(in.w);
+      n_prot += sr::in_protected_profile(sr::instr_op(in.w)) ? 1 : 0;
+      cached = cached || (sr::instr_load(in.w) && sr::instr_leaf_kind(in.w) == sr::kLeafR) ||
+               sr::instr_b_kind(in.w) == sr::kBR;
+    }
+    in_profile[c] = n_prot;
+    refs[c] = cached ? 1 : 0;
+  };
+  ctx->workers.run(nt, nt, compile_chunk);
   for (int c = 0; c < nt; ++c)
     if (st[static_cast<size_t>(c)] != SR_OK)
       return ctx->fail(st[static_cast<size_t>(c)],
@@ -140,16 +155,12 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
     pos += static_cast<int64_t>(c.size());
   }
   ps.h_code.p[total] = Instr{0, 0, 0, 0};  // prefetch padding
-  int64_t in_profile = 0;
-  bool cache_refs = false;
-  for (int64_t i = 0; i < total; ++i) {
-    const uint32_t w = ps.h_code.p[i].w;
-    in_profile += sr::in_protected_profile(sr::instr_op(w)) ? 1 : 0;
-    cache_refs = cache_refs || (sr::instr_load(w) && sr::instr_leaf_kind(w) == sr::kLeafR) ||
-                 sr::instr_b_kind(w) == sr::kBR;
+  ps.n_instr_protected = 0;
+  ps.cache_refs = false;
+  for (size_t c = 0; c < codes.size(); ++c) {
+    ps.n_instr_protected += in_profile[c];
+    ps.cache_refs = ps.cache_refs || refs[c] != 0;
   }
-  ps.n_instr_protected = in_profile;
-  ps.cache_refs = cache_refs;
   int64_t o = 0;
   for (int x = 0; x < E; ++x) {
     const auto &in = infos[static_cast<size_t>(x)];
@@ -175,6 +186,28 @@ constexpr int64_t kMinSpan = 256;
 bool protected_profile(const ProgramSet &ps) {
   return ps.n_instr > 0 &&
          static_cast<double>(ps.n_instr_protected) >= sr::kProtectedShare * ps.n_instr;
+}
+
+// The expressions in decreasing cost, equal ones in index order: a counting
+// sort over half units of cost (all costs are multiples of one; those above the
+// last bucket, far beyond any program that differs in rank, keep index order).
+static void cost_order(const std::vector<float> &cost, int E, int32_t *order) {
+  if (E < 1024) {  // fewer than the buckets' own cost
+    std::iota(order, order + E, 0);
+    std::stable_sort(order, order + E, [&](int32_t a, int32_t b) {
+      return cost[static_cast<size_t>(a)] > cost[static_cast<size_t>(b)];
+    });
+    return;
+  }
+  constexpr int kBuckets = 1 << 14;
+  std::vector<int32_t> start(kBuckets + 1, 0);
+  const auto bucket = [&](int x) {
+    return kBuckets - 1 -
+           static_cast<int>(std::min(2.0f * cost[static_cast<size_t>(x)], kBuckets - 1.0f));
+  };
+  for (int x = 0; x < E; ++x) ++start[static_cast<size_t>(bucket(x)) + 1];
+  for (int b = 0; b < kBuckets; ++b) start[static_cast<size_t>(b) + 1] += start[static_cast<size_t>(b)];
+  for (int x = 0; x < E; ++x) order[start[static_cast<size_t>(bucket(x))]++] = x;
 }
 
 // Size class of a launch, from its 256-datapoint tiles of expressions per SM:
@@ -309,13 +342,8 @@ sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, i
   // Group table: expressions in decreasing modelled cost, G per group, so
   // every group holds similar work and hands out its largest first.
   if (p.G > sr::kMaxGroup) return ctx->fail(SR_ERR_UNSUPPORTED, "expression group too large");
-  std::vector<int32_t> order(static_cast<size_t>(E));
-  std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
-    return ps.cost[static_cast<size_t>(a)] > ps.cost[static_cast<size_t>(b)];
-  });
-  for (int64_t k = 0; k < static_cast<int64_t>(p.n_groups) * p.G; ++k)
-    ps.h_group.p[k] = k < E ? order[static_cast<size_t>(k)] : -1;
+  cost_order(ps.cost, E, ps.h_group.p);
+  for (int64_t k = E; k < static_cast<int64_t>(p.n_groups) * p.G; ++k) ps.h_group.p[k] = -1;
   ps.plan = p;
   return SR_OK;
 }

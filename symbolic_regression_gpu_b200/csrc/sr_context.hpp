@@ -15,6 +15,7 @@
 #include "sr_detect.hpp"
 #include "sr_eval.h"
 #include "sr_internal.hpp"
+#include "sr_parallel.hpp"
 #include "sr_program.hpp"
 
 namespace sr {
@@ -344,6 +345,8 @@ struct sr_context {
 
   // statistics of the prepared population
   sr_stats prep_stats{};
+
+  sr::WorkerPool workers;  // host passes over the population
 
   // resident blocks per SM of the interpreter shapes planned so far (the
   // occupancy query costs microseconds, a small call plans three shapes)

@@ -99,6 +99,23 @@ float op_cost(int tok) {
 
 namespace {
 
+// Cost and declared work per device opcode (reversed opcodes like their
+// operator), looked up once per instruction.
+struct OpTables {
+  float cost[64];
+  float sfu[64], fp32[64];
+  OpTables() {
+    for (int k = 0; k < 64; ++k) {
+      const int op = k > static_cast<int>(kOpReversed) ? k - static_cast<int>(kOpReversed) : k;
+      double s, f;
+      declared_op_work(op, &s, &f);
+      cost[k] = 2.0f + op_cost(op);
+      sfu[k] = static_cast<float>(s);
+      fp32[k] = static_cast<float>(f);
+    }
+  }
+};
+
 struct Node {
   bool leaf = false;
   int32_t op = 0;          // operator token
@@ -133,13 +150,24 @@ inline uint32_t reversed(int tok) {
                                    : kOpReversed + static_cast<uint32_t>(tok);
 }
 
+// Writes one program (its instruction count is known: one per operator node,
+// one for a single leaf) and adds up its modelled cost.
 struct Emitter {
-  const std::vector<Node> &nodes;
-  std::vector<Instr> &out;
-  size_t first = 0;          // index of this program's first instruction in `out`
+  const Node *nodes;
+  const OpTables &tab;
+  int n_const;               // constants of the expression
+  Instr *out;                // the program's first instruction
+  int count = 0;
+  float cost = 0.f, sfu = 0.f, fp32 = 0.f;
   int pending_spill = -1;
   int sp = 0;
   int spill_at[kMaxSpillSlots + 1] = {};  // instruction that spilled into each slot
+
+  // Constants are numbered in token order; the parse meets them from the right.
+  uint32_t const_index(uint32_t from_right) const {
+    return from_right == kNoConst ? kNoConst
+                                  : static_cast<uint32_t>(n_const - 1) - from_right;
+  }
 
   // [spill] [T = load] [b = operand] T = op(T, b)
   void emit(uint32_t op, const Node *load, uint32_t bk, uint32_t bp, uint32_t bc) {
@@ -147,22 +175,27 @@ struct Emitter {
     ins.w = (op & 63u) | ((bk & 7u) << 9);
     uint32_t ac = kNoConst;
     ins.a = 0;
+    cost += tab.cost[op & 63u];
+    sfu += tab.sfu[op & 63u];
+    fp32 += tab.fp32[op & 63u];
     if (load) {
       ins.w |= kLoadBit | ((load->lk & 3u) << 7);
       ins.a = load->lp;
-      ac = load->lconst;
+      ac = const_index(load->lconst);
+      if (load->lk != kLeafC) cost += 0.5f;
     }
-    const int index = static_cast<int>(out.size() - first);
     if (pending_spill >= 0) {
       ins.w |= kSpillBit | (static_cast<uint32_t>(pending_spill) << 13);
-      spill_at[pending_spill] = index;
+      spill_at[pending_spill] = count;
       pending_spill = -1;
+      cost += 0.5f;
     }
+    if (bk == kBS || bk == kBX || bk == kBR) cost += 0.5f;
     ins.b = bp;
     // A spilled operand is the accumulator value right before its spill.
     const uint32_t producer = (bk == kBS) ? static_cast<uint32_t>(spill_at[bp] - 1) : 0u;
-    ins.c = (ac & 0x3FFu) | ((bc & 0x3FFu) << 10) | ((producer & 0x3FFu) << 20);
-    out.push_back(ins);
+    ins.c = (ac & 0x3FFu) | ((const_index(bc) & 0x3FFu) << 10) | ((producer & 0x3FFu) << 20);
+    out[count++] = ins;
   }
 
   void emit_b_leaf(uint32_t op, const Node *load, const Node &b) {
@@ -230,141 +263,103 @@ sr_status compile_expression(const int32_t *tok, const double *val, int len,
                     std::to_string(SR_MAX_TOKENS) + ")";
     return SR_ERR_EXPRESSION_TOO_LONG;
   }
-  // Validate the original token stream: known tokens, no underflow, exactly
-  // one value left.
-  {
-    int depth = 0;
-    for (int i = len - 1; i >= 0; --i) {
-      const int t = tok[i];
-      if (t == SR_TOK_CONST || t == SR_TOK_VAR) {
-        ++depth;
-      } else if (is_binary_token(t)) {
-        if (depth < 2) {
-          if (err) *err = "stack underflow at token " + std::to_string(i);
-          return SR_ERR_MALFORMED_EXPRESSION;
-        }
-        --depth;
-      } else if (is_unary_token(t)) {
-        if (depth < 1) {
-          if (err) *err = "stack underflow at token " + std::to_string(i);
-          return SR_ERR_MALFORMED_EXPRESSION;
-        }
+  // One pass from the right: validation of the original token stream (known
+  // tokens, no underflow, exactly one value left), constant numbering and the
+  // tree, with cached subtrees (hints) collapsed to one leaf at their root.
+  // Children get lower node ids than their parent, and a node's spill-slot
+  // label (Sethi-Ullman) is known when it is made.
+  static const OpTables tab;
+  thread_local std::vector<Node> node_store;
+  thread_local std::vector<int32_t> stack_store;
+  if (static_cast<int>(node_store.size()) < len) {
+    node_store.resize(static_cast<size_t>(len));
+    stack_store.resize(static_cast<size_t>(len) + 1);
+  }
+  Node *nodes = node_store.data();
+  int32_t *stk = stack_store.data();
+  int n_nodes = 0, sp = 0, depth = 0, n_ops = 0;
+  uint32_t n_const = 0;
+  bool bad_skeleton = false;
+  for (int i = len - 1; i >= 0; --i) {
+    const int t = tok[i];
+    const int hint = hints ? hints[i] : -1;
+    // hint >= 0: root of a cached subtree; -2: inside one; -1: neither.
+    if (t == SR_TOK_CONST || t == SR_TOK_VAR) {
+      ++depth;
+      const uint32_t ci = n_const;
+      if (t == SR_TOK_CONST) ++n_const;
+      if (hint == -2) continue;
+      Node &nd = nodes[n_nodes];
+      nd.leaf = true;
+      nd.need = 0;
+      nd.lconst = kNoConst;
+      if (hint >= 0) {
+        nd.lk = kLeafR;
+        nd.lp = static_cast<uint32_t>(hint);
+      } else if (t == SR_TOK_CONST) {
+        nd.lk = kLeafC;
+        nd.lp = float_bits(static_cast<float>(val[i]));
+        nd.lconst = ci;
       } else {
-        if (err) *err = "unknown token " + std::to_string(t) + " at position " +
-                        std::to_string(i);
-        return SR_ERR_BAD_TOKEN;
+        const int v = var_index(val[i]);
+        const bool ok = v >= 0 && v < num_vars;
+        nd.lk = ok ? kLeafX : kLeafC;  // reference CPU pushes 0.0f (cl_cpu_eval.cpp:73-75)
+        nd.lp = ok ? static_cast<uint32_t>(v) : float_bits(0.0f);
       }
+      stk[sp++] = n_nodes++;
+      continue;
     }
-    if (depth != 1) {
-      if (err) *err = "expression leaves " + std::to_string(depth) +
-                      " values on the stack";
+    const bool binary = is_binary_token(t);
+    if (!binary && !is_unary_token(t)) {
+      if (err) *err = "unknown token " + std::to_string(t) + " at position " + std::to_string(i);
+      return SR_ERR_BAD_TOKEN;
+    }
+    if (depth < (binary ? 2 : 1)) {
+      if (err) *err = "stack underflow at token " + std::to_string(i);
       return SR_ERR_MALFORMED_EXPRESSION;
     }
-  }
-
-  // Constant numbering in token order, and subtree sizes for cache hints.
-  thread_local std::vector<int32_t> const_idx, sizes, seq;
-  thread_local std::vector<Node> nodes;
-  thread_local std::vector<int32_t> stk;
-  const_idx.assign(len, static_cast<int32_t>(kNoConst));
-  int n_const = 0;
-  for (int i = 0; i < len; ++i)
-    if (tok[i] == SR_TOK_CONST) const_idx[i] = n_const++;
-  info.n_const = n_const;
-
-  // Skeleton positions: cached subtrees collapse to one leaf at their root.
-  seq.clear();
-  if (hints) {
-    sizes.resize(len);
-    subtree_sizes(tok, len, sizes.data());
-    for (int k = 0; k < len; ++k) {
-      const int h = hints[k];
-      if (h >= 0) {
-        seq.push_back(-(k + 1));  // negative = cached-subtree leaf at k
-        k += sizes[k] - 1;
-      } else if (h == -2) {
-        continue;
-      } else {
-        seq.push_back(k);
-      }
-    }
-  } else {
-    seq.resize(len);
-    for (int k = 0; k < len; ++k) seq[k] = k;
-  }
-
-  // Parse right to left into a tree; children get lower node ids than their
-  // parent, so node-id order is a post-order.
-  nodes.clear();
-  stk.clear();
-  for (int s = static_cast<int>(seq.size()) - 1; s >= 0; --s) {
-    const int e = seq[s];
-    Node nd;
-    if (e < 0) {
-      const int k = -e - 1;
+    if (binary) --depth;
+    if (hint == -2 || bad_skeleton) continue;
+    Node &nd = nodes[n_nodes];
+    nd.lconst = kNoConst;
+    if (hint >= 0) {
       nd.leaf = true;
+      nd.need = 0;
       nd.lk = kLeafR;
-      nd.lp = static_cast<uint32_t>(hints[k]);
-    } else {
-      const int t = tok[e];
-      if (t == SR_TOK_CONST) {
-        nd.leaf = true;
-        nd.lk = kLeafC;
-        nd.lp = float_bits(static_cast<float>(val[e]));
-        nd.lconst = static_cast<uint32_t>(const_idx[e]);
-      } else if (t == SR_TOK_VAR) {
-        nd.leaf = true;
-        const int v = var_index(val[e]);
-        if (v >= 0 && v < num_vars) {
-          nd.lk = kLeafX;
-          nd.lp = static_cast<uint32_t>(v);
-        } else {
-          nd.lk = kLeafC;  // reference CPU pushes 0.0f (cl_cpu_eval.cpp:73-75)
-          nd.lp = float_bits(0.0f);
-        }
-      } else {
-        nd.op = t;
-        if (stk.empty()) {
-          if (err) *err = "cache marking produced an invalid skeleton";
-          return SR_ERR_MALFORMED_EXPRESSION;
-        }
-        nd.left = stk.back();
-        stk.pop_back();
-        if (is_binary_token(t)) {
-          if (stk.empty()) {
-            if (err) *err = "cache marking produced an invalid skeleton";
-            return SR_ERR_MALFORMED_EXPRESSION;
-          }
-          nd.right = stk.back();
-          stk.pop_back();
-        }
-      }
+      nd.lp = static_cast<uint32_t>(hint);
+      stk[sp++] = n_nodes++;
+      continue;
     }
-    nodes.push_back(nd);
-    stk.push_back(static_cast<int32_t>(nodes.size() - 1));
+    if (sp < (binary ? 2 : 1)) {
+      bad_skeleton = true;
+      continue;
+    }
+    nd.leaf = false;
+    nd.op = t;
+    nd.left = stk[--sp];
+    nd.right = -1;
+    const Node &L = nodes[nd.left];
+    nd.need = L.need;  // a leaf's is 0
+    if (binary) {
+      nd.right = stk[--sp];
+      const Node &R = nodes[nd.right];
+      if (R.leaf) nd.need = L.need;
+      else if (L.leaf) nd.need = R.need;
+      else nd.need = (L.need == R.need) ? L.need + 1 : std::max(L.need, R.need);
+    }
+    ++n_ops;
+    stk[sp++] = n_nodes++;
   }
-  if (stk.size() != 1) {
+  if (depth != 1) {
+    if (err) *err = "expression leaves " + std::to_string(depth) + " values on the stack";
+    return SR_ERR_MALFORMED_EXPRESSION;
+  }
+  if (bad_skeleton || sp != 1) {
     if (err) *err = "cache marking produced an invalid skeleton";
     return SR_ERR_MALFORMED_EXPRESSION;
   }
   const int root = stk[0];
-
-  // Spill-slot labels (post-order).
-  for (auto &nd : nodes) {
-    if (nd.leaf) {
-      nd.need = 0;
-    } else if (nd.right < 0) {
-      const Node &c = nodes[nd.left];
-      nd.need = c.leaf ? 0 : c.need;
-    } else {
-      const Node &L = nodes[nd.left];
-      const Node &R = nodes[nd.right];
-      if (L.leaf && R.leaf) nd.need = 0;
-      else if (R.leaf) nd.need = L.need;
-      else if (L.leaf) nd.need = R.need;
-      else nd.need = (L.need == R.need) ? L.need + 1 : std::max(L.need, R.need);
-    }
-  }
+  info.n_const = static_cast<int>(n_const);
   info.need = nodes[root].need;
   if (info.need > kMaxSpillSlots) {
     if (err) *err = "expression needs " + std::to_string(info.need) +
@@ -373,30 +368,13 @@ sr_status compile_expression(const int32_t *tok, const double *val, int len,
   }
 
   const size_t first = out.size();
-  Emitter em{nodes, out, first};
+  info.n_instr = std::max(n_ops, 1);
+  out.resize(first + static_cast<size_t>(info.n_instr));
+  Emitter em{nodes, tab, info.n_const, out.data() + first};
   em.gen(root);
-  info.n_instr = static_cast<int32_t>(out.size() - first);
-
-  // Cost model and declared work, over the executed instructions.
-  float cost = 0.f;
-  double sfu = 0, fp = 0;
-  for (size_t i = first; i < out.size(); ++i) {
-    const uint32_t w = out[i].w;
-    uint32_t op = instr_op(w);
-    if (op > kOpReversed) op -= kOpReversed;
-    cost += 2.0f + op_cost(static_cast<int>(op));
-    if (instr_load(w) && instr_leaf_kind(w) != kLeafC) cost += 0.5f;
-    const uint32_t bk = instr_b_kind(w);
-    if (bk == kBS || bk == kBX || bk == kBR) cost += 0.5f;
-    if (instr_spill(w)) cost += 0.5f;
-    double s, f;
-    declared_op_work(static_cast<int>(op), &s, &f);
-    sfu += s;
-    fp += f;
-  }
-  info.cost = cost + 6.0f;  // epilogue
-  info.sfu_ops = sfu;
-  info.fp32_ops = fp + 3.0;  // MSE epilogue per datapoint (declared model)
+  info.cost = em.cost + 6.0f;           // epilogue
+  info.sfu_ops = em.sfu;
+  info.fp32_ops = em.fp32 + 3.0;        // MSE epilogue per datapoint (declared model)
   return SR_OK;
 }
 
