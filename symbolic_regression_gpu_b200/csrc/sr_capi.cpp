@@ -90,8 +90,12 @@ sr_status check_population(sr_context *ctx, const sr_population *pop) {
 }
 
 // Compile expressions [0, E) of a CSR population into ps (pinned staging).
+// With `share` equal expressions are compiled once and folded subtrees and
+// derived rows collapse to leaves; folded subtrees, there and under kHintFold
+// hints, are added to ctx->folds.
 sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *val,
-                      const int64_t *off, const int32_t *hints, ProgramSet &ps) {
+                      const int64_t *off, const int32_t *hints, ProgramSet &ps,
+                      const sr::Sharing *share) {
   SR_TRACE("sr: compile");
   ps.E = E;
   ps.cost.assign(static_cast<size_t>(E), 0.f);
@@ -100,67 +104,106 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
   ps.n_instr = 0;
   ps.n_tokens = 0;
   ps.sfu_per_dp = ps.fp32_per_dp = 0.0;
+  ps.n_derived = 0;
   // About 20 ns a token, and tens of microseconds to wake the workers: chunks
   // of 2,500 tokens or more, one thread below two of them.
   const int64_t n_tok = E > 0 ? off[E] - off[0] : 0;
   const int nt = static_cast<int>(
       std::max<int64_t>(1, std::min<int64_t>({host_threads(ctx), E, n_tok / 2500})));
-  std::vector<std::vector<Instr>> codes(static_cast<size_t>(nt));
+  struct Chunk {
+    std::vector<Instr> code;
+    std::vector<sr::FoldSet::Ref> folds;  // loc and first relative to the chunk
+    std::vector<uint2> fold_tokens;
+    sr_status st = SR_OK;
+    std::string msg;
+    int64_t bad = -1, in_profile = 0;
+    bool refs = false;
+  };
+  std::vector<Chunk> chunks(static_cast<size_t>(nt));
   std::vector<sr::ExprInfo> infos(static_cast<size_t>(E));
-  std::vector<sr_status> st(static_cast<size_t>(nt), SR_OK);
-  std::vector<std::string> msg(static_cast<size_t>(nt));
-  std::vector<int64_t> bad(static_cast<size_t>(nt), -1);
-  std::vector<int64_t> in_profile(static_cast<size_t>(nt), 0);
-  std::vector<char> refs(static_cast<size_t>(nt), 0);
+  std::vector<int32_t> reps(share ? static_cast<size_t>(E) : 0);
   const auto compile_chunk = [&](int ci) {
-    const size_t c = static_cast<size_t>(ci);
+    Chunk &c = chunks[static_cast<size_t>(ci)];
     const int64_t x0 = static_cast<int64_t>(E) * ci / nt, x1 = static_cast<int64_t>(E) * (ci + 1) / nt;
-    auto &code = codes[c];
-    code.reserve(static_cast<size_t>((off[x1] - off[x0]) * 2 / 3 + 8));
-    std::string err;
+    c.code.reserve(static_cast<size_t>((off[x1] - off[x0]) * 2 / 3 + 8));
+    std::vector<int32_t> marks(share ? SR_MAX_TOKENS : 0);
+    std::vector<sr::FoldRef> refs;
     for (int64_t x = x0; x < x1; ++x) {
-      const sr_status s = sr::compile_expression(
-          tok + off[x], val + off[x], static_cast<int>(off[x + 1] - off[x]), ctx->V,
-          hints ? hints + off[x] : nullptr, code, infos[static_cast<size_t>(x)], &err);
+      sr::ExprInfo &info = infos[static_cast<size_t>(x)];
+      const int len = static_cast<int>(off[x + 1] - off[x]);
+      const int32_t *h = hints ? hints + off[x] : nullptr;
+      if (share) {
+        const int r = share->rep(static_cast<int>(x));
+        reps[static_cast<size_t>(x)] = r;
+        if (r == x && share->mark(static_cast<int>(x), marks.data())) h = marks.data();
+        if (r != x) {
+          info.n_tokens = len;
+          sr::declared_work(tok + off[x], len, &info.sfu_ops, &info.fp32_ops);
+          info.fp32_ops += 3.0;
+          continue;
+        }
+      }
+      const int64_t i0 = static_cast<int64_t>(c.code.size());
+      refs.clear();
+      const sr_status s = sr::compile_expression(tok + off[x], val + off[x], len, ctx->V, h, c.code,
+                                                 info, &c.msg, ctx->V + 1, &refs);
       if (s != SR_OK) {
-        st[c] = s;
-        msg[c] = err;
-        bad[c] = x;
+        c.st = s;
+        c.bad = x;
         return;
       }
+      if (share) {  // the declared work is that of the whole expression
+        sr::declared_work(tok + off[x], len, &info.sfu_ops, &info.fp32_ops);
+        info.fp32_ops += 3.0;
+      }
+      for (const sr::FoldRef &f : refs) {
+        const int64_t t0 = off[x] + f.tok;
+        uint32_t n = 0;
+        for (int need = 1; need > 0; ++n) {
+          const int t = tok[t0 + n];
+          need += t <= 0 ? -1 : (sr::is_binary_token(t) ? 1 : 0);
+          uint2 w{static_cast<uint32_t>(t), 0u};
+          const float v = static_cast<float>(val[t0 + n]);
+          if (t == SR_TOK_CONST) std::memcpy(&w.y, &v, sizeof v);
+          c.fold_tokens.push_back(w);
+        }
+        c.folds.push_back(sr::FoldSet::Ref{&ps, (i0 << 1) + f.loc,
+                                           static_cast<uint32_t>(c.fold_tokens.size()) - n, n});
+      }
     }
-    int64_t n_prot = 0;
-    bool cached = false;
-    for (Instr &in : code) {
+    for (Instr &in : c.code) {
       in.w = sr::with_dispatch(in.w);
-      n_prot += sr::in_protected_profile(sr::instr_op(in.w)) ? 1 : 0;
-      cached = cached || (sr::instr_load(in.w) && sr::instr_leaf_kind(in.w) == sr::kLeafR) ||
+      c.in_profile += sr::in_protected_profile(sr::instr_op(in.w)) ? 1 : 0;
+      c.refs = c.refs || (sr::instr_load(in.w) && sr::instr_leaf_kind(in.w) == sr::kLeafR) ||
                sr::instr_b_kind(in.w) == sr::kBR;
     }
-    in_profile[c] = n_prot;
-    refs[c] = cached ? 1 : 0;
   };
   ctx->workers.run(nt, nt, compile_chunk);
-  for (int c = 0; c < nt; ++c)
-    if (st[static_cast<size_t>(c)] != SR_OK)
-      return ctx->fail(st[static_cast<size_t>(c)],
-                       "expression " + std::to_string(bad[static_cast<size_t>(c)]) + ": " +
-                           msg[static_cast<size_t>(c)]);
   int64_t total = 0;
-  for (auto &c : codes) total += static_cast<int64_t>(c.size());
+  for (const Chunk &c : chunks) {
+    if (c.st != SR_OK)
+      return ctx->fail(c.st, "expression " + std::to_string(c.bad) + ": " + c.msg);
+    total += static_cast<int64_t>(c.code.size());
+  }
   SR_TRY_CUDA(ctx, ps.layout_host(static_cast<size_t>(total + 1), static_cast<size_t>(E)));
   int64_t pos = 0;
-  for (auto &c : codes) {
-    std::memcpy(ps.h_code.p + pos, c.data(), c.size() * sizeof(Instr));
-    pos += static_cast<int64_t>(c.size());
-  }
-  ps.h_code.p[total] = Instr{0, 0, 0, 0};  // prefetch padding
   ps.n_instr_protected = 0;
   ps.cache_refs = false;
-  for (size_t c = 0; c < codes.size(); ++c) {
-    ps.n_instr_protected += in_profile[c];
-    ps.cache_refs = ps.cache_refs || refs[c] != 0;
+  for (const Chunk &c : chunks) {
+    const uint32_t t0 = static_cast<uint32_t>(ctx->folds.tokens.size());
+    for (sr::FoldSet::Ref r : c.folds) {
+      r.loc += pos << 1;
+      r.first += t0;
+      ctx->folds.refs.push_back(r);
+    }
+    ctx->folds.tokens.insert(ctx->folds.tokens.end(), c.fold_tokens.begin(), c.fold_tokens.end());
+    std::memcpy(ps.h_code.p + pos, c.code.data(), c.code.size() * sizeof(Instr));
+    pos += static_cast<int64_t>(c.code.size());
+    ps.n_instr_protected += c.in_profile;
+    ps.cache_refs = ps.cache_refs || c.refs;
   }
+  ps.h_code.p[total] = Instr{0, 0, 0, 0};  // prefetch padding
+  ps.n_listed = E;
   int64_t o = 0;
   for (int x = 0; x < E; ++x) {
     const auto &in = infos[static_cast<size_t>(x)];
@@ -173,8 +216,107 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
     ps.n_tokens += in.n_tokens;
     ps.sfu_per_dp += in.sfu_ops;
     ps.fp32_per_dp += in.fp32_ops;
+    if (share) {
+      ps.h_row.p[x] = reps[static_cast<size_t>(x)];
+      if (reps[static_cast<size_t>(x)] != x) --ps.n_listed;
+    }
   }
+  ps.shared = ps.n_listed < E;
   ps.n_instr = total;
+  return SR_OK;
+}
+
+// Copies the folded subtrees collected by compile_set and has the device
+// compute them into the (uploaded) programs.
+static sr_status upload_folds(sr_context *ctx) {
+  sr::FoldSet &f = ctx->folds;
+  if (f.refs.empty()) return SR_OK;
+  const size_t ib = f.refs.size() * sizeof(sr::FoldItem), tb = f.tokens.size() * sizeof(uint2);
+  SR_TRY_CUDA(ctx, f.h_pack.ensure(ib + tb));
+  SR_TRY_CUDA(ctx, f.pack.ensure(ib + tb));
+  auto *items = reinterpret_cast<sr::FoldItem *>(f.h_pack.p);
+  for (size_t i = 0; i < f.refs.size(); ++i) {
+    const sr::FoldSet::Ref &r = f.refs[i];
+    Instr *in = r.set->code.p + (r.loc >> 1);
+    items[i] = sr::FoldItem{r.first, r.len, (r.loc & 1) ? &in->b : &in->a};
+  }
+  std::memcpy(f.h_pack.p + ib, f.tokens.data(), tb);
+  ctx->prep_stats.h2d_bytes += static_cast<int64_t>(ib + tb);
+  SR_TRY_CUDA(ctx, cudaMemcpyAsync(f.pack.p, f.h_pack.p, ib + tb, cudaMemcpyHostToDevice,
+                                   ctx->stream));
+  SR_TRY_CUDA(ctx, sr::launch_fold(reinterpret_cast<const sr::FoldItem *>(f.pack.p),
+                                   reinterpret_cast<const uint2 *>(f.pack.p + ib),
+                                   static_cast<int>(f.refs.size()), ctx->stream));
+  return SR_OK;
+}
+
+// Derived rows of a population, at most: 23 rows of 512-datapoint spans, twice
+// buffered, fit in shared memory beside four spill slots for each of 31 warps.
+// More rows leave 256-datapoint spans, whose items cost what the rows save
+// (batched population, interpreter: none 42.9 ms, 16 rows 37.7, 32 rows at 256
+// datapoints 37.5; 24 rows with two spill slots, deeper ones in global scratch,
+// 46.9).  A bounded part of the device's memory too.
+static int derived_row_limit(const sr_context *ctx) {
+  int r = std::min(16, 22 - ctx->V);
+  const double row = static_cast<double>(ctx->ldx) * sizeof(float);
+  const double room = std::min(1073741824.0, static_cast<double>(ctx->device_memory) / 16.0);
+  r = std::min(r, static_cast<int>(room / row));
+  return r < 4 ? 0 : std::min(r, sr::kMaxDerivedRows);
+}
+
+// Whether finding shared work pays: the search and the two more kernels cost
+// 0.1 to 0.2 ms of a call at 15,000 tokens and 0.8 ms at 170,000, and the
+// evaluation, 0.3 ms per 1e9 tokens x datapoints, becomes a fifth to a third
+// shorter (1,000 ramped trees x 100k, 1.5e9: 811 -> 770 us a call; 1,531 bred
+// trees x 250k, 6.9e9: 2.40 -> 2.34 ms; 10,000 x 1M, 1.7e11: 49.8 -> 39.8 ms).
+static bool sharing_pays(const sr_context *ctx, const sr_population *pop) {
+  return static_cast<double>(pop->offsets[pop->num_exprs]) * static_cast<double>(ctx->N) >= 1e9;
+}
+
+// Batched programs: shared work found and taken out where that pays, then
+// compiled, planned and uploaded.
+static sr_status prepare_batched(sr_context *ctx, const sr_population *pop) {
+  const int E = pop->num_exprs;
+  const double tc0 = now_ms();
+  sr::Sharing &sh = ctx->sharing;
+  ctx->rows.plan = sr::Plan{};
+  bool share = sharing_pays(ctx, pop);
+  if (share) {
+    SR_TRACE("sr: share");
+    share = sh.find(E, pop->tokens, pop->values, pop->offsets, derived_row_limit(ctx),
+                    ctx->workers, host_threads(ctx));
+    // Rows are an option: without the memory for them they are evaluated in
+    // place like everything else.
+    if (share && !sh.rows().empty() &&
+        ctx->derived.ensure(sh.rows().size() * static_cast<size_t>(ctx->ldx)) != cudaSuccess) {
+      cudaGetLastError();
+      sh.drop_rows();
+    }
+  }
+  SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, nullptr, ctx->main,
+                     share ? &sh : nullptr));
+  if (share && !sh.rows().empty()) {
+    std::vector<int32_t> tok, hints;
+    std::vector<double> val;
+    std::vector<int64_t> off{0};
+    for (const auto &r : sh.rows()) {
+      tok.insert(tok.end(), pop->tokens + r.tok, pop->tokens + r.tok + r.size);
+      val.insert(val.end(), pop->values + r.tok, pop->values + r.tok + r.size);
+      hints.resize(tok.size());
+      sh.mark_row(r, hints.data() + off.back());
+      off.push_back(static_cast<int64_t>(tok.size()));
+    }
+    const int R = static_cast<int>(sh.rows().size());
+    SR_TRY(compile_set(ctx, R, tok.data(), val.data(), off.data(), hints.data(), ctx->rows));
+    for (int r = 0; r < R; ++r) ctx->rows.h_row.p[r] = r;
+    SR_TRY(plan_set(ctx, ctx->rows, true, 8, sr::kMaxWarps));
+    SR_TRY(upload_set(ctx, ctx->rows, true));
+    ctx->main.n_derived = R;
+  }
+  ctx->prep_stats.host_compile_time_ms = now_ms() - tc0;
+  SR_TRY(prepare_main_shape(ctx, true, false));
+  ctx->prep_stats.node_evals = ctx->main.n_tokens * ctx->N;
+  ctx->prep_stats.node_evals_executed = ctx->prep_stats.node_evals;
   return SR_OK;
 }
 
@@ -188,14 +330,20 @@ bool protected_profile(const ProgramSet &ps) {
          static_cast<double>(ps.n_instr_protected) >= sr::kProtectedShare * ps.n_instr;
 }
 
-// The expressions in decreasing cost, equal ones in index order: a counting
-// sort over half units of cost (all costs are multiples of one; those above the
-// last bucket, far beyond any program that differs in rank, keep index order).
-static void cost_order(const std::vector<float> &cost, int E, int32_t *order) {
-  if (E < 1024) {  // fewer than the buckets' own cost
-    std::iota(order, order + E, 0);
-    std::stable_sort(order, order + E, [&](int32_t a, int32_t b) {
-      return cost[static_cast<size_t>(a)] > cost[static_cast<size_t>(b)];
+// The listed expressions in decreasing cost, equal ones in index order: a
+// counting sort over half units of cost (all costs are multiples of one; those
+// above the last bucket, far beyond any program that differs in rank, keep
+// index order).
+static void cost_order(const ProgramSet &ps, sr::GroupRec *order) {
+  const std::vector<float> &cost = ps.cost;
+  const auto listed = [&](int x) { return !ps.shared || ps.h_row.p[x] == x; };
+  const auto rec = [&](int x) { return sr::GroupRec{x, ps.h_len.p[x], ps.h_off.p[x]}; };
+  if (ps.E < 1024) {  // fewer than the buckets' own cost
+    int n = 0;
+    for (int x = 0; x < ps.E; ++x)
+      if (listed(x)) order[n++] = rec(x);
+    std::stable_sort(order, order + n, [&](const sr::GroupRec &a, const sr::GroupRec &b) {
+      return cost[static_cast<size_t>(a.e)] > cost[static_cast<size_t>(b.e)];
     });
     return;
   }
@@ -205,9 +353,11 @@ static void cost_order(const std::vector<float> &cost, int E, int32_t *order) {
     return kBuckets - 1 -
            static_cast<int>(std::min(2.0f * cost[static_cast<size_t>(x)], kBuckets - 1.0f));
   };
-  for (int x = 0; x < E; ++x) ++start[static_cast<size_t>(bucket(x)) + 1];
+  for (int x = 0; x < ps.E; ++x)
+    if (listed(x)) ++start[static_cast<size_t>(bucket(x)) + 1];
   for (int b = 0; b < kBuckets; ++b) start[static_cast<size_t>(b) + 1] += start[static_cast<size_t>(b)];
-  for (int x = 0; x < E; ++x) order[start[static_cast<size_t>(bucket(x))]++] = x;
+  for (int x = 0; x < ps.E; ++x)
+    if (listed(x)) order[start[static_cast<size_t>(bucket(x))]++] = rec(x);
 }
 
 // Size class of a launch, from its 256-datapoint tiles of expressions per SM:
@@ -257,15 +407,23 @@ sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, i
   p.W = W;
   p.ops = (!pred && protected_profile(ps)) ? sr::kOpsProtected : sr::kOpsAll;
   p.smax = std::max(ps.smax, 0);
-  p.s_smem = std::min(p.smax, split < 0 ? sr::smem_spill_slots(dpt) : split);
+  const int slots = sr::smem_spill_slots(dpt);
+  p.s_smem = std::min(p.smax, split >= 0 ? split : slots);
   p.general = !pred && (ps.cache_refs || p.s_smem < p.smax);
   const int64_t tile = 32 * dpt;
-  const int E = ps.E;
+  const int E = ps.n_listed;
+  const int rows = ctx->V + ps.n_derived;  // besides y
   const bool by_size = per_warp <= 0;
   if (by_size) {
     const int size = launch_size(ctx, E);
     per_warp = size <= 1 ? 1 : (size == 2 ? 2 : 4);
     if (size <= 1) span_target = static_cast<int>(std::max<int64_t>(tile, kMinSpan));
+    // Derived rows fill shared memory: spans of 512 at most, and at a middle
+    // size twice the expressions for them.
+    if (ps.n_derived > 0 && span_target > 512) {
+      span_target = 512;
+      per_warp = 4;
+    }
   }
   p.G = std::max(1, W * per_warp);
   p.n_groups = (E + p.G - 1) / p.G;
@@ -273,7 +431,7 @@ sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, i
   // Span: the target, shrunk to the data and to the shared-memory budget.
   int64_t span = std::min<int64_t>(span_target, std::max<int64_t>(tile, round_up(ctx->N, tile)));
   auto smem_at = [&](int64_t sp) {
-    return sr::interp_smem_bytes(dpt, W, ctx->V, p.s_smem, static_cast<int>(sp), p.G, pred);
+    return sr::interp_smem_bytes(dpt, W, rows, p.s_smem, static_cast<int>(sp), p.G, pred);
   };
   while (span > tile && smem_at(span) > max_smem) span = std::max<int64_t>(tile, (span / 2) / tile * tile);
   // Then, while the span's shared memory (the X buffers grow with the
@@ -315,7 +473,7 @@ sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, i
   // x span groups.  It is sized against the device's memory (the allocation
   // itself reports SR_ERR_OUT_OF_MEMORY when the free memory is short).
   if (!pred) {
-    const double need = static_cast<double>(p.n_span_groups()) * E * 32.0;
+    const double need = static_cast<double>(p.n_span_groups()) * ps.E * 32.0;
     if (need > 0.9 * static_cast<double>(ctx->device_memory))
       return ctx->fail(SR_ERR_UNSUPPORTED,
                        "partial-sum buffer (" + std::to_string(static_cast<int64_t>(need)) +
@@ -342,8 +500,9 @@ sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, i
   // Group table: expressions in decreasing modelled cost, G per group, so
   // every group holds similar work and hands out its largest first.
   if (p.G > sr::kMaxGroup) return ctx->fail(SR_ERR_UNSUPPORTED, "expression group too large");
-  cost_order(ps.cost, E, ps.h_group.p);
-  for (int64_t k = E; k < static_cast<int64_t>(p.n_groups) * p.G; ++k) ps.h_group.p[k] = -1;
+  cost_order(ps, ps.h_group.p);
+  for (int64_t k = ps.n_listed; k < static_cast<int64_t>(p.n_groups) * p.G; ++k)
+    ps.h_group.p[k] = sr::GroupRec{-1, 0, 0};
   ps.plan = p;
   return SR_OK;
 }
@@ -351,8 +510,8 @@ sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, i
 sr_status upload_groups(sr_context *ctx, ProgramSet &ps) {
   SR_TRACE("sr: upload groups");
   const size_t ng = static_cast<size_t>(std::max(ps.plan.n_groups * ps.plan.G, 1));
-  ctx->prep_stats.h2d_bytes += static_cast<int64_t>(ng * sizeof(int32_t));
-  SR_TRY_CUDA(ctx, cudaMemcpyAsync(ps.group.p, ps.h_group.p, ng * sizeof(int32_t),
+  ctx->prep_stats.h2d_bytes += static_cast<int64_t>(ng * sizeof(sr::GroupRec));
+  SR_TRY_CUDA(ctx, cudaMemcpyAsync(ps.group.p, ps.h_group.p, ng * sizeof(sr::GroupRec),
                                    cudaMemcpyHostToDevice, ctx->stream));
   return SR_OK;
 }
@@ -394,7 +553,7 @@ sr::EvalArgs make_args(sr_context *ctx, ProgramSet &ps, int32_t *counter) {
   a.code = ps.code.p;
   a.code_off = ps.off.p;
   a.code_len = ps.len.p;
-  a.group_expr = ps.group.p;
+  a.groups = ps.group.p;
   a.partial = ctx->partial.p;
   a.work_counter = counter;
   a.error = ctx->d_error;
@@ -402,6 +561,9 @@ sr::EvalArgs make_args(sr_context *ctx, ProgramSet &ps, int32_t *counter) {
   a.ldc = ctx->ldx;
   a.V = ctx->V;
   a.E = ps.E;
+  a.derived = ctx->derived.p;
+  a.n_derived = ps.n_derived;
+  a.n_listed = ps.n_listed;
   a.W = ps.plan.W;
   a.smax = ps.plan.smax;
   a.G = ps.plan.G;
@@ -427,6 +589,13 @@ sr_status launch_set(sr_context *ctx, ProgramSet &ps, bool pred, int32_t *counte
   return SR_OK;
 }
 
+// Derived rows of the prepared population, if it has any.
+static sr_status launch_rows(sr_context *ctx) {
+  if (ctx->main.n_derived == 0) return SR_OK;
+  return launch_set(ctx, ctx->rows, true, ctx->d_counter + 1, ctx->derived.p, ctx->ldx,
+                    ctx->rows.row.p);
+}
+
 // ---- launch-shape tuning ---------------------------------------------------
 
 std::string tune_key(const sr_context *ctx, const ProgramSet &ps) {
@@ -438,6 +607,7 @@ std::string tune_key(const sr_context *ctx, const ProgramSet &ps) {
   k << ctx->device_name << "|V" << ctx->V << "|N" << lg_n << "|E" << lg_e << "|I"
     << static_cast<int>(std::lround(std::log2(1.0 + mean_instr) * 4.0)) << "|S" << ps.smax
     << "|P" << (prot ? sr::kOpsProtected : sr::kOpsAll);
+  if (ps.n_derived > 0) k << "|R" << ps.n_derived;
   return k.str();
 }
 
@@ -564,8 +734,13 @@ sr_status prepare_main_shape(sr_context *ctx, bool allow_tune, bool on_device) {
     const std::string key = tune_key(ctx, ps);
     auto it = ctx->tuned.find(key);
     if (it == ctx->tuned.end() && allow_tune && ctx->opts.autotune && ps.E > 0 && ctx->N > 0) {
-      if (!on_device) SR_TRY(upload_set(ctx, ps, false));
-      on_device = true;
+      if (!on_device) {
+        SR_TRY(upload_set(ctx, ps, false));
+        SR_TRY(upload_folds(ctx));
+        SR_TRY(begin_sequence(ctx));
+        SR_TRY(launch_rows(ctx));
+        on_device = true;
+      }
       SR_TRY(autotune_main(ctx, key));
       it = ctx->tuned.find(key);
     }
@@ -580,14 +755,15 @@ sr_status prepare_main_shape(sr_context *ctx, bool allow_tune, bool on_device) {
     const bool have = it != ctx->tuned.end();
     int wide = 8;
     if (prot) {
-      const int s_smem = std::min(std::max(ps.smax, 0), sr::smem_spill_slots(8));
+      const int s_smem = std::min(std::max(ps.smax, 0),
+                                  ps.n_derived > 0 ? 2 : sr::smem_spill_slots(8));
       const int W = sr::kMaxInterpWarps;
-      if (sr::interp_smem_bytes(8, W, ctx->V, s_smem, 32 * 8 * 2, W * 4, false) <=
+      if (sr::interp_smem_bytes(8, W, ctx->V + ps.n_derived, s_smem, 32 * 8 * 2, W * 4, false) <=
           static_cast<size_t>(ctx->max_smem))
         wide = W;
     }
     const int tdpt = have ? it->second.dpt : (prot ? 8 : 4);
-    const bool small = launch_size(ctx, ps.E) == 0;
+    const bool small = launch_size(ctx, ps.n_listed) == 0;
     const int tw = have ? it->second.W : (small ? 8 : (prot ? wide : 16));
     // the tuned split belongs to the tuned shape only
     if (have && (dpt == 0 || dpt == tdpt) && (W == 0 || W == tw)) {
@@ -599,10 +775,12 @@ sr_status prepare_main_shape(sr_context *ctx, bool allow_tune, bool on_device) {
   }
   if (ctx->opts.smem_spill_slots >= 0) split = ctx->opts.smem_spill_slots;
   SR_TRY(plan_set(ctx, ps, false, dpt, W, split, per_warp));
-  if (on_device)
+  if (on_device) {
     SR_TRY(upload_groups(ctx, ps));
-  else
+  } else {
     SR_TRY(upload_set(ctx, ps, true));
+    SR_TRY(upload_folds(ctx));
+  }
   SR_TRY_CUDA(ctx, ctx->partial.ensure(static_cast<size_t>(std::max<int64_t>(
                        2 * static_cast<int64_t>(ps.plan.n_span_groups()) * ps.E, 1))));
   return SR_OK;
@@ -625,6 +803,8 @@ cudaError_t sr::capi::record_event(sr_context *ctx, int k) {
 // point into buffers that the next prepare / set_data may move).
 void sr::capi::reset_prepared(sr_context *ctx) {
   ctx->mode = sr::Mode::kNone;
+  ctx->folds.refs.clear();
+  ctx->folds.tokens.clear();
   ctx->launched = false;
   ctx->cache.rollback();  // subtrees of a launch that never ran hold no values
   if (ctx->graph_exec) {
@@ -1158,16 +1338,16 @@ sr_status sr_prepare(sr_context *ctx, const sr_population *pop, uint32_t flags) 
     SR_TRY(prepare_cached(ctx, pop, flags));
     ctx->mode = sr::Mode::kCached;
   } else {
-    const double tc0 = now_ms();
-    SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, nullptr, ctx->main));
-    ctx->prep_stats.host_compile_time_ms = now_ms() - tc0;
-    SR_TRY(prepare_main_shape(ctx, true, false));
-    ctx->prep_stats.node_evals = ctx->main.n_tokens * ctx->N;
-    ctx->prep_stats.node_evals_executed = ctx->prep_stats.node_evals;
+    SR_TRY(prepare_batched(ctx, pop));
     ctx->mode = sr::Mode::kBatched;
   }
   SR_TRY_CUDA(ctx, cudaEventRecord(ctx->ev[5], ctx->stream));
   return SR_OK;
+}
+
+// Where each expression's result is, when equal ones share an evaluation.
+static const int32_t *representatives(const sr_context *ctx) {
+  return ctx->mode == sr::Mode::kBatched && ctx->main.shared ? ctx->main.row.p : nullptr;
 }
 
 // Enqueue the prepared launch sequence on the context stream.
@@ -1195,13 +1375,18 @@ static sr_status enqueue_launch(sr_context *ctx, int *launches_out) {
                         ctx->sub.row.p));
       ++launches;
     }
+    if (ctx->mode == sr::Mode::kBatched && ctx->main.n_derived > 0 && ctx->rows.plan.items() > 0) {
+      SR_TRY(launch_rows(ctx));
+      ++launches;
+    }
     SR_TRY_CUDA(ctx, record_event(ctx, 1));
     if (ctx->main.plan.items() > 0) {
       SR_TRY(launch_set(ctx, ctx->main, false, ctx->d_counter, nullptr, 0, nullptr));
       ++launches;
     }
     SR_TRY_CUDA(ctx, record_event(ctx, 2));
-    SR_TRY_CUDA(ctx, sr::launch_finalize_groups(ctx->partial.p, ctx->main.plan.n_span_groups(),
+    SR_TRY_CUDA(ctx, sr::launch_finalize_groups(ctx->partial.p, representatives(ctx),
+                                                ctx->main.plan.n_span_groups(),
                                                 ctx->E, ctx->mse.p, nullptr, sequence_end(ctx),
                                                 s));
     ctx->counters_used = false;
@@ -1346,7 +1531,7 @@ sr_status sr_read_sums(sr_context *ctx, double *sum_out, double *count_out) {
   else if (ctx->mode == sr::Mode::kGrad)
     ;  // the gradient finalize kernels wrote ctx->sums
   else
-    SR_TRY_CUDA(ctx, sr::launch_finalize_groups(ctx->partial.p, n_spans, E, nullptr,
+    SR_TRY_CUDA(ctx, sr::launch_finalize_groups(ctx->partial.p, representatives(ctx), n_spans, E, nullptr,
                                                 ctx->sums.p, sr::SequenceEnd{}, ctx->stream));
   SR_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->h_sums.p, ctx->sums.p, E * sizeof(double2),
                                    cudaMemcpyDeviceToHost, ctx->stream));

@@ -225,8 +225,9 @@ sr_status sr_prepare_device_population(sr_context *ctx, const int32_t *tokens,
   const size_t n_code = static_cast<size_t>(E) * (static_cast<size_t>(stride) + 1) + 1;
   SR_TRY_CUDA(ctx, ps.layout_device(n_code, static_cast<size_t>(E)));
   SR_TRY_CUDA(ctx, ps.layout_host(0, static_cast<size_t>(E)));  // the group table only
-  SR_TRY_CUDA(ctx, ctx->evo_summary.ensure(8));
-  SR_TRY_CUDA(ctx, ctx->h_evo_summary.ensure(8));
+  const size_t n_summary = 8 + 2 * static_cast<size_t>(E);
+  SR_TRY_CUDA(ctx, ctx->evo_summary.ensure(n_summary));
+  SR_TRY_CUDA(ctx, ctx->h_evo_summary.ensure(n_summary));
   SR_TRY_CUDA(ctx, ctx->mse.ensure(static_cast<size_t>(E) + 1));
   SR_TRY_CUDA(ctx, ctx->h_mse.ensure(static_cast<size_t>(E) + 1));
   // The interpreter prefetches one instruction past a program: keep the
@@ -235,7 +236,7 @@ sr_status sr_prepare_device_population(sr_context *ctx, const int32_t *tokens,
   SR_TRY_CUDA(ctx, sr::launch_compile_device(tokens, values, lengths, E, stride, ctx->V,
                                              ps.code.p, ps.off.p, ps.len.p, ctx->evo_summary.p,
                                              ctx->stream));
-  SR_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->h_evo_summary.p, ctx->evo_summary.p, 8 * sizeof(int32_t),
+  SR_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->h_evo_summary.p, ctx->evo_summary.p, n_summary * sizeof(int32_t),
                                    cudaMemcpyDeviceToHost, ctx->stream));
   SR_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   const int32_t *sm = ctx->h_evo_summary.p;
@@ -251,7 +252,15 @@ sr_status sr_prepare_device_population(sr_context *ctx, const int32_t *tokens,
   ps.n_instr = n_ins;
   ps.n_instr_protected = sm[6];
   ps.cache_refs = false;  // compiled without cache hints
-  ps.cost.assign(static_cast<size_t>(E), 0.0f);  // groups in population order
+  ps.n_listed = E;
+  ps.shared = false;
+  ps.n_derived = 0;
+  ps.cost.resize(static_cast<size_t>(E));
+  for (int x = 0; x < E; ++x) {
+    ps.h_off.p[x] = static_cast<int64_t>(x) * (stride + 1);
+    ps.h_len.p[x] = sm[8 + 2 * x];
+    std::memcpy(&ps.cost[static_cast<size_t>(x)], sm + 9 + 2 * x, sizeof(float));
+  }
   ps.n_const.assign(static_cast<size_t>(E), 0);
   ps.sfu_per_dp = 0.0;
   ps.fp32_per_dp = 0.0;

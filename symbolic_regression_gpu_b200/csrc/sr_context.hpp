@@ -17,6 +17,7 @@
 #include "sr_internal.hpp"
 #include "sr_parallel.hpp"
 #include "sr_program.hpp"
+#include "sr_share.hpp"
 
 namespace sr {
 
@@ -134,19 +135,21 @@ struct ProgramSet {
   Region<int64_t> off, h_off;
   Region<int32_t> len, h_len;
   Region<int32_t> row, h_row;
-  Region<int32_t> group, h_group;  // the last region: E + kMaxGroup entries
-  template <class B>
+  Region<GroupRec> group, h_group;  // the last region: E + kMaxGroup entries
   static void place(unsigned char *base, size_t n_code, size_t E, Region<Instr> &c,
-                    Region<int64_t> &o, Region<int32_t> &l, Region<int32_t> &r, B &g) {
+                    Region<int64_t> &o, Region<int32_t> &l, Region<int32_t> &r,
+                    Region<GroupRec> &g) {
     c.p = reinterpret_cast<Instr *>(base);
     o.p = reinterpret_cast<int64_t *>(base + n_code * sizeof(Instr));
     l.p = reinterpret_cast<int32_t *>(o.p + E);
     r.p = l.p + E;
-    g.p = r.p + E;
+    g.p = reinterpret_cast<GroupRec *>(base + groups_at(n_code, E));
+  }
+  static size_t groups_at(size_t n_code, size_t E) {
+    return (n_code * sizeof(Instr) + E * (sizeof(int64_t) + 2 * sizeof(int32_t)) + 15) / 16 * 16;
   }
   static size_t pack_bytes(size_t n_code, size_t E) {
-    return n_code * sizeof(Instr) + E * (sizeof(int64_t) + 3 * sizeof(int32_t)) +
-           kMaxGroup * sizeof(int32_t);
+    return groups_at(n_code, E) + (E + kMaxGroup) * sizeof(GroupRec);
   }
   // Room for n_code instructions (the padding one included) and n expressions.
   cudaError_t layout_host(size_t n_code, size_t n) {
@@ -169,7 +172,23 @@ struct ProgramSet {
   int64_t n_tokens = 0;      // tokens represented (skeleton-equivalent)
   double sfu_per_dp = 0.0;   // declared work, summed over expressions
   double fp32_per_dp = 0.0;
+  int n_listed = 0;    // distinct expressions: the ones in the group table
+  bool shared = false; // row holds each expression's representative
+  int n_derived = 0;   // derived rows its programs read
   Plan plan;
+};
+
+// Folded constant subtrees of a prepared population: items, then tokens.
+struct FoldSet {
+  struct Ref {
+    ProgramSet *set;
+    int64_t loc;   // (instruction << 1) | (operand b)
+    uint32_t first, len;
+  };
+  std::vector<Ref> refs;
+  std::vector<uint2> tokens;
+  DevBuf<unsigned char> pack;
+  PinnedBuf<unsigned char> h_pack;
 };
 
 // Buffers of the plain baseline kernel.
@@ -289,6 +308,10 @@ struct sr_context {
   // compiled work
   sr::ProgramSet main;   // expressions (or skeletons)
   sr::ProgramSet sub;    // new cached subtrees of this call
+  sr::ProgramSet rows;   // derived rows of the prepared population
+  sr::DevBuf<float> derived;  // their values, [rows][ldx]
+  sr::FoldSet folds;
+  sr::Sharing sharing;
   sr::PlainSet plain;
   sr::Mode mode = sr::Mode::kNone;
   int E = 0;
@@ -329,7 +352,7 @@ struct sr_context {
   sr::DevBuf<int32_t> evo_idx;     // [E]
   sr::DevBuf<int32_t> evo_order;   // [E]
   sr::DevBuf<float> evo_fit;       // [E] fitness in rank order
-  sr::DevBuf<int32_t> evo_summary; // [8] see launch_compile_device
+  sr::DevBuf<int32_t> evo_summary; // [8 + 2E] see launch_compile_device
   sr::PinnedBuf<int32_t> h_evo_summary;
 
   // timing

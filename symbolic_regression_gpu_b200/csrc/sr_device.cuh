@@ -928,24 +928,29 @@ struct FoldArgs {
   int64_t C;
 };
 
-// The producer thread of a block: claims work items from the global counter
+// The producer warp of a block: lane 0 claims work items from the global counter
 // (item = span group x expression group, numbered expression-group-major: the
 // most expensive groups, which come first in the cost-sorted group table, are
 // claimed first and the last items are the cheapest; span-major numbering ended
-// on expensive ones, 1,000 x 100k: 818 against 710 us), and copies each of the item's spans
-// (k_spans consecutive spans, the last group shorter) with every row of X
-// into one of kBufs shared-memory buffers with the bulk-copy engine;
-// publishes item -1 when the work runs out.  A span lies in its buffer as
+// on expensive ones, 1,000 x 100k: 818 against 710 us), and its lanes copy each
+// of the item's spans (k_spans consecutive spans, the last group shorter) with
+// every row of X into one of kBufs shared-memory buffers with the bulk-copy
+// engine; it
+// publishes item -1 when the work runs out.  The first n_x of a span's rows
+// come from X, the others from `derived`.  A span lies in its buffer as
 // [span / chunk][rows][chunk] (`chunk` divides the span and is a multiple of 4
 // floats): with chunk = the tile of a warp, variable rows and spill slots have
-// the same stride, so one address computation serves both.  With FOLD (MSE launches) it also
-// folds, once the warps have released a buffer, the span slots written for it
-// into the item's accumulators (in span order) and writes each finished
-// item's sums out.  Every wait is bounded.
+// the same stride, so one address computation serves both.  With FOLD (MSE
+// launches) it also folds, once the warps have released a buffer, the span
+// slots written for it into the item's accumulators (in span order) and writes
+// each finished item's sums out, the expressions of the group over its lanes (one
+// thread folding the 124 slots of a span took thousands of issue slots a span).
+// Every wait is bounded.
 template <bool FOLD>
-__device__ __noinline__ void run_producer(int n_groups, int n_items, int k_spans, int n_spans,
-                                          int32_t *work_counter, int32_t *error, const float *X,
-                                          int64_t ldx, int rows, int span, int chunk, float *xbuf,
+__device__ __noinline__ void run_producer(int lane, int n_groups, int n_items, int k_spans,
+                                          int n_spans, int32_t *work_counter, int32_t *error, const float *X,
+                                          const float *derived, int n_x, int64_t ldx, int rows,
+                                          int span, int chunk, float *xbuf,
                                           ItemDesc *desc, uint64_t *full, uint64_t *empty,
                                           FoldArgs fa) {
   uint32_t buf = 0, phase = 0;
@@ -960,7 +965,7 @@ __device__ __noinline__ void run_producer(int n_groups, int n_items, int k_spans
   auto flush = [&]() {
     if constexpr (FOLD) {
       if (acc_item < 0) return;
-      for (int j = 0; j < acc_n; ++j) {
+      for (int j = lane; j < acc_n; j += 32) {
         const GroupAcc a = fa.acc[j];
         double2 *o = fa.out + 2 * (static_cast<int64_t>(acc_sg) * fa.E + a.e);
         o[0] = make_double2(a.hi, a.lo);
@@ -983,31 +988,44 @@ __device__ __noinline__ void run_producer(int n_groups, int n_items, int k_spans
         acc_sg = it % ((n_spans + k_spans - 1) / k_spans);
         const int g = held_group[b];
         acc_n = min(fa.G, fa.n_valid - g * fa.G);  // groups are padded at their end only
-        for (int j = 0; j < acc_n; ++j) fa.acc[j] = GroupAcc{0.0, 0.0, 0.0, 0, 0};
-        for (int j = 0; j < acc_n * fa.K; ++j) fa.gacc[j] = 0.0;
+        for (int j = lane; j < acc_n; j += 32) {
+          fa.acc[j] = GroupAcc{0.0, 0.0, 0.0, 0, 0};
+          for (int c = 0; c < fa.K; ++c) fa.gacc[j * fa.K + c] = 0.0;
+        }
       }
       const SpanPart *q = fa.part + static_cast<size_t>(b) * fa.G;
-      for (int j = 0; j < acc_n; ++j) {
+      const double *gq = fa.gpart + static_cast<size_t>(b) * fa.G * fa.K;
+      for (int j = lane; j < acc_n; j += 32) {  // a lane keeps its expressions
         const SpanPart v = q[j];
-        dd_add(fa.acc[j].hi, fa.acc[j].lo, v.sum);
-        fa.acc[j].cnt += static_cast<double>(v.cnt);
-        fa.acc[j].e = v.e;
-      }
-      if (fa.K > 0) {
-        const double *gq = fa.gpart + static_cast<size_t>(b) * fa.G * fa.K;
-        for (int j = 0; j < acc_n * fa.K; ++j) fa.gacc[j] += gq[j];
+        GroupAcc a = fa.acc[j];
+        dd_add(a.hi, a.lo, v.sum);
+        a.cnt += static_cast<double>(v.cnt);
+        a.e = v.e;
+        fa.acc[j] = a;
+        for (int c = 0; c < fa.K; ++c) fa.gacc[j * fa.K + c] += gq[j * fa.K + c];
       }
       held[b] = false;
     }
   };
+  // Lane 0 waits; what it then sees the others see (the shuffle orders memory
+  // among them).
+  auto wait = [&](uint64_t *bar, uint32_t parity) {
+    bool ok = true;
+    if (lane == 0) ok = mbar_wait(bar, parity, error);
+    __syncwarp();
+    return __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+  };
   auto drain = [&]() {
     // Let copies already issued land before the block exits.
+    if (lane != 0) return;
     if (armed & 1u) mbar_drain(&full[0], fill_phase[0]);
     if (armed & 2u) mbar_drain(&full[1], fill_phase[1]);
   };
 
   for (;;) {
-    const int item = atomicAdd(work_counter, 1);
+    int item = 0;
+    if (lane == 0) item = atomicAdd(work_counter, 1);
+    item = __shfl_sync(0xffffffffu, item, 0);
     const bool last = item >= n_items;
     const int n_sg = (n_spans + k_spans - 1) / k_spans;
     const int group = last ? 0 : item / n_sg;
@@ -1015,7 +1033,7 @@ __device__ __noinline__ void run_producer(int n_groups, int n_items, int k_spans
     const int s_begin = sgi * k_spans;
     const int s_end = last ? 1 : min(n_spans, s_begin + k_spans);
     for (int sp = s_begin; sp < s_end; ++sp) {
-      if (!mbar_wait(&empty[buf], phase ^ 1u, error)) {
+      if (!wait(&empty[buf], phase ^ 1u)) {
         drain();
         return;
       }
@@ -1023,13 +1041,16 @@ __device__ __noinline__ void run_producer(int n_groups, int n_items, int k_spans
       // its span slots are complete.
       armed &= ~(1u << buf);
       if (held[buf]) fold(buf);
+      __syncwarp();  // the slots have been read: the warps may write them again
       if (last) {
-        desc[buf] = ItemDesc{-1, 0, 0, 0};
-        mbar_arrive(&full[buf]);
+        if (lane == 0) {
+          desc[buf] = ItemDesc{-1, 0, 0, 0};
+          mbar_arrive(&full[buf]);
+        }
         if (FOLD) {
           const uint32_t other = buf ^ 1u;
           if (held[other]) {
-            if (!mbar_wait(&empty[other], fill_phase[other], error)) {
+            if (!wait(&empty[other], fill_phase[other])) {
               drain();
               return;
             }
@@ -1039,14 +1060,20 @@ __device__ __noinline__ void run_producer(int n_groups, int n_items, int k_spans
         }
         return;
       }
-      desc[buf] = ItemDesc{item, group, sp, 0};
-      mbar_arrive_expect_tx(&full[buf], row_bytes * rows);
+      if (lane == 0) {
+        desc[buf] = ItemDesc{item, group, sp, 0};
+        mbar_arrive_expect_tx(&full[buf], row_bytes * rows);
+      }
+      __syncwarp();  // the expected bytes are set before any copy
       const float *src = X + static_cast<int64_t>(sp) * span;
+      const float *src_d = derived + static_cast<int64_t>(sp) * span;
       float *dst = xbuf + static_cast<size_t>(buf) * rows * span;
-      for (int c = 0; c < span; c += chunk)
-        for (int v = 0; v < rows; ++v)
-          bulk_g2s(dst + static_cast<size_t>(c) * rows + static_cast<size_t>(v) * chunk,
-                   src + v * ldx + c, chunk_bytes, &full[buf]);
+      const int n_chunks = rows * (span / chunk);  // [chunk of the span][row]
+      for (int k = lane; k < n_chunks; k += 32) {
+        const int v = k % rows, c = (k / rows) * chunk;
+        bulk_g2s(dst + static_cast<size_t>(k) * chunk,
+                 (v < n_x ? src + v * ldx : src_d + (v - n_x) * ldx) + c, chunk_bytes, &full[buf]);
+      }
       armed |= 1u << buf;
       fill_phase[buf] = phase;
       held[buf] = FOLD;

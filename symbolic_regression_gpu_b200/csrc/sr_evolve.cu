@@ -552,11 +552,15 @@ __global__ void compile_kernel(const int32_t *__restrict__ tok, const float *__r
   }
   code_len[i] = count;
   int prot = 0;
+  float cost = 6.0f;  // the host compiler's model: its group table is built from these
   for (int k = 0; k < count; ++k) {
     const uint32_t w = with_dispatch(code[base + k].w);
     code[base + k].w = w;
     prot += in_protected_profile(instr_op(w)) ? 1 : 0;
+    cost += instr_cost(w);
   }
+  summary[8 + 2 * i] = count;
+  summary[9 + 2 * i] = __float_as_int(cost);
   if (prot) atomicAdd(&summary[6], prot);
   atomicMax(&summary[0], need);
   atomicAdd(reinterpret_cast<unsigned long long *>(summary + 2), static_cast<unsigned long long>(n));

@@ -133,10 +133,65 @@ SR_HD uint32_t with_dispatch(uint32_t w) {
   return (w & ~(31u << kDShift)) | (d << kDShift);
 }
 
+// Modelled relative device cost of one operator per datapoint (used only to
+// order and balance work; calibrated by hand against instruction counts).
+SR_HD float operator_cost(int tok) {
+  switch (tok) {
+    case 4: return 10.f;              // DIV
+    case 8: return 12.f;              // LOOSE_DIV
+    case 18: return 8.f;              // INV
+    case 23: return 10.f;             // LOOSE_INV
+    case 26: return 8.f;              // SQRT
+    case 27: return 9.f;              // LOOSE_SQRT
+    case 10: case 11: return 24.f;    // SIN, COS
+    case 12: return 36.f;             // TAN
+    case 13: return 26.f;             // SINH
+    case 14: return 22.f;             // COSH
+    case 15: return 18.f;             // TANH
+    case 16: return 12.f;             // EXP
+    case 32: return 13.f;             // EXP_CLAMP
+    case 17: return 16.f;             // LOG
+    case 22: return 18.f;             // LOOSE_LOG
+    case 5: return 50.f;              // POW
+    case 9: return 52.f;              // LOOSE_POW
+    case 19: return 20.f;             // ASIN
+    case 20: case 21: return 22.f;    // ACOS, ATAN
+    default: return 1.f;
+  }
+}
+
+// Modelled cost of one instruction beside its operator: dispatch, operands in
+// memory, a spill.
+SR_HD float instr_cost(uint32_t w) {
+  uint32_t op = instr_op(w);
+  if (op > kOpReversed) op -= kOpReversed;
+  float c = 2.0f + operator_cost(static_cast<int>(op));
+  if (instr_load(w) && instr_leaf_kind(w) != kLeafC) c += 0.5f;
+  const uint32_t bk = instr_b_kind(w);
+  if (bk != kBNone && bk != kBC) c += 0.5f;
+  if (instr_spill(w)) c += 0.5f;
+  return c;
+}
+
 // Device-side error word bits.
 enum : int32_t {
   kDevErrTimeout = 1,   // a bounded mbarrier wait gave up
   kDevErrBounds = 2,    // a device bounds check fired (debug builds)
+};
+
+// One expression of a group: its program's place beside its index, so that
+// claiming an expression reads one 16-byte word (index, offset and length
+// were three loads one after the other).  e = -1 pads the last group.
+struct alignas(16) GroupRec {
+  int32_t e, len;
+  int64_t off;
+};
+
+// One folded subtree: its tokens (opcode, float bits) evaluated from the right
+// give the constant stored at dst.
+struct FoldItem {
+  uint32_t first, len;
+  uint32_t *dst;
 };
 
 // Argument block of the interpreter kernel (passed by value).
@@ -157,7 +212,8 @@ struct EvalArgs {
   const Instr *code;     // all programs back to back
   const int64_t *code_off;   // [E] first instruction of each expression
   const int32_t *code_len;   // [E] instruction count
-  const int32_t *group_expr; // [n_groups * G] expression index or -1 (tail)
+  const int32_t *group_expr; // [n_groups * G] expression index or -1 (tail): gradient launches
+  const GroupRec *groups;    // [n_groups * G] the same with its program: interpreter launches
   double2 *partial;      // [n_span_groups][E] x 2 (MSE launches; see span_per_item)
   int32_t *work_counter; // zeroed before each launch
   int32_t *error;        // device error word
@@ -174,6 +230,11 @@ struct EvalArgs {
   int32_t n_groups;
   int32_t span;          // datapoints per span, multiple of 32*DPT
   int32_t n_spans;
+  // Derived rows (values of shared subtrees over the dataset): rows V + 1 ..
+  // V + n_derived of a program's operands, [n_derived][ldx].
+  const float *derived;
+  int32_t n_derived;
+  int32_t n_listed;      // expressions in the group table
   // Spill slots [0, s_smem) of each warp live in shared memory, slots
   // [s_smem, smax) in this global scratch: per resident warp
   // (blockIdx.x * W + warp), (smax - s_smem) tiles of 32*DPT floats.

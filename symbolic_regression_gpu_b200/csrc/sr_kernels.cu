@@ -56,7 +56,7 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) interp_kernel(const Eva
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int W = p.W;
-  const int rows = p.V + 1;
+  const int rows = p.V + 1 + p.n_derived;
   const int span = p.span;
   float *xbuf = reinterpret_cast<float *>(smem_raw);
   float *sreg = xbuf + static_cast<size_t>(kBufs) * rows * span;
@@ -80,10 +80,9 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) interp_kernel(const Eva
   const int n_items = p.n_groups * ((p.n_spans + k_spans - 1) / k_spans);
 
   if (warp == W) {
-    if (lane == 0)
-      run_producer<!PRED>(p.n_groups, n_items, k_spans, p.n_spans, p.work_counter, p.error, p.X,
-                          p.ldx, rows, span, TILE, xbuf, desc, full, empty,
-                          FoldArgs{part, gacc, p.partial, p.G, p.E, p.E, 0, nullptr, nullptr, nullptr,
+    run_producer<!PRED>(lane, p.n_groups, n_items, k_spans, p.n_spans, p.work_counter, p.error, p.X,
+                          p.derived, p.V + 1, p.ldx, rows, span, TILE, xbuf, desc, full, empty,
+                          FoldArgs{part, gacc, p.partial, p.G, p.E, p.n_listed, 0, nullptr, nullptr, nullptr,
                                    nullptr, nullptr, 0});
     return;
   }
@@ -107,10 +106,14 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) interp_kernel(const Eva
       if (lane == 0) j = atomicAdd(&desc[buf].claim, 1);
       j = __shfl_sync(0xffffffffu, j, 0);
       if (j >= p.G) break;
-      const int e = p.group_expr[static_cast<int64_t>(d.group) * p.G + j];
+      // One 16-byte record: the expression and its program's place.
+      const int4 rec = __ldg(reinterpret_cast<const int4 *>(
+          p.groups + static_cast<int64_t>(d.group) * p.G + j));
+      const int e = rec.x;
       if (e < 0) break;  // groups are padded at their end only
-      const Instr *code = p.code + p.code_off[e];
-      const int len = p.code_len[e];
+      const int len = rec.y;
+      const Instr *code = p.code + ((static_cast<int64_t>(rec.w) << 32) |
+                                    static_cast<uint32_t>(rec.z));
       double acc = 0.0;
       int cnt = 0;
       for (int t = 0; t < tiles; ++t) {
@@ -139,10 +142,8 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) interp_kernel(const Eva
       }
       if constexpr (!PRED) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          acc += __shfl_xor_sync(0xffffffffu, acc, o);
-          cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        }
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
         if (lane == 0) part[static_cast<size_t>(buf) * p.G + j] = SpanPart{acc, cnt, e};
       }
     }
@@ -155,6 +156,32 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) interp_kernel(const Eva
   }
 }
 
+// The value of each folded constant subtree into the instruction word that
+// holds it: one thread per subtree, its tokens from the right over a small
+// stack, with the operators every kernel of this library evaluates
+// (op_apply).  At most kMaxFoldDepth values wait at a time (64 tokens).
+constexpr int kMaxFoldDepth = 40;
+__global__ void __launch_bounds__(128)
+    fold_kernel(const FoldItem *__restrict__ items, const uint2 *__restrict__ tokens, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const FoldItem it = items[i];
+  float stk[kMaxFoldDepth];
+  int sp = 0;
+  for (uint32_t k = it.len; k-- > 0;) {
+    const uint2 t = tokens[it.first + k];
+    if (t.x == 0) {
+      stk[sp++] = __uint_as_float(t.y);
+    } else {
+      const float v1 = stk[--sp];
+      float v2 = 0.0f;
+      if (t.x < 10) v2 = stk[--sp];
+      stk[sp++] = op_apply(static_cast<int>(t.x), v1, v2);
+    }
+  }
+  *it.dst = __float_as_uint(stk[0]);
+}
+
 // mse and (sum, count) of the interpreter's entries ([n_groups][E] x (hi, lo),
 // (count, 0)): one warp per expression, its lanes the span groups lane,
 // lane + 32, ..., their double-doubles merged over the warp in a fixed order;
@@ -162,15 +189,17 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) interp_kernel(const Eva
 // together, where one thread per expression walked the span groups one after
 // the other (1,000 expressions x 391 span groups: 100 -> 6 us).
 __global__ void __launch_bounds__(256)
-    finalize_dd_kernel(const double2 *__restrict__ partial, int n_groups, int E,
-                       float *__restrict__ mse, double2 *__restrict__ sums, SequenceEnd end) {
+    finalize_dd_kernel(const double2 *__restrict__ partial, const int32_t *__restrict__ rep,
+                       int n_groups, int E, float *__restrict__ mse, double2 *__restrict__ sums,
+                       SequenceEnd end) {
   end_sequence(end);
   const int e = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (e >= E) return;  // warp-uniform
+  const int src = rep ? rep[e] : e;  // equal expressions share one evaluation
   double hi = 0.0, lo = 0.0, c = 0.0;
   for (int k = lane; k < n_groups; k += 32) {
-    const double2 *q = partial + 2 * (static_cast<int64_t>(k) * E + e);
+    const double2 *q = partial + 2 * (static_cast<int64_t>(k) * E + src);
     const double2 a = q[0];
     dd_add(hi, lo, a.x);
     dd_add(hi, lo, a.y);
@@ -545,10 +574,17 @@ cudaError_t launch_finalize(const double2 *partial, int n_spans, int E,
   return cudaGetLastError();
 }
 
-cudaError_t launch_finalize_groups(const double2 *partial, int n_groups, int E, float *mse,
-                                   double2 *sums, SequenceEnd end, cudaStream_t stream) {
+cudaError_t launch_finalize_groups(const double2 *partial, const int32_t *rep, int n_groups, int E,
+                                   float *mse, double2 *sums, SequenceEnd end,
+                                   cudaStream_t stream) {
   if (E <= 0) return cudaSuccess;
-  finalize_dd_kernel<<<(E + 7) / 8, 256, 0, stream>>>(partial, n_groups, E, mse, sums, end);
+  finalize_dd_kernel<<<(E + 7) / 8, 256, 0, stream>>>(partial, rep, n_groups, E, mse, sums, end);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fold(const FoldItem *items, const uint2 *tokens, int n, cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  fold_kernel<<<(n + 127) / 128, 128, 0, stream>>>(items, tokens, n);
   return cudaGetLastError();
 }
 

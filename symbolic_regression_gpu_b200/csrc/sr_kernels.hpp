@@ -51,8 +51,13 @@ cudaError_t launch_finalize(const double2 *partial, int n_spans, int E,
 // The interpreter's MSE entries ([n_groups][E] x 2 double2 per span group,
 // see EvalArgs::span_per_item): mse = sum / count (NaN without a valid
 // datapoint) into `mse`, and (sum, count) into `sums`; either may be NULL.
-cudaError_t launch_finalize_groups(const double2 *partial, int n_groups, int E, float *mse,
-                                   double2 *sums, SequenceEnd end, cudaStream_t stream);
+// rep (nullable): the expression whose entries each expression's result is
+// taken from (equal expressions are evaluated once).
+cudaError_t launch_finalize_groups(const double2 *partial, const int32_t *rep, int n_groups, int E,
+                                   float *mse, double2 *sums, SequenceEnd end,
+                                   cudaStream_t stream);
+// Values of n folded constant subtrees into their instruction words.
+cudaError_t launch_fold(const FoldItem *items, const uint2 *tokens, int n, cudaStream_t stream);
 // (sum of valid squared errors, valid count) per expression, combined over
 // the span partials in the order launch_finalize uses (plain and gradient
 // launches).

@@ -15,6 +15,8 @@
 // receives exactly the same operand values.
 #include "sr_program.hpp"
 
+#include "sr_share.hpp"
+
 #include <cmath>
 #include <cstring>
 
@@ -68,34 +70,7 @@ void declared_op_work(int tok, double *sfu, double *fp32) {
   *fp32 = f;
 }
 
-float op_cost(int tok) {
-  switch (tok) {
-    case 0: return 1.f;
-    case SR_OP_ADD: case SR_OP_SUB: case SR_OP_MUL: case SR_OP_MIN:
-    case SR_OP_MAX: case SR_OP_NEG: case SR_OP_ABS: return 1.f;
-    case SR_OP_DIV: return 10.f;
-    case SR_OP_LOOSE_DIV: return 12.f;
-    case SR_OP_INV: return 8.f;
-    case SR_OP_LOOSE_INV: return 10.f;
-    case SR_OP_SQRT: return 8.f;
-    case SR_OP_LOOSE_SQRT: return 9.f;
-    case SR_OP_SIN: case SR_OP_COS: return 24.f;
-    case SR_OP_TAN: return 36.f;
-    case SR_OP_SINH: return 26.f;
-    case SR_OP_COSH: return 22.f;
-    case SR_OP_TANH: return 18.f;
-    case SR_OP_EXP: return 12.f;
-    case SR_OP_EXP_CLAMP: return 13.f;
-    case SR_OP_LOG: return 16.f;
-    case SR_OP_LOOSE_LOG: return 18.f;
-    case SR_OP_POW: return 50.f;
-    case SR_OP_LOOSE_POW: return 52.f;
-    case SR_OP_ASIN: return 20.f;
-    case SR_OP_ACOS: return 22.f;
-    case SR_OP_ATAN: return 22.f;
-    default: return 1.f;
-  }
-}
+float op_cost(int tok) { return operator_cost(tok); }
 
 namespace {
 
@@ -122,6 +97,7 @@ struct Node {
   uint32_t lk = kLeafC;    // leaf kind (kLeafX / kLeafC / kLeafR)
   uint32_t lp = 0;         // leaf payload
   uint32_t lconst = kNoConst;
+  int32_t fold = -1;       // token of a folded subtree this leaf stands for
   int32_t left = -1;       // first popped operand (operators)
   int32_t right = -1;      // second popped operand (binary)
   int32_t need = 0;
@@ -156,6 +132,7 @@ struct Emitter {
   const Node *nodes;
   const OpTables &tab;
   int n_const;               // constants of the expression
+  std::vector<FoldRef> *folds;
   Instr *out;                // the program's first instruction
   int count = 0;
   float cost = 0.f, sfu = 0.f, fp32 = 0.f;
@@ -183,6 +160,7 @@ struct Emitter {
       ins.a = load->lp;
       ac = const_index(load->lconst);
       if (load->lk != kLeafC) cost += 0.5f;
+      if (load->fold >= 0) folds->push_back(FoldRef{load->fold, count << 1});
     }
     if (pending_spill >= 0) {
       ins.w |= kSpillBit | (static_cast<uint32_t>(pending_spill) << 13);
@@ -199,6 +177,7 @@ struct Emitter {
   }
 
   void emit_b_leaf(uint32_t op, const Node *load, const Node &b) {
+    if (b.fold >= 0) folds->push_back(FoldRef{b.fold, (count << 1) | 1});
     emit(op, load, b_kind_of_leaf(b.lk), b.lp, b.lconst);
   }
 
@@ -246,12 +225,29 @@ struct Emitter {
   }
 };
 
+const OpTables &op_tables() {
+  static const OpTables tab;
+  return tab;
+}
+
 }  // namespace
+
+void declared_work(const int32_t *tok, int len, double *sfu, double *fp32) {
+  const OpTables &tab = op_tables();
+  float s = 0.f, f = 0.f;
+  for (int i = 0; i < len; ++i)
+    if (tok[i] > 0) {
+      s += tab.sfu[tok[i] & 63];
+      f += tab.fp32[tok[i] & 63];
+    }
+  *sfu = s;
+  *fp32 = f;
+}
 
 sr_status compile_expression(const int32_t *tok, const double *val, int len,
                              int num_vars, const int32_t *hints,
                              std::vector<Instr> &out, ExprInfo &info,
-                             std::string *err) {
+                             std::string *err, int first_row, std::vector<FoldRef> *folds) {
   info = ExprInfo{};
   info.n_tokens = len;
   if (len <= 0) {
@@ -268,7 +264,7 @@ sr_status compile_expression(const int32_t *tok, const double *val, int len,
   // tree, with cached subtrees (hints) collapsed to one leaf at their root.
   // Children get lower node ids than their parent, and a node's spill-slot
   // label (Sethi-Ullman) is known when it is made.
-  static const OpTables tab;
+  const OpTables &tab = op_tables();
   thread_local std::vector<Node> node_store;
   thread_local std::vector<int32_t> stack_store;
   if (static_cast<int>(node_store.size()) < len) {
@@ -280,10 +276,29 @@ sr_status compile_expression(const int32_t *tok, const double *val, int len,
   int n_nodes = 0, sp = 0, depth = 0, n_ops = 0;
   uint32_t n_const = 0;
   bool bad_skeleton = false;
+  // The leaf a collapsed subtree becomes.
+  const auto collapse = [&](Node &nd, int hint, int i) {
+    nd.leaf = true;
+    nd.need = 0;
+    nd.lconst = kNoConst;
+    nd.fold = -1;
+    if (hint >= 0) {
+      nd.lk = kLeafR;
+      nd.lp = static_cast<uint32_t>(hint);
+    } else if (hint == kHintFold) {
+      nd.lk = kLeafC;
+      nd.lp = 0;
+      nd.fold = i;
+    } else {
+      nd.lk = kLeafX;
+      nd.lp = static_cast<uint32_t>(first_row + (kHintRow0 - hint));
+    }
+  };
   for (int i = len - 1; i >= 0; --i) {
     const int t = tok[i];
     const int hint = hints ? hints[i] : -1;
-    // hint >= 0: root of a cached subtree; -2: inside one; -1: neither.
+    const bool collapsed = hint >= 0 || hint == kHintFold || hint <= kHintRow0;
+    // -2: inside a collapsed subtree; -1: neither.
     if (t == SR_TOK_CONST || t == SR_TOK_VAR) {
       ++depth;
       const uint32_t ci = n_const;
@@ -293,9 +308,9 @@ sr_status compile_expression(const int32_t *tok, const double *val, int len,
       nd.leaf = true;
       nd.need = 0;
       nd.lconst = kNoConst;
-      if (hint >= 0) {
-        nd.lk = kLeafR;
-        nd.lp = static_cast<uint32_t>(hint);
+      nd.fold = -1;
+      if (collapsed) {
+        collapse(nd, hint, i);
       } else if (t == SR_TOK_CONST) {
         nd.lk = kLeafC;
         nd.lp = float_bits(static_cast<float>(val[i]));
@@ -322,11 +337,9 @@ sr_status compile_expression(const int32_t *tok, const double *val, int len,
     if (hint == -2 || bad_skeleton) continue;
     Node &nd = nodes[n_nodes];
     nd.lconst = kNoConst;
-    if (hint >= 0) {
-      nd.leaf = true;
-      nd.need = 0;
-      nd.lk = kLeafR;
-      nd.lp = static_cast<uint32_t>(hint);
+    nd.fold = -1;
+    if (collapsed) {
+      collapse(nd, hint, i);
       stk[sp++] = n_nodes++;
       continue;
     }
@@ -370,7 +383,7 @@ sr_status compile_expression(const int32_t *tok, const double *val, int len,
   const size_t first = out.size();
   info.n_instr = std::max(n_ops, 1);
   out.resize(first + static_cast<size_t>(info.n_instr));
-  Emitter em{nodes, tab, info.n_const, out.data() + first};
+  Emitter em{nodes, tab, info.n_const, folds, out.data() + first};
   em.gen(root);
   info.cost = em.cost + 6.0f;           // epilogue
   info.sfu_ops = em.sfu;

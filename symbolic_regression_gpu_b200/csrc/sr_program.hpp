@@ -33,16 +33,28 @@ void subtree_sizes(const int32_t *tok, int len, int32_t *sizes);
 //   cache: hints[i] >= 0 marks the root of a cached subtree held in cache slot
 //   hints[i]; -2 marks the body of such a subtree; -1 elsewhere (reference
 //   mark_cached_subtrees_from_state, src/cleaned/cl_gpu_eval.cu:294-329).
+//   Two more marks (sr_share.hpp) collapse a subtree to another leaf:
+//   kHintFold to a constant whose value the device fills in (its token and
+//   the instruction word that holds it go to `folds`), kHintRow0 - r to the
+//   variable row first_row + r.
 // Appends the program to `out`.  Returns SR_OK or an error with `*err` set.
+struct FoldRef {
+  int32_t tok;   // root of the folded subtree in the expression
+  int32_t loc;   // (instruction of the program << 1) | (operand b)
+};
 sr_status compile_expression(const int32_t *tok, const double *val, int len,
                              int num_vars, const int32_t *hints,
                              std::vector<Instr> &out, ExprInfo &info,
-                             std::string *err);
+                             std::string *err, int first_row = 0,
+                             std::vector<FoldRef> *folds = nullptr);
 
 // Declared per-datapoint work of one operator token (project cost model:
 // SFU / FP32 operation counts), used for the roofline; not CUDA's
 // implementation.
 void declared_op_work(int tok, double *sfu, double *fp32);
+
+// The same for a whole token run.
+void declared_work(const int32_t *tok, int len, double *sfu, double *fp32);
 
 // Modelled relative device cost of one operator per datapoint (used only to
 // balance warps; calibrated by hand against instruction counts).

@@ -1,0 +1,340 @@
+// sr_share.cpp — equal expressions, constant subtrees and frequent subtrees of
+// a population (sr_share.hpp).
+//
+// Three passes.  (1) On the workers: a structural hash and size per token,
+// from the right, and a count per distinct subtree in one open-addressed table
+// (keys are claimed with a compare-and-swap; a hash is only ever a hint, every
+// use compares the tokens).  (2) On the caller: the rows, chosen greedily by
+// the evaluations they save, most first; choosing one takes its occurrences
+// away from the subtrees inside it and its cost from the subtrees around it.
+// (3) While compiling: each expression's tokens are marked, outermost first.
+#include "sr_share.hpp"
+
+#include <algorithm>
+#include <cstring>
+
+#include "sr_internal.hpp"
+#include "sr_program.hpp"
+
+namespace sr {
+
+namespace {
+
+inline uint64_t mix(uint64_t z) {
+  z ^= z >> 30;
+  z *= 0xBF58476D1CE4E5B9ull;
+  z ^= z >> 27;
+  z *= 0x94D049BB133111EBull;
+  return z ^ (z >> 31);
+}
+
+inline uint32_t bits_of(double v) {
+  const float f = static_cast<float>(v);
+  uint32_t u;
+  std::memcpy(&u, &f, sizeof u);
+  return u;
+}
+
+inline int64_t index_of(double v) {
+  return v > -2147483648.0 && v < 2147483648.0 ? static_cast<int64_t>(v) : -1;
+}
+
+// Device cost of one operator instruction in warp instructions per 8
+// datapoints a lane: its arithmetic and about 25 of dispatch.
+inline float token_cost(int t) { return 25.0f + 6.0f * op_cost(t); }
+constexpr float kRowLoadCost = 8.0f;  // reading a row instead
+
+constexpr uint64_t kRootSalt = 0x9E3779B97F4A7C15ull;
+
+}  // namespace
+
+Sharing::Entry *Sharing::insert(uint64_t key) {
+  size_t i = key & mask_;
+  for (;;) {
+    uint64_t k = table_[i].key.load(std::memory_order_relaxed);
+    if (k == key) return &table_[i];
+    if (k == 0 &&
+        (table_[i].key.compare_exchange_strong(k, key, std::memory_order_relaxed) || k == key))
+      return &table_[i];
+    i = (i + 1) & mask_;
+  }
+}
+
+const Sharing::Entry *Sharing::lookup(uint64_t key) const {
+  for (size_t i = key & mask_;; i = (i + 1) & mask_) {
+    const uint64_t k = table_[i].key.load(std::memory_order_relaxed);
+    if (k == key) return &table_[i];
+    if (k == 0) return nullptr;
+  }
+}
+
+// Same operators, same constants (as floats, bit for bit), same variables.
+bool Sharing::equal_runs(int64_t a, int64_t b, int32_t n) const {
+  for (int32_t i = 0; i < n; ++i) {
+    const int32_t t = tok_[a + i];
+    if (t != tok_[b + i]) return false;
+    if (t == SR_TOK_CONST && bits_of(val_[a + i]) != bits_of(val_[b + i])) return false;
+    if (t == SR_TOK_VAR && index_of(val_[a + i]) != index_of(val_[b + i])) return false;
+  }
+  return true;
+}
+
+bool Sharing::hash_expression(int x, std::vector<uint32_t> &frequent) {
+  const int64_t o = off_[x];
+  const int len = static_cast<int>(off_[x + 1] - o);
+  int depth = 0;  // values to the right: an operator finds its operands there
+  for (int i = len - 1; i >= 0; --i) {
+    const int64_t p = o + i;
+    const int32_t t = tok_[p];
+    if (t == SR_TOK_CONST || t == SR_TOK_VAR) {
+      ++depth;
+    } else if (is_binary_token(t)) {
+      if (--depth < 1) return false;
+    } else if (!is_unary_token(t) || depth < 1) {
+      return false;
+    }
+    if (t == SR_TOK_CONST) {
+      hash_[static_cast<size_t>(p)] = mix(0x100000000ull | bits_of(val_[p]));
+      size_[static_cast<size_t>(p)] = -1;
+      continue;
+    }
+    if (t == SR_TOK_VAR) {
+      hash_[static_cast<size_t>(p)] = mix(0x200000000ull ^ static_cast<uint64_t>(index_of(val_[p])));
+      size_[static_cast<size_t>(p)] = 1;
+      continue;
+    }
+    const int16_t sl = size_[static_cast<size_t>(p + 1)];
+    const int nl = sl < 0 ? -sl : sl;
+    uint64_t h = mix(hash_[static_cast<size_t>(p + 1)] + 0x632BE59BD9B4E019ull * static_cast<uint64_t>(t));
+    int n = 1 + nl;
+    bool constant = sl < 0;
+    if (is_binary_token(t)) {
+      const int16_t sr = size_[static_cast<size_t>(p + 1 + nl)];
+      n += sr < 0 ? -sr : sr;
+      constant = constant && sr < 0;
+      h = mix(h ^ (hash_[static_cast<size_t>(p + 1 + nl)] * 0xD6E8FEB86659FD93ull));
+    }
+    h |= 1;  // never 0, the table's empty key
+    hash_[static_cast<size_t>(p)] = h;
+    size_[static_cast<size_t>(p)] = static_cast<int16_t>(constant ? -n : n);
+    if (constant || n > kMaxSharedTokens) continue;
+    Entry *e = insert(h);
+    const uint32_t before = e->count.fetch_add(1, std::memory_order_relaxed);
+    if (before == 0) e->at.store(static_cast<uint32_t>(p), std::memory_order_relaxed);
+    if (before + 1 == min_count_) frequent.push_back(static_cast<uint32_t>(e - table_.get()));
+  }
+  // The expression itself: the lowest index of each distinct one.
+  Entry *e = insert(mix(hash_[static_cast<size_t>(o)] ^ kRootSalt) | 1);
+  uint32_t cur = e->at.load(std::memory_order_relaxed);
+  const uint32_t mine = static_cast<uint32_t>(x) + 1;  // 0: not set yet
+  while ((cur == 0 || mine < cur) &&
+         !e->at.compare_exchange_weak(cur, mine, std::memory_order_relaxed)) {
+  }
+  return depth == 1;
+}
+
+void Sharing::choose(std::vector<uint32_t> &frequent, int max_rows) {
+  drop_rows();
+  struct Candidate {
+    uint64_t key;
+    int64_t at;
+    int32_t n;
+    float occ, cost;
+    bool taken;
+  };
+  std::vector<Candidate> cs;
+  cs.reserve(frequent.size());
+  for (const uint32_t i : frequent) {
+    const Entry &e = table_[i];
+    Candidate c{};
+    c.key = e.key.load(std::memory_order_relaxed);
+    c.at = e.at.load(std::memory_order_relaxed);
+    if (c.at >= n_tokens_ || hash_[static_cast<size_t>(c.at)] != c.key) continue;
+    c.n = size_[static_cast<size_t>(c.at)];
+    if (c.n < 2) continue;
+    c.occ = static_cast<float>(e.count.load(std::memory_order_relaxed));
+    for (int32_t q = 0; q < c.n;) {
+      const int16_t s = size_[static_cast<size_t>(c.at + q)];
+      if (s < -1) {
+        q += -s;  // folded
+        continue;
+      }
+      if (tok_[c.at + q] > 0) c.cost += token_cost(tok_[c.at + q]);
+      ++q;
+    }
+    cs.push_back(c);
+  }
+  // Most saving first; the hash breaks ties, so the choice does not depend on
+  // which worker met a subtree first.
+  const auto gain = [](const Candidate &c) { return (c.occ - 1.0f) * (c.cost - kRowLoadCost); };
+  const auto before = [&](const Candidate &a, const Candidate &b) {
+    const float ga = gain(a), gb = gain(b);
+    return ga != gb ? ga > gb : a.key < b.key;
+  };
+  constexpr size_t kCandidates = 384;
+  if (cs.size() > kCandidates) {
+    std::nth_element(cs.begin(), cs.begin() + kCandidates, cs.end(), before);
+    cs.resize(kCandidates);
+  }
+  std::sort(cs.begin(), cs.end(), before);
+  const auto find_candidate = [&](uint64_t key) -> Candidate * {
+    for (auto &c : cs)
+      if (c.key == key) return &c;
+    return nullptr;
+  };
+  while (static_cast<int>(rows_.size()) < max_rows) {
+    Candidate *best = nullptr;
+    for (auto &c : cs)
+      if (!c.taken && (!best || before(c, *best))) best = &c;
+    // A row costs its own evaluation and a copy per group of expressions: it
+    // has to save several of them.
+    if (!best || best->occ < static_cast<float>(min_count_) || best->cost <= 2.0f * kRowLoadCost)
+      break;
+    best->taken = true;
+    const int r = static_cast<int>(rows_.size());
+    rows_.push_back(Row{best->at, best->n, static_cast<int32_t>(best->occ)});
+    size_t slot = best->key & 255;
+    while (row_key_[slot] != 0) slot = (slot + 1) & 255;
+    row_key_[slot] = best->key;
+    row_of_[slot] = static_cast<int16_t>(r);
+    const auto is_row = [&](uint64_t key) {
+      for (size_t i = key & 255; row_key_[i] != 0; i = (i + 1) & 255)
+        if (row_key_[i] == key) return true;
+      return false;
+    };
+    // Inside it: those occurrences go.
+    for (int32_t q = 1; q < best->n;) {
+      const size_t p = static_cast<size_t>(best->at + q);
+      const int16_t s = size_[p];
+      if (s < 0 || tok_[p] <= 0) {
+        q += s < 0 ? -s : 1;
+        continue;
+      }
+      if (is_row(hash_[p])) {
+        q += s;
+        continue;
+      }
+      if (Candidate *c = find_candidate(hash_[p])) c->occ -= best->occ;
+      ++q;
+    }
+    // Around it: it is read, not evaluated.
+    const float saved = best->cost - kRowLoadCost;
+    for (auto &c : cs) {
+      if (c.taken || c.n <= best->n) continue;
+      for (int32_t q = 1; q + best->n <= c.n; ++q)
+        if (hash_[static_cast<size_t>(c.at + q)] == best->key) c.cost -= saved;
+    }
+  }
+}
+
+void Sharing::drop_rows() {
+  rows_.clear();
+  std::memset(row_key_, 0, sizeof row_key_);
+}
+
+bool Sharing::find(int E, const int32_t *tok, const double *val, const int64_t *off, int max_rows,
+                   WorkerPool &pool, int threads) {
+  tok_ = tok;
+  val_ = val;
+  off_ = off;
+  rows_.clear();
+  const size_t T = static_cast<size_t>(off[E]);
+  if (T >= (1ull << 31)) return false;
+  n_tokens_ = static_cast<int64_t>(T);
+  if (hash_.size() < T) hash_.resize(T);
+  if (size_.size() < T) size_.resize(T);
+  size_t cap = 1024;
+  while (cap < T + static_cast<size_t>(E)) cap *= 2;  // at most 2/3 full: leaves are not entered
+  if (cap > cap_) {
+    table_.reset(new Entry[cap]);
+    cap_ = cap;
+  }
+  mask_ = cap - 1;
+  // Rows serve every group of expressions; one used by few is no gain.
+  min_count_ = static_cast<uint32_t>(std::max(4, E / 512));
+  const int chunks = static_cast<int>(
+      std::max<int64_t>(1, std::min<int64_t>({threads, E, static_cast<int64_t>(T) / 2500})));
+  Entry *table = table_.get();
+  pool.run(chunks, threads, [&](int c) {
+    const size_t a = cap * static_cast<size_t>(c) / chunks, b = cap * (static_cast<size_t>(c) + 1) / chunks;
+    std::memset(static_cast<void *>(table + a), 0, (b - a) * sizeof(Entry));
+  });
+  std::vector<std::vector<uint32_t>> frequent(static_cast<size_t>(chunks));
+  std::vector<char> bad(static_cast<size_t>(chunks), 0);
+  pool.run(chunks, threads, [&](int c) {
+    const int x0 = static_cast<int>(static_cast<int64_t>(E) * c / chunks);
+    const int x1 = static_cast<int>(static_cast<int64_t>(E) * (c + 1) / chunks);
+    for (int x = x0; x < x1; ++x)
+      if (!hash_expression(x, frequent[static_cast<size_t>(c)])) {
+        bad[static_cast<size_t>(c)] = 1;
+        return;
+      }
+  });
+  if (std::find(bad.begin(), bad.end(), 1) != bad.end()) return false;
+  std::vector<uint32_t> all;
+  for (const auto &f : frequent) all.insert(all.end(), f.begin(), f.end());
+  choose(all, max_rows);
+  return true;
+}
+
+bool Sharing::mark(int x, int32_t *hints) const {
+  const int64_t o = off_[x];
+  const int len = static_cast<int>(off_[x + 1] - o);
+  bool any = false;
+  for (int i = 0; i < len;) {
+    const size_t p = static_cast<size_t>(o + i);
+    hints[i] = -1;
+    const int16_t s = size_[p];
+    int32_t mark = -1;
+    int n = s < 0 ? -s : s;
+    if (tok_[p] > 0 && n <= kMaxSharedTokens) {
+      if (s < 0) {
+        mark = kHintFold;
+      } else {
+        const uint64_t key = hash_[p];
+        for (size_t k = key & 255; row_key_[k] != 0; k = (k + 1) & 255)
+          if (row_key_[k] == key) {
+            const Row &r = rows_[static_cast<size_t>(row_of_[k])];
+            if (r.size == n && equal_runs(r.tok, o + i, n)) mark = kHintRow0 - row_of_[k];
+            break;
+          }
+      }
+    }
+    if (mark == -1) {
+      ++i;
+      continue;
+    }
+    any = true;
+    hints[i] = mark;
+    for (int k = 1; k < n; ++k) hints[i + k] = -2;
+    i += n;
+  }
+  return any;
+}
+
+void Sharing::mark_row(const Row &r, int32_t *hints) const {
+  for (int i = 0; i < r.size;) {
+    const size_t p = static_cast<size_t>(r.tok + i);
+    const int16_t s = size_[p];
+    hints[i] = -1;
+    if (s < -1) {
+      hints[i] = kHintFold;
+      for (int k = 1; k < -s; ++k) hints[i + k] = -2;
+      i += -s;
+    } else {
+      ++i;
+    }
+  }
+}
+
+int Sharing::rep(int x) const {
+  const int64_t o = off_[x];
+  const Entry *e = lookup(mix(hash_[static_cast<size_t>(o)] ^ kRootSalt) | 1);
+  if (!e) return x;
+  const int first = static_cast<int>(e->at.load(std::memory_order_relaxed)) - 1;
+  const int64_t n = off_[x + 1] - o;
+  if (first < 0 || first >= x || off_[first + 1] - off_[first] != n) return x;
+  return equal_runs(off_[first], o, static_cast<int32_t>(n)) ? first : x;
+}
+
+}  // namespace sr

@@ -408,9 +408,8 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) tan_kernel(const TanArg
   const int k_spans = p.span_per_item;
   const int n_items = p.n_groups * ((p.n_spans + k_spans - 1) / k_spans);
   if (warp == W) {
-    if (lane == 0)
-      run_producer<true>(p.n_groups, n_items, k_spans, p.n_spans, p.work_counter, p.error, p.X,
-                         p.ldx, rows, span, span, xbuf, desc, full, empty,
+    run_producer<true>(lane, p.n_groups, n_items, k_spans, p.n_spans, p.work_counter, p.error, p.X,
+                         nullptr, rows, p.ldx, rows, span, span, xbuf, desc, full, empty,
                          FoldArgs{part, gacc, p.partial, p.G, p.E, a.n_valid, K, gpart, ggacc,
                                   a.gout, a.const_off, a.const_cnt, a.C});
     return;
