@@ -2,6 +2,7 @@
 // passes, and a pool of waiting workers for the passes of every call.
 #pragma once
 #include <algorithm>
+#include <atomic>
 #include <condition_variable>
 #include <cstdint>
 #include <functional>
@@ -30,8 +31,10 @@ void parallel_for(int64_t n, int threads, F &&fn) {
 
 // Workers owned by one context, started when a pass first needs them and
 // joined with the context.  Starting a thread costs about 20 us, so forking 15
-// of them took 0.3 ms of every call.  One thread at a time calls run() (a
-// context serves one caller at a time).
+// of them took 0.3 ms of every call; waking one costs tens of microseconds, so
+// a worker that has finished looks out for the next pass of the call for a
+// moment before it sleeps.  One thread at a time calls run() (a context serves
+// one caller at a time).
 class WorkerPool {
  public:
   WorkerPool() = default;
@@ -41,6 +44,7 @@ class WorkerPool {
     {
       std::lock_guard<std::mutex> lock(m_);
       stop_ = true;
+      generation_.fetch_add(1);
     }
     wake_.notify_all();
     for (auto &t : workers_) t.join();
@@ -54,22 +58,33 @@ class WorkerPool {
       return;
     }
     grow(std::min(threads, chunks) - 1);
+    fn_ = &fn;
+    chunks_ = chunks;
+    next_.store(0);
+    pending_.store(chunks);
+    open_.store(true);
     {
       std::lock_guard<std::mutex> lock(m_);
-      fn_ = &fn;
-      chunks_ = chunks;
-      next_ = 0;
-      pending_ = chunks;
-      ++generation_;
+      generation_.fetch_add(1);
     }
-    wake_.notify_all();
-    work(fn);
-    std::unique_lock<std::mutex> lock(m_);
-    done_.wait(lock, [&] { return pending_ == 0; });
-    fn_ = nullptr;
+    if (sleepers_.load() > 0) wake_.notify_all();
+    work();
+    // Every chunk done, then no worker left inside the pass: the next one may
+    // change its description.
+    for (int spin = 0; pending_.load() > 0; ++spin) pause(spin);
+    open_.store(false);
+    for (int spin = 0; inside_.load() > 0; ++spin) pause(spin);
   }
 
  private:
+  static constexpr int kSpins = 4000;  // about 50 us
+
+  static void pause(int spin) {
+    if (spin < kSpins)
+      __builtin_ia32_pause();
+    else
+      std::this_thread::yield();
+  }
   void grow(int want) {
     while (static_cast<int>(workers_.size()) < want) {
       try {
@@ -79,42 +94,40 @@ class WorkerPool {
       }
     }
   }
-  // Takes chunks until none is left.
-  void work(const std::function<void(int)> &fn) {
-    for (;;) {
-      int c;
-      {
-        std::lock_guard<std::mutex> lock(m_);
-        if (fn_ != &fn || next_ >= chunks_) return;
-        c = next_++;
-      }
-      fn(c);
-      std::lock_guard<std::mutex> lock(m_);
-      if (--pending_ == 0) done_.notify_all();
+  void work() {
+    for (int c; (c = next_.fetch_add(1)) < chunks_;) {
+      (*fn_)(c);
+      pending_.fetch_sub(1);
     }
   }
   void loop() {
     uint64_t seen = 0;
     for (;;) {
-      const std::function<void(int)> *fn;
-      {
+      for (int spin = 0; generation_.load() == seen && spin < kSpins; ++spin) pause(spin);
+      if (generation_.load() == seen) {
         std::unique_lock<std::mutex> lock(m_);
-        wake_.wait(lock, [&] { return stop_ || (fn_ && generation_ != seen); });
-        if (stop_) return;
-        seen = generation_;
-        fn = fn_;
+        sleepers_.fetch_add(1);
+        wake_.wait(lock, [&] { return generation_.load() != seen; });
+        sleepers_.fetch_sub(1);
       }
-      work(*fn);
+      seen = generation_.load();
+      if (stop_.load()) return;
+      // The pass's description is read only between entering and leaving, and
+      // only while it is open (run() closes it, then waits for both).
+      inside_.fetch_add(1);
+      if (open_.load()) work();
+      inside_.fetch_sub(1);
     }
   }
 
   std::mutex m_;
-  std::condition_variable wake_, done_;
+  std::condition_variable wake_;
   std::vector<std::thread> workers_;
   const std::function<void(int)> *fn_ = nullptr;
-  int chunks_ = 0, next_ = 0, pending_ = 0;
-  uint64_t generation_ = 0;
-  bool stop_ = false;
+  int chunks_ = 0;
+  std::atomic<int> next_{0}, pending_{0}, inside_{0}, sleepers_{0};
+  std::atomic<bool> open_{false}, stop_{false};
+  std::atomic<uint64_t> generation_{0};
 };
 
 }  // namespace sr

@@ -21,11 +21,10 @@ namespace sr {
 namespace {
 
 inline uint64_t mix(uint64_t z) {
-  z ^= z >> 30;
-  z *= 0xBF58476D1CE4E5B9ull;
-  z ^= z >> 27;
-  z *= 0x94D049BB133111EBull;
-  return z ^ (z >> 31);
+  z *= 0x9E3779B97F4A7C15ull;
+  z ^= z >> 32;
+  z *= 0xD6E8FEB86659FD93ull;
+  return z ^ (z >> 29);
 }
 
 inline uint32_t bits_of(double v) {
@@ -47,6 +46,26 @@ constexpr float kRowLoadCost = 8.0f;  // reading a row instead
 constexpr uint64_t kRootSalt = 0x9E3779B97F4A7C15ull;
 
 }  // namespace
+
+// A worker's own counts of the subtrees it met last: the frequent ones (sin x0)
+// would otherwise have every worker add to the same few words.
+struct Sharing::Local {
+  static constexpr int kSlots = 256;
+  uint64_t key[kSlots] = {};
+  uint32_t count[kSlots] = {};
+  uint32_t at[kSlots] = {};
+  std::vector<uint32_t> frequent;  // table entries that reached min_count_
+};
+
+void Sharing::flush(Local &local, int s) {
+  if (local.count[s] == 0) return;
+  Entry *e = insert(local.key[s]);
+  const uint32_t before = e->count.fetch_add(local.count[s], std::memory_order_relaxed);
+  if (before == 0) e->at.store(local.at[s], std::memory_order_relaxed);
+  if (before < min_count_ && before + local.count[s] >= min_count_)
+    local.frequent.push_back(static_cast<uint32_t>(e - table_.get()));
+  local.count[s] = 0;
+}
 
 Sharing::Entry *Sharing::insert(uint64_t key) {
   size_t i = key & mask_;
@@ -79,7 +98,7 @@ bool Sharing::equal_runs(int64_t a, int64_t b, int32_t n) const {
   return true;
 }
 
-bool Sharing::hash_expression(int x, std::vector<uint32_t> &frequent) {
+bool Sharing::hash_expression(int x, Local &local) {
   const int64_t o = off_[x];
   const int len = static_cast<int>(off_[x + 1] - o);
   int depth = 0;  // values to the right: an operator finds its operands there
@@ -105,23 +124,27 @@ bool Sharing::hash_expression(int x, std::vector<uint32_t> &frequent) {
     }
     const int16_t sl = size_[static_cast<size_t>(p + 1)];
     const int nl = sl < 0 ? -sl : sl;
-    uint64_t h = mix(hash_[static_cast<size_t>(p + 1)] + 0x632BE59BD9B4E019ull * static_cast<uint64_t>(t));
+    uint64_t h = hash_[static_cast<size_t>(p + 1)] + 0x632BE59BD9B4E019ull * static_cast<uint64_t>(t);
     int n = 1 + nl;
     bool constant = sl < 0;
     if (is_binary_token(t)) {
       const int16_t sr = size_[static_cast<size_t>(p + 1 + nl)];
       n += sr < 0 ? -sr : sr;
       constant = constant && sr < 0;
-      h = mix(h ^ (hash_[static_cast<size_t>(p + 1 + nl)] * 0xD6E8FEB86659FD93ull));
+      const uint64_t r = hash_[static_cast<size_t>(p + 1 + nl)];
+      h = mix(h) ^ ((r << 23) | (r >> 41));
     }
-    h |= 1;  // never 0, the table's empty key
+    h = mix(h) | 1;  // never 0, the table's empty key
     hash_[static_cast<size_t>(p)] = h;
     size_[static_cast<size_t>(p)] = static_cast<int16_t>(constant ? -n : n);
     if (constant || n > kMaxSharedTokens) continue;
-    Entry *e = insert(h);
-    const uint32_t before = e->count.fetch_add(1, std::memory_order_relaxed);
-    if (before == 0) e->at.store(static_cast<uint32_t>(p), std::memory_order_relaxed);
-    if (before + 1 == min_count_) frequent.push_back(static_cast<uint32_t>(e - table_.get()));
+    const int slot = static_cast<int>((h >> 1) & (Local::kSlots - 1));
+    if (local.key[slot] != h) {
+      flush(local, slot);
+      local.key[slot] = h;
+      local.at[slot] = static_cast<uint32_t>(p);
+    }
+    ++local.count[slot];
   }
   // The expression itself: the lowest index of each distinct one.
   Entry *e = insert(mix(hash_[static_cast<size_t>(o)] ^ kRootSalt) | 1);
@@ -171,15 +194,23 @@ void Sharing::choose(std::vector<uint32_t> &frequent, int max_rows) {
     const float ga = gain(a), gb = gain(b);
     return ga != gb ? ga > gb : a.key < b.key;
   };
-  constexpr size_t kCandidates = 384;
+  // The rows come from the first of them: choosing one only lowers the others.
+  constexpr size_t kCandidates = 128;
   if (cs.size() > kCandidates) {
     std::nth_element(cs.begin(), cs.begin() + kCandidates, cs.end(), before);
     cs.resize(kCandidates);
   }
-  std::sort(cs.begin(), cs.end(), before);
+  // Candidates by hash, open-addressed.
+  int16_t of_key[512];
+  std::memset(of_key, 0xff, sizeof of_key);
+  for (size_t i = 0; i < cs.size(); ++i) {
+    size_t k = cs[i].key & 511;
+    while (of_key[k] >= 0) k = (k + 1) & 511;
+    of_key[k] = static_cast<int16_t>(i);
+  }
   const auto find_candidate = [&](uint64_t key) -> Candidate * {
-    for (auto &c : cs)
-      if (c.key == key) return &c;
+    for (size_t k = key & 511; of_key[k] >= 0; k = (k + 1) & 511)
+      if (cs[static_cast<size_t>(of_key[k])].key == key) return &cs[static_cast<size_t>(of_key[k])];
     return nullptr;
   };
   while (static_cast<int>(rows_.size()) < max_rows) {
@@ -192,6 +223,7 @@ void Sharing::choose(std::vector<uint32_t> &frequent, int max_rows) {
       break;
     best->taken = true;
     const int r = static_cast<int>(rows_.size());
+    max_row_size_ = std::max(max_row_size_, best->n);
     rows_.push_back(Row{best->at, best->n, static_cast<int32_t>(best->occ)});
     size_t slot = best->key & 255;
     while (row_key_[slot] != 0) slot = (slot + 1) & 255;
@@ -229,6 +261,7 @@ void Sharing::choose(std::vector<uint32_t> &frequent, int max_rows) {
 
 void Sharing::drop_rows() {
   rows_.clear();
+  max_row_size_ = 0;
   std::memset(row_key_, 0, sizeof row_key_);
 }
 
@@ -237,14 +270,17 @@ bool Sharing::find(int E, const int32_t *tok, const double *val, const int64_t *
   tok_ = tok;
   val_ = val;
   off_ = off;
-  rows_.clear();
+  drop_rows();
   const size_t T = static_cast<size_t>(off[E]);
   if (T >= (1ull << 31)) return false;
   n_tokens_ = static_cast<int64_t>(T);
   if (hash_.size() < T) hash_.resize(T);
   if (size_.size() < T) size_.resize(T);
+  // Room for every operator and expression, were they all different.
+  size_t n_ops = 0;
+  for (size_t i = 0; i < T; ++i) n_ops += tok[i] > 0 ? 1 : 0;
   size_t cap = 1024;
-  while (cap < T + static_cast<size_t>(E)) cap *= 2;  // at most 2/3 full: leaves are not entered
+  while (cap * 7 < (n_ops + static_cast<size_t>(E)) * 8) cap *= 2;
   if (cap > cap_) {
     table_.reset(new Entry[cap]);
     cap_ = cap;
@@ -255,24 +291,27 @@ bool Sharing::find(int E, const int32_t *tok, const double *val, const int64_t *
   const int chunks = static_cast<int>(
       std::max<int64_t>(1, std::min<int64_t>({threads, E, static_cast<int64_t>(T) / 2500})));
   Entry *table = table_.get();
-  pool.run(chunks, threads, [&](int c) {
-    const size_t a = cap * static_cast<size_t>(c) / chunks, b = cap * (static_cast<size_t>(c) + 1) / chunks;
+  const int zero_chunks = cap < 65536 ? 1 : chunks;  // 1 MB
+  pool.run(zero_chunks, threads, [&](int c) {
+    const size_t a = cap * static_cast<size_t>(c) / zero_chunks, b = cap * (static_cast<size_t>(c) + 1) / zero_chunks;
     std::memset(static_cast<void *>(table + a), 0, (b - a) * sizeof(Entry));
   });
-  std::vector<std::vector<uint32_t>> frequent(static_cast<size_t>(chunks));
+  std::vector<Local> locals(static_cast<size_t>(chunks));
   std::vector<char> bad(static_cast<size_t>(chunks), 0);
   pool.run(chunks, threads, [&](int c) {
     const int x0 = static_cast<int>(static_cast<int64_t>(E) * c / chunks);
     const int x1 = static_cast<int>(static_cast<int64_t>(E) * (c + 1) / chunks);
+    Local &local = locals[static_cast<size_t>(c)];
     for (int x = x0; x < x1; ++x)
-      if (!hash_expression(x, frequent[static_cast<size_t>(c)])) {
+      if (!hash_expression(x, local)) {
         bad[static_cast<size_t>(c)] = 1;
         return;
       }
+    for (int k = 0; k < Local::kSlots; ++k) flush(local, k);
   });
   if (std::find(bad.begin(), bad.end(), 1) != bad.end()) return false;
   std::vector<uint32_t> all;
-  for (const auto &f : frequent) all.insert(all.end(), f.begin(), f.end());
+  for (const auto &l : locals) all.insert(all.end(), l.frequent.begin(), l.frequent.end());
   choose(all, max_rows);
   return true;
 }
@@ -290,7 +329,7 @@ bool Sharing::mark(int x, int32_t *hints) const {
     if (tok_[p] > 0 && n <= kMaxSharedTokens) {
       if (s < 0) {
         mark = kHintFold;
-      } else {
+      } else if (n <= max_row_size_) {
         const uint64_t key = hash_[p];
         for (size_t k = key & 255; row_key_[k] != 0; k = (k + 1) & 255)
           if (row_key_[k] == key) {

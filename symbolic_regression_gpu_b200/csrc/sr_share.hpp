@@ -64,7 +64,9 @@ class Sharing {
   Entry *insert(uint64_t key);
   const Entry *lookup(uint64_t key) const;
   bool equal_runs(int64_t a, int64_t b, int32_t n) const;
-  bool hash_expression(int x, std::vector<uint32_t> &frequent);
+  struct Local;
+  bool hash_expression(int x, Local &local);
+  void flush(Local &local, int slot);
   void choose(std::vector<uint32_t> &frequent, int max_rows);
 
   const int32_t *tok_ = nullptr;
@@ -77,6 +79,7 @@ class Sharing {
   std::unique_ptr<Entry[]> table_;
   size_t cap_ = 0, mask_ = 0;
   std::vector<Row> rows_;
+  int max_row_size_ = 0;
   uint64_t row_key_[256];        // open-addressed set of the rows' hashes
   int16_t row_of_[256];
 };
