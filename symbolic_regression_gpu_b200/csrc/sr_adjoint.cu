@@ -73,6 +73,32 @@ __device__ __forceinline__ void gacc_add(double *gacc, uint32_t c, uint32_t ncon
   gacc[c * 32 + lane] += s;
 }
 
+// The adjoint g of a folded constant subtree's value, carried on to each of its
+// constants along the subtree's partials (the products the sweep would form if
+// it walked the subtree).
+struct FoldedConsts {
+  const int4 *cinfo;  // of the expression's constants
+  const float *path;
+};
+template <int DPT>
+__device__ __noinline__ void gacc_add_folded(double *gacc, uint32_t c0, uint32_t nconst, int lane,
+                                             const float *g, FoldedConsts fc) {
+  if (c0 >= nconst) return;
+  const int nc = fc.cinfo[c0].z;
+  for (int j = 0; j < nc; ++j) {
+    const int4 info = fc.cinfo[c0 + j];
+    float t[DPT];
+#pragma unroll
+    for (int k = 0; k < DPT; ++k) t[k] = g[k];
+    for (int q = 0; q < info.y; ++q) {
+      const float d = fc.path[info.x + q];
+#pragma unroll
+      for (int k = 0; k < DPT; ++k) t[k] = strong_mul(t[k], d);
+    }
+    gacc_add<DPT>(gacc, c0 + static_cast<uint32_t>(j), nconst, lane, t);
+  }
+}
+
 __device__ __forceinline__ bool needs_db(uint32_t bk) { return bk == kBC || bk == kBS; }
 
 // One forward instruction: [spill] [T = leaf] [b = operand] T = op(T, b),
@@ -99,7 +125,8 @@ __device__ __forceinline__ uint32_t fwd_instr(const uint4 ins, float (&T)[DPT], 
 template <int DPT>
 __device__ __forceinline__ void bwd_instr(const uint4 ins, float (&gT)[DPT], const float *dT_at,
                                           const float *db_at, const SpillStack &adj,
-                                          double *gacc, uint32_t nconst, int lane) {
+                                          double *gacc, uint32_t nconst, int lane,
+                                          const FoldedConsts &fc) {
   const uint32_t w = ins.x;
   const uint32_t bk = instr_b_kind(w);
   float dT[DPT], gi[DPT];
@@ -111,13 +138,28 @@ __device__ __forceinline__ void bwd_instr(const uint4 ins, float (&gT)[DPT], con
     lds_vec<DPT>(db_at, lane, db);
 #pragma unroll
     for (int k = 0; k < DPT; ++k) gb[k] = strong_mul(gT[k], db[k]);
-    if (bk == kBC)
-      gacc_add<DPT>(gacc, (ins.w >> 10) & 0x3FFu, nconst, lane, gb);
-    else
+    if (bk != kBC) {
       spill_store<DPT>(adj, ins.z, lane, gb);
+    } else if (ins.w & kFoldB) {
+      float t[DPT];
+#pragma unroll
+      for (int k = 0; k < DPT; ++k) t[k] = gb[k];
+      gacc_add_folded<DPT>(gacc, (ins.w >> 10) & 0x3FFu, nconst, lane, t, fc);
+    } else {
+      gacc_add<DPT>(gacc, (ins.w >> 10) & 0x3FFu, nconst, lane, gb);
+    }
   }
   if (instr_load(w)) {
-    if (instr_leaf_kind(w) == kLeafC) gacc_add<DPT>(gacc, ins.w & 0x3FFu, nconst, lane, gi);
+    if (instr_leaf_kind(w) == kLeafC) {
+      if (ins.w & kFoldA) {
+        float t[DPT];
+#pragma unroll
+        for (int k = 0; k < DPT; ++k) t[k] = gi[k];
+        gacc_add_folded<DPT>(gacc, ins.w & 0x3FFu, nconst, lane, t, fc);
+      } else {
+        gacc_add<DPT>(gacc, ins.w & 0x3FFu, nconst, lane, gi);
+      }
+    }
     if (instr_spill(w)) {
       spill_load<DPT>(adj, instr_spill_slot(w), lane, gT);
     } else {
@@ -217,6 +259,7 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1) adj_kernel(const AdjA
       const int len = p.code_len[e];
       const int lo = a.bwd_lo[e];  // lowest instruction holding a constant (len: none)
       const uint32_t nconst = static_cast<uint32_t>(a.const_cnt[e]);
+      const FoldedConsts fc{a.cinfo + a.const_off[e], a.path};
       // Checkpoint: partials of [t_lo, len).  Recompute: of the last segment.
       const int last_seg = RECOMP ? ((len - 1) / kSeg) * kSeg : 0;
       const int t_lo = RECOMP ? max(lo, last_seg) : lo;
@@ -282,7 +325,7 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1) adj_kernel(const AdjA
             const uint4 ins = ldg_instr(code + i);
             if (needs_db(instr_b_kind(ins.x))) --kb;
             bwd_instr<DPT>(ins, gT, tape + (i - lo) * TILE, tape + (db_base + kb) * TILE, adj,
-                           gacc, nconst, lane);
+                           gacc, nconst, lane, fc);
           }
         } else {
           for (int s0 = last_seg; s0 >= 0 && s0 + kSeg > lo; s0 -= kSeg) {
@@ -317,7 +360,7 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1) adj_kernel(const AdjA
               const uint4 ins = ldg_instr(code + i);
               if (needs_db(instr_b_kind(ins.x))) --kb;
               bwd_instr<DPT>(ins, gT, tape + (i - s0) * TILE, tape + (db_base + kb) * TILE, adj,
-                             gacc, nconst, lane);
+                             gacc, nconst, lane, fc);
             }
           }
         }
@@ -404,6 +447,7 @@ __global__ void adam_kernel(int64_t C, const float *__restrict__ grad, float *__
   const float nv = consts[c] - lr * mhat / (sqrtf(vhat) + eps);
   consts[c] = nv;
   const int64_t l = loc[c];
+  if (l < 0) return;  // in a folded subtree: its value follows consts
   uint32_t *word = reinterpret_cast<uint32_t *>(code + (l >> 1)) + ((l & 1) ? 2 : 1);
   *word = __float_as_uint(nv);
 }

@@ -19,6 +19,8 @@ struct AdjArgs {
   float *gtape;               // per-warp tapes in global memory, or null (shared memory)
   int32_t tape_len;           // tape entries per warp (>= the tape of any program)
   int32_t gmax;               // gradient accumulators per warp (>= constants of any program)
+  const int4 *cinfo;          // [C] path offset, length, constants of a folded subtree
+  const float *path;          // partials from a folded subtree's root to each constant
   int32_t seg_cap;            // recompute mode: segment-tape entries (min(segment, longest))
   int32_t reserved0;
 };
@@ -36,12 +38,19 @@ struct TanArgs {
   const uint32_t *tmask;      // [instructions + 1] mask words, aligned with the code
   const int64_t *const_off;   // [E] first constant (global index) of each expression
   const int32_t *const_cnt;   // [E] constants of each expression
+  const float *tinit;         // [C] tangent a constant enters with
   double *gout;               // [span groups][C] gradient sums per span group
   int64_t C;                  // constants of the population
   int32_t n_valid;            // expressions in the group table
   int32_t K;                  // tangent rows per warp (>= the constants of any expression)
 };
 
+// Values of n folded constant subtrees into their instruction words, the
+// tangents their constants enter with (tinit) and the partials from each
+// subtree's root down to each constant (path, at cinfo[c].x).
+cudaError_t launch_fold_grad(const GradFold *items, const uint2 *tokens, int n,
+                             const float *consts, const int4 *cinfo, float *tinit, float *path,
+                             cudaStream_t stream);
 int tan_dpt();         // datapoints per thread
 int tan_warps(int K);  // evaluating warps per block (at most) for K tangent rows
 size_t tan_smem_bytes(int K, int W, int V, int s_smem, int span, int G);

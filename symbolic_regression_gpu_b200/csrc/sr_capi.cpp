@@ -91,11 +91,12 @@ sr_status check_population(sr_context *ctx, const sr_population *pop) {
 
 // Compile expressions [0, E) of a CSR population into ps (pinned staging).
 // With `share` equal expressions are compiled once and folded subtrees and
-// derived rows collapse to leaves; folded subtrees, there and under kHintFold
-// hints, are added to ctx->folds.
+// derived rows collapse to leaves; fold_constants (gradient programs) folds
+// constant subtrees alone.  Folded subtrees, there and under kHintFold hints,
+// are added to ctx->folds.
 sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *val,
                       const int64_t *off, const int32_t *hints, ProgramSet &ps,
-                      const sr::Sharing *share) {
+                      const sr::Sharing *share, bool fold_constants) {
   SR_TRACE("sr: compile");
   ps.E = E;
   ps.cost.assign(static_cast<size_t>(E), 0.f);
@@ -126,7 +127,7 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
     Chunk &c = chunks[static_cast<size_t>(ci)];
     const int64_t x0 = static_cast<int64_t>(E) * ci / nt, x1 = static_cast<int64_t>(E) * (ci + 1) / nt;
     c.code.reserve(static_cast<size_t>((off[x1] - off[x0]) * 2 / 3 + 8));
-    std::vector<int32_t> marks(share ? SR_MAX_TOKENS : 0);
+    std::vector<int32_t> marks(share || fold_constants ? SR_MAX_TOKENS : 0);
     std::vector<sr::FoldRef> refs;
     for (int64_t x = x0; x < x1; ++x) {
       sr::ExprInfo &info = infos[static_cast<size_t>(x)];
@@ -143,6 +144,8 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
           continue;
         }
       }
+      if (fold_constants && sr::mark_constant_subtrees(tok + off[x], len, marks.data()))
+        h = marks.data();
       const int64_t i0 = static_cast<int64_t>(c.code.size());
       refs.clear();
       const sr_status s = sr::compile_expression(tok + off[x], val + off[x], len, ctx->V, h, c.code,
@@ -159,8 +162,11 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
       for (const sr::FoldRef &f : refs) {
         const int64_t t0 = off[x] + f.tok;
         uint32_t n = 0;
+        int32_t c0 = 0, nc = 0;
+        for (int32_t k = 0; k < f.tok; ++k) c0 += tok[off[x] + k] == SR_TOK_CONST ? 1 : 0;
         for (int need = 1; need > 0; ++n) {
           const int t = tok[t0 + n];
+          nc += t == SR_TOK_CONST ? 1 : 0;
           need += t <= 0 ? -1 : (sr::is_binary_token(t) ? 1 : 0);
           uint2 w{static_cast<uint32_t>(t), 0u};
           const float v = static_cast<float>(val[t0 + n]);
@@ -168,7 +174,8 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
           c.fold_tokens.push_back(w);
         }
         c.folds.push_back(sr::FoldSet::Ref{&ps, (i0 << 1) + f.loc,
-                                           static_cast<uint32_t>(c.fold_tokens.size()) - n, n});
+                                           static_cast<uint32_t>(c.fold_tokens.size()) - n, n,
+                                           static_cast<int32_t>(x), c0, nc});
       }
     }
     for (Instr &in : c.code) {

@@ -37,7 +37,9 @@ constexpr int kNumTanWidths = 2;
 // the constants (token-order indices, all below kMaxTangentConsts here) under
 // the accumulator before each operator (A) and under its operand b (B), and
 // the constant-load flag.
-void tangent_masks(const Instr *code, int len, uint32_t *out) {
+// A folded constant subtree enters with all its constants (fold_n: their number,
+// per instruction leaf A and operand b).
+void tangent_masks(const Instr *code, int len, const uint8_t *fold_n, uint32_t *out) {
   uint32_t mT = 0;
   uint32_t mS[32] = {};
   for (int i = 0; i < len; ++i) {
@@ -47,13 +49,14 @@ void tangent_masks(const Instr *code, int len, uint32_t *out) {
     if (sr::instr_load(in.w)) {
       const uint32_t ca = in.c & 0x3FFu;
       const bool cl = sr::instr_leaf_kind(in.w) == sr::kLeafC && ca < 8u;
-      A = cl ? (1u << ca) : 0u;
+      A = cl ? (((1u << ((in.c & sr::kFoldA) ? fold_n[2 * i] : 1)) - 1u) << ca) & 0xFFu : 0u;
       L = cl ? sr::kTanLoadConst : 0u;
     }
     uint32_t B = 0;
     const uint32_t bk = sr::instr_b_kind(in.w);
     const uint32_t cb = (in.c >> 10) & 0x3FFu;
-    if (bk == sr::kBC && cb < 8u) B = 1u << cb;
+    if (bk == sr::kBC && cb < 8u)
+      B = (((1u << ((in.c & sr::kFoldB) ? fold_n[2 * i + 1] : 1)) - 1u) << cb) & 0xFFu;
     if (bk == sr::kBS) B = mS[in.b & 31u];
     mT = A | B;
     out[i] = A | (B << 8) | L;
@@ -63,7 +66,7 @@ void tangent_masks(const Instr *code, int len, uint32_t *out) {
 // Kernel launches of one gradient evaluation (forward-mode launches, reverse
 // classes, finalize kernels).
 int grad_launch_count(const sr::GradSet &g) {
-  int n = 0;
+  int n = g.n_folds > 0 ? 1 : 0;
   for (const sr::TanSet &t : g.tsets) n += (t.plan.items() > 0 ? 1 : 0) + 1;
   for (const sr::AdjClass &cl : g.classes) n += cl.plan.items() > 0 ? 1 : 0;
   return n + (g.n_rev > 0 ? 1 : 0);
@@ -77,7 +80,17 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
   g.recompute = recompute;
   ProgramSet &ps = ctx->main;
   const int E = pop->num_exprs;
-  SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, nullptr, ps));
+  SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, nullptr, ps, nullptr, true));
+  // The first constant of each folded subtree stands in its instruction.
+  const std::vector<sr::FoldSet::Ref> &folds = ctx->folds.refs;
+  std::vector<uint8_t> fold_n(2 * static_cast<size_t>(ps.n_instr), 0);
+  for (const auto &f : folds) {
+    Instr &in = ps.h_code.p[f.loc >> 1];
+    const uint32_t c0 = static_cast<uint32_t>(f.c0) & 0x3FFu;
+    in.c = (f.loc & 1) ? (in.c & ~(0x3FFu << 10)) | (c0 << 10) | sr::kFoldB
+                       : (in.c & ~0x3FFu) | c0 | sr::kFoldA;
+    fold_n[static_cast<size_t>(f.loc)] = static_cast<uint8_t>(f.nc);
+  }
   SR_TRY(upload_set(ctx, ps, false));
   // Constants: CSR offsets and the bytecode word that holds each one.
   SR_TRY_CUDA(ctx, g.h_const_off.ensure(static_cast<size_t>(E) + 1));
@@ -99,20 +112,23 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
   g.C = C;
   SR_TRY_CUDA(ctx, g.h_const_loc.ensure(static_cast<size_t>(std::max<int64_t>(C, 1))));
   SR_TRY_CUDA(ctx, g.h_consts.ensure(static_cast<size_t>(std::max<int64_t>(C, 1))));
+  {
+    int64_t c = 0;
+    for (int64_t i = 0; i < pop->offsets[E]; ++i)
+      if (pop->tokens[i] == SR_TOK_CONST) g.h_consts.p[c++] = static_cast<float>(pop->values[i]);
+  }
+  for (int64_t c = 0; c < C; ++c) g.h_const_loc.p[c] = -1;  // in a folded subtree
   for (int x = 0; x < E; ++x) {
     const int64_t i0 = ps.h_off.p[x];
     const int64_t base = g.h_const_off.p[x];
     for (int i = 0; i < ps.h_len.p[x]; ++i) {
       const Instr &in = ps.h_code.p[i0 + i];
       const uint32_t ca = in.c & 0x3FFu, cb = (in.c >> 10) & 0x3FFu;
-      if (sr::instr_load(in.w) && sr::instr_leaf_kind(in.w) == sr::kLeafC && ca != sr::kNoConst) {
+      if (sr::instr_load(in.w) && sr::instr_leaf_kind(in.w) == sr::kLeafC && ca != sr::kNoConst &&
+          !(in.c & sr::kFoldA))
         g.h_const_loc.p[base + ca] = ((i0 + i) << 1);
-        std::memcpy(&g.h_consts.p[base + ca], &in.a, sizeof(float));
-      }
-      if (sr::instr_b_kind(in.w) == sr::kBC && cb != sr::kNoConst) {
+      if (sr::instr_b_kind(in.w) == sr::kBC && cb != sr::kNoConst && !(in.c & sr::kFoldB))
         g.h_const_loc.p[base + cb] = ((i0 + i) << 1) | 1;
-        std::memcpy(&g.h_consts.p[base + cb], &in.b, sizeof(float));
-      }
     }
   }
   // Forward mode for the expressions with at most kMaxTangentConsts
@@ -134,7 +150,8 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
   std::memset(g.h_tmask.p, 0, (static_cast<size_t>(ps.n_instr) + 1) * sizeof(uint32_t));
   for (const auto &mem : tan_members)
     for (int32_t x : mem)
-      tangent_masks(ps.h_code.p + ps.h_off.p[x], ps.h_len.p[x], g.h_tmask.p + ps.h_off.p[x]);
+      tangent_masks(ps.h_code.p + ps.h_off.p[x], ps.h_len.p[x], fold_n.data() + 2 * ps.h_off.p[x],
+                    g.h_tmask.p + ps.h_off.p[x]);
 
   // Backward range and Jacobian-tape length of each reverse-mode program:
   // the sweep runs from the last instruction down to the lowest one holding
@@ -349,6 +366,60 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
                            " bytes) exceed the device memory; split the population or the "
                            "datapoints");
   }
+  // Folded subtrees: items, tokens, and per constant its place in the path
+  // partials (a plain constant: tangent 1, no path), in one copy.
+  {
+    const size_t nf = folds.size(), nt = ctx->folds.tokens.size(), nC = static_cast<size_t>(C);
+    const size_t b_items = nf * sizeof(sr::GradFold), b_tok = nt * sizeof(uint2);
+    const size_t b_info = nC * sizeof(int4), b_init = nC * sizeof(float);
+    g.n_folds = static_cast<int>(nf);
+    SR_TRY_CUDA(ctx, g.folds.ensure(std::max<size_t>(nf, 1)));
+    SR_TRY_CUDA(ctx, g.fold_tokens.ensure(std::max<size_t>(nt, 1)));
+    SR_TRY_CUDA(ctx, g.cinfo.ensure(std::max<size_t>(nC, 1)));
+    SR_TRY_CUDA(ctx, g.tinit.ensure(std::max<size_t>(nC, 1)));
+    SR_TRY_CUDA(ctx, g.h_fold.ensure(std::max<size_t>(b_items + b_tok + b_info + b_init, 1)));
+    auto *items = reinterpret_cast<sr::GradFold *>(g.h_fold.p);
+    // Widest alignment first (GradFold 32 bytes, int4 16, uint2 8, float 4).
+    auto *info = reinterpret_cast<int4 *>(g.h_fold.p + b_items);
+    auto *tokens = reinterpret_cast<uint2 *>(g.h_fold.p + b_items + b_info);
+    auto *init = reinterpret_cast<float *>(g.h_fold.p + b_items + b_info + b_tok);
+    if (nt > 0) std::memcpy(tokens, ctx->folds.tokens.data(), b_tok);
+    for (size_t c = 0; c < nC; ++c) {
+      info[c] = int4{0, 0, 1, 0};
+      init[c] = 1.0f;
+    }
+    int n_path = 0;
+    for (size_t i = 0; i < nf; ++i) {
+      const auto &f = folds[i];
+      const int64_t c0 = g.h_const_off.p[f.expr] + f.c0;
+      Instr *in = ps.code.p + (f.loc >> 1);
+      items[i] = sr::GradFold{f.first, f.len, c0, f.nc, 0, (f.loc & 1) ? &in->b : &in->a};
+      // Depth of each constant under the subtree's root (tokens from the
+      // left: an operator opens its operands one level down).
+      int left[sr::kMaxSharedTokens + 1];  // operands still to come, per open operator
+      int level = 0, k = 0;
+      for (uint32_t q = 0; q < f.len; ++q) {
+        const uint32_t t = tokens[f.first + q].x;
+        if (t != 0) {
+          left[level++] = t < 10 ? 2 : 1;
+          continue;
+        }
+        info[c0 + k] = int4{n_path, level, f.nc, 0};
+        n_path += level;
+        ++k;
+        while (level > 0 && --left[level - 1] == 0) --level;
+      }
+    }
+    SR_TRY_CUDA(ctx, g.path.ensure(static_cast<size_t>(std::max(n_path, 1))));
+    if (nf > 0) {
+      SR_TRY_CUDA(ctx, cudaMemcpyAsync(g.folds.p, items, b_items, cudaMemcpyHostToDevice, ctx->stream));
+      SR_TRY_CUDA(ctx, cudaMemcpyAsync(g.fold_tokens.p, tokens, b_tok, cudaMemcpyHostToDevice, ctx->stream));
+    }
+    if (nC > 0) {
+      SR_TRY_CUDA(ctx, cudaMemcpyAsync(g.cinfo.p, info, b_info, cudaMemcpyHostToDevice, ctx->stream));
+      SR_TRY_CUDA(ctx, cudaMemcpyAsync(g.tinit.p, init, b_init, cudaMemcpyHostToDevice, ctx->stream));
+    }
+  }
   // Uploads.
   const size_t Cs = static_cast<size_t>(std::max<int64_t>(C, 1));
   SR_TRY_CUDA(ctx, g.h_groups.ensure(std::max<size_t>(table.size(), 1)));
@@ -435,6 +506,8 @@ sr_status launch_grad(sr_context *ctx) {
   }
   SR_TRY_CUDA(ctx, record_event(ctx, 1));
   SR_TRY(begin_sequence(ctx));
+  SR_TRY_CUDA(ctx, sr::launch_fold_grad(g.folds.p, g.fold_tokens.p, g.n_folds, g.consts.p, g.cinfo.p,
+                                        g.tinit.p, g.path.p, s));
   int32_t *counter = ctx->d_counter + 2;  // one per launch of the sequence
   for (const sr::TanSet &ts : g.tsets) {
     if (ts.plan.items() == 0) continue;
@@ -453,6 +526,7 @@ sr_status launch_grad(sr_context *ctx) {
     a.tmask = g.tmask.p;
     a.const_off = g.const_off.p;
     a.const_cnt = g.const_cnt.p;
+    a.tinit = g.tinit.p;
     a.gout = g.tan_gout.p + ts.gout_off;
     a.C = g.C;
     a.n_valid = ts.n_exprs;
@@ -474,6 +548,8 @@ sr_status launch_grad(sr_context *ctx) {
     a.const_off = g.const_off.p;
     a.const_cnt = g.const_cnt.p;
     a.bwd_lo = g.bwd_lo.p;
+    a.cinfo = g.cinfo.p;
+    a.path = g.path.p;
     a.grad_acc = g.grad_acc.p;
     a.gtape = cl.global_tape ? g.gtape.p : nullptr;
     a.tape_len = cl.tape_len;

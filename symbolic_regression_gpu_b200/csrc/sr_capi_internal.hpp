@@ -39,7 +39,7 @@ int64_t round_up(int64_t a, int64_t b);
 sr_status check_population(sr_context *ctx, const sr_population *pop);
 sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *val,
                       const int64_t *off, const int32_t *hints, ProgramSet &ps,
-                      const sr::Sharing *share = nullptr);
+                      const sr::Sharing *share = nullptr, bool fold_constants = false);
 // Operator profile of a compiled set (evaluation launches).
 bool protected_profile(const ProgramSet &ps);
 // Launch shape: groups of G cost-sorted expressions x spans of datapoints.

@@ -184,6 +184,7 @@ struct FoldSet {
     ProgramSet *set;
     int64_t loc;   // (instruction << 1) | (operand b)
     uint32_t first, len;
+    int32_t expr, c0, nc;  // its expression; its constants there (token order)
   };
   std::vector<Ref> refs;
   std::vector<uint2> tokens;
@@ -249,7 +250,17 @@ struct TanSet {
 struct GradSet {
   DevBuf<int64_t> const_off;
   DevBuf<int32_t> const_cnt;
-  DevBuf<int64_t> const_loc;  // (instruction << 1) | (operand b)
+  DevBuf<int64_t> const_loc;  // (instruction << 1) | (operand b); -1: in a folded subtree
+  // Constant subtrees are folded in gradient launches too: fold_grad_kernel
+  // evaluates them from the current constants, with the partials on the way
+  // from each constant to the subtree's root.
+  DevBuf<GradFold> folds;     // one per folded subtree
+  DevBuf<uint2> fold_tokens;
+  DevBuf<int4> cinfo;         // [C] path offset, path length, constants of the subtree (at its first)
+  DevBuf<float> tinit;        // [C] d subtree / d constant (1 for a constant of its own)
+  DevBuf<float> path;         // partials from the root down to each folded constant
+  PinnedBuf<unsigned char> h_fold;
+  int n_folds = 0;
   DevBuf<double> grad_acc;
   DevBuf<float> grad;
   DevBuf<float> consts;

@@ -36,8 +36,9 @@
 //   Instr.a  payload of leaf A, Instr.b payload of operand b: spill slot /
 //            variable row / float bits of the constant / cache slot
 //   Instr.c  bits 0..9 / 10..19: constant index (token order) of leaf A /
-//            operand b when it is a constant, 0x3FF otherwise; bits 20..29:
-//            when b is a spill slot, the program-relative index of the
+//            operand b when it is a constant, 0x3FF otherwise (bits 30 / 31:
+//            that constant is the first of a folded constant subtree, kFoldA /
+//            kFoldB; gradient programs only); bits 20..29: when b is a spill slot, the program-relative index of the
 //            instruction whose output was spilled there (the adjoint reads
 //            that value back from its tape).
 #pragma once
@@ -193,6 +194,20 @@ struct FoldItem {
   uint32_t first, len;
   uint32_t *dst;
 };
+
+// A folded constant subtree of a gradient launch: its tokens, its constants
+// [c0, c0 + nc) (indices into the population's constants, token order) and the
+// instruction word that holds its value.
+struct GradFold {
+  uint32_t first, len;
+  int64_t c0;
+  int32_t nc, reserved0;
+  uint32_t *dst;
+};
+static_assert(sizeof(GradFold) == 32, "packed before 16-byte words");
+// Instr.c flags: the constant index of leaf A / operand b is the first
+// constant of a folded subtree.
+constexpr uint32_t kFoldA = 1u << 30, kFoldB = 1u << 31;
 
 // Argument block of the interpreter kernel (passed by value).
 //

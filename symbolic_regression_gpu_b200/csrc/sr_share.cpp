@@ -47,6 +47,47 @@ constexpr uint64_t kRootSalt = 0x9E3779B97F4A7C15ull;
 
 }  // namespace
 
+bool mark_constant_subtrees(const int32_t *tok, int len, int32_t *hints) {
+  // size: tokens of the subtree at each position, negative when constant.
+  int16_t size[SR_MAX_TOKENS];
+  if (len > SR_MAX_TOKENS) return false;
+  int depth = 0;
+  for (int i = len - 1; i >= 0; --i) {
+    const int32_t t = tok[i];
+    if (t == SR_TOK_CONST || t == SR_TOK_VAR) {
+      ++depth;
+      size[i] = t == SR_TOK_CONST ? -1 : 1;
+      continue;
+    }
+    const bool binary = is_binary_token(t);
+    if (binary ? --depth < 1 : !is_unary_token(t) || depth < 1) return false;
+    const int16_t a = size[i + 1];
+    int n = 1 + (a < 0 ? -a : a);
+    bool constant = a < 0;
+    if (binary) {
+      const int16_t b = size[i + n];
+      n += b < 0 ? -b : b;
+      constant = constant && b < 0;
+    }
+    size[i] = static_cast<int16_t>(constant ? -n : n);
+  }
+  if (depth != 1) return false;
+  bool any = false;
+  for (int i = 0; i < len;) {
+    hints[i] = -1;
+    const int n = -size[i];
+    if (n < 2 || n > kMaxSharedTokens) {
+      ++i;
+      continue;
+    }
+    any = true;
+    hints[i] = kHintFold;
+    for (int k = 1; k < n; ++k) hints[i + k] = -2;
+    i += n;
+  }
+  return any;
+}
+
 // A worker's own counts of the subtrees it met last: the frequent ones (sin x0)
 // would otherwise have every worker add to the same few words.
 struct Sharing::Local {

@@ -31,6 +31,11 @@ constexpr int32_t kHintRow0 = -16;     // root of derived row r: kHintRow0 - r
 constexpr int kMaxDerivedRows = 64;
 constexpr int kMaxSharedTokens = 64;   // largest subtree folded or made a row
 
+// Marks the maximal subtrees of constants of one expression (operators over
+// constants only, at most kMaxSharedTokens tokens) for folding; returns
+// whether there is one, false as well for a malformed expression.
+bool mark_constant_subtrees(const int32_t *tok, int len, int32_t *hints);
+
 class Sharing {
  public:
   struct Row {

@@ -313,6 +313,7 @@ __device__ __forceinline__ void run_tangent_program(const Instr *__restrict__ co
                                                     const uint32_t *__restrict__ tmask, int len,
                                                     const float *xs, int xrs,
                                                     const SpillStack &st, int lane, float *tan,
+                                                    const float *__restrict__ tinit,
                                                     float (&T)[DPT]) {
   constexpr int TILE = 32 * DPT;
   uint4 ins = ldg_instr(code);
@@ -336,7 +337,8 @@ __device__ __forceinline__ void run_tangent_program(const Instr *__restrict__ co
     tan_apply<DPT>(instr_op(w), (A | B) != 0, T, b, dT, db, dk, bkn);
     if (A | B) {
       // Constants that enter here (a constant leaf, a constant operand b)
-      // start from tangent 1; rows of an operator whose partial is exactly 1
+      // start from tangent 1, those of a folded subtree from the subtree's
+      // derivative by them; rows of an operator whose partial is exactly 1
       // stay as they are.  (One loop for both masks: a second copy of it
       // costs more in instruction-cache misses than its branches.)
       const uint32_t fresh = (m & kTanLoadConst ? A : 0u) | (bk == kBC ? B : 0u);
@@ -349,8 +351,9 @@ __device__ __forceinline__ void run_tangent_program(const Instr *__restrict__ co
         float *row = tan + c * TILE;
         float tv[DPT];
         if (is_fresh) {
+          const float t0 = __ldg(tinit + c);
 #pragma unroll
-          for (int k = 0; k < DPT; ++k) tv[k] = 1.0f;
+          for (int k = 0; k < DPT; ++k) tv[k] = t0;
         } else {
           lds_vec<DPT>(row, lane, tv);
         }
@@ -441,6 +444,7 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) tan_kernel(const TanArg
       const uint32_t *tm = a.tmask + p.code_off[e];
       const int len = p.code_len[e];
       const int nconst = min(a.const_cnt[e], K);
+      const float *tinit = a.tinit + a.const_off[e];
       double acc = 0.0;
       int cnt = 0;
       for (int c = 0; c < nconst; ++c) gl[c * 32 + lane] = 0.0;
@@ -449,7 +453,7 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) tan_kernel(const TanArg
         if (dp0 >= p.N) break;  // tail of the last span
         const float *xs = xb + t * TILE;
         float T[DPT];
-        run_tangent_program<DPT>(code, tm, len, xs, span, st, lane, tan, T);
+        run_tangent_program<DPT>(code, tm, len, xs, span, st, lane, tan, tinit, T);
         float y[DPT], sd[DPT];
         lds_vec<DPT>(xs + p.V * span, lane, y);
         const bool full_tile = dp0 + TILE <= p.N;  // warp-uniform
@@ -508,6 +512,70 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) tan_kernel(const TanArg
       buf = 0;
       phase ^= 1u;
     }
+  }
+}
+
+// Folded constant subtrees of a gradient launch, one thread each: the value
+// and, constant by constant, the derivative from the constant up to the root,
+// through the tangent kernel's own operators and zero rule (the rows of these
+// constants would hold the same products at the subtree's root), and the
+// partials met on the way.  A subtree's work is that of a few datapoints; the
+// launch over all of them is latency-bound (5 us).
+constexpr int kMaxFoldDepth = 40;  // values waiting in a subtree of 64 tokens
+__global__ void __launch_bounds__(64)
+    fold_grad_kernel(const GradFold *__restrict__ items, const uint2 *__restrict__ tokens, int n,
+                     const float *__restrict__ consts, const int4 *__restrict__ cinfo,
+                     float *__restrict__ tinit, float *__restrict__ path) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const GradFold it = items[i];
+  float val[kMaxFoldDepth], tan[kMaxFoldDepth];
+  bool on[kMaxFoldDepth];  // the constant lies under it
+  for (int j = 0; j < it.nc; ++j) {
+    const int64_t cj = it.c0 + j;
+    const int4 info = cinfo[cj];
+    int sp = 0, seen = 0, step = info.y;
+    for (uint32_t k = it.len; k-- > 0;) {
+      const uint32_t op = tokens[it.first + k].x;
+      if (op == 0) {
+        const int idx = it.nc - 1 - seen++;
+        val[sp] = consts[it.c0 + idx];
+        tan[sp] = 1.0f;
+        on[sp] = idx == j;
+        ++sp;
+        continue;
+      }
+      const int a = --sp;
+      const int b = op < 10 ? --sp : a;
+      float T[2] = {val[a], val[a]}, B[2] = {val[b], val[b]};
+      float dT[2], dB[2];
+      int kt, kb;
+      tan_apply<2>(op, true, T, B, dT, dB, kt, kb);
+      const bool under_b = op < 10 && on[b];
+      const bool under = on[a] || under_b;
+      if (under) {
+        float t[2] = {under_b ? tan[b] : tan[a], 0.0f};
+        t[1] = t[0];
+        const int kind = under_b ? kb : kt;
+        float d = kind == kDOne ? 1.0f : -1.0f;
+        if (kind == kDGen) {
+          d = under_b ? dB[0] : dT[0];
+          if (under_b)
+            kill_mul<2>(t, dB);
+          else
+            kill_mul<2>(t, dT);
+        } else if (kind == kDNeg) {
+          t[0] = -t[0];
+        }
+        path[info.x + --step] = d;
+        tan[sp] = t[0];
+      }
+      on[sp] = under;
+      val[sp] = T[0];
+      ++sp;
+    }
+    tinit[cj] = tan[0];
+    if (j == 0) *it.dst = __float_as_uint(val[0]);
   }
 }
 
@@ -615,6 +683,14 @@ cudaError_t launch_tangent(const TanArgs &args, int blocks, size_t smem, cudaStr
   if (args.e.W < 1 || args.e.W > tan_max_warps(args.K)) return cudaErrorInvalidValue;
   void *params[] = {const_cast<TanArgs *>(&args)};
   return cudaLaunchKernel(fn, dim3(blocks), dim3((args.e.W + 1) * 32), params, smem, stream);
+}
+
+cudaError_t launch_fold_grad(const GradFold *items, const uint2 *tokens, int n,
+                             const float *consts, const int4 *cinfo, float *tinit, float *path,
+                             cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  fold_grad_kernel<<<(n + 63) / 64, 64, 0, stream>>>(items, tokens, n, consts, cinfo, tinit, path);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_tan_finalize(const double2 *partial, const double *gout, int n_groups, int E,
