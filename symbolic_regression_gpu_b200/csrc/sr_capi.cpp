@@ -914,6 +914,8 @@ sr_status sr_create(const sr_options *opts, sr_context **out) {
   ctx->num_sms = prop.multiProcessorCount;
   ctx->device_memory = prop.totalGlobalMem;
   ctx->max_smem = static_cast<int>(prop.sharedMemPerBlockOptin);
+  ctx->sm_smem = static_cast<int>(prop.sharedMemPerMultiprocessor);
+  ctx->block_smem = static_cast<int>(prop.reservedSharedMemPerBlock);
   ctx->device_name = prop.name;
   ctx->cache.capacity = o.cache_capacity;
   cudaError_t e = cudaSuccess;

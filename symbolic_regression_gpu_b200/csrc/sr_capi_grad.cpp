@@ -72,6 +72,13 @@ int grad_launch_count(const sr::GradSet &g) {
   return n + (g.n_rev > 0 ? 1 : 0);
 }
 
+// Expressions per group and evaluating warp, as the interpreter's launches
+// choose them.
+static int group_depth(const sr_context *ctx, int E) {
+  const int size = launch_size(ctx, E);
+  return size <= 1 ? 1 : (size == 2 ? 2 : 4);
+}
+
 // Compile, lay out constants, split expressions into tape-length classes and
 // upload everything the adjoint launches need.
 sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute,
@@ -207,7 +214,7 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
   // One span for every class (the MSE partials are laid out per span): the
   // largest of 1024 / 512 / 256 / 128 datapoints whose double-buffered X
   // stage fits in 48 KB.
-  int span = 1024;
+  int span = launch_size(ctx, g.n_rev) <= 1 ? 256 : 1024;
   while (span > tile && 2 * static_cast<int64_t>(ctx->V + 1) * span * 4 > 48 * 1024) span /= 2;
   g.span = static_cast<int>(std::min<int64_t>(span, std::max<int64_t>(tile, round_up(ctx->N, tile))));
   g.n_spans = (ctx->N == 0) ? 0 : static_cast<int>((ctx->N + g.span - 1) / g.span);
@@ -244,8 +251,13 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
         const size_t smem =
             sr::adj_smem_bytes(W, ctx->V, s_smem, g.span, cl.tape_len, cl.gmax, gt);
         if (smem > static_cast<size_t>(dev_max_smem)) continue;
-        int bps = 0;
-        SR_TRY_CUDA(ctx, sr::adj_configure(smem, W, gt, recompute, &bps));
+        // Resident blocks: the registers' limit, asked for once per warp count
+        // (the query costs microseconds and 32 shapes are looked at), and
+        // shared memory's.
+        int &reg_blocks = ctx->adj_blocks[gt ? 1 : 0][recompute ? 1 : 0][W];
+        if (reg_blocks == 0) SR_TRY_CUDA(ctx, sr::adj_configure(0, W, gt, recompute, &reg_blocks));
+        const size_t block = (smem + 127) / 128 * 128 + static_cast<size_t>(ctx->block_smem);
+        const int bps = std::min(reg_blocks, static_cast<int>(static_cast<size_t>(ctx->sm_smem) / block));
         if (bps <= 0) continue;
         const int64_t resident_tape =
             static_cast<int64_t>(W) * bps * ctx->num_sms * cl.tape_len * tile * 4;
@@ -258,6 +270,12 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
         }
       }
     }
+    if (best_w > 0) {
+      int bps = 0;  // the chosen shape as the driver counts it
+      SR_TRY_CUDA(ctx, sr::adj_configure(best_smem, best_w, cl.global_tape, recompute, &bps));
+      best_res = best_w * bps;
+      if (bps <= 0) best_w = 0;
+    }
     if (best_w == 0)
       return ctx->fail(SR_ERR_UNSUPPORTED, "no adjoint launch shape fits " +
                                                std::to_string(cl.tape_len) + " tape entries");
@@ -266,7 +284,7 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
     p.W = best_w;
     p.smax = ps.smax;
     p.s_smem = s_smem;
-    p.G = best_w * 4;
+    p.G = best_w * group_depth(ctx, static_cast<int>(mem.size()));
     p.n_groups = static_cast<int>((mem.size() + p.G - 1) / p.G);
     p.span = g.span;
     p.n_spans = g.n_spans;
@@ -305,7 +323,8 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
     // Wider sets keep one spill slot per warp in shared memory (the others in
     // per-warp global scratch): the tangent rows need the room.
     p.s_smem = std::min(ps.smax, ts.K > 4 ? 1 : sr::smem_spill_slots(p.dpt));
-    int64_t tspan = 1024;
+    const int depth = group_depth(ctx, static_cast<int>(mem.size()));
+    int64_t tspan = launch_size(ctx, static_cast<int>(mem.size())) <= 1 ? 256 : 1024;
     while (tspan > ttile && 2 * static_cast<int64_t>(ctx->V + 1) * tspan * 4 > 48 * 1024)
       tspan /= 2;
     tspan = std::min<int64_t>(tspan, std::max<int64_t>(ttile, round_up(ctx->N, ttile)));
@@ -313,13 +332,13 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
     // block's shared memory does not fit, then fewer evaluating warps.
     const size_t budget = static_cast<size_t>(dev_max_smem);
     while (tspan / 2 >= std::max<int64_t>(ttile, 512) && (tspan / 2) % ttile == 0 &&
-           sr::tan_smem_bytes(ts.K, p.W, ctx->V, p.s_smem, static_cast<int>(tspan), p.W * 4) >
+           sr::tan_smem_bytes(ts.K, p.W, ctx->V, p.s_smem, static_cast<int>(tspan), p.W * depth) >
                budget)
       tspan /= 2;
     while (p.W > 4 && sr::tan_smem_bytes(ts.K, p.W, ctx->V, p.s_smem, static_cast<int>(tspan),
-                                         p.W * 4) > budget)
+                                         p.W * depth) > budget)
       --p.W;
-    p.G = p.W * 4;
+    p.G = p.W * depth;
     p.n_groups = static_cast<int>((mem.size() + p.G - 1) / p.G);
     p.span = static_cast<int>(tspan);
     p.n_spans = (ctx->N == 0) ? 0 : static_cast<int>((ctx->N + tspan - 1) / tspan);

@@ -42,6 +42,8 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
                       const sr::Sharing *share = nullptr, bool fold_constants = false);
 // Operator profile of a compiled set (evaluation launches).
 bool protected_profile(const ProgramSet &ps);
+// Size class of a launch of E expressions over the dataset, 0 (small) .. 3.
+int launch_size(const sr_context *ctx, int E);
 // Launch shape: groups of G cost-sorted expressions x spans of datapoints.
 // `split`: spill slots per warp kept in shared memory (-1 = the default for
 // the dpt); `per_warp`: expressions per group and evaluating warp (0: by the

@@ -304,6 +304,8 @@ struct sr_context {
   int device = 0;
   int num_sms = 0;
   int max_smem = 0;          // opt-in shared memory per block
+  int sm_smem = 0;           // shared memory per SM, and what each block reserves
+  int block_smem = 0;
   size_t device_memory = 0;  // bytes of device memory (cudaDeviceProp::totalGlobalMem)
   std::string device_name;
   cudaStream_t stream = nullptr;
@@ -385,6 +387,9 @@ struct sr_context {
   // resident blocks per SM of the interpreter shapes planned so far (the
   // occupancy query costs microseconds, a small call plans three shapes)
   std::map<std::array<int64_t, 6>, int> occupancy;
+  // the same of the reverse-mode kernels without shared memory, [tape in
+  // global memory][recompute][evaluating warps]
+  int adj_blocks[2][2][32] = {};
 
   // tuned launch shapes: key -> (dpt, W, spill slots in shared memory (-1 =
   // the default for the dpt), expressions per group and warp)
