@@ -514,10 +514,93 @@ constexpr int kInlineMaxDpt = 8;  // wider launches call them (16 copies overflo
   SR_C_INL_OR(CASE, T[k] = expf(fminf(T[k], 80.0f)),                             \
               _Pragma("unroll") for (int k = 0; k < DPT; ++k) T[k] = fminf(T[k], 80.0f); \
               SR_MAP1(v_exp, T, T))
+// The out-of-line rest of the paired forms below: a lane with an argument
+// outside their range evaluates its datapoints one by one.
+template <int DPT>
+__device__ __noinline__ void lsqrt_cold(float *T) {
+#pragma unroll
+  for (int k = 0; k < DPT; ++k) T[k] = __fsqrt_rn(fabsf(T[k]));
+}
+template <int DPT>
+__device__ __noinline__ void llog_cold(float *T) {
+#pragma unroll
+  for (int k = 0; k < DPT; ++k) T[k] = sr_loose_logf(T[k]);
+}
+template <int DPT>
+__device__ __noinline__ void ldiv_cold(float *T, const float *b) {
+#pragma unroll
+  for (int k = 0; k < DPT; ++k) T[k] = __fdiv_rn(T[k], loose_denom(b[k]));
+}
+// sqrt|T|
+template <int DPT>
+__device__ __forceinline__ void lsqrt_wide(float (&T)[DPT]) {
+  if (min_abs<DPT>(T) >= kSqrtMin && max_abs<DPT>(T) <= kSqrtMax) {
+#pragma unroll
+    for (int k = 0; k < DPT; k += 2) {
+      const float2 r = sqrt2_mid(make_float2(fabsf(T[k]), fabsf(T[k + 1])));
+      T[k] = r.x;
+      T[k + 1] = r.y;
+    }
+  } else {
+    float t[DPT];
+#pragma unroll
+    for (int k = 0; k < DPT; ++k) t[k] = T[k];
+    lsqrt_cold<DPT>(t);
+#pragma unroll
+    for (int k = 0; k < DPT; ++k) T[k] = t[k];
+  }
+}
+// -1e9 at 0, else log|T|
+template <int DPT>
+__device__ __forceinline__ void llog_wide(float (&T)[DPT]) {
+  if (min_abs<DPT>(T) >= kMinNormal && max_abs_nan<DPT>(T) < INFINITY) {
+#pragma unroll
+    for (int k = 0; k < DPT; k += 2) {
+      const float2 r = sr_log_normal2(fabsf(T[k]), fabsf(T[k + 1]));
+      T[k] = r.x;
+      T[k + 1] = r.y;
+    }
+  } else {
+    float t[DPT];
+#pragma unroll
+    for (int k = 0; k < DPT; ++k) t[k] = T[k];
+    llog_cold<DPT>(t);
+#pragma unroll
+    for (int k = 0; k < DPT; ++k) T[k] = t[k];
+  }
+}
+// T / protected(b): outside the protected region the denominator is b itself.
+template <int DPT>
+__device__ __forceinline__ void ldiv_wide(float (&T)[DPT], const float (&b)[DPT]) {
+  const float largest = fmaxf(max_abs<DPT>(T), max_abs<DPT>(b));
+  if (largest <= kDivMax && min_abs<DPT>(T) >= kDivMin && min_abs<DPT>(b) > 1e-9f) {
+#pragma unroll
+    for (int k = 0; k < DPT; k += 2) {
+      const float2 r = div2_mid(make_float2(T[k], T[k + 1]), make_float2(b[k], b[k + 1]));
+      T[k] = r.x;
+      T[k + 1] = r.y;
+    }
+  } else {
+    float t[DPT], u[DPT];
+#pragma unroll
+    for (int k = 0; k < DPT; ++k) {
+      t[k] = T[k];
+      u[k] = b[k];
+    }
+    ldiv_cold<DPT>(t, u);
+#pragma unroll
+    for (int k = 0; k < DPT; ++k) T[k] = t[k];
+  }
+}
 #define SR_LSQRT_INL(CASE)                                                     \
-  SR_C_INL_OR(CASE, T[k] = __fsqrt_rn(fabsf(T[k])),                              \
-              _Pragma("unroll") for (int k = 0; k < DPT; ++k) T[k] = fabsf(T[k]); \
-              SR_MAP1(v_sqrt, T, T))
+  case CASE:                                                                   \
+    if constexpr (DPT <= kInlineMaxDpt) {                                      \
+      lsqrt_wide<DPT>(T);                                                      \
+    } else {                                                                   \
+      _Pragma("unroll") for (int k = 0; k < DPT; ++k) T[k] = fabsf(T[k]);      \
+      SR_MAP1(v_sqrt, T, T)                                                    \
+    }                                                                          \
+    break;
 #define SR_C_LDIV_INL                                                          \
   SR_C_INL_OR(8, T[k] = __fdiv_rn(T[k], loose_denom(b[k])),                    \
               _Pragma("unroll") for (int k = 0; k < DPT; ++k) b[k] = loose_denom(b[k]); \
@@ -540,9 +623,7 @@ __device__ __noinline__ void sincos_cold(float *T, int q_offset) {
 #define SR_C_SINCOS_INL(CASE, QOFF, NAME)                                      \
   case CASE:                                                                   \
     if constexpr (DPT <= kInlineMaxDpt) {                                      \
-      bool slow_ = false;                                                      \
-      _Pragma("unroll") for (int k = 0; k < DPT; ++k) slow_ |= !sincos_fast_ok(T[k]); \
-      if (slow_) {                                                             \
+      if (!(max_abs<DPT>(T) <= kSinCosFastMax)) {                                                             \
         float t_[DPT];                                                         \
         _Pragma("unroll") for (int k = 0; k < DPT; ++k) t_[k] = T[k];          \
         sincos_cold<DPT>(t_, QOFF);                                            \
@@ -561,20 +642,19 @@ __device__ __noinline__ void sincos_cold(float *T, int q_offset) {
     }                                                                          \
     break;
 #define SR_LLOG_INL(CASE)                                                      \
-  SR_C_INL_OR(CASE, if ((k & 1) == 0) {                                          \
-                const float2 l_ = sr_log_nonneg2(fabsf(T[k]), fabsf(T[k + 1])); \
-                T[k] = T[k] == 0.0f ? -1e9f : l_.x;                            \
-                T[k + 1] = T[k + 1] == 0.0f ? -1e9f : l_.y;                    \
-              },                                                               \
-              {                                                                \
-                bool z_[DPT];                                                  \
-                _Pragma("unroll") for (int k = 0; k < DPT; ++k) {              \
-                  z_[k] = (T[k] == 0.0f);                                      \
-                  T[k] = fabsf(T[k]);                                          \
-                }                                                              \
-                SR_MAP1(v_log, T, T)                                           \
-                _Pragma("unroll") for (int k = 0; k < DPT; ++k) T[k] = z_[k] ? -1e9f : T[k]; \
-              })
+  case CASE:                                                                   \
+    if constexpr (DPT <= kInlineMaxDpt) {                                      \
+      llog_wide<DPT>(T);                                                       \
+    } else {                                                                   \
+      bool z_[DPT];                                                            \
+      _Pragma("unroll") for (int k = 0; k < DPT; ++k) {                        \
+        z_[k] = (T[k] == 0.0f);                                                \
+        T[k] = fabsf(T[k]);                                                    \
+      }                                                                        \
+      SR_MAP1(v_log, T, T)                                                     \
+      _Pragma("unroll") for (int k = 0; k < DPT; ++k) T[k] = z_[k] ? -1e9f : T[k]; \
+    }                                                                          \
+    break;
 
 // Operator profiles (kOpsAll / kOpsProtected and the host-side membership
 // test live in sr_internal.hpp).  kOpsAll dispatches every operator inline;
@@ -640,13 +720,15 @@ __device__ __noinline__ void apply_op_cold(uint32_t op, float *T, float *b) {
 // ones, for launches whose programs have none (dispatch stays short).
 //
 // Issue-bound: the schedulers issue on nearly every cycle, so time is the
-// number of instructions.  Each bytecode instruction costs one test of the
-// load / spill flags, one operand address and one indirect branch on its
-// dispatch code, whose case loads the operand where the operator takes it
-// (+ - * straight into the paired operations; a constant is not spread over
-// DPT registers first).  Batched population (10,000 x 1M) 55.1 -> 49.2 ms,
-// 8,000 long programs x 4M 326 -> 287 ms against separate branches for the
-// operand's kind and the opcode.
+// number of instructions (an addition of a variable row took 50 of them for 8
+// datapoints a lane with a switch over the dispatch codes, which the compiler
+// turns into a tree of branches; 45 here, six of them the loads and adds).  Each
+// instruction costs one test of the load / spill flags, one operand address and
+// tests of single bits of its dispatch code; + - * need two or three.  Batched
+// population (10,000 x 1M) 55.1 -> 49.2 ms with dispatch codes instead of separate
+// branches for the operand's kind and the opcode, 37.6 -> 36.1 ms with bit tests
+// on a uniform word, -> 35.1 ms with the paired division, square root and
+// logarithm; 8,000 long programs x 4M 326 -> 287 -> 222 -> 215 ms.
 template <int DPT, int OPS, bool GEN>
 __device__ __forceinline__ void run_program(const Instr *__restrict__ code, int len,
                                             const float *xs, const SpillStack &st, int lane,
@@ -658,10 +740,14 @@ __device__ __forceinline__ void run_program(const Instr *__restrict__ code, int 
   // Every program starts with an instruction that loads T.
   uint4 ins = ldg_instr(code);
   for (int i = 0; i < len; ++i) {
-    // The code buffer ends with a padding instruction, so this prefetch of
-    // the next word is always in bounds.
-    const uint4 nxt = ldg_instr(code + i + 1);
-    const uint32_t w = ins.x;
+    // The code buffer ends with a padding instruction, so this prefetch of the
+    // next word is always in bounds.  (General launches fetch it below, once
+    // this word's registers are free: their operands need them.)
+    uint4 nxt;
+    if constexpr (!GEN) nxt = ldg_instr(code + i + 1);
+    // The word is the same in every lane; the reduction says so to the compiler
+    // (a uniform register).
+    const uint32_t w = __reduce_or_sync(0xffffffffu, ins.x);
     if (w & (kLoadBit | kSpillBit)) {
       if (GEN) {
         if (instr_spill(w)) spill_store<DPT>(st, instr_spill_slot(w), lane, T);
@@ -681,8 +767,8 @@ __device__ __forceinline__ void run_program(const Instr *__restrict__ code, int 
       }
     }
     const uint32_t d = instr_dispatch(w);
-    const float cb = __uint_as_float(ins.z);
-    const float2 c2 = make_float2(cb, cb);
+    const uint32_t bw = ins.z;
+    const float cb = __uint_as_float(bw);
     // Operand b in shared memory: a spill slot (kind 1) or a variable row (2).
     const float *bp = ((w & (2u << 9)) ? xl : sl) + ins.z * TILE;
     // General launches read a memory operand into registers by its kind.
@@ -694,56 +780,15 @@ __device__ __forceinline__ void run_program(const Instr *__restrict__ code, int 
       else if (bk == kBS)
         spill_load<DPT>(st, ins.z, lane, bg);
       else if (bk == kBX)
-        lds_vec<DPT>(bp, 0, bg);
+        lds_vec<DPT>(xs + ins.z * TILE, lane, bg);
     }
+    if constexpr (GEN) ins = ldg_instr(code + i + 1);
     auto quad_b = [&](int h) {
       if constexpr (GEN)
         return make_float4(bg[4 * h], bg[4 * h + 1], bg[4 * h + 2], bg[4 * h + 3]);
       else
         return *reinterpret_cast<const float4 *>(bp + h * 128);
     };
-#define SR_F_MEM(EXPR)                                                         \
-  {                                                                            \
-    _Pragma("unroll") for (int h = 0; h < DPT / 4; ++h) {                      \
-      const float4 q = quad_b(h);                                              \
-      {                                                                        \
-        const float2 t_ = make_float2(T[4 * h], T[4 * h + 1]);                 \
-        const float2 u_ = make_float2(q.x, q.y);                               \
-        const float2 r_ = (EXPR);                                              \
-        T[4 * h] = r_.x;                                                       \
-        T[4 * h + 1] = r_.y;                                                   \
-      }                                                                        \
-      {                                                                        \
-        const float2 t_ = make_float2(T[4 * h + 2], T[4 * h + 3]);             \
-        const float2 u_ = make_float2(q.z, q.w);                               \
-        const float2 r_ = (EXPR);                                              \
-        T[4 * h + 2] = r_.x;                                                   \
-        T[4 * h + 3] = r_.y;                                                   \
-      }                                                                        \
-    }                                                                          \
-  }                                                                            \
-  break;
-#define SR_F_CONST(EXPR)                                                       \
-  {                                                                            \
-    _Pragma("unroll") for (int k = 0; k < DPT; k += 2) {                       \
-      const float2 t_ = make_float2(T[k], T[k + 1]);                           \
-      const float2 u_ = c2;                                                    \
-      const float2 r_ = (EXPR);                                                \
-      T[k] = r_.x;                                                             \
-      T[k + 1] = r_.y;                                                         \
-    }                                                                          \
-  }                                                                            \
-  break;
-#define SR_F_CHEAP                                                             \
-  case kDNone: break;                                                          \
-  case kDAddM: SR_F_MEM(__fadd2_rn(t_, u_))                                    \
-  case kDSubM: SR_F_MEM(__fadd2_rn(t_, make_float2(-u_.x, -u_.y)))             \
-  case kDRSubM: SR_F_MEM(__fadd2_rn(u_, make_float2(-t_.x, -t_.y)))            \
-  case kDMulM: SR_F_MEM(__fmul2_rn(t_, u_))                                    \
-  case kDAddC: SR_F_CONST(__fadd2_rn(t_, u_))                                  \
-  case kDSubC: SR_F_CONST(__fadd2_rn(t_, make_float2(-u_.x, -u_.y)))           \
-  case kDRSubC: SR_F_CONST(__fadd2_rn(u_, make_float2(-t_.x, -t_.y)))          \
-  case kDMulC: SR_F_CONST(__fmul2_rn(t_, u_))
     auto memory_b = [&](float (&b)[DPT]) {
 #pragma unroll
       for (int h = 0; h < DPT / 4; ++h) unquad<DPT>(b, h, quad_b(h));
@@ -757,9 +802,41 @@ __device__ __forceinline__ void run_program(const Instr *__restrict__ code, int 
         memory_b(b);
       }
     };
-    if constexpr (OPS == kOpsProtected) {
+#define SR_LINEAR_M(EXPR)                                                      \
+  _Pragma("unroll") for (int h = 0; h < DPT / 4; ++h) {                        \
+    const float4 q = quad_b(h);                                                \
+    _Pragma("unroll") for (int g = 0; g < 2; ++g) {                            \
+      const float2 t_ = make_float2(T[4 * h + 2 * g], T[4 * h + 2 * g + 1]);   \
+      const float2 u_ = g ? make_float2(q.z, q.w) : make_float2(q.x, q.y);     \
+      const float2 r_ = (EXPR);                                                \
+      T[4 * h + 2 * g] = r_.x;                                                 \
+      T[4 * h + 2 * g + 1] = r_.y;                                             \
+    }                                                                          \
+  }
+    if (d & kDLinear) {
+      // + - * as one fused multiply-add each, two datapoints at a time: T + b
+      // = 1 b + T, T - b = -1 b + T, b - T = -1 T + b and T b = T b + (-0) are
+      // the correctly rounded operations themselves, zeros' signs included.
+      if (d & kDConst) {
+        const float mul = (d & kDMul) ? cb : ((d & kDRSub) ? -1.0f : 1.0f);
+        const float add = (d & kDMul) ? -0.0f : ((d & kDSub) ? -cb : cb);
+#pragma unroll
+        for (int k = 0; k < DPT; k += 2) {
+          const float2 r = __ffma2_rn(make_float2(T[k], T[k + 1]), f2(mul), f2(add));
+          T[k] = r.x;
+          T[k + 1] = r.y;
+        }
+      } else if (d & kDMul) {
+        SR_LINEAR_M(__fmul2_rn(t_, u_))
+      } else if (d & kDRSub) {
+        SR_LINEAR_M(__ffma2_rn(t_, f2(-1.0f), u_))
+      } else {
+        const float2 sign = f2((d & kDSub) ? -1.0f : 1.0f);
+        SR_LINEAR_M(__ffma2_rn(u_, sign, t_))
+      }
+    } else if constexpr (OPS == kOpsProtected) {
       switch (d) {
-        SR_F_CHEAP
+        case kDNone: break;
         case kDLDivM:
         case kDRLDivM:
         case kDLDivC:
@@ -779,12 +856,11 @@ __device__ __forceinline__ void run_program(const Instr *__restrict__ code, int 
               b[k] = t;
             }
           }
-#pragma unroll
-          for (int k = 0; k < DPT; ++k) b[k] = loose_denom(b[k]);
           if constexpr (DPT <= kInlineMaxDpt) {
-#pragma unroll
-            for (int k = 0; k < DPT; ++k) T[k] = __fdiv_rn(T[k], b[k]);
+            ldiv_wide<DPT>(T, b);
           } else {
+#pragma unroll
+            for (int k = 0; k < DPT; ++k) b[k] = loose_denom(b[k]);
             SR_MAP2(v_div, T, T, b)
           }
         } break;
@@ -804,19 +880,13 @@ __device__ __forceinline__ void run_program(const Instr *__restrict__ code, int 
         }
       }
     } else {
-      switch (d) {
-        SR_F_CHEAP
-        default: {
-          float b[DPT];
-          operand(b);
-          apply_op_any<DPT>(instr_op(w), T, b);
-        }
+      if (d != kDNone) {
+        float b[DPT];
+        operand(b);
+        apply_op_any<DPT>(instr_op(w), T, b);
       }
     }
-#undef SR_F_CHEAP
-#undef SR_F_MEM
-#undef SR_F_CONST
-    ins = nxt;
+    if constexpr (!GEN) ins = nxt;
   }
 }
 #undef SR_EACH

@@ -101,27 +101,29 @@ SR_HD bool in_protected_profile(uint32_t op) {
          op == 27;
 }
 
-// Dispatch codes: the frequent operators with the place of operand b folded
-// in (M: memory, a variable row, a spill slot or a cached subtree; C: a
-// constant), so that one branch reaches code that loads the operand and
-// applies the operator.  kDAny: every other combination (operand by kind, then a switch
-// over the opcodes).
+// Dispatch codes: what the interpreter branches on, operator and place of
+// operand b in one (M: memory, a variable row, a spill slot or a cached
+// subtree; C: a constant).  kDLinear: + - * with an operand, one bit for the
+// operator (kDSub, kDRSub, kDMul; none of them adds) and kDConst for a
+// constant operand.  kDAny: every other combination (operand by kind, then a
+// switch over the opcodes).
 enum : uint32_t {
-  kDAny = 0, kDNone, kDAddM, kDSubM, kDRSubM, kDMulM, kDAddC, kDSubC, kDRSubC, kDMulC,
-  kDLDivM, kDRLDivM, kDLDivC, kDRLDivC, kDSin, kDCos, kDExpC, kDLLog, kDLSqrt
+  kDAny = 0, kDNone, kDLDivM, kDRLDivM, kDLDivC, kDRLDivC, kDSin, kDCos, kDExpC, kDLLog, kDLSqrt,
+  kDSub = 1, kDRSub = 2, kDMul = 4, kDConst = 8, kDLinear = 16
 };
 constexpr int kDShift = 18;
 SR_HD uint32_t instr_dispatch(uint32_t w) { return (w >> kDShift) & 31u; }
 SR_HD uint32_t with_dispatch(uint32_t w) {
   const uint32_t bk = instr_b_kind(w);
   const bool m = bk == kBS || bk == kBX || bk == kBR, c = bk == kBC;
+  const uint32_t linear = kDLinear | (c ? kDConst : 0u);
   uint32_t d = kDAny;
   switch (instr_op(w)) {
     case 0: d = kDNone; break;
-    case 1: d = m ? kDAddM : (c ? kDAddC : kDAny); break;
-    case 2: d = m ? kDSubM : (c ? kDSubC : kDAny); break;
-    case kOpReversed + 2: d = m ? kDRSubM : (c ? kDRSubC : kDAny); break;
-    case 3: d = m ? kDMulM : (c ? kDMulC : kDAny); break;
+    case 1: d = m || c ? linear : kDAny; break;
+    case 2: d = m || c ? linear | kDSub : kDAny; break;
+    case kOpReversed + 2: d = m || c ? linear | kDRSub : kDAny; break;
+    case 3: d = m || c ? linear | kDMul : kDAny; break;
     case 8: d = m ? kDLDivM : (c ? kDLDivC : kDAny); break;
     case kOpReversed + 8: d = m ? kDRLDivM : (c ? kDRLDivC : kDAny); break;
     case 10: d = kDSin; break;

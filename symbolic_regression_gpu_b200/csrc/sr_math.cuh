@@ -142,6 +142,90 @@ __device__ __forceinline__ void sincos_parts2(float2 x, SinCosParts &p0, SinCosP
   p0.s = s.x; p1.s = s.y; p0.c = c.x; p1.c = c.y;
 }
 
+// Largest and smallest magnitude of N values (at least 3), two values an
+// instruction; _nan: NaN when one is, otherwise NaNs are passed over.
+__device__ __forceinline__ float max3_abs(float a, float b, float c) {
+  float r;
+  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float min3_abs(float a, float b, float c) {
+  float r;
+  asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float max3_abs_nan(float a, float b, float c) {
+  float r;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+template <int N>
+__device__ __forceinline__ float max_abs(const float (&v)[N]) {
+  float m = max3_abs(v[0], v[1], v[2]);
+#pragma unroll
+  for (int k = 3; k < N; k += 2) m = max3_abs(m, v[k], v[k + 1 < N ? k + 1 : k]);
+  return m;
+}
+template <int N>
+__device__ __forceinline__ float max_abs_nan(const float (&v)[N]) {
+  float m = max3_abs_nan(v[0], v[1], v[2]);
+#pragma unroll
+  for (int k = 3; k < N; k += 2) m = max3_abs_nan(m, v[k], v[k + 1 < N ? k + 1 : k]);
+  return m;
+}
+template <int N>
+__device__ __forceinline__ float min_abs(const float (&v)[N]) {
+  float m = min3_abs(v[0], v[1], v[2]);
+#pragma unroll
+  for (int k = 3; k < N; k += 2) m = min3_abs(m, v[k], v[k + 1 < N ? k + 1 : k]);
+  return m;
+}
+
+// Correctly rounded division and square root of two values at once for
+// arguments of middling magnitude, in paired operations: an approximate
+// reciprocal (reciprocal square root), one Newton step, and exact residuals by
+// fused multiply-add (P. Markstein, IA-64 and Elementary Functions, 2000;
+// J.-M. Muller et al., Handbook of Floating-Point Arithmetic, ch. 4).  Within
+// the ranges below no intermediate over- or underflows, so the last step
+// rounds correctly, as __fdiv_rn and __fsqrt_rn do; every other argument goes to
+// those.  tests/test_gpu_interpreter.py compares them with IEEE results on the
+// quotients closest to a rounding boundary and on every mantissa.
+constexpr float kDivMin = 8.67361738e-19f, kDivMax = 1.15292150e18f;     // 2^-60, 2^60
+constexpr float kSqrtMin = 7.88860905e-31f, kSqrtMax = 1.26765060e30f;   // 2^-100, 2^100
+
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// a / b, |a| and |b| in [kDivMin, kDivMax] (NaN gives NaN).
+__device__ __forceinline__ float2 div2_mid(float2 a, float2 b) {
+  const float2 nb = __fmul2_rn(b, f2(-1.0f));
+  float2 r = make_float2(rcp_approx(b.x), rcp_approx(b.y));
+  r = __ffma2_rn(r, __ffma2_rn(nb, r, f2(1.0f)), r);
+  float2 q = __fmul2_rn(a, r);
+  q = __ffma2_rn(__ffma2_rn(nb, q, a), r, q);
+  return __ffma2_rn(__ffma2_rn(nb, q, a), r, q);
+}
+
+// sqrt(x), x in [kSqrtMin, kSqrtMax] (NaN gives NaN).
+__device__ __forceinline__ float2 sqrt2_mid(float2 x) {
+  const float2 nx = __fmul2_rn(x, f2(-1.0f));
+  const float2 y = make_float2(rsqrt_approx(x.x), rsqrt_approx(x.y));
+  float2 g = __fmul2_rn(x, y);          // sqrt x
+  float2 nh = __fmul2_rn(y, f2(-0.5f)); // -1 / (2 sqrt x)
+  const float2 e = __ffma2_rn(nh, g, f2(0.5f));
+  g = __ffma2_rn(g, e, g);
+  nh = __ffma2_rn(nh, e, nh);
+  return __ffma2_rn(__ffma2_rn(g, g, nx), nh, g);
+}
+
 // log(1 + f) = f + f^2 (-1/2 + f R(f)), R(f) = kR0 + f (kR1 + ... f kR7)
 constexpr float kR0 = 0.333333317078f;
 constexpr float kR1 = -0.250008210321f;
@@ -205,6 +289,31 @@ __device__ __forceinline__ float2 sr_log_nonneg2(float a0, float a1) {
       (a0 == 0.0f) ? __int_as_float(0xff800000) : (a0 < INFINITY ? r.x : a0),
       (a1 == 0.0f) ? __int_as_float(0xff800000) : (a1 < INFINITY ? r.y : a1));
 }
+
+// The same for two positive normal arguments: no scaling, no special cases
+// (the exponent becomes a float by adding it to the low bits of 1.5 * 2^23).
+__device__ __forceinline__ float2 sr_log_normal2(float a0, float a1) {
+  const int ia0 = __float_as_int(a0), ia1 = __float_as_int(a1);
+  const int k0 = ia0 - 0x3f3504f3, k1 = ia1 - 0x3f3504f3;
+  const float2 m = make_float2(__int_as_float(ia0 - (k0 & 0xff800000)),
+                               __int_as_float(ia1 - (k1 & 0xff800000)));
+  const float2 f = __fadd2_rn(m, f2(-1.0f));
+  const int magic = __float_as_int(kRoundMagic);
+  const float2 ef = __fadd2_rn(make_float2(__int_as_float((k0 >> 23) + magic),
+                                           __int_as_float((k1 >> 23) + magic)),
+                               f2(-kRoundMagic));
+  float2 p = __ffma2_rn(f2(kR7), f, f2(kR6));
+  p = __ffma2_rn(p, f, f2(kR5));
+  p = __ffma2_rn(p, f, f2(kR4));
+  p = __ffma2_rn(p, f, f2(kR3));
+  p = __ffma2_rn(p, f, f2(kR2));
+  p = __ffma2_rn(p, f, f2(kR1));
+  p = __ffma2_rn(p, f, f2(kR0));
+  p = __ffma2_rn(p, f, f2(-0.5f));
+  const float2 y = __ffma2_rn(__fmul2_rn(f, f), p, f);
+  return __ffma2_rn(ef, f2(kLn2Hi), __ffma2_rn(ef, f2(kLn2Lo), y));
+}
+constexpr float kMinNormal = 1.17549435e-38f;
 
 // logf semantics: NaN for negative arguments.
 __device__ __forceinline__ float sr_logf(float x) {

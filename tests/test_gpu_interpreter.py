@@ -98,3 +98,88 @@ def test_mse_is_the_mean_of_the_predictions_squares(n, opts):
             _agree(np.where(cnt > 0, s / cnt, np.nan).astype(np.float32), want)
         _agree(ev.eval_mse(pop, cache=True, clear_cache=True), want)
         _agree(ev.eval_grad(pop)[0], want)
+
+
+def _hard_quotients(r):
+    """(a, b) whose quotient lies r / (b 2^24) (a >= b) or r / (b 2^25) (a < b)
+    from the middle between two floats, for every odd 24-bit b: a 2^24 = r
+    (mod b) by halving r 24 (25) times modulo b."""
+    b = np.arange((1 << 23) + 1, 1 << 24, 2, dtype=np.int64)
+    x = np.full(b.shape, r, np.int64) % b
+    out = []
+    for k in range(25):
+        x = np.where(x % 2 == 0, x // 2, (x + b) // 2)
+        if k == 23:
+            a = x + b
+            ok = a < (1 << 24)
+            out.append((a[ok], b[ok]))
+    ok = (x >= (1 << 23)) & (x < b)
+    out.append((x[ok], b[ok]))
+    return (np.concatenate([o[0] for o in out]).astype(np.float32),
+            np.concatenate([o[1] for o in out]).astype(np.float32))
+
+
+def _zero_error(exprs, X, n_valid=None):
+    """Every prediction equals the target bit for bit: the sum of squares is 0
+    over all datapoints."""
+    with sg.Evaluator(device=0) as ev:
+        ev.set_data(X)
+        mse = ev.eval_mse(sg.Population.from_lists(exprs))
+        s, n = ev.read_sums()
+    assert np.all(n == (X.shape[1] if n_valid is None else n_valid))
+    assert np.all(s == 0.0) and np.all(mse == 0.0)
+
+
+_DIV = [([op.LOOSE_DIV, -1, -1], [0.0, 0.0, 1.0]),
+        # the accumulator as the divisor and as the dividend, products that are exact
+        ([op.LOOSE_DIV, -1, op.MUL, -1, 0], [0.0, 0.0, 0.0, 1.0, 1.0]),
+        ([op.LOOSE_DIV, op.MUL, -1, 0, -1], [0.0, 0.0, 0.0, 1.0, 1.0])]
+
+
+@pytest.mark.parametrize("r", [1, -1, 3, -5])
+def test_division_rounds_correctly_next_to_the_midpoints(r):
+    a, b = _hard_quotients(r)
+    assert a.size > 1_000_000
+    _zero_error(_DIV, np.stack([a, b, a / b]))
+
+
+@pytest.mark.parametrize("lo,hi", [(-60, 60), (-126, 127), (-149, 20), (-61, -59), (59, 61)])
+def test_division_rounds_correctly_over_its_range(lo, hi):
+    rng = np.random.default_rng(abs(hi))
+    n = 1_500_001
+    with np.errstate(all="ignore"):
+        a, b = (np.ldexp(rng.uniform(1, 2, n), rng.integers(lo, hi + 1, n)).astype(np.float32)
+                * rng.choice([-1, 1], n).astype(np.float32) for _ in range(2))
+        a[::1001] = 0.0
+        b[::1013] = -0.0
+        d = np.where(np.abs(b) <= np.float32(1e-9),
+                     np.where(b < 0, np.float32(-1e-9), np.float32(1e-9)), b).astype(np.float32)
+        y = a / d
+    keep = np.isfinite(y) & (np.abs(y) < 1e19)
+    a, b, y = a[keep], b[keep], y[keep]
+    _zero_error(_DIV, np.stack([a, b, y]))
+
+
+@pytest.mark.parametrize("case", ["mantissas", "range"])
+def test_square_root_rounds_correctly(case):
+    if case == "mantissas":  # every one, both parities of the exponent
+        x = np.arange(0x3F800000, 0x40800000, dtype=np.uint32).view(np.float32)
+    else:
+        rng = np.random.default_rng(3)
+        x = rng.integers(0, 0x7F800000, 3_000_001, dtype=np.int64).astype(np.uint32).view(np.float32)
+        x[:4] = [0.0, 1e-45, 1.17549435e-38, 3.4e38]
+    x = x * np.where(np.arange(x.size) % 3 == 0, np.float32(-1), np.float32(1))
+    _zero_error([([op.LOOSE_SQRT, -1], [0.0, 0.0])], np.stack([x, np.sqrt(np.abs(x))]))
+
+
+def test_protected_log_is_the_same_in_every_path():
+    """log|x| of the MSE launch against the prediction launch's (scalar form)."""
+    rng = np.random.default_rng(4)
+    x = rng.integers(0, 0x7F800000, 4_000_003, dtype=np.int64).astype(np.uint32).view(np.float32)
+    x[:6] = [0.0, -0.0, 1e-45, 1.17549435e-38, 1.1754942e-38, 3.4028235e38]
+    x[1::2] *= -1
+    pop = sg.Population.from_lists([([op.LOOSE_LOG, -1], [0.0, 0.0])])
+    with sg.Evaluator(device=0) as ev:
+        ev.set_data(np.stack([x, x]))
+        y = ev.predictions(pop)[0]
+    _zero_error([([op.LOOSE_LOG, -1], [0.0, 0.0])], np.stack([x, y]))
