@@ -142,7 +142,7 @@ __device__ __forceinline__ void sincos_parts2(float2 x, SinCosParts &p0, SinCosP
   p0.s = s.x; p1.s = s.y; p0.c = c.x; p1.c = c.y;
 }
 
-// Largest and smallest magnitude of N values (at least 3), two values an
+// Largest and smallest magnitude of N values (at least 2), two values an
 // instruction; _nan: NaN when one is, otherwise NaNs are passed over.
 __device__ __forceinline__ float max3_abs(float a, float b, float c) {
   float r;
@@ -161,21 +161,21 @@ __device__ __forceinline__ float max3_abs_nan(float a, float b, float c) {
 }
 template <int N>
 __device__ __forceinline__ float max_abs(const float (&v)[N]) {
-  float m = max3_abs(v[0], v[1], v[2]);
+  float m = max3_abs(v[0], v[1], v[N > 2 ? 2 : 1]);
 #pragma unroll
   for (int k = 3; k < N; k += 2) m = max3_abs(m, v[k], v[k + 1 < N ? k + 1 : k]);
   return m;
 }
 template <int N>
 __device__ __forceinline__ float max_abs_nan(const float (&v)[N]) {
-  float m = max3_abs_nan(v[0], v[1], v[2]);
+  float m = max3_abs_nan(v[0], v[1], v[N > 2 ? 2 : 1]);
 #pragma unroll
   for (int k = 3; k < N; k += 2) m = max3_abs_nan(m, v[k], v[k + 1 < N ? k + 1 : k]);
   return m;
 }
 template <int N>
 __device__ __forceinline__ float min_abs(const float (&v)[N]) {
-  float m = min3_abs(v[0], v[1], v[2]);
+  float m = min3_abs(v[0], v[1], v[N > 2 ? 2 : 1]);
 #pragma unroll
   for (int k = 3; k < N; k += 2) m = min3_abs(m, v[k], v[k + 1 < N ? k + 1 : k]);
   return m;
@@ -212,6 +212,15 @@ __device__ __forceinline__ float2 div2_mid(float2 a, float2 b) {
   float2 q = __fmul2_rn(a, r);
   q = __ffma2_rn(__ffma2_rn(nb, q, a), r, q);
   return __ffma2_rn(__ffma2_rn(nb, q, a), r, q);
+}
+
+// 1 / b, |b| in [kDivMin, kDivMax] (NaN gives NaN).
+__device__ __forceinline__ float2 rcp2_mid(float2 b) {
+  const float2 nb = __fmul2_rn(b, f2(-1.0f));
+  float2 r = make_float2(rcp_approx(b.x), rcp_approx(b.y));
+  r = __ffma2_rn(r, __ffma2_rn(nb, r, f2(1.0f)), r);
+  const float2 q = __ffma2_rn(__ffma2_rn(nb, r, f2(1.0f)), r, r);
+  return __ffma2_rn(__ffma2_rn(nb, q, f2(1.0f)), r, q);
 }
 
 // sqrt(x), x in [kSqrtMin, kSqrtMax] (NaN gives NaN).

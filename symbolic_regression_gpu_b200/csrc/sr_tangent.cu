@@ -100,6 +100,61 @@ __device__ __noinline__ void tan_sincos_cold(float *T, float *dT, int q_offset) 
   }
 }
 
+// Division and reciprocal, two datapoints at a time where the lane's arguments
+// are of middling magnitude, one by one out of line elsewhere: one short copy
+// of each in the kernel's hot code (its instruction-cache misses were its second
+// stall).
+template <int DPT>
+__device__ __noinline__ void div_cold(float *T, const float *b) {
+#pragma unroll
+  for (int k = 0; k < DPT; ++k) T[k] = __fdiv_rn(T[k], b[k]);
+}
+template <int DPT>
+__device__ __noinline__ void rcp_cold(const float *b, float *r) {
+#pragma unroll
+  for (int k = 0; k < DPT; ++k) r[k] = __frcp_rn(b[k]);
+}
+template <int DPT>
+__device__ __forceinline__ void div_wide(float (&T)[DPT], const float (&b)[DPT]) {
+  if (fmaxf(max_abs<DPT>(T), max_abs<DPT>(b)) <= kDivMax &&
+      min_abs<DPT>(T) >= kDivMin && min_abs<DPT>(b) >= kDivMin) {
+#pragma unroll
+    for (int k = 0; k < DPT; k += 2) {
+      const float2 r = div2_mid(make_float2(T[k], T[k + 1]), make_float2(b[k], b[k + 1]));
+      T[k] = r.x;
+      T[k + 1] = r.y;
+    }
+  } else {
+    float t[DPT], u[DPT];
+#pragma unroll
+    for (int k = 0; k < DPT; ++k) {
+      t[k] = T[k];
+      u[k] = b[k];
+    }
+    div_cold<DPT>(t, u);
+#pragma unroll
+    for (int k = 0; k < DPT; ++k) T[k] = t[k];
+  }
+}
+template <int DPT>
+__device__ __forceinline__ void rcp_wide(const float (&b)[DPT], float (&r)[DPT]) {
+  if (max_abs<DPT>(b) <= kDivMax && min_abs<DPT>(b) >= kDivMin) {
+#pragma unroll
+    for (int k = 0; k < DPT; k += 2) {
+      const float2 q = rcp2_mid(make_float2(b[k], b[k + 1]));
+      r[k] = q.x;
+      r[k + 1] = q.y;
+    }
+  } else {
+    float u[DPT], q[DPT];
+#pragma unroll
+    for (int k = 0; k < DPT; ++k) u[k] = b[k];
+    rcp_cold<DPT>(u, q);
+#pragma unroll
+    for (int k = 0; k < DPT; ++k) r[k] = q[k];
+  }
+}
+
 // T = op(T, b) with the partials the tangent update needs (only when `live`:
 // instructions off every constant's path skip them).  dk / bk_: how dT / db
 // are known.  The IEEE divisions and reciprocals of the protected division
@@ -185,10 +240,7 @@ __device__ __forceinline__ void tan_apply(uint32_t op, bool live, float (&T)[DPT
     case 10:
     case 11: {
       const int qoff = (op == 11) ? 1 : 0;
-      bool slow = false;
-#pragma unroll
-      for (int k = 0; k < DPT; ++k) slow |= !sincos_fast_ok(T[k]);
-      if (slow) {
+      if (!(max_abs<DPT>(T) <= kSinCosFastMax)) {
         float t_[DPT], d_[DPT];
 #pragma unroll
         for (int k = 0; k < DPT; ++k) t_[k] = T[k];
@@ -226,24 +278,19 @@ __device__ __forceinline__ void tan_apply(uint32_t op, bool live, float (&T)[DPT
       break;
     case 22:  // protected log: -1e9 at 0, else log|x|; derivative 0 at 0, else 1/x
 #pragma unroll
-      for (int k = 0; k < DPT; k += 2) {
-        const float x0 = T[k], x1 = T[k + 1];
-        const float2 l = sr_log_nonneg2(fabsf(x0), fabsf(x1));
-        b[k] = x0;
-        b[k + 1] = x1;
-        T[k] = x0 == 0.0f ? -1e9f : l.x;
-        T[k + 1] = x1 == 0.0f ? -1e9f : l.y;
-      }
+      for (int k = 0; k < DPT; ++k) b[k] = T[k];
+      llog_wide<DPT>(T);
       post = 2;
       break;
     case 27:  // sqrt|x|: derivative 0 at 0, else sign(x) / (2 out)
 #pragma unroll
+      for (int k = 0; k < DPT; ++k) dT[k] = T[k];
+      lsqrt_wide<DPT>(T);
+#pragma unroll
       for (int k = 0; k < DPT; ++k) {
-        const float x = T[k];
-        const float o = __fsqrt_rn(fabsf(x));
-        b[k] = x == 0.0f ? 1.0f : 2.0f * o;  // at 0: sign 0 times 1
-        dT[k] = signf(x);                     // times 1 / (2 out) below
-        T[k] = o;
+        const float x = dT[k];
+        b[k] = x == 0.0f ? 1.0f : 2.0f * T[k];  // at 0: sign 0 times 1
+        dT[k] = signf(x);                        // times 1 / (2 out) below
       }
       post = 2;
       break;
@@ -270,14 +317,10 @@ __device__ __forceinline__ void tan_apply(uint32_t op, bool live, float (&T)[DPT
       break;
     }
   }
-  if (post & 1) {
-#pragma unroll
-    for (int k = 0; k < DPT; ++k) T[k] = __fdiv_rn(T[k], b[k]);
-  }
+  if (post & 1) div_wide<DPT>(T, b);
   if ((post & 2) && live) {
     float rc[DPT];
-#pragma unroll
-    for (int k = 0; k < DPT; ++k) rc[k] = __frcp_rn(b[k]);
+    rcp_wide<DPT>(b, rc);
     // Partials from the reciprocal (the reverse-mode routines' formulas).
     if (op == 8) {  // d/dT = 1/den, d/db = -out/den (0 in the flat region)
 #pragma unroll

@@ -183,3 +183,21 @@ def test_protected_log_is_the_same_in_every_path():
         ev.set_data(np.stack([x, x]))
         y = ev.predictions(pop)[0]
     _zero_error([([op.LOOSE_LOG, -1], [0.0, 0.0])], np.stack([x, y]))
+
+
+def test_reciprocals_of_the_gradient_round_correctly():
+    """d/dc of c / (k x) at c = x = 1, y = 0, one datapoint: the FP32 product of
+    the seed 2 / k and the partial 1 / k, both of which are correctly rounded."""
+    rng = np.random.default_rng(6)
+    n = 60_000
+    k = np.ldexp(rng.uniform(1, 2, n), rng.integers(-62, 63, n)).astype(np.float32)
+    k[:2000] = (0x3FFFFFFF - np.arange(2000)).astype(np.uint32).view(np.float32)  # just below 2
+    k[2000:4000] = (0x3F800000 + np.arange(2000)).astype(np.uint32).view(np.float32)
+    k = k[np.abs(k) > 1e-9]
+    pop = sg.Population.from_lists([([op.LOOSE_DIV, 0, op.MUL, 0, -1], [0.0, 1.0, 0.0, float(v), 0.0])
+                                    for v in k])
+    with sg.Evaluator(device=0) as ev:
+        ev.set_data(np.array([[1.0], [0.0]], np.float32))
+        _, grad = ev.eval_grad(pop)
+    r = np.float32(1) / k
+    assert np.array_equal(grad[::2], (np.float32(2) * r) * r)
