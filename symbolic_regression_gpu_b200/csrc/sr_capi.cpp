@@ -91,8 +91,8 @@ sr_status check_population(sr_context *ctx, const sr_population *pop) {
 
 // Compile expressions [0, E) of a CSR population into ps (pinned staging).
 // With `share` equal expressions are compiled once and folded subtrees and
-// derived rows collapse to leaves; fold_constants (gradient programs) folds
-// constant subtrees alone.  Folded subtrees, there and under kHintFold hints,
+// derived rows collapse to leaves; fold_constants (gradient and cached programs)
+// folds constant subtrees alone.  Folded subtrees, there and under kHintFold hints,
 // are added to ctx->folds.
 sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *val,
                       const int64_t *off, const int32_t *hints, ProgramSet &ps,
@@ -144,8 +144,10 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
           continue;
         }
       }
-      if (fold_constants && sr::mark_constant_subtrees(tok + off[x], len, marks.data()))
+      if (fold_constants && sr::mark_constant_subtrees(tok + off[x], len, marks.data())) {
+        if (h) sr::merge_hints(h, len, marks.data());
         h = marks.data();
+      }
       const int64_t i0 = static_cast<int64_t>(c.code.size());
       refs.clear();
       const sr_status s = sr::compile_expression(tok + off[x], val + off[x], len, ctx->V, h, c.code,
@@ -257,14 +259,16 @@ static sr_status upload_folds(sr_context *ctx) {
   return SR_OK;
 }
 
-// Derived rows of a population, at most: 23 rows of 512-datapoint spans, twice
-// buffered, fit in shared memory beside four spill slots for each of 31 warps.
-// More rows leave 256-datapoint spans, whose items cost what the rows save
-// (batched population, interpreter: none 42.9 ms, 16 rows 37.7, 32 rows at 256
-// datapoints 37.5; 24 rows with two spill slots, deeper ones in global scratch,
-// 46.9).  A bounded part of the device's memory too.
-static int derived_row_limit(const sr_context *ctx) {
-  int r = std::min(16, 22 - ctx->V);
+// Derived rows of a population whose programs spill at most `slots` values, at
+// most: what 512-datapoint spans, twice buffered, leave of shared memory beside
+// the spill slots of 31 warps (31 KB a slot) and the span sums.  More rows leave
+// 256-datapoint spans, whose items cost what the rows save (batched population,
+// interpreter at the time: no rows 42.9 ms, 16 rows 37.7, 32 rows at 256
+// datapoints 37.5; 24 rows with two of the three spill slots it needs, the other
+// in global scratch, 46.9).  A bounded part of the device's memory too.
+static int derived_row_limit(const sr_context *ctx, int slots) {
+  const int fit = (ctx->max_smem - 9 * 1024 - slots * 31 * 1024) / 4096;
+  int r = std::min(24, fit - (ctx->V + 1));
   const double row = static_cast<double>(ctx->ldx) * sizeof(float);
   const double room = std::min(1073741824.0, static_cast<double>(ctx->device_memory) / 16.0);
   r = std::min(r, static_cast<int>(room / row));
@@ -290,7 +294,7 @@ static sr_status prepare_batched(sr_context *ctx, const sr_population *pop) {
   bool share = sharing_pays(ctx, pop);
   if (share) {
     SR_TRACE("sr: share");
-    share = sh.find(E, pop->tokens, pop->values, pop->offsets, derived_row_limit(ctx),
+    share = sh.find(E, pop->tokens, pop->values, pop->offsets, derived_row_limit(ctx, 3),
                     ctx->workers, host_threads(ctx));
     // Rows are an option: without the memory for them they are evaluated in
     // place like everything else.
@@ -302,6 +306,14 @@ static sr_status prepare_batched(sr_context *ctx, const sr_population *pop) {
   }
   SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, nullptr, ctx->main,
                      share ? &sh : nullptr));
+  // Programs of long expressions can need a fourth spill slot: fewer rows then.
+  if (share && ctx->main.smax > 3 &&
+      static_cast<int>(sh.rows().size()) > derived_row_limit(ctx, 4)) {
+    sh.keep_rows(derived_row_limit(ctx, 4));
+    ctx->folds.refs.clear();
+    ctx->folds.tokens.clear();
+    SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, nullptr, ctx->main, &sh));
+  }
   if (share && !sh.rows().empty()) {
     std::vector<int32_t> tok, hints;
     std::vector<double> val;
@@ -1291,7 +1303,10 @@ sr_status prepare_cached(sr_context *ctx, const sr_population *pop, uint32_t fla
 
   // Subtrees to evaluate into the cache this call.
   const double tc0 = now_ms();
-  SR_TRY(compile_set(ctx, n_new, sub_tok.data(), sub_val.data(), sub_off.data(), nullptr, ctx->sub));
+  // Constant subtrees are folded in both sets (a cached one too, where it lies in
+  // a larger subtree of constants or is one: a constant costs no load).
+  SR_TRY(compile_set(ctx, n_new, sub_tok.data(), sub_val.data(), sub_off.data(), nullptr, ctx->sub,
+                     nullptr, true));
   for (int k = 0; k < n_new; ++k) ctx->sub.h_row.p[k] = sub_slot[static_cast<size_t>(k)];
   if (n_new > 0) {
     SR_TRY(plan_set(ctx, ctx->sub, true, 8, sr::kMaxWarps));
@@ -1305,7 +1320,8 @@ sr_status prepare_cached(sr_context *ctx, const sr_population *pop, uint32_t fla
   ctx->hints.resize(static_cast<size_t>(T));
   const int64_t removed = sr::mark_cached_subtrees(E, pop->tokens, pop->values, pop->offsets,
                                                    ctx->cache, threads, ctx->hints.data());
-  SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, ctx->hints.data(), ctx->main));
+  SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, ctx->hints.data(), ctx->main,
+                     nullptr, true));
   ctx->prep_stats.host_compile_time_ms = now_ms() - tc0;
   SR_TRY(prepare_main_shape(ctx, false, false));
   ctx->prep_stats.node_evals = T * ctx->N;

@@ -1092,10 +1092,14 @@ __device__ __noinline__ void run_producer(int lane, int n_groups, int n_items, i
     if (armed & 2u) mbar_drain(&full[1], fill_phase[1]);
   };
 
-  for (;;) {
-    int item = 0;
-    if (lane == 0) item = atomicAdd(work_counter, 1);
-    item = __shfl_sync(0xffffffffu, item, 0);
+  // A block's first item is its own index; the counter hands out the rest (none
+  // when there is a block for every item).
+  for (bool first = true;; first = false) {
+    int item = first ? static_cast<int>(blockIdx.x) : n_items;
+    if (!first && n_items > static_cast<int>(gridDim.x)) {
+      if (lane == 0) item = atomicAdd(work_counter, 1) + static_cast<int>(gridDim.x);
+      item = __shfl_sync(0xffffffffu, item, 0);
+    }
     const bool last = item >= n_items;
     const int n_sg = (n_spans + k_spans - 1) / k_spans;
     const int group = last ? 0 : item / n_sg;

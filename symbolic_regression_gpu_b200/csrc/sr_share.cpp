@@ -88,6 +88,20 @@ bool mark_constant_subtrees(const int32_t *tok, int len, int32_t *hints) {
   return any;
 }
 
+void merge_hints(const int32_t *hints, int len, int32_t *marks) {
+  for (int i = 0; i < len;) {
+    if (marks[i] == kHintFold) {  // over whatever is cached inside
+      for (++i; i < len && marks[i] == -2; ++i) {
+      }
+    } else if (hints[i] >= 0) {   // over whatever would be folded inside
+      marks[i] = hints[i];
+      for (++i; i < len && hints[i] == -2; ++i) marks[i] = -2;
+    } else {
+      ++i;
+    }
+  }
+}
+
 // A worker's own counts of the subtrees it met last: the frequent ones (sin x0)
 // would otherwise have every worker add to the same few words.
 struct Sharing::Local {
@@ -264,12 +278,8 @@ void Sharing::choose(std::vector<uint32_t> &frequent, int max_rows) {
       break;
     best->taken = true;
     const int r = static_cast<int>(rows_.size());
-    max_row_size_ = std::max(max_row_size_, best->n);
     rows_.push_back(Row{best->at, best->n, static_cast<int32_t>(best->occ)});
-    size_t slot = best->key & 255;
-    while (row_key_[slot] != 0) slot = (slot + 1) & 255;
-    row_key_[slot] = best->key;
-    row_of_[slot] = static_cast<int16_t>(r);
+    enter_row(best->key, r);
     const auto is_row = [&](uint64_t key) {
       for (size_t i = key & 255; row_key_[i] != 0; i = (i + 1) & 255)
         if (row_key_[i] == key) return true;
@@ -300,10 +310,20 @@ void Sharing::choose(std::vector<uint32_t> &frequent, int max_rows) {
   }
 }
 
-void Sharing::drop_rows() {
-  rows_.clear();
+void Sharing::enter_row(uint64_t key, int r) {
+  size_t slot = key & 255;
+  while (row_key_[slot] != 0) slot = (slot + 1) & 255;
+  row_key_[slot] = key;
+  row_of_[slot] = static_cast<int16_t>(r);
+  max_row_size_ = std::max(max_row_size_, rows_[static_cast<size_t>(r)].size);
+}
+
+void Sharing::keep_rows(int n) {
+  if (static_cast<int>(rows_.size()) > n) rows_.resize(static_cast<size_t>(n));
   max_row_size_ = 0;
   std::memset(row_key_, 0, sizeof row_key_);
+  for (size_t r = 0; r < rows_.size(); ++r)
+    enter_row(hash_[static_cast<size_t>(rows_[r].tok)], static_cast<int>(r));
 }
 
 bool Sharing::find(int E, const int32_t *tok, const double *val, const int64_t *off, int max_rows,

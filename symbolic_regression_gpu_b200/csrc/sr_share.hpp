@@ -36,6 +36,10 @@ constexpr int kMaxSharedTokens = 64;   // largest subtree folded or made a row
 // whether there is one, false as well for a malformed expression.
 bool mark_constant_subtrees(const int32_t *tok, int len, int32_t *hints);
 
+// Adds an expression's cache hints to its fold marks: cached subtrees outside
+// the folded ones stay collapsed.
+void merge_hints(const int32_t *hints, int len, int32_t *marks);
+
 class Sharing {
  public:
   struct Row {
@@ -58,7 +62,9 @@ class Sharing {
   int rep(int x) const;
 
   const std::vector<Row> &rows() const { return rows_; }
-  void drop_rows();
+  void drop_rows() { keep_rows(0); }
+  // The first n rows only (the most saving ones).
+  void keep_rows(int n);
 
  private:
   struct Entry {
@@ -85,6 +91,7 @@ class Sharing {
   size_t cap_ = 0, mask_ = 0;
   std::vector<Row> rows_;
   int max_row_size_ = 0;
+  void enter_row(uint64_t key, int r);
   uint64_t row_key_[256];        // open-addressed set of the rows' hashes
   int16_t row_of_[256];
 };
