@@ -15,7 +15,8 @@
 //                          prefix -> bytecode translation (Sethi-Ullman
 //                          evaluation order, leaf operands folded, reversed
 //                          opcodes, spill slots), so a population bred on the
-//                          device is evaluated without a host round trip.
+//                          device is evaluated without a host round trip;
+//                          subtrees of constants become one constant.
 //
 // Random numbers: every child draws from its own counter-based stream (a
 // SplitMix64 sequence seeded from (seed, generation, child)), so a step is
@@ -32,6 +33,7 @@
 #include "sr_eval.h"
 #include "sr_evolve.hpp"
 #include "sr_internal.hpp"
+#include "sr_ops.cuh"
 
 namespace sr {
 namespace {
@@ -420,6 +422,15 @@ __device__ int compile_one(const int32_t *tok, const float *val, int len, int nu
       nd.op = t;
       nd.left = stk[--ns];
       if (is_binary_token(t)) nd.right = stk[--ns];
+      // Constants only: the value now, with the operators every kernel
+      // evaluates, instead of at every datapoint.
+      const DNode &l = nodes[nd.left];
+      const DNode &r = nodes[nd.right < 0 ? nd.left : nd.right];
+      if (l.op < 0 && l.lk == kLeafC && r.op < 0 && r.lk == kLeafC) {
+        nd.op = -1;
+        nd.lp = __float_as_uint(op_apply(t, __uint_as_float(l.lp), __uint_as_float(r.lp)));
+        nd.left = nd.right = -1;
+      }
     }
     nodes[nn] = nd;
     stk[ns++] = static_cast<int16_t>(nn);

@@ -91,3 +91,28 @@ def test_shared_work_changes_no_result(V, N, every):
         assert np.array_equal(np.where(n > 0, s / n, np.nan).astype(np.float32), got, equal_nan=True)
     for other in (again, launched, graphed):
         assert np.array_equal(other, got, equal_nan=True)
+
+
+def test_device_populations_fold_constants_to_the_same_values():
+    """The device compiler evaluates subtrees of constants; the host's small
+    launches evaluate them at every datapoint."""
+    from symbolic_regression_gpu_b200.evolution import DeviceEvolution, evolve_options
+
+    V, N = 3, 5003
+    pop = _population(77, 800, V, True)
+    keep = [i for i in range(pop.num_exprs) if pop.offsets[i + 1] - pop.offsets[i] <= 120]
+    pop = pop.subset(keep)
+    X = np.random.default_rng(7).uniform(-3.0, 3.0, (V + 1, N)).astype(np.float32)
+    assert pop.num_tokens * N < 1e9  # nothing shared on the host's side
+    with sg.Evaluator(device=0) as ev:
+        ev.set_data(X)
+        want = ev.eval_mse(pop)
+        de = DeviceEvolution(ev, pop.num_exprs, evolve_options(V, seed=1), stride=130)
+        de.load(pop)
+        de.evaluate()
+        got = de.fitness()
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(np.isinf(got), np.isinf(want))
+    f = np.isfinite(want)
+    ulp = np.abs(got[f].view(np.int32).astype(np.int64) - want[f].view(np.int32).astype(np.int64))
+    assert ulp.max() <= 1
