@@ -275,13 +275,18 @@ static int derived_row_limit(const sr_context *ctx, int slots) {
   return r < 4 ? 0 : std::min(r, sr::kMaxDerivedRows);
 }
 
-// Whether finding shared work pays: the search and the two more kernels cost
-// 0.1 to 0.2 ms of a call at 15,000 tokens and 0.8 ms at 170,000, and the
-// evaluation, 0.3 ms per 1e9 tokens x datapoints, becomes a fifth to a third
-// shorter (1,000 ramped trees x 100k, 1.5e9: 811 -> 770 us a call; 1,531 bred
-// trees x 250k, 6.9e9: 2.40 -> 2.34 ms; 10,000 x 1M, 1.7e11: 49.8 -> 39.8 ms).
+// Whether finding shared work pays.  The search and the two more kernels cost
+// about 0.15 ms and 4 ns a token; the evaluation, 0.28 ms per 1e9 tokens x
+// datapoints, becomes a quarter shorter, 0.07 ps a token and datapoint: even at
+// 60,000 datapoints for the tokens' part, and 3e9 leaves room for the rest.
+// A call without and with it, us:
+//   1,000 ramped trees x 100k    660 / 750       1,500 bred x 200k   1,689 / 1,629
+//   500 ramped x 400k          1,017 / 1,080     5,000 bred x 100k   2,941 / 2,876
+//   1,500 ramped x 200k        1,465 / 1,460     1,500 bred x 400k   3,113 / 2,697
+//   500 long x 200k            1,039 / 1,034     5,000 long x 200k   8,990 / 7,440
 static bool sharing_pays(const sr_context *ctx, const sr_population *pop) {
-  return static_cast<double>(pop->offsets[pop->num_exprs]) * static_cast<double>(ctx->N) >= 1e9;
+  const double tokens = static_cast<double>(pop->offsets[pop->num_exprs]);
+  return tokens * (static_cast<double>(ctx->N) - 60000.0) >= 3e9;
 }
 
 // Batched programs: shared work found and taken out where that pays, then
