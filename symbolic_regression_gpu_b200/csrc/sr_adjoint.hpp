@@ -26,16 +26,15 @@ struct AdjArgs {
 };
 
 // Forward-mode (tangent) launch: the expressions with at most
-// kMaxTangentConsts constants.  Per instruction one mask word: bits 0..7 A
-// (constants under the accumulator before the operator), 8..15 B (constants
-// under the operand b), bit 24 set when the instruction loads a constant leaf
-// (its bit in A).
+// kMaxTangentConsts constants.  Per instruction one mask word, in Instr.c: bits
+// 0..7 A (constants under the accumulator before the operator), 8..15 B
+// (constants under the operand b), bit 24 set when the instruction loads a
+// constant leaf (its bits in A).
 constexpr int kMaxTangentConsts = 8;
 constexpr uint32_t kTanLoadConst = 1u << 24;
 
 struct TanArgs {
   EvalArgs e;                 // forward part (dataset, programs, group table, spans, MSE sums)
-  const uint32_t *tmask;      // [instructions + 1] mask words, aligned with the code
   const int64_t *const_off;   // [E] first constant (global index) of each expression
   const int32_t *const_cnt;   // [E] constants of each expression
   const float *tinit;         // [C] tangent a constant enters with

@@ -33,17 +33,17 @@ constexpr int kMaxAdjConsts = 64;  // constants per expression with a gradient
 constexpr int kTanWidths[] = {4, sr::kMaxTangentConsts};
 constexpr int kNumTanWidths = 2;
 
-// Mask words of one program for the forward-mode kernel (TanArgs::tmask):
-// the constants (token-order indices, all below kMaxTangentConsts here) under
+// Mask words of one program for the forward-mode kernel, in place of the constant
+// indices (Instr.c), which it does not read: the constants (token-order indices, all below kMaxTangentConsts here) under
 // the accumulator before each operator (A) and under its operand b (B), and
 // the constant-load flag.
 // A folded constant subtree enters with all its constants (fold_n: their number,
 // per instruction leaf A and operand b).
-void tangent_masks(const Instr *code, int len, const uint8_t *fold_n, uint32_t *out) {
+void tangent_masks(Instr *code, int len, const uint8_t *fold_n) {
   uint32_t mT = 0;
   uint32_t mS[32] = {};
   for (int i = 0; i < len; ++i) {
-    const Instr &in = code[i];
+    Instr &in = code[i];
     if (sr::instr_spill(in.w)) mS[sr::instr_spill_slot(in.w) & 31u] = mT;
     uint32_t A = mT, L = 0;
     if (sr::instr_load(in.w)) {
@@ -59,7 +59,7 @@ void tangent_masks(const Instr *code, int len, const uint8_t *fold_n, uint32_t *
       B = (((1u << ((in.c & sr::kFoldB) ? fold_n[2 * i + 1] : 1)) - 1u) << cb) & 0xFFu;
     if (bk == sr::kBS) B = mS[in.b & 31u];
     mT = A | B;
-    out[i] = A | (B << 8) | L;
+    in.c = A | (B << 8) | L;
   }
 }
 
@@ -98,7 +98,6 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
                        : (in.c & ~0x3FFu) | c0 | sr::kFoldA;
     fold_n[static_cast<size_t>(f.loc)] = static_cast<uint8_t>(f.nc);
   }
-  SR_TRY(upload_set(ctx, ps, false));
   // Constants: CSR offsets and the bytecode word that holds each one.
   SR_TRY_CUDA(ctx, g.h_const_off.ensure(static_cast<size_t>(E) + 1));
   SR_TRY_CUDA(ctx, g.h_const_cnt.ensure(static_cast<size_t>(std::max(E, 1))));
@@ -153,12 +152,10 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
       rev_members.push_back(x);
   }
   g.n_rev = static_cast<int>(rev_members.size());
-  SR_TRY_CUDA(ctx, g.h_tmask.ensure(static_cast<size_t>(ps.n_instr) + 1));
-  std::memset(g.h_tmask.p, 0, (static_cast<size_t>(ps.n_instr) + 1) * sizeof(uint32_t));
   for (const auto &mem : tan_members)
     for (int32_t x : mem)
-      tangent_masks(ps.h_code.p + ps.h_off.p[x], ps.h_len.p[x], fold_n.data() + 2 * ps.h_off.p[x],
-                    g.h_tmask.p + ps.h_off.p[x]);
+      tangent_masks(ps.h_code.p + ps.h_off.p[x], ps.h_len.p[x], fold_n.data() + 2 * ps.h_off.p[x]);
+  SR_TRY(upload_set(ctx, ps, false));
 
   // Backward range and Jacobian-tape length of each reverse-mode program:
   // the sweep runs from the last instruction down to the lowest one holding
@@ -167,7 +164,8 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
   // spilled subtree.
   SR_TRY_CUDA(ctx, g.h_bwd_lo.ensure(static_cast<size_t>(std::max(E, 1))));
   std::vector<int32_t> tape_need(static_cast<size_t>(E));
-  for (int x = 0; x < E; ++x) {
+  std::fill_n(g.h_bwd_lo.p, E, 0);
+  for (int32_t x : rev_members) {
     const Instr *code = ps.h_code.p + ps.h_off.p[x];
     const int len = ps.h_len.p[x];
     int lo = len;
@@ -317,14 +315,14 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
     for (int32_t x : mem) ts.K = std::max(ts.K, ps.n_const[static_cast<size_t>(x)]);
     sr::Plan &p = ts.plan;
     p.dpt = sr::tan_dpt();
-    const int64_t ttile = 32 * p.dpt;
+    const int64_t tile = 32 * p.dpt, ttile = 2 * tile;  // tiles are summed in pairs
     p.W = sr::tan_warps(ts.K);
     p.smax = ps.smax;
     // Wider sets keep one spill slot per warp in shared memory (the others in
     // per-warp global scratch): the tangent rows need the room.
     p.s_smem = std::min(ps.smax, ts.K > 4 ? 1 : sr::smem_spill_slots(p.dpt));
     const int depth = group_depth(ctx, static_cast<int>(mem.size()));
-    int64_t tspan = launch_size(ctx, static_cast<int>(mem.size())) <= 1 ? 256 : 1024;
+    int64_t tspan = launch_size(ctx, static_cast<int>(mem.size())) <= 1 ? ttile : 1024;
     while (tspan > ttile && 2 * static_cast<int64_t>(ctx->V + 1) * tspan * 4 > 48 * 1024)
       tspan /= 2;
     tspan = std::min<int64_t>(tspan, std::max<int64_t>(ttile, round_up(ctx->N, ttile)));
@@ -358,7 +356,7 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
     p.blocks = static_cast<int>(std::min<int64_t>(static_cast<int64_t>(bps) * ctx->num_sms,
                                                   std::max<int64_t>(p.items(), 1)));
     spill_floats = std::max<int64_t>(spill_floats, static_cast<int64_t>(p.blocks) * p.W *
-                                                       (p.smax - p.s_smem) * ttile);
+                                                       (p.smax - p.s_smem) * tile);
     std::stable_sort(mem.begin(), mem.end(), [&](int32_t a, int32_t b) {
       return ps.cost[static_cast<size_t>(a)] > ps.cost[static_cast<size_t>(b)];
     });
@@ -460,7 +458,6 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
   if (g.n_rev > 0)
     SR_TRY_CUDA(ctx, ctx->partial.ensure(static_cast<size_t>(
                          std::max<int64_t>(static_cast<int64_t>(g.n_spans) * E, 1))));
-  SR_TRY_CUDA(ctx, g.tmask.ensure(static_cast<size_t>(ps.n_instr) + 1));
   SR_TRY_CUDA(ctx, g.h_exprs.ensure(std::max<size_t>(expr_list.size(), 1)));
   if (!expr_list.empty())
     std::memcpy(g.h_exprs.p, expr_list.data(), expr_list.size() * sizeof(int32_t));
@@ -469,9 +466,6 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
   SR_TRY_CUDA(ctx, ctx->mse.ensure(static_cast<size_t>(E) + 1));
   SR_TRY_CUDA(ctx, ctx->h_mse.ensure(static_cast<size_t>(E) + 1));
   cudaStream_t s = ctx->stream;
-  SR_TRY_CUDA(ctx, cudaMemcpyAsync(g.tmask.p, g.h_tmask.p,
-                                   (static_cast<size_t>(ps.n_instr) + 1) * sizeof(uint32_t),
-                                   cudaMemcpyHostToDevice, s));
   if (!expr_list.empty())
     SR_TRY_CUDA(ctx, cudaMemcpyAsync(g.exprs.p, g.h_exprs.p, expr_list.size() * sizeof(int32_t),
                                      cudaMemcpyHostToDevice, s));
@@ -542,7 +536,6 @@ sr_status launch_grad(sr_context *ctx) {
     a.e.span_per_item = ts.plan.k_spans;
     a.e.group_expr = g.groups.p + ts.group_off;
     a.e.partial = g.tan_partial.p + ts.part_off;
-    a.tmask = g.tmask.p;
     a.const_off = g.const_off.p;
     a.const_cnt = g.const_cnt.p;
     a.tinit = g.tinit.p;

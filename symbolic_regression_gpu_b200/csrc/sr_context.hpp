@@ -279,8 +279,6 @@ struct GradSet {
   // the code) and span-group sums; the expression lists (tangent sets first,
   // then the reverse-mode expressions) that the finalize kernels walk.
   std::vector<TanSet> tsets;
-  DevBuf<uint32_t> tmask;
-  PinnedBuf<uint32_t> h_tmask;
   DevBuf<double2> tan_partial;
   DevBuf<double> tan_gout;
   DevBuf<int32_t> exprs;

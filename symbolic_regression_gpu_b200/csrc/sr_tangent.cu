@@ -161,7 +161,7 @@ __device__ __forceinline__ void rcp_wide(const float (&b)[DPT], float (&r)[DPT])
 // (both operand orders), the protected log's and sqrt|x|'s derivatives run
 // in one shared loop each after the switch, so the code holds one copy of
 // each (instruction-cache footprint).
-template <int DPT>
+template <int DPT, bool LINEAR>
 __device__ __forceinline__ void tan_apply(uint32_t op, bool live, float (&T)[DPT],
                                           float (&b)[DPT], float (&dT)[DPT], float (&db)[DPT],
                                           int &dk, int &bk_) {
@@ -171,53 +171,58 @@ __device__ __forceinline__ void tan_apply(uint32_t op, bool live, float (&T)[DPT
   // these operators b holds the divisor (the protected denominator) or, for
   // the unary ones, the value to invert.
   int post = 0;
+  if constexpr (LINEAR) {
+    switch (op) {
+      // + - * in paired FP32 instructions (each half correctly rounded, a - b
+      // as a + (-b)): the forward interpreter's values.
+      case 1:
+#pragma unroll
+        for (int k = 0; k < DPT; k += 2) {
+          const float2 r = __fadd2_rn(make_float2(T[k], T[k + 1]), make_float2(b[k], b[k + 1]));
+          T[k] = r.x;
+          T[k + 1] = r.y;
+        }
+        dk = kDOne;
+        bk_ = kDOne;
+        return;
+      case 2:
+#pragma unroll
+        for (int k = 0; k < DPT; k += 2) {
+          const float2 r = __fadd2_rn(make_float2(T[k], T[k + 1]), make_float2(-b[k], -b[k + 1]));
+          T[k] = r.x;
+          T[k + 1] = r.y;
+        }
+        dk = kDOne;
+        bk_ = kDNeg;
+        return;
+      case kOpReversed + 2:
+#pragma unroll
+        for (int k = 0; k < DPT; k += 2) {
+          const float2 r = __fadd2_rn(make_float2(b[k], b[k + 1]), make_float2(-T[k], -T[k + 1]));
+          T[k] = r.x;
+          T[k + 1] = r.y;
+        }
+        dk = kDNeg;
+        bk_ = kDOne;
+        return;
+      case 3:
+#pragma unroll
+        for (int k = 0; k < DPT; k += 2) {
+          dT[k] = b[k];
+          dT[k + 1] = b[k + 1];
+          db[k] = T[k];
+          db[k + 1] = T[k + 1];
+          const float2 r = __fmul2_rn(make_float2(T[k], T[k + 1]), make_float2(b[k], b[k + 1]));
+          T[k] = r.x;
+          T[k + 1] = r.y;
+        }
+        return;
+      default: break;
+    }
+  }
   switch (op) {
     case 0:
       dk = kDOne;
-      break;
-    // + - * in paired FP32 instructions (each half correctly rounded, a - b
-    // as a + (-b)): the forward interpreter's values.
-    case 1:
-#pragma unroll
-      for (int k = 0; k < DPT; k += 2) {
-        const float2 r = __fadd2_rn(make_float2(T[k], T[k + 1]), make_float2(b[k], b[k + 1]));
-        T[k] = r.x;
-        T[k + 1] = r.y;
-      }
-      dk = kDOne;
-      bk_ = kDOne;
-      break;
-    case 2:
-#pragma unroll
-      for (int k = 0; k < DPT; k += 2) {
-        const float2 r = __fadd2_rn(make_float2(T[k], T[k + 1]), make_float2(-b[k], -b[k + 1]));
-        T[k] = r.x;
-        T[k + 1] = r.y;
-      }
-      dk = kDOne;
-      bk_ = kDNeg;
-      break;
-    case kOpReversed + 2:
-#pragma unroll
-      for (int k = 0; k < DPT; k += 2) {
-        const float2 r = __fadd2_rn(make_float2(b[k], b[k + 1]), make_float2(-T[k], -T[k + 1]));
-        T[k] = r.x;
-        T[k + 1] = r.y;
-      }
-      dk = kDNeg;
-      bk_ = kDOne;
-      break;
-    case 3:
-#pragma unroll
-      for (int k = 0; k < DPT; k += 2) {
-        dT[k] = b[k];
-        dT[k + 1] = b[k + 1];
-        db[k] = T[k];
-        db[k + 1] = T[k + 1];
-        const float2 r = __fmul2_rn(make_float2(T[k], T[k + 1]), make_float2(b[k], b[k + 1]));
-        T[k] = r.x;
-        T[k + 1] = r.y;
-      }
       break;
     case 8:  // T / protected(b)
 #pragma unroll
@@ -344,29 +349,90 @@ __device__ __forceinline__ void tan_apply(uint32_t op, bool live, float (&T)[DPT
   }
 }
 
-// One program over the warp's tile: values in T (registers), tangents in the
-// warp's shared-memory rows tan[c][TILE] (c = constant index; the loops over
-// a mask's set bits index them directly, one copy of each update in the code).
-// A spilled subtree's tangents stay in their rows: the instructions that
-// follow it (up to the one that takes it back as operand b) belong to other
-// subtrees, whose constants are other constants, so they never write its
-// rows; the instruction that consumes it multiplies them by db in place.
+// The tangents of the constants under one operand of an instruction times the
+// operator's partial by it.  These constants are the ones of a subtree, so they
+// are neighbours: `mask` is one run of bits and their rows follow one another.
+// Constants that enter here (`fresh`: a constant leaf, a constant operand b)
+// start from lane c's `tinit` (1, or a folded subtree's derivative by constant
+// c); rows of an operator whose partial is exactly 1 stay as they are, and -1
+// negates them.  A partial that is zero somewhere in the lane takes the zero
+// rule's selects, out of line; the others need none.
 template <int DPT>
-__device__ __forceinline__ void run_tangent_program(const Instr *__restrict__ code,
-                                                    const uint32_t *__restrict__ tmask, int len,
+__device__ __noinline__ void tan_rows_zero(float *row, int n, const float *d) {
+  float f[DPT];
+#pragma unroll
+  for (int k = 0; k < DPT; ++k) f[k] = d[k];
+#pragma unroll 1
+  for (int c = 0; c < n; ++c, row += 32 * DPT) {
+    float tv[DPT];
+    lds_vec<DPT>(row, 0, tv);
+    kill_mul<DPT>(tv, f);
+    sts_vec<DPT>(row, 0, tv);
+  }
+}
+template <int DPT>
+__device__ __forceinline__ void tan_rows(float *tan, uint32_t mask, int lane, int kind,
+                                         float (&d)[DPT], bool fresh, float tinit) {
+  if (kind == kDOne && !fresh) return;
+  const int c0 = __ffs(mask) - 1, n = __popc(mask);
+  float *row = tan + c0 * (32 * DPT) + lane * 4;
+  if (fresh) {
+    float *q = row;
+#pragma unroll 1
+    for (int c = 0; c < n; ++c, q += 32 * DPT) {
+      float t0 = __shfl_sync(0xffffffffu, tinit, c0 + c), tv[DPT];
+      if (kind == kDNeg) t0 = -t0;
+#pragma unroll
+      for (int k = 0; k < DPT; ++k) tv[k] = t0;
+      sts_vec<DPT>(q, 0, tv);
+    }
+    if (kind != kDGen) return;
+  }
+  if (kind == kDNeg) {
+#pragma unroll
+    for (int k = 0; k < DPT; ++k) d[k] = -1.0f;
+  }
+  if (min_abs<DPT>(d) > 0.0f) {
+#pragma unroll 1
+    for (int c = 0; c < n; ++c, row += 32 * DPT) {
+      float tv[DPT];
+      lds_vec<DPT>(row, 0, tv);
+#pragma unroll
+      for (int k = 0; k < DPT; k += 2) {
+        const float2 r = __fmul2_rn(make_float2(d[k], d[k + 1]), make_float2(tv[k], tv[k + 1]));
+        tv[k] = r.x;
+        tv[k + 1] = r.y;
+      }
+      sts_vec<DPT>(row, 0, tv);
+    }
+  } else {
+    float f[DPT];
+#pragma unroll
+    for (int k = 0; k < DPT; ++k) f[k] = d[k];
+    tan_rows_zero<DPT>(row, n, f);
+  }
+}
+
+// One program over the warp's tile: values in T (registers), tangents in the
+// warp's shared-memory rows tan[c][TILE] (c = constant index).  A spilled
+// subtree's tangents stay in their rows: the instructions that follow it (up to
+// the one that takes it back as operand b) belong to other subtrees, whose
+// constants are other constants, so they never write its rows; the instruction
+// that consumes it multiplies them by db in place.
+template <int DPT>
+__device__ __forceinline__ void run_tangent_program(const Instr *__restrict__ code, int len,
                                                     const float *xs, int xrs,
                                                     const SpillStack &st, int lane, float *tan,
-                                                    const float *__restrict__ tinit,
-                                                    float (&T)[DPT]) {
-  constexpr int TILE = 32 * DPT;
+                                                    float tinit, float (&T)[DPT]) {
   uint4 ins = ldg_instr(code);
-  uint32_t m = __ldg(tmask);
   for (int i = 0; i < len; ++i) {
-    // The code and mask buffers end with a padding entry, so these prefetches
-    // of the next entry are always in bounds.
+    // The code buffer ends with a padding entry, so this prefetch of the next
+    // entry is always in bounds.
     const uint4 nxt = ldg_instr(code + i + 1);
-    const uint32_t mn = __ldg(tmask + i + 1);
-    const uint32_t w = ins.x;
+    // Word and masks are the same in every lane; the reductions say so to the
+    // compiler (uniform registers).
+    const uint32_t w = __reduce_or_sync(0xffffffffu, ins.x);
+    const uint32_t m = __reduce_or_sync(0xffffffffu, ins.w);
     const uint32_t A = m & 0xFFu, B = (m >> 8) & 0xFFu;
     if (w & (kLoadBit | kSpillBit)) {
       if (instr_spill(w)) spill_store<DPT>(st, instr_spill_slot(w), lane, T);
@@ -376,44 +442,45 @@ __device__ __forceinline__ void run_tangent_program(const Instr *__restrict__ co
     float b[DPT], dT[DPT], db[DPT];
     const uint32_t bk = instr_b_kind(w);
     if (bk != kBNone) load_operand<DPT, false>(bk, ins.z, b, xs, xrs, st, lane, nullptr, 0, 0);
-    int dk, bkn;
-    tan_apply<DPT>(instr_op(w), (A | B) != 0, T, b, dT, db, dk, bkn);
-    if (A | B) {
-      // Constants that enter here (a constant leaf, a constant operand b)
-      // start from tangent 1, those of a folded subtree from the subtree's
-      // derivative by them; rows of an operator whose partial is exactly 1
-      // stay as they are.  (One loop for both masks: a second copy of it
-      // costs more in instruction-cache misses than its branches.)
-      const uint32_t fresh = (m & kTanLoadConst ? A : 0u) | (bk == kBC ? B : 0u);
-      for (uint32_t u = A | B; u; u &= u - 1) {
-        const int c = __ffs(u) - 1;
-        const bool on_b = (B >> c) & 1u;
-        const int kind = on_b ? bkn : dk;
-        const bool is_fresh = (fresh >> c) & 1u;
-        if (kind == kDOne && !is_fresh) continue;
-        float *row = tan + c * TILE;
-        float tv[DPT];
-        if (is_fresh) {
-          const float t0 = __ldg(tinit + c);
+    const uint32_t d = instr_dispatch(w);
+    int dk = kDOne, bkn = kDOne;
+    if (d & kDLinear) {
+      // + - * as the interpreter's fused multiply-adds, with its values.
+      if (d & kDMul) {
+        dk = bkn = kDGen;
 #pragma unroll
-          for (int k = 0; k < DPT; ++k) tv[k] = t0;
-        } else {
-          lds_vec<DPT>(row, lane, tv);
+        for (int k = 0; k < DPT; k += 2) {
+          const float2 t = make_float2(T[k], T[k + 1]), u = make_float2(b[k], b[k + 1]);
+          const float2 r = __fmul2_rn(t, u);
+          dT[k] = u.x;
+          dT[k + 1] = u.y;
+          db[k] = t.x;
+          db[k + 1] = t.y;
+          T[k] = r.x;
+          T[k + 1] = r.y;
         }
-        if (kind == kDNeg) {
+      } else {
+        const float st_ = (d & kDRSub) ? -1.0f : 1.0f;
+        if (d & kDRSub) dk = kDNeg;
+        if (d & kDSub) bkn = kDNeg;
+        if (d & kDSub) {
 #pragma unroll
-          for (int k = 0; k < DPT; ++k) tv[k] = -tv[k];
-        } else if (kind == kDGen) {
-          if (on_b)
-            kill_mul<DPT>(tv, db);
-          else
-            kill_mul<DPT>(tv, dT);
+          for (int k = 0; k < DPT; ++k) b[k] = -b[k];
         }
-        sts_vec<DPT>(row, lane, tv);
+#pragma unroll
+        for (int k = 0; k < DPT; k += 2) {
+          const float2 r = __ffma2_rn(make_float2(T[k], T[k + 1]), make_float2(st_, st_),
+                                      make_float2(b[k], b[k + 1]));
+          T[k] = r.x;
+          T[k + 1] = r.y;
+        }
       }
+    } else {
+      tan_apply<DPT, false>(instr_op(w), (A | B) != 0, T, b, dT, db, dk, bkn);
     }
+    if (A) tan_rows<DPT>(tan, A, lane, dk, dT, (m & kTanLoadConst) != 0, tinit);
+    if (B) tan_rows<DPT>(tan, B, lane, bkn, db, bk == kBC, tinit);
     ins = nxt;
-    m = mn;
   }
 }
 
@@ -434,7 +501,8 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) tan_kernel(const TanArg
   float *sreg = xbuf + static_cast<size_t>(kBufs) * rows * span;
   float *tans = sreg + static_cast<size_t>(W) * p.s_smem * TILE;  // [W][K][TILE]
   double *gsm = reinterpret_cast<double *>(tans + static_cast<size_t>(W) * K * TILE);  // [W][K][32]
-  ItemDesc *desc = reinterpret_cast<ItemDesc *>(gsm + static_cast<size_t>(W) * K * 32);
+  float *csm = reinterpret_cast<float *>(gsm + static_cast<size_t>(W) * K * 32);  // [W][K][32]
+  ItemDesc *desc = reinterpret_cast<ItemDesc *>(csm + static_cast<size_t>(W) * K * 32);
   uint64_t *full = reinterpret_cast<uint64_t *>(desc + kBufs);
   uint64_t *empty = full + kBufs;
   SpanPart *part = reinterpret_cast<SpanPart *>(empty + kBufs);
@@ -467,7 +535,8 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) tan_kernel(const TanArg
                         static_cast<size_t>(p.smax - p.s_smem) * TILE;
   st.s_smem = p.s_smem;
   float *tan = tans + static_cast<size_t>(warp) * K * TILE;
-  double *gl = gsm + static_cast<size_t>(warp) * K * 32;  // per-lane gradient sums
+  double *gl = gsm + static_cast<size_t>(warp) * K * 32 + lane;  // per-lane gradient sums
+  float *half = csm + static_cast<size_t>(warp) * K * 32 + lane;  // of a pair's first tile
   const int tiles = span / TILE;
   uint32_t buf = 0, phase = 0;
   for (;;) {
@@ -484,19 +553,19 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) tan_kernel(const TanArg
       const int e = p.group_expr[static_cast<int64_t>(d.group) * p.G + j];
       if (e < 0) break;  // groups are padded at their end only
       const Instr *code = p.code + p.code_off[e];
-      const uint32_t *tm = a.tmask + p.code_off[e];
       const int len = p.code_len[e];
       const int nconst = min(a.const_cnt[e], K);
-      const float *tinit = a.tinit + a.const_off[e];
+      // Lane c holds what the tangent of constant c starts from.
+      const float tinit = lane < nconst ? __ldg(a.tinit + a.const_off[e] + lane) : 1.0f;
       double acc = 0.0;
       int cnt = 0;
-      for (int c = 0; c < nconst; ++c) gl[c * 32 + lane] = 0.0;
+      for (int c = 0; c < nconst; ++c) gl[c * 32] = 0.0;
       for (int t = 0; t < tiles; ++t) {
         const int64_t dp0 = dp_span + static_cast<int64_t>(t) * TILE;
         if (dp0 >= p.N) break;  // tail of the last span
         const float *xs = xb + t * TILE;
         float T[DPT];
-        run_tangent_program<DPT>(code, tm, len, xs, span, st, lane, tan, tinit, T);
+        run_tangent_program<DPT>(code, len, xs, span, st, lane, tan, tinit, T);
         float y[DPT], sd[DPT];
         lds_vec<DPT>(xs + p.V * span, lane, y);
         const bool full_tile = dp0 + TILE <= p.N;  // warp-uniform
@@ -510,29 +579,47 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) tan_kernel(const TanArg
           dsq[k] = sq2.x;
           dsq[k + 1] = sq2.y;
         }
+        const int before = cnt;
         add_squares<DPT>(T, dsq, full_tile, dp0, lane, p.N, acc, cnt);
 #pragma unroll
-        for (int k = 0; k < DPT; ++k) {
-          const bool valid =
-              (full_tile || dp0 + (k / 4) * 128 + lane * 4 + (k % 4) < p.N) && isfinite(T[k]);
-          sd[k] = valid ? 2.0f * dfs[k] : 0.0f;
+        for (int k = 0; k < DPT; ++k) sd[k] = 2.0f * dfs[k];
+        if (cnt - before != DPT) {
+#pragma unroll
+          for (int k = 0; k < DPT; ++k) {
+            const bool valid =
+                (full_tile || dp0 + (k / 4) * 128 + lane * 4 + (k % 4) < p.N) && isfinite(T[k]);
+            sd[k] = valid ? sd[k] : 0.0f;
+          }
         }
         // d MSE / d c (times the count): seed * t_c, zero where the seed is;
-        // each lane adds its DPT products in order in FP32, FP64 from there
-        // on (an FP32 lane sum overflows only for products beyond ~4e37).
+        // each lane adds its products of a pair of tiles (2 DPT) in order in
+        // FP32, FP64 from there on (an FP32 lane sum overflows only for products
+        // beyond ~4e37).  Spans hold whole pairs; the last one may lack its
+        // second tile.
+        const bool odd = (t & 1) != 0;
+        const bool pair_end = odd || dp0 + TILE >= p.N;
+        const bool seeded = min_abs<DPT>(sd) > 0.0f;
+#pragma unroll 1
         for (int cc = 0; cc < nconst; ++cc) {
           float tv[DPT];
           lds_vec<DPT>(tan + cc * TILE, lane, tv);
 #pragma unroll
           for (int k = 0; k < DPT; k += 2) {
             const float2 r = __fmul2_rn(make_float2(sd[k], sd[k + 1]), make_float2(tv[k], tv[k + 1]));
-            tv[k] = sd[k] == 0.0f ? 0.0f : r.x;
-            tv[k + 1] = sd[k + 1] == 0.0f ? 0.0f : r.y;
+            tv[k] = r.x;
+            tv[k + 1] = r.y;
           }
-          float g = tv[0];
+          if (!seeded) {
+#pragma unroll
+            for (int k = 0; k < DPT; ++k) tv[k] = sd[k] == 0.0f ? 0.0f : tv[k];
+          }
+          float g = odd ? __fadd_rn(half[cc * 32], tv[0]) : tv[0];
 #pragma unroll
           for (int k = 1; k < DPT; ++k) g = __fadd_rn(g, tv[k]);
-          gl[cc * 32 + lane] += static_cast<double>(g);
+          if (pair_end)
+            gl[cc * 32] += static_cast<double>(g);
+          else
+            half[cc * 32] = g;
         }
       }
 #pragma unroll
@@ -542,7 +629,7 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) tan_kernel(const TanArg
       }
       double *gp = gpart + (static_cast<size_t>(buf) * p.G + j) * K;
       for (int cc = 0; cc < K; ++cc) {
-        double g = cc < nconst ? gl[cc * 32 + lane] : 0.0;
+        double g = cc < nconst ? gl[cc * 32] : 0.0;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
         if (lane == 0) gp[cc] = g;
@@ -593,7 +680,7 @@ __global__ void __launch_bounds__(64)
       float T[2] = {val[a], val[a]}, B[2] = {val[b], val[b]};
       float dT[2], dB[2];
       int kt, kb;
-      tan_apply<2>(op, true, T, B, dT, dB, kt, kb);
+      tan_apply<2, true>(op, true, T, B, dT, dB, kt, kb);
       const bool under_b = op < 10 && on[b];
       const bool under = on[a] || under_b;
       if (under) {
@@ -681,16 +768,19 @@ const void *tan_fn() {
   return reinterpret_cast<const void *>(&tan_kernel<DPT, MAXW, MINB>);
 }
 
-// Launch shapes: 8 datapoints per thread, one block per SM with as many
-// evaluating warps as the register file holds beside the producer warp: up
-// to 19 (96 registers per thread) for up to 4 tangent rows, 15 (120) for more.
-// The kernel is latency-bound on dependent chains; one large block keeps
-// more warps resident than two blocks of 8 + 1 or 7 + 1 warps did (16 and 12
-// evaluating warps per SM).
-constexpr int kTanDpt = 8;
-constexpr int tan_max_warps(int K) { return K <= 4 ? 19 : 15; }
+// Launch shapes: 4 datapoints per thread, one block per SM with as many
+// evaluating warps as the register file holds beside the producer warp: 31 (64
+// registers per thread) for up to 4 tangent rows, 27 (72) for more, as far as
+// their tangent rows fit in shared memory.  The kernel lives on resident warps:
+// 8 datapoints per thread and 19 or 15 warps issued on 61 and 53 % of the cycles
+// (dependent chains, instruction fetches), these on 83 and 75 %, which outweighs
+// a quarter more instructions: 4,096 x 262,144 19.8 -> 18.9 ms, 1,000 x 20,001
+// 0.65 -> 0.55 ms a pass.  Widths of 2, 4, 6 and 8 rows in four launches give
+// 18.4 and 0.59 ms; 3, 5 and 8 18.7 and 0.56.
+constexpr int kTanDpt = 4;
+constexpr int tan_max_warps(int K) { return K <= 4 ? 31 : 27; }
 const void *select_tan(int K) {
-  return K <= 4 ? tan_fn<kTanDpt, 19, 1>() : tan_fn<kTanDpt, 15, 1>();
+  return K <= 4 ? tan_fn<kTanDpt, 31, 1>() : tan_fn<kTanDpt, 27, 1>();
 }
 
 }  // namespace
@@ -702,7 +792,7 @@ size_t tan_smem_bytes(int K, int W, int V, int s_smem, int span, int G) {
   const size_t tile = 32u * static_cast<size_t>(kTanDpt);
   return (static_cast<size_t>(kBufs) * (V + 1) * span +
           static_cast<size_t>(W) * (s_smem + K) * tile) * sizeof(float) +
-         static_cast<size_t>(W) * K * 32 * sizeof(double) +
+         static_cast<size_t>(W) * K * 32 * (sizeof(double) + sizeof(float)) +
          kBufs * sizeof(ItemDesc) + 2 * kBufs * sizeof(uint64_t) +
          static_cast<size_t>(G) * (kBufs * sizeof(SpanPart) + sizeof(GroupAcc)) +
          static_cast<size_t>(G) * K * (kBufs + 1) * sizeof(double);
