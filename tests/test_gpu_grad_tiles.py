@@ -1,6 +1,7 @@
-"""Forward-mode gradients at the edges of tiles and of pairs of tiles (whose
-products are summed together), with 1 to 8 constants and partials that are zero
-somewhere, against the FP32 bytecode emulator.
+"""Gradients in both modes at the edges of tiles and of forward mode's pairs of
+tiles (whose products are summed together), with 1 to 8 constants, partials that
+are zero somewhere and datapoints whose residual is, against the FP32 bytecode
+emulator.
 
 Tolerance, derived: as for the larger emulator comparison, only the FP64
 summation order (at most (N + 64) 2^-53 of the summed magnitudes) and the FP32 rounding
@@ -8,8 +9,8 @@ of the returned gradient (half an ulp) differ."""
 import numpy as np
 import pytest
 
-from emulate import tangent_bytecode
-from symbolic_regression_gpu_b200 import Evaluator, Population
+from emulate import adjoint_bytecode, tangent_bytecode
+from symbolic_regression_gpu_b200 import Evaluator, Population, _lib
 from symbolic_regression_gpu_b200 import opcodes as op
 from symbolic_regression_gpu_b200.evaluator import compile_population
 
@@ -43,23 +44,27 @@ def _population(V):
     return Population.from_lists(out)
 
 
+@pytest.mark.parametrize("reverse", [False, True])
 @pytest.mark.parametrize("N", [1, 127, 128, 129, 256, 257, 384, 641])
-def test_tile_pairs_match_the_emulator(N):
+def test_tile_edges_match_the_emulator(N, reverse):
     V = 3
     rng = np.random.default_rng(N)
     X = rng.uniform(-2.0, 2.0, (V + 1, N)).astype(np.float32)
     X[2, ::5] = 0.0
     pop = _population(V)
+    X[V, ::3] = X[0, ::3] + np.float32(0.5)  # the first expression's value: a zero residual
+    mode = _lib.SR_GRAD_CHECKPOINT | (_lib.SR_GRAD_REVERSE_ONLY if reverse else 0)
+    emulate = adjoint_bytecode if reverse else tangent_bytecode
     with Evaluator(device=0) as ev:
         ev.set_data(X)
-        mse, g = ev.eval_grad(pop)
+        mse, g = ev.eval_grad(pop, mode=mode)
     code, offs, _ = compile_population(pop, V)
     co = pop.constant_offsets()
     for e in range(pop.num_exprs):
         nc = int(co[e + 1] - co[e])
         with np.errstate(all="ignore"):
-            m_e, g_e, gabs = tangent_bytecode(code[offs[e]:offs[e + 1]], X, V, nc,
-                                              dtype=np.float32, with_abs=True)
+            m_e, g_e, gabs = emulate(code[offs[e]:offs[e + 1]], X, V, nc, dtype=np.float32,
+                                     with_abs=True)
         got = g[co[e]:co[e + 1]]
         assert np.array_equal(np.isfinite(got), np.isfinite(g_e))
         f = np.isfinite(g_e)
