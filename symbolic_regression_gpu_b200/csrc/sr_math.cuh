@@ -223,6 +223,19 @@ __device__ __forceinline__ float2 rcp2_mid(float2 b) {
   return __ffma2_rn(__ffma2_rn(nb, q, f2(1.0f)), r, q);
 }
 
+// a / b into a and 1 / b into r: both from one reciprocal, the same values as
+// div2_mid and rcp2_mid.
+__device__ __forceinline__ void div_rcp2_mid(float2 &a, float2 b, float2 &r) {
+  const float2 nb = __fmul2_rn(b, f2(-1.0f));
+  r = make_float2(rcp_approx(b.x), rcp_approx(b.y));
+  r = __ffma2_rn(r, __ffma2_rn(nb, r, f2(1.0f)), r);
+  float2 q = __fmul2_rn(a, r);
+  q = __ffma2_rn(__ffma2_rn(nb, q, a), r, q);
+  a = __ffma2_rn(__ffma2_rn(nb, q, a), r, q);
+  q = __ffma2_rn(__ffma2_rn(nb, r, f2(1.0f)), r, r);
+  r = __ffma2_rn(__ffma2_rn(nb, q, f2(1.0f)), r, q);
+}
+
 // sqrt(x), x in [kSqrtMin, kSqrtMax] (NaN gives NaN).
 __device__ __forceinline__ float2 sqrt2_mid(float2 x) {
   const float2 nx = __fmul2_rn(x, f2(-1.0f));
