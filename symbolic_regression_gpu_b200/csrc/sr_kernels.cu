@@ -1,23 +1,27 @@
 // sr_kernels.cu — sm_100a kernels of the population evaluator.
 //
-//  interp_kernel<DPT, PRED, MAXW, MINB, OPS>
+//  interp_kernel<DPT, PRED, MAXW, MINB, OPS, GEN>
 //                             persistent interpreter (OPS: the operator
 //                             profile its switch dispatches inline,
-//                             sr_internal.hpp).  One producer thread
-//                             per block claims work items (span, group) from
-//                             a global counter and copies the item's X span
+//                             sr_internal.hpp; GEN: cached subtrees or spill
+//                             slots in global scratch).  One producer warp per
+//                             block claims work items (span group, expression
+//                             group) and copies each of the item's X spans
 //                             (every row) into one of two shared-memory
 //                             buffers with the bulk-copy (TMA) engine, one
-//                             cp.async.bulk per row, completion tracked by
-//                             mbarrier transaction counts.  The W evaluating
-//                             warps claim the group's expressions from a
-//                             shared counter and run each over the whole span:
-//                             32 lanes x DPT datapoints per instruction fetch,
-//                             accumulator in registers, spilled values in a
-//                             per-warp shared stack.  The epilogue either
+//                             cp.async.bulk per row and tile, completion
+//                             tracked by mbarrier transaction counts.  The W
+//                             evaluating warps claim the group's expressions
+//                             from a shared counter and run each over the whole
+//                             span: 32 lanes x DPT datapoints per instruction
+//                             fetch, accumulator in registers, spilled values
+//                             in a per-warp shared stack.  The epilogue either
 //                             accumulates the squared error (FP32 squares, FP64
-//                             sums)
-//                             or stores the predictions.
+//                             sums) or stores the predictions.
+//  fold_kernel                values of constant subtrees, into the instruction
+//                             words that hold them.
+//  finalize_dd_kernel         per-expression combination of the span groups'
+//                             double-doubles in a fixed order.
 //  finalize_kernel            per-expression combination of span partials in
 //                             a fixed order: mse = sum / count.
 //  sums_kernel                the same combination kept as (sum, count), for
@@ -511,8 +515,9 @@ static const void *interp_mse(int ops, bool general) {
 // register budget), larger W the wide ones (up to 16 warps; at 8 datapoints
 // per thread MSE launches also come as 2 blocks of up to 15 + 1 warps and 1
 // block of up to 31 + 1 warps, both at 64 registers: on the batched
-// population the interpreter is latency-bound, and 30 or 31 evaluating warps
-// per SM beat 24 at 72 registers: 65.2 -> 60.1 and 58.8 ms).  MSE launches
+// population 30 or 31 evaluating warps per SM beat 24 at 72 registers: 65.2 ->
+// 60.1 and 58.8 ms at the time; now 38.5 and 34.1, 16 datapoints per thread 47 to
+// 85).  MSE launches
 // come in both operator profiles, with and without the general operand paths
 // (cached subtrees, spill slots in global scratch); prediction launches (cache
 // fills, predictions) in kOpsAll with them.

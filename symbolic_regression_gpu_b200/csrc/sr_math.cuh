@@ -1,4 +1,5 @@
-// sr_math.cuh — the evaluator's own single-precision sin, cos and log.
+// sr_math.cuh — the evaluator's own single-precision sin, cos and log, and paired
+// division, reciprocal and square root.
 //
 // CUDA's accurate sinf / cosf / logf are general-purpose routines (each with
 // a slow path for arguments its fast path cannot reduce) that cost 30+
