@@ -5,10 +5,12 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstdint>
+#include <exception>
 #include <functional>
 #include <mutex>
 #include <system_error>
 #include <thread>
+#include <utility>
 #include <vector>
 
 namespace sr {
@@ -51,7 +53,9 @@ class WorkerPool {
   }
 
   // fn(0) .. fn(chunks - 1), each once, on the caller and up to `threads` - 1
-  // workers; returns when all are done.
+  // workers; returns when all are done.  An exception of fn leaves the pool
+  // usable and reaches the caller once no worker is inside the pass any more
+  // (the first one, when several chunks throw).
   void run(int chunks, int threads, const std::function<void(int)> &fn) {
     if (chunks <= 1 || threads <= 1) {
       for (int c = 0; c < chunks; ++c) fn(c);
@@ -62,6 +66,8 @@ class WorkerPool {
     chunks_ = chunks;
     next_.store(0);
     pending_.store(chunks);
+    failure_ = nullptr;
+    failed_.store(false);
     open_.store(true);
     {
       std::lock_guard<std::mutex> lock(m_);
@@ -74,6 +80,7 @@ class WorkerPool {
     for (int spin = 0; pending_.load() > 0; ++spin) pause(spin);
     open_.store(false);
     for (int spin = 0; inside_.load() > 0; ++spin) pause(spin);
+    if (failure_) std::rethrow_exception(std::exchange(failure_, nullptr));
   }
 
  private:
@@ -96,7 +103,11 @@ class WorkerPool {
   }
   void work() {
     for (int c; (c = next_.fetch_add(1)) < chunks_;) {
-      (*fn_)(c);
+      try {
+        (*fn_)(c);
+      } catch (...) {
+        if (!failed_.exchange(true)) failure_ = std::current_exception();
+      }
       pending_.fetch_sub(1);
     }
   }
@@ -126,7 +137,8 @@ class WorkerPool {
   const std::function<void(int)> *fn_ = nullptr;
   int chunks_ = 0;
   std::atomic<int> next_{0}, pending_{0}, inside_{0}, sleepers_{0};
-  std::atomic<bool> open_{false}, stop_{false};
+  std::atomic<bool> open_{false}, stop_{false}, failed_{false};
+  std::exception_ptr failure_;  // of the pass: written by the one that set failed_
   std::atomic<uint64_t> generation_{0};
 };
 

@@ -12,6 +12,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <new>
 
 #include "sr_internal.hpp"
 #include "sr_program.hpp"
@@ -328,6 +329,22 @@ void Sharing::keep_rows(int n) {
 
 bool Sharing::find(int E, const int32_t *tok, const double *val, const int64_t *off, int max_rows,
                    WorkerPool &pool, int threads) {
+  // Sharing is an option: a population whose hashes and table (up to about 50
+  // bytes a token) do not fit host memory is evaluated without it.
+  try {
+    return search(E, tok, val, off, max_rows, pool, threads);
+  } catch (const std::bad_alloc &) {
+    drop_rows();
+    std::vector<uint64_t>().swap(hash_);
+    std::vector<int16_t>().swap(size_);
+    table_.reset();
+    cap_ = 0;
+    return false;
+  }
+}
+
+bool Sharing::search(int E, const int32_t *tok, const double *val, const int64_t *off,
+                     int max_rows, WorkerPool &pool, int threads) {
   tok_ = tok;
   val_ = val;
   off_ = off;
@@ -343,6 +360,8 @@ bool Sharing::find(int E, const int32_t *tok, const double *val, const int64_t *
   size_t cap = 1024;
   while (cap * 7 < (n_ops + static_cast<size_t>(E)) * 8) cap *= 2;
   if (cap > cap_) {
+    table_.reset();
+    cap_ = 0;
     table_.reset(new Entry[cap]);
     cap_ = cap;
   }

@@ -50,7 +50,7 @@ class Sharing {
 
   // Hashes, counts and chooses up to max_rows rows for expressions [0, E) of a
   // CSR population.  False when an expression is malformed (compiling it
-  // reports how).  The arrays are read until the last mark() / rep().
+  // reports how) or host memory runs out.  The arrays are read until the last mark() / rep().
   bool find(int E, const int32_t *tok, const double *val, const int64_t *off, int max_rows,
             WorkerPool &pool, int threads);
   // Marks expression x's tokens (hints has its length) and returns whether
@@ -76,6 +76,8 @@ class Sharing {
   const Entry *lookup(uint64_t key) const;
   bool equal_runs(int64_t a, int64_t b, int32_t n) const;
   struct Local;
+  bool search(int E, const int32_t *tok, const double *val, const int64_t *off, int max_rows,
+              WorkerPool &pool, int threads);
   bool hash_expression(int x, Local &local);
   void flush(Local &local, int slot);
   void choose(std::vector<uint32_t> &frequent, int max_rows);
