@@ -191,9 +191,9 @@ const char *sr_status_string(sr_status s);
 const char *sr_last_error(const sr_context *ctx);
 int32_t sr_abi_version(void);
 /* Fault injection for tests (process-wide): with n > 0 the n-th following
- * device or pinned-host allocation made by the library fails as if the
- * memory were exhausted (the call returns SR_ERR_OUT_OF_MEMORY and the
- * context stays usable); n = 0 disables it.  The reference has no
+ * device or pinned-host allocation or graph instantiation made by the
+ * library fails as if the memory were exhausted (the call returns
+ * SR_ERR_OUT_OF_MEMORY and the context stays usable); n = 0 disables it.  The reference has no
  * counterpart (its CUDA_CHECK exits the process on any failure,
  * cl_gpu_common.h:15-23). */
 sr_status sr_inject_allocation_failure(int64_t n);

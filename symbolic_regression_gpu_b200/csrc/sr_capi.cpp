@@ -552,12 +552,30 @@ sr_status upload_set(sr_context *ctx, ProgramSet &ps, bool groups) {
   return SR_OK;
 }
 
-sr_status begin_sequence(sr_context *ctx) {
-  if (ctx->counters_used)
+// Work counters at zero, by a memset where the last sequence has not left them
+// so.  counters_used follows what has been enqueued for execution: on a stream
+// that its owner is capturing the memset goes into the capture, whose replays
+// meet whatever ran before them, and the flag stays set.
+static sr_status zero_counters(sr_context *ctx) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  SR_TRY_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capture));
+  ctx->outer_capture = capture != cudaStreamCaptureStatusNone;
+  if (ctx->outer_capture || ctx->counters_used)
     SR_TRY_CUDA(ctx, cudaMemsetAsync(ctx->d_counter, 0, sr::kCounters * sizeof(int32_t),
                                      ctx->stream));
+  ctx->counters_used = ctx->outer_capture;
+  return SR_OK;
+}
+
+sr_status begin_sequence(sr_context *ctx) {
+  if (ctx->capturing) return SR_OK;  // the launch of the graph sees to it
+  SR_TRY(zero_counters(ctx));
   ctx->counters_used = true;
   return SR_OK;
+}
+
+void finish_sequence(sr_context *ctx) {
+  if (!ctx->capturing && !ctx->outer_capture) ctx->counters_used = false;
 }
 
 sr::SequenceEnd sequence_end(sr_context *ctx) {
@@ -1419,7 +1437,7 @@ static sr_status enqueue_launch(sr_context *ctx, int *launches_out) {
                                                 ctx->main.plan.n_span_groups(),
                                                 ctx->E, ctx->mse.p, nullptr, sequence_end(ctx),
                                                 s));
-    ctx->counters_used = false;
+    finish_sequence(ctx);
     ++launches;
   }
   SR_TRY_CUDA(ctx, record_event(ctx, 3));
@@ -1455,12 +1473,15 @@ static sr_status launch_prepared(sr_context *ctx, bool allow_graph) {
         return st;
       }
       SR_TRY_CUDA(ctx, ce);
-      const cudaError_t ie = cudaGraphInstantiate(&ctx->graph_exec, graph, 0);
+      const cudaError_t ie = sr::alloc_fault_fires()
+                                 ? cudaErrorMemoryAllocation
+                                 : cudaGraphInstantiate(&ctx->graph_exec, graph, 0);
       cudaGraphDestroy(graph);
       if (ie != cudaSuccess) ctx->graph_exec = nullptr;
       SR_TRY_CUDA(ctx, ie);
       ctx->graph_launches = launches;
     }
+    SR_TRY(zero_counters(ctx));  // the captured sequence only leaves them at zero
     SR_TRY_CUDA(ctx, cudaGraphLaunch(ctx->graph_exec, s));
     launches = ctx->graph_launches;
   } else {

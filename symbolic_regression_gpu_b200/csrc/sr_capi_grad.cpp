@@ -584,7 +584,7 @@ sr_status launch_grad(sr_context *ctx) {
                                               g.exprs.p + g.rev_expr_off, g.n_rev, g.const_off.p,
                                               g.const_cnt.p, g.grad_acc.p, ctx->mse.p, g.grad.p,
                                               ctx->sums.p, end, s));
-  if (!g.tsets.empty() || g.n_rev > 0) ctx->counters_used = false;
+  if (!g.tsets.empty() || g.n_rev > 0) finish_sequence(ctx);
   return SR_OK;
 }
 

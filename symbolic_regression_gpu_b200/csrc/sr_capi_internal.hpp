@@ -53,10 +53,11 @@ sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, i
 sr_status upload_groups(sr_context *ctx, ProgramSet &ps);
 // The set's packed buffer, with or without its group table, in one copy.
 sr_status upload_set(sr_context *ctx, ProgramSet &ps, bool groups);
-// Work counters at zero before a launch sequence, and what its last kernel
-// does for the next one.
+// Work counters at zero before a launch sequence, what its last kernel does for
+// the next one, and the note that this kernel is enqueued.
 sr_status begin_sequence(sr_context *ctx);
 sr::SequenceEnd sequence_end(sr_context *ctx);
+void finish_sequence(sr_context *ctx);
 EvalArgs make_args(sr_context *ctx, ProgramSet &ps, int32_t *counter);
 sr_status launch_set(sr_context *ctx, ProgramSet &ps, bool pred, int32_t *counter,
                      float *pred_out, int64_t ldp, const int32_t *pred_row);

@@ -22,8 +22,9 @@
 namespace sr {
 
 // Host-side fault injection for tests (sr_inject_allocation_failure): when the
-// countdown is n > 0, the n-th following DevBuf / PinnedBuf allocation fails
-// with cudaErrorMemoryAllocation without reaching the allocator (once).
+// countdown is n > 0, the n-th following DevBuf / PinnedBuf allocation or graph
+// instantiation fails with cudaErrorMemoryAllocation without reaching the
+// allocator (once).
 inline std::atomic<int64_t> &alloc_fault_countdown() {
   static std::atomic<int64_t> countdown{0};
   return countdown;
@@ -333,9 +334,11 @@ struct sr_context {
   sr::PinnedBuf<float> h_mse;
   // Work counters: [0] main, [1] subtree launches, [2..] gradient launches.
   // They are zero before a launch sequence: its last kernel (a finalize)
-  // zeroes them for the next one; counters_used marks sequences that had none.
+  // zeroes them for the next one.  counters_used: the last sequence enqueued had
+  // no such kernel, or nothing is known of it (zero_counters).
   int32_t *d_counter = nullptr;
   bool counters_used = false;
+  bool outer_capture = false;     // the stream's owner is capturing the current sequence
   int32_t *d_error = nullptr;
   int32_t *h_error = nullptr;     // pinned
 
