@@ -289,18 +289,52 @@ static bool sharing_pays(const sr_context *ctx, const sr_population *pop) {
   return tokens * (static_cast<double>(ctx->N) - 60000.0) >= 3e9;
 }
 
-// Batched programs: shared work found and taken out where that pays, then
-// compiled, planned and uploaded.
-static sr_status prepare_batched(sr_context *ctx, const sr_population *pop) {
+// Batched programs with the shared work found (sh, or null) taken out: compiled,
+// planned and uploaded.
+static sr_status prepare_programs(sr_context *ctx, const sr_population *pop, sr::Sharing *sh) {
   const int E = pop->num_exprs;
+  const double tc0 = now_ms();
+  SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, nullptr, ctx->main, sh));
+  // Programs of long expressions can need a fourth spill slot: fewer rows then.
+  if (sh && ctx->main.smax > 3 &&
+      static_cast<int>(sh->rows().size()) > derived_row_limit(ctx, 4)) {
+    sh->keep_rows(derived_row_limit(ctx, 4));
+    ctx->folds.refs.clear();
+    ctx->folds.tokens.clear();
+    SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, nullptr, ctx->main, sh));
+  }
+  if (sh && !sh->rows().empty()) {
+    std::vector<int32_t> tok, hints;
+    std::vector<double> val;
+    std::vector<int64_t> off{0};
+    for (const auto &r : sh->rows()) {
+      tok.insert(tok.end(), pop->tokens + r.tok, pop->tokens + r.tok + r.size);
+      val.insert(val.end(), pop->values + r.tok, pop->values + r.tok + r.size);
+      hints.resize(tok.size());
+      sh->mark_row(r, hints.data() + off.back());
+      off.push_back(static_cast<int64_t>(tok.size()));
+    }
+    const int R = static_cast<int>(sh->rows().size());
+    SR_TRY(compile_set(ctx, R, tok.data(), val.data(), off.data(), hints.data(), ctx->rows));
+    for (int r = 0; r < R; ++r) ctx->rows.h_row.p[r] = r;
+    SR_TRY(plan_set(ctx, ctx->rows, true, 8, sr::kMaxWarps));
+    SR_TRY(upload_set(ctx, ctx->rows, true));
+    ctx->main.n_derived = R;
+  }
+  ctx->prep_stats.host_compile_time_ms += now_ms() - tc0;
+  return prepare_main_shape(ctx, true, false);
+}
+
+// Batched programs, shared work found and taken out where that pays.
+static sr_status prepare_batched(sr_context *ctx, const sr_population *pop) {
   const double tc0 = now_ms();
   sr::Sharing &sh = ctx->sharing;
   ctx->rows.plan = sr::Plan{};
   bool share = sharing_pays(ctx, pop);
   if (share) {
     SR_TRACE("sr: share");
-    share = sh.find(E, pop->tokens, pop->values, pop->offsets, derived_row_limit(ctx, 3),
-                    ctx->workers, host_threads(ctx));
+    share = sh.find(pop->num_exprs, pop->tokens, pop->values, pop->offsets,
+                    derived_row_limit(ctx, 3), ctx->workers, host_threads(ctx));
     // Rows are an option: without the memory for them they are evaluated in
     // place like everything else.
     if (share && !sh.rows().empty() &&
@@ -309,36 +343,19 @@ static sr_status prepare_batched(sr_context *ctx, const sr_population *pop) {
       sh.drop_rows();
     }
   }
-  SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, nullptr, ctx->main,
-                     share ? &sh : nullptr));
-  // Programs of long expressions can need a fourth spill slot: fewer rows then.
-  if (share && ctx->main.smax > 3 &&
-      static_cast<int>(sh.rows().size()) > derived_row_limit(ctx, 4)) {
-    sh.keep_rows(derived_row_limit(ctx, 4));
+  ctx->prep_stats.host_compile_time_ms = now_ms() - tc0;
+  sr_status st = prepare_programs(ctx, pop, share ? &sh : nullptr);
+  // derived_row_limit counts the spill slots of the shapes chosen here; a shape
+  // given from outside may leave the rows no shared memory.
+  if (st == SR_ERR_UNSUPPORTED && share && !sh.rows().empty()) {
+    SR_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // the rows' upload
+    ctx->last_error.clear();
     ctx->folds.refs.clear();
     ctx->folds.tokens.clear();
-    SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, nullptr, ctx->main, &sh));
+    sh.drop_rows();
+    st = prepare_programs(ctx, pop, &sh);
   }
-  if (share && !sh.rows().empty()) {
-    std::vector<int32_t> tok, hints;
-    std::vector<double> val;
-    std::vector<int64_t> off{0};
-    for (const auto &r : sh.rows()) {
-      tok.insert(tok.end(), pop->tokens + r.tok, pop->tokens + r.tok + r.size);
-      val.insert(val.end(), pop->values + r.tok, pop->values + r.tok + r.size);
-      hints.resize(tok.size());
-      sh.mark_row(r, hints.data() + off.back());
-      off.push_back(static_cast<int64_t>(tok.size()));
-    }
-    const int R = static_cast<int>(sh.rows().size());
-    SR_TRY(compile_set(ctx, R, tok.data(), val.data(), off.data(), hints.data(), ctx->rows));
-    for (int r = 0; r < R; ++r) ctx->rows.h_row.p[r] = r;
-    SR_TRY(plan_set(ctx, ctx->rows, true, 8, sr::kMaxWarps));
-    SR_TRY(upload_set(ctx, ctx->rows, true));
-    ctx->main.n_derived = R;
-  }
-  ctx->prep_stats.host_compile_time_ms = now_ms() - tc0;
-  SR_TRY(prepare_main_shape(ctx, true, false));
+  SR_TRY(st);
   ctx->prep_stats.node_evals = ctx->main.n_tokens * ctx->N;
   ctx->prep_stats.node_evals_executed = ctx->prep_stats.node_evals;
   return SR_OK;
@@ -458,6 +475,9 @@ sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, i
     return sr::interp_smem_bytes(dpt, W, rows, p.s_smem, static_cast<int>(sp), p.G, pred);
   };
   while (span > tile && smem_at(span) > max_smem) span = std::max<int64_t>(tile, (span / 2) / tile * tile);
+  if (smem_at(span) > max_smem)
+    return ctx->fail(SR_ERR_UNSUPPORTED, "launch shape needs " + std::to_string(smem_at(span)) +
+                                             " bytes of shared memory");
   // Then, while the span's shared memory (the X buffers grow with the
   // variable count) rather than the registers limits the resident blocks,
   // halve it: more resident warps pay for more, shorter work items
@@ -476,9 +496,6 @@ sr_status plan_set(sr_context *ctx, ProgramSet &ps, bool pred, int dpt, int W, i
   if (span % tile != 0) return ctx->fail(SR_ERR_UNSUPPORTED, "span is not a multiple of the tile");
   p.span = static_cast<int>(span);
   p.smem = smem_at(p.span);
-  if (p.smem > max_smem)
-    return ctx->fail(SR_ERR_UNSUPPORTED, "launch shape needs " + std::to_string(p.smem) +
-                                             " bytes of shared memory");
   p.n_spans = (ctx->N == 0 || E == 0) ? 0 : static_cast<int>((ctx->N + span - 1) / span);
   // Spans per work item: as many as keep about 32 items of 32 expressions
   // per SM (up to 32 spans), so the per-(span group, expression) entries stay
