@@ -326,7 +326,7 @@ static sr_status prepare_programs(sr_context *ctx, const sr_population *pop, sr:
 }
 
 // Batched programs, shared work found and taken out where that pays.
-static sr_status prepare_batched(sr_context *ctx, const sr_population *pop) {
+static sr_status prepare_batched(sr_context *ctx, const sr_population *pop, bool with_rows) {
   const double tc0 = now_ms();
   sr::Sharing &sh = ctx->sharing;
   ctx->rows.plan = sr::Plan{};
@@ -334,7 +334,7 @@ static sr_status prepare_batched(sr_context *ctx, const sr_population *pop) {
   if (share) {
     SR_TRACE("sr: share");
     share = sh.find(pop->num_exprs, pop->tokens, pop->values, pop->offsets,
-                    derived_row_limit(ctx, 3), ctx->workers, host_threads(ctx));
+                    with_rows ? derived_row_limit(ctx, 3) : 0, ctx->workers, host_threads(ctx));
     // Rows are an option: without the memory for them they are evaluated in
     // place like everything else.
     if (share && !sh.rows().empty() &&
@@ -873,6 +873,17 @@ void sr::capi::reset_prepared(sr_context *ctx) {
   ctx->graph_launches = 0;
 }
 
+// Derived rows are an option: a call that fails for want of memory (and drops
+// the prepared launch anyway) gives theirs back and tries once more.
+bool sr::capi::give_back_rows(sr_context *ctx, sr_status st) {
+  if (st != SR_ERR_OUT_OF_MEMORY || !ctx->derived.p) return false;
+  if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return false;
+  reset_prepared(ctx);
+  ctx->derived.release();
+  ctx->last_error.clear();
+  return true;
+}
+
 // Drop the dataset, the cache built on it and every prepared launch.
 void sr::capi::invalidate_data(sr_context *ctx) {
   reset_prepared(ctx);
@@ -1007,8 +1018,8 @@ sr_status sr_destroy(sr_context *ctx) {
   return SR_OK;
 }
 
-sr_status sr_set_data_device(sr_context *ctx, const float *X_dev, int64_t ld, int32_t num_vars,
-                             int64_t num_dps) {
+static sr_status set_data_device(sr_context *ctx, const float *X_dev, int64_t ld, int32_t num_vars,
+                                 int64_t num_dps) {
   SR_TRACE("sr_set_data_device");
   if (!ctx) return SR_ERR_INVALID_ARGUMENT;
   if (num_vars < 0 || num_dps < 0 || (num_dps > 0 && !X_dev) || ld < num_dps)
@@ -1035,6 +1046,12 @@ sr_status sr_set_data_device(sr_context *ctx, const float *X_dev, int64_t ld, in
   ctx->V = num_vars;
   ctx->N = num_dps;
   return SR_OK;
+}
+
+sr_status sr_set_data_device(sr_context *ctx, const float *X_dev, int64_t ld, int32_t num_vars,
+                             int64_t num_dps) {
+  const sr_status st = set_data_device(ctx, X_dev, ld, num_vars, num_dps);
+  return ctx && give_back_rows(ctx, st) ? set_data_device(ctx, X_dev, ld, num_vars, num_dps) : st;
 }
 
 static sr_status set_data_host(sr_context *ctx, const float *X, const float *const *rows_ptr,
@@ -1076,14 +1093,20 @@ static sr_status set_data_host(sr_context *ctx, const float *X, const float *con
   return SR_OK;
 }
 
+static sr_status set_data(sr_context *ctx, const float *X, const float *const *rows,
+                          int32_t num_vars, int64_t num_dps) {
+  const sr_status st = set_data_host(ctx, X, rows, num_vars, num_dps);
+  return ctx && give_back_rows(ctx, st) ? set_data_host(ctx, X, rows, num_vars, num_dps) : st;
+}
+
 sr_status sr_set_data(sr_context *ctx, const float *X, int32_t num_vars, int64_t num_dps) {
-  return set_data_host(ctx, X, nullptr, num_vars, num_dps);
+  return set_data(ctx, X, nullptr, num_vars, num_dps);
 }
 
 sr_status sr_set_data_rows(sr_context *ctx, const float *const *rows, int32_t num_vars,
                            int64_t num_dps) {
   if (ctx && num_dps > 0 && !rows) return ctx->fail(SR_ERR_INVALID_ARGUMENT, "rows is NULL");
-  return set_data_host(ctx, nullptr, rows, num_vars, num_dps);
+  return set_data(ctx, nullptr, rows, num_vars, num_dps);
 }
 
 }  // extern "C"
@@ -1374,13 +1397,9 @@ sr_status prepare_cached(sr_context *ctx, const sr_population *pop, uint32_t fla
 
 extern "C" {
 
-sr_status sr_prepare(sr_context *ctx, const sr_population *pop, uint32_t flags) {
-  SR_TRACE("sr_prepare");
-  if (!ctx) return SR_ERR_INVALID_ARGUMENT;
-  ctx->last_error.clear();
-  SR_TRY(check_population(ctx, pop));
-  if (ctx->V < 0) return ctx->fail(SR_ERR_NO_DATA, "no dataset: call sr_set_data first");
-  DeviceScope scope(ctx->device);
+// One attempt; without derived rows (with_rows = false) after memory ran out.
+static sr_status prepare_once(sr_context *ctx, const sr_population *pop, uint32_t flags,
+                              bool with_rows) {
   SR_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   reset_prepared(ctx);
   ctx->prep_stats = sr_stats{};
@@ -1403,11 +1422,22 @@ sr_status sr_prepare(sr_context *ctx, const sr_population *pop, uint32_t flags) 
     SR_TRY(prepare_cached(ctx, pop, flags));
     ctx->mode = sr::Mode::kCached;
   } else {
-    SR_TRY(prepare_batched(ctx, pop));
+    SR_TRY(prepare_batched(ctx, pop, with_rows));
     ctx->mode = sr::Mode::kBatched;
   }
   SR_TRY_CUDA(ctx, cudaEventRecord(ctx->ev[5], ctx->stream));
   return SR_OK;
+}
+
+sr_status sr_prepare(sr_context *ctx, const sr_population *pop, uint32_t flags) {
+  SR_TRACE("sr_prepare");
+  if (!ctx) return SR_ERR_INVALID_ARGUMENT;
+  ctx->last_error.clear();
+  SR_TRY(check_population(ctx, pop));
+  if (ctx->V < 0) return ctx->fail(SR_ERR_NO_DATA, "no dataset: call sr_set_data first");
+  DeviceScope scope(ctx->device);
+  const sr_status st = prepare_once(ctx, pop, flags, true);
+  return give_back_rows(ctx, st) ? prepare_once(ctx, pop, flags, false) : st;
 }
 
 // Where each expression's result is, when equal ones share an evaluation.
@@ -1683,6 +1713,22 @@ sr_status sr_eval_mse(sr_context *ctx, const sr_population *pop, uint32_t flags,
   return SR_OK;
 }
 
+// Programs, shape and output buffer of a prediction launch.
+static sr_status prepare_predictions(sr_context *ctx, const sr_population *pop) {
+  const int E = pop->num_exprs;
+  SR_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  reset_prepared(ctx);
+  SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, nullptr, ctx->main));
+  for (int x = 0; x < E; ++x) ctx->main.h_row.p[x] = x;
+  int dpt = ctx->opts.dpt ? ctx->opts.dpt : 8;
+  int W = ctx->opts.warps_per_block ? std::min(ctx->opts.warps_per_block, sr::kMaxWarps)
+                                     : sr::kMaxWarps;
+  SR_TRY(plan_set(ctx, ctx->main, true, dpt, W));
+  SR_TRY(upload_set(ctx, ctx->main, true));
+  SR_TRY_CUDA(ctx, ctx->pred.ensure(static_cast<size_t>(E) * ctx->ldx));
+  return SR_OK;
+}
+
 sr_status sr_eval_predictions(sr_context *ctx, const sr_population *pop, int64_t dp_begin,
                               int64_t dp_count, float *pred_out) {
   SR_TRACE("sr_eval_predictions");
@@ -1699,16 +1745,8 @@ sr_status sr_eval_predictions(sr_context *ctx, const sr_population *pop, int64_t
   if (bytes > 16.0 * (1ull << 30))
     return ctx->fail(SR_ERR_UNSUPPORTED, "prediction buffer would exceed 16 GiB");
   DeviceScope scope(ctx->device);
-  SR_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  reset_prepared(ctx);
-  SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, nullptr, ctx->main));
-  for (int x = 0; x < E; ++x) ctx->main.h_row.p[x] = x;
-  int dpt = ctx->opts.dpt ? ctx->opts.dpt : 8;
-  int W = ctx->opts.warps_per_block ? std::min(ctx->opts.warps_per_block, sr::kMaxWarps)
-                                     : sr::kMaxWarps;
-  SR_TRY(plan_set(ctx, ctx->main, true, dpt, W));
-  SR_TRY(upload_set(ctx, ctx->main, true));
-  SR_TRY_CUDA(ctx, ctx->pred.ensure(static_cast<size_t>(E) * ctx->ldx));
+  const sr_status st = prepare_predictions(ctx, pop);
+  SR_TRY(give_back_rows(ctx, st) ? prepare_predictions(ctx, pop) : st);
   SR_TRY(begin_sequence(ctx));
   SR_TRY(launch_set(ctx, ctx->main, true, ctx->d_counter, ctx->pred.p, ctx->ldx, ctx->main.row.p));
   SR_TRY_CUDA(ctx, cudaMemcpy2DAsync(pred_out, dp_count * sizeof(float), ctx->pred.p + dp_begin,

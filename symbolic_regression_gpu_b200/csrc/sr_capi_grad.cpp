@@ -640,8 +640,12 @@ sr_status sr_optimize_constants(sr_context *ctx, const sr_population *pop,
   reset_prepared(ctx);
   ctx->prep_stats = sr_stats{};
   ctx->E = pop->num_exprs;
-  SR_TRY(prepare_grad(ctx, pop, store == SR_GRAD_RECOMPUTE,
-                      (adam->mode & SR_GRAD_REVERSE_ONLY) != 0));
+  const auto prepare = [&] {
+    return prepare_grad(ctx, pop, store == SR_GRAD_RECOMPUTE,
+                        (adam->mode & SR_GRAD_REVERSE_ONLY) != 0);
+  };
+  const sr_status st = prepare();
+  SR_TRY(give_back_rows(ctx, st) ? prepare() : st);
   ctx->mode = sr::Mode::kGrad;
   sr::GradSet &g = ctx->grad;
   cudaStream_t s = ctx->stream;

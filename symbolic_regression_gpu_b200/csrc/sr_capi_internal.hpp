@@ -65,6 +65,9 @@ sr_status launch_set(sr_context *ctx, ProgramSet &ps, bool pred, int32_t *counte
 sr_status prepare_main_shape(sr_context *ctx, bool allow_tune, bool on_device);
 cudaError_t record_event(sr_context *ctx, int k);
 void reset_prepared(sr_context *ctx);
+// After a step that returned st: whether the derived rows' memory has been given
+// back, so that the step is worth another try.  Nothing is prepared then.
+bool give_back_rows(sr_context *ctx, sr_status st);
 void invalidate_data(sr_context *ctx);
 sr_status check_device_error(sr_context *ctx);
 void fill_stats(sr_context *ctx, sr_stats *st);

@@ -201,18 +201,9 @@ sr_status sr_evolve_step(sr_context *ctx, const sr_evolve_options *opts, int32_t
   return SR_OK;
 }
 
-sr_status sr_prepare_device_population(sr_context *ctx, const int32_t *tokens,
-                                       const float *values, const int32_t *lengths,
-                                       int32_t num_exprs, int32_t stride) {
-  SR_TRACE("sr_prepare_device_population");
-  if (!ctx) return SR_ERR_INVALID_ARGUMENT;
-  ctx->last_error.clear();
-  if (num_exprs < 0 || stride < 1 || stride > SR_EVOLVE_MAX_STRIDE)
-    return ctx->fail(SR_ERR_INVALID_ARGUMENT, "bad population size or stride");
-  if (num_exprs > 0 && (!tokens || !values || !lengths))
-    return ctx->fail(SR_ERR_INVALID_ARGUMENT, "NULL buffer");
-  if (ctx->V < 0) return ctx->fail(SR_ERR_NO_DATA, "no dataset: call sr_set_data first");
-  DeviceScope scope(ctx->device);
+static sr_status prepare_device_population(sr_context *ctx, const int32_t *tokens,
+                                           const float *values, const int32_t *lengths,
+                                           int32_t num_exprs, int32_t stride) {
   SR_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   reset_prepared(ctx);
   ctx->prep_stats = sr_stats{};
@@ -273,6 +264,25 @@ sr_status sr_prepare_device_population(sr_context *ctx, const int32_t *tokens,
   ctx->prep_stats.node_evals_executed = ctx->prep_stats.node_evals;
   ctx->mode = sr::Mode::kBatched;
   return SR_OK;
+}
+
+sr_status sr_prepare_device_population(sr_context *ctx, const int32_t *tokens,
+                                       const float *values, const int32_t *lengths,
+                                       int32_t num_exprs, int32_t stride) {
+  SR_TRACE("sr_prepare_device_population");
+  if (!ctx) return SR_ERR_INVALID_ARGUMENT;
+  ctx->last_error.clear();
+  if (num_exprs < 0 || stride < 1 || stride > SR_EVOLVE_MAX_STRIDE)
+    return ctx->fail(SR_ERR_INVALID_ARGUMENT, "bad population size or stride");
+  if (num_exprs > 0 && (!tokens || !values || !lengths))
+    return ctx->fail(SR_ERR_INVALID_ARGUMENT, "NULL buffer");
+  if (ctx->V < 0) return ctx->fail(SR_ERR_NO_DATA, "no dataset: call sr_set_data first");
+  DeviceScope scope(ctx->device);
+  const sr_status st =
+      prepare_device_population(ctx, tokens, values, lengths, num_exprs, stride);
+  return give_back_rows(ctx, st)
+             ? prepare_device_population(ctx, tokens, values, lengths, num_exprs, stride)
+             : st;
 }
 
 sr_status sr_get_stream(sr_context *ctx, void **stream) {
