@@ -398,9 +398,11 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1) adj_kernel(const AdjA
         acc += __shfl_xor_sync(0xffffffffu, acc, o);
         cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
       }
+      // By the expression's place in the list of reverse-mode ones: a few among
+      // many need little memory, whatever the population's size.
       if (lane == 0)
-        p.partial[static_cast<int64_t>(d.span) * p.E + e] =
-            make_double2(acc, static_cast<double>(cnt));
+        p.partial[static_cast<int64_t>(d.span) * a.n_rev + static_cast<int64_t>(d.group) * p.G +
+                  j] = make_double2(acc, static_cast<double>(cnt));
       const int64_t coff = a.const_off[e];
       for (uint32_t c = 0; c < nconst; ++c) {
         double g = gacc[c * 32 + lane];
@@ -420,7 +422,7 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1) adj_kernel(const AdjA
 
 // One warp per expression, its lanes the spans (see finalize_dd_kernel).
 __global__ void __launch_bounds__(256)
-    grad_finalize_kernel(const double2 *__restrict__ partial, int n_spans, int E,
+    grad_finalize_kernel(const double2 *__restrict__ partial, int n_spans,
                          const int32_t *__restrict__ exprs, int n_exprs,
                          const int64_t *__restrict__ const_off,
                          const int32_t *__restrict__ const_cnt,
@@ -434,7 +436,7 @@ __global__ void __launch_bounds__(256)
   const int e = exprs[q_];
   double s = 0.0, c = 0.0;
   for (int k = lane; k < n_spans; k += 32) {
-    const double2 q = partial[static_cast<int64_t>(k) * E + e];
+    const double2 q = partial[static_cast<int64_t>(k) * n_exprs + q_];
     s += q.x;
     c += q.y;
   }
@@ -522,14 +524,14 @@ cudaError_t launch_adjoint(const AdjArgs &args, bool recompute, int blocks, size
 
 int adj_segment() { return kSeg; }
 
-cudaError_t launch_grad_finalize(const double2 *partial, int n_spans, int E,
+cudaError_t launch_grad_finalize(const double2 *partial, int n_spans,
                                  const int32_t *exprs, int n_exprs, const int64_t *const_off,
                                  const int32_t *const_cnt, const double *grad_acc, float *mse,
                                  float *grad, double2 *sums, SequenceEnd end,
                                  cudaStream_t stream) {
   if (n_exprs <= 0) return cudaSuccess;
   grad_finalize_kernel<<<(n_exprs + 7) / 8, 256, 0, stream>>>(
-      partial, n_spans, E, exprs, n_exprs, const_off, const_cnt, grad_acc, mse, grad, sums, end);
+      partial, n_spans, exprs, n_exprs, const_off, const_cnt, grad_acc, mse, grad, sums, end);
   return cudaGetLastError();
 }
 

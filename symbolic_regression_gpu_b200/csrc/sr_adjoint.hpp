@@ -22,7 +22,7 @@ struct AdjArgs {
   const int4 *cinfo;          // [C] path offset, length, constants of a folded subtree
   const float *path;          // partials from a folded subtree's root to each constant
   int32_t seg_cap;            // recompute mode: segment-tape entries (min(segment, longest))
-  int32_t reserved0;
+  int32_t n_rev;              // reverse-mode expressions of all classes (e.partial: [span][n_rev])
 };
 
 // Forward-mode (tangent) launch: the expressions with at most
@@ -80,7 +80,7 @@ cudaError_t launch_adjoint(const AdjArgs &args, bool recompute, int blocks, size
                            cudaStream_t stream);
 // mse / grad (and the (sum, count) sums) of the n_exprs reverse-mode
 // expressions listed in exprs.
-cudaError_t launch_grad_finalize(const double2 *partial, int n_spans, int E,
+cudaError_t launch_grad_finalize(const double2 *partial, int n_spans,
                                  const int32_t *exprs, int n_exprs, const int64_t *const_off,
                                  const int32_t *const_cnt, const double *grad_acc, float *mse,
                                  float *grad, double2 *sums, SequenceEnd end,

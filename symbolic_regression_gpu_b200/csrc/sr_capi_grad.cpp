@@ -219,7 +219,7 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
   g.span = static_cast<int>(std::min<int64_t>(span, std::max<int64_t>(tile, round_up(ctx->N, tile))));
   g.n_spans = (ctx->N == 0) ? 0 : static_cast<int>((ctx->N + g.span - 1) / g.span);
   g.classes.clear();
-  std::vector<int32_t> table;
+  std::vector<int32_t> table, rev_list;
   int64_t spill_floats = 0, gtape_floats = 0;
   const int s_smem = std::min(ps.smax, sr::smem_spill_slots(dpt));
   for (int k = 0; k < kNumClasses; ++k) {
@@ -302,6 +302,8 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
     cl.group_off = static_cast<int64_t>(table.size());
     for (int64_t q = 0; q < static_cast<int64_t>(p.n_groups) * p.G; ++q)
       table.push_back(q < static_cast<int64_t>(mem.size()) ? mem[static_cast<size_t>(q)] : -1);
+    cl.rev_off = static_cast<int64_t>(rev_list.size());
+    rev_list.insert(rev_list.end(), mem.begin(), mem.end());
     g.classes.push_back(cl);
   }
   // Forward-mode launches: the interpreter's shape (span groups folded by
@@ -375,13 +377,16 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
     g.tsets.push_back(ts);
   }
   g.rev_expr_off = static_cast<int64_t>(expr_list.size());
-  expr_list.insert(expr_list.end(), rev_members.begin(), rev_members.end());
+  expr_list.insert(expr_list.end(), rev_list.begin(), rev_list.end());
+  // Reverse-mode span sums: one (sum, count) per span and reverse-mode
+  // expression, at its place in the list.
+  const int64_t rev_part = static_cast<int64_t>(g.n_spans) * g.n_rev;
   {
-    const double need = static_cast<double>(tan_part) * sizeof(double2) +
+    const double need = static_cast<double>(tan_part + rev_part) * sizeof(double2) +
                         static_cast<double>(tan_gout) * sizeof(double);
     if (need > 0.9 * static_cast<double>(ctx->device_memory))
       return ctx->fail(SR_ERR_UNSUPPORTED,
-                       "forward-mode span sums (" + std::to_string(static_cast<int64_t>(need)) +
+                       "gradient span sums (" + std::to_string(static_cast<int64_t>(need)) +
                            " bytes) exceed the device memory; split the population or the "
                            "datapoints");
   }
@@ -458,8 +463,7 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
   if (tan_part > 0) SR_TRY_CUDA(ctx, g.tan_partial.ensure(static_cast<size_t>(tan_part)));
   if (tan_gout > 0) SR_TRY_CUDA(ctx, g.tan_gout.ensure(static_cast<size_t>(tan_gout)));
   if (g.n_rev > 0)
-    SR_TRY_CUDA(ctx, ctx->partial.ensure(static_cast<size_t>(
-                         std::max<int64_t>(static_cast<int64_t>(g.n_spans) * E, 1))));
+    SR_TRY_CUDA(ctx, ctx->partial.ensure(static_cast<size_t>(std::max<int64_t>(rev_part, 1))));
   SR_TRY_CUDA(ctx, g.h_exprs.ensure(std::max<size_t>(expr_list.size(), 1)));
   if (!expr_list.empty())
     std::memcpy(g.h_exprs.p, expr_list.data(), expr_list.size() * sizeof(int32_t));
@@ -559,6 +563,8 @@ sr_status launch_grad(sr_context *ctx) {
     a.e.span = cl.plan.span;
     a.e.n_spans = cl.plan.n_spans;
     a.e.group_expr = g.groups.p + cl.group_off;
+    a.e.partial = ctx->partial.p + cl.rev_off;
+    a.n_rev = g.n_rev;
     a.const_off = g.const_off.p;
     a.const_cnt = g.const_cnt.p;
     a.bwd_lo = g.bwd_lo.p;
@@ -580,7 +586,7 @@ sr_status launch_grad(sr_context *ctx) {
                          g.const_off.p, g.const_cnt.p, ts.K, ctx->mse.p, g.grad.p, g.grad_acc.p,
                          ctx->sums.p, end, s));
   if (g.n_rev > 0)
-    SR_TRY_CUDA(ctx, sr::launch_grad_finalize(ctx->partial.p, g.n_spans, ps.E,
+    SR_TRY_CUDA(ctx, sr::launch_grad_finalize(ctx->partial.p, g.n_spans,
                                               g.exprs.p + g.rev_expr_off, g.n_rev, g.const_off.p,
                                               g.const_cnt.p, g.grad_acc.p, ctx->mse.p, g.grad.p,
                                               ctx->sums.p, end, s));

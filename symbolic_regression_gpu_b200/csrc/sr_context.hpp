@@ -215,6 +215,7 @@ struct AdjClass {
   bool global_tape = false;  // tape in per-warp global scratch instead of shared memory
   int seg_cap = 0;           // recompute mode: segment-tape entries
   int64_t group_off = 0;     // into the concatenated group table
+  int64_t rev_off = 0;       // into the list of reverse-mode expressions
   Plan plan;
 };
 
