@@ -39,7 +39,8 @@ struct TanArgs {
   const int32_t *const_cnt;   // [E] constants of each expression
   const float *tinit;         // [C] tangent a constant enters with
   double *gout;               // [span groups][C] gradient sums per span group
-  int64_t C;                  // constants of the population
+  const int64_t *gout_off;    // [E] first constant of each expression there
+  int64_t C;                  // constants of the launch's expressions
   int32_t n_valid;            // expressions in the group table
   int32_t K;                  // tangent rows per warp (>= the constants of any expression)
 };
@@ -61,9 +62,10 @@ cudaError_t tan_configure(int K, size_t smem, int W, int *blocks_per_sm);
 // sequence is valid on its own.
 cudaError_t tan_set_smem_limit(int K, size_t smem);
 cudaError_t launch_tangent(const TanArgs &args, int blocks, size_t smem, cudaStream_t stream);
-cudaError_t launch_tan_finalize(const double2 *partial, const double *gout, int n_groups, int E,
+cudaError_t launch_tan_finalize(const double2 *partial, const double *gout, int n_groups,
                                 int64_t C, const int32_t *exprs, int n_exprs,
-                                const int64_t *const_off, const int32_t *const_cnt, int K,
+                                const int64_t *const_off, const int64_t *gout_off,
+                                const int32_t *const_cnt, int K,
                                 float *mse, float *grad, double *gsum, double2 *sums,
                                 SequenceEnd end, cudaStream_t stream);
 

@@ -99,7 +99,7 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
     fold_n[static_cast<size_t>(f.loc)] = static_cast<uint8_t>(f.nc);
   }
   // Constants: CSR offsets and the bytecode word that holds each one.
-  SR_TRY_CUDA(ctx, g.h_const_off.ensure(static_cast<size_t>(E) + 1));
+  SR_TRY_CUDA(ctx, g.h_const_off.ensure(2 * static_cast<size_t>(E) + 1));
   SR_TRY_CUDA(ctx, g.h_const_cnt.ensure(static_cast<size_t>(std::max(E, 1))));
   int64_t C = 0;
   int gmax = 0;
@@ -307,7 +307,11 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
     g.classes.push_back(cl);
   }
   // Forward-mode launches: the interpreter's shape (span groups folded by
-  // each block's producer).
+  // each block's producer).  Their sums count the set's own expressions and
+  // constants: a few among many need little memory, whatever the population's
+  // size.
+  int64_t *set_off = g.h_const_off.p + E + 1;
+  std::fill_n(set_off, E, 0);
   g.tsets.clear();
   std::vector<int32_t> expr_list;
   int64_t tan_part = 0, tan_gout = 0;
@@ -370,10 +374,14 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
     ts.n_exprs = static_cast<int>(mem.size());
     ts.expr_off = static_cast<int64_t>(expr_list.size());
     expr_list.insert(expr_list.end(), mem.begin(), mem.end());
+    for (int32_t x : mem) {
+      set_off[x] = ts.C;
+      ts.C += ps.n_const[static_cast<size_t>(x)];
+    }
     ts.part_off = tan_part;
-    tan_part += 2 * static_cast<int64_t>(p.n_span_groups()) * E;
+    tan_part += 2 * static_cast<int64_t>(p.n_span_groups()) * ts.n_exprs;
     ts.gout_off = tan_gout;
-    tan_gout += static_cast<int64_t>(p.n_span_groups()) * C;
+    tan_gout += static_cast<int64_t>(p.n_span_groups()) * ts.C;
     g.tsets.push_back(ts);
   }
   g.rev_expr_off = static_cast<int64_t>(expr_list.size());
@@ -449,7 +457,7 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
   SR_TRY_CUDA(ctx, g.h_groups.ensure(std::max<size_t>(table.size(), 1)));
   if (!table.empty()) std::memcpy(g.h_groups.p, table.data(), table.size() * sizeof(int32_t));
   SR_TRY_CUDA(ctx, g.groups.ensure(std::max<size_t>(table.size(), 1)));
-  SR_TRY_CUDA(ctx, g.const_off.ensure(static_cast<size_t>(E) + 1));
+  SR_TRY_CUDA(ctx, g.const_off.ensure(2 * static_cast<size_t>(E) + 1));
   SR_TRY_CUDA(ctx, g.const_cnt.ensure(static_cast<size_t>(std::max(E, 1))));
   SR_TRY_CUDA(ctx, g.bwd_lo.ensure(static_cast<size_t>(std::max(E, 1))));
   if (gtape_floats > 0) SR_TRY_CUDA(ctx, g.gtape.ensure(static_cast<size_t>(gtape_floats)));
@@ -478,7 +486,8 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
   if (!table.empty())
     SR_TRY_CUDA(ctx, cudaMemcpyAsync(g.groups.p, g.h_groups.p, table.size() * sizeof(int32_t),
                                      cudaMemcpyHostToDevice, s));
-  SR_TRY_CUDA(ctx, cudaMemcpyAsync(g.const_off.p, g.h_const_off.p, (E + 1) * sizeof(int64_t),
+  SR_TRY_CUDA(ctx, cudaMemcpyAsync(g.const_off.p, g.h_const_off.p,
+                                   (2 * static_cast<size_t>(E) + 1) * sizeof(int64_t),
                                    cudaMemcpyHostToDevice, s));
   SR_TRY_CUDA(ctx, cudaMemcpyAsync(g.const_cnt.p, g.h_const_cnt.p, E * sizeof(int32_t),
                                    cudaMemcpyHostToDevice, s));
@@ -546,7 +555,8 @@ sr_status launch_grad(sr_context *ctx) {
     a.const_cnt = g.const_cnt.p;
     a.tinit = g.tinit.p;
     a.gout = g.tan_gout.p + ts.gout_off;
-    a.C = g.C;
+    a.gout_off = g.const_off.p + ps.E + 1;
+    a.C = ts.C;
     a.n_valid = ts.n_exprs;
     a.K = ts.K;
     SR_TRY_CUDA(ctx, sr::launch_tangent(a, ts.plan.blocks, ts.plan.smem, s));
@@ -582,9 +592,9 @@ sr_status launch_grad(sr_context *ctx) {
   for (const sr::TanSet &ts : g.tsets)
     SR_TRY_CUDA(ctx, sr::launch_tan_finalize(
                          g.tan_partial.p + ts.part_off, g.tan_gout.p + ts.gout_off,
-                         ts.plan.n_span_groups(), ps.E, g.C, g.exprs.p + ts.expr_off, ts.n_exprs,
-                         g.const_off.p, g.const_cnt.p, ts.K, ctx->mse.p, g.grad.p, g.grad_acc.p,
-                         ctx->sums.p, end, s));
+                         ts.plan.n_span_groups(), ts.C, g.exprs.p + ts.expr_off, ts.n_exprs,
+                         g.const_off.p, g.const_off.p + ps.E + 1, g.const_cnt.p, ts.K, ctx->mse.p,
+                         g.grad.p, g.grad_acc.p, ctx->sums.p, end, s));
   if (g.n_rev > 0)
     SR_TRY_CUDA(ctx, sr::launch_grad_finalize(ctx->partial.p, g.n_spans,
                                               g.exprs.p + g.rev_expr_off, g.n_rev, g.const_off.p,

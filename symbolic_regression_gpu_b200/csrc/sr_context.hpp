@@ -242,6 +242,7 @@ struct DetectBufs {
 struct TanSet {
   int K = 0;
   int n_exprs = 0;
+  int64_t C = 0;          // constants of its expressions
   int64_t group_off = 0;  // into the concatenated group table
   int64_t expr_off = 0;   // into the expression lists
   int64_t part_off = 0;   // double2 offset of its MSE sums in tan_partial
@@ -250,7 +251,8 @@ struct TanSet {
 };
 
 struct GradSet {
-  DevBuf<int64_t> const_off;
+  DevBuf<int64_t> const_off;  // [E + 1] first constant of each expression, then [E]
+                              // the same among its forward-mode set's constants
   DevBuf<int32_t> const_cnt;
   DevBuf<int64_t> const_loc;  // (instruction << 1) | (operand b); -1: in a folded subtree
   // Constant subtrees are folded in gradient launches too: fold_grad_kernel

@@ -983,7 +983,9 @@ __device__ __forceinline__ void end_sequence(const SequenceEnd &end) {
 // group table (groups are padded at their end only).  Gradient launches
 // (K > 0) also fold each expression's constant gradients: K doubles per span
 // slot, added in span order into K doubles per expression, written out to
-// gout[span group][C] at the expression's constant offset.
+// gout[span group][C] at the expression's constant offset.  Theirs cover part of
+// a population: E, C and the offsets count that part alone, and an expression's
+// entry is its place in the group table.
 struct FoldArgs {
   SpanPart *part;  // [kBufs][G]
   GroupAcc *acc;   // [G]
@@ -993,8 +995,8 @@ struct FoldArgs {
   const double *gpart;       // [kBufs][G][K]
   double *gacc;              // [G][K]
   double *gout;              // [span groups][C]
-  const int64_t *const_off;  // [E]
-  const int32_t *const_cnt;  // [E]
+  const int64_t *const_off;  // per expression of the population
+  const int32_t *const_cnt;
   int64_t C;
 };
 
@@ -1028,7 +1030,7 @@ __device__ __noinline__ void run_producer(int lane, int n_groups, int n_items, i
   uint32_t fill_phase[kBufs] = {0, 0};
   bool held[kBufs] = {false, false};  // a span whose slots are still to fold
   int held_item[kBufs] = {0, 0}, held_group[kBufs] = {0, 0};
-  int acc_item = -1, acc_sg = 0, acc_n = 0;
+  int acc_item = -1, acc_sg = 0, acc_n = 0, acc_group = 0;
   const uint32_t row_bytes = static_cast<uint32_t>(span) * sizeof(float);
   const uint32_t chunk_bytes = static_cast<uint32_t>(chunk) * sizeof(float);
 
@@ -1037,7 +1039,8 @@ __device__ __noinline__ void run_producer(int lane, int n_groups, int n_items, i
       if (acc_item < 0) return;
       for (int j = lane; j < acc_n; j += 32) {
         const GroupAcc a = fa.acc[j];
-        double2 *o = fa.out + 2 * (static_cast<int64_t>(acc_sg) * fa.E + a.e);
+        const int at = fa.K > 0 ? acc_group * fa.G + j : a.e;
+        double2 *o = fa.out + 2 * (static_cast<int64_t>(acc_sg) * fa.E + at);
         o[0] = make_double2(a.hi, a.lo);
         o[1] = make_double2(a.cnt, 0.0);
         if (fa.K > 0) {
@@ -1056,8 +1059,8 @@ __device__ __noinline__ void run_producer(int lane, int n_groups, int n_items, i
         flush();
         acc_item = it;
         acc_sg = it % ((n_spans + k_spans - 1) / k_spans);
-        const int g = held_group[b];
-        acc_n = min(fa.G, fa.n_valid - g * fa.G);  // groups are padded at their end only
+        acc_group = held_group[b];
+        acc_n = min(fa.G, fa.n_valid - acc_group * fa.G);  // groups are padded at their end only
         for (int j = lane; j < acc_n; j += 32) {
           fa.acc[j] = GroupAcc{0.0, 0.0, 0.0, 0, 0};
           for (int c = 0; c < fa.K; ++c) fa.gacc[j * fa.K + c] = 0.0;

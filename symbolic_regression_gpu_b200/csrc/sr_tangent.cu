@@ -237,8 +237,8 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) tan_kernel(const TanArg
   if (warp == W) {
     run_producer<true>(lane, p.n_groups, n_items, k_spans, p.n_spans, p.work_counter, p.error, p.X,
                          nullptr, rows, p.ldx, rows, span, span, xbuf, desc, full, empty,
-                         FoldArgs{part, gacc, p.partial, p.G, p.E, a.n_valid, K, gpart, ggacc,
-                                  a.gout, a.const_off, a.const_cnt, a.C});
+                         FoldArgs{part, gacc, p.partial, p.G, a.n_valid, a.n_valid, K, gpart, ggacc,
+                                  a.gout, a.gout_off, a.const_cnt, a.C});
     return;
   }
 
@@ -430,8 +430,9 @@ __global__ void __launch_bounds__(64)
 // so that their loads overlap.
 __global__ void __launch_bounds__(256)
     tan_finalize_kernel(const double2 *__restrict__ partial, const double *__restrict__ gout,
-                        int n_groups, int E, int64_t C, const int32_t *__restrict__ exprs,
+                        int n_groups, int64_t C, const int32_t *__restrict__ exprs,
                         int n_exprs, const int64_t *__restrict__ const_off,
+                        const int64_t *__restrict__ gout_off,
                         const int32_t *__restrict__ const_cnt, int K, float *__restrict__ mse,
                         float *__restrict__ grad, double *__restrict__ gsum,
                         double2 *__restrict__ sums, SequenceEnd end) {
@@ -441,18 +442,18 @@ __global__ void __launch_bounds__(256)
   if (q >= n_exprs) return;  // warp-uniform
   const int e = exprs[q];
   const int nc = min(const_cnt[e], K);
-  const int64_t o = const_off[e];
+  const int64_t o = const_off[e], og = gout_off[e];
   double hi = 0.0, lo = 0.0, cnt = 0.0;
   double g[kMaxTangentConsts];
 #pragma unroll
   for (int c = 0; c < kMaxTangentConsts; ++c) g[c] = 0.0;
   for (int k = lane; k < n_groups; k += 32) {
-    const double2 *pp = partial + 2 * (static_cast<int64_t>(k) * E + e);
+    const double2 *pp = partial + 2 * (static_cast<int64_t>(k) * n_exprs + q);
     const double2 v = pp[0];
     dd_add(hi, lo, v.x);
     dd_add(hi, lo, v.y);
     cnt += pp[1].x;
-    const double *gk = gout + static_cast<int64_t>(k) * C + o;
+    const double *gk = gout + static_cast<int64_t>(k) * C + og;
 #pragma unroll
     for (int c = 0; c < kMaxTangentConsts; ++c)
       if (c < nc) g[c] += gk[c];
@@ -539,15 +540,16 @@ cudaError_t launch_fold_grad(const GradFold *items, const uint2 *tokens, int n,
   return cudaGetLastError();
 }
 
-cudaError_t launch_tan_finalize(const double2 *partial, const double *gout, int n_groups, int E,
+cudaError_t launch_tan_finalize(const double2 *partial, const double *gout, int n_groups,
                                 int64_t C, const int32_t *exprs, int n_exprs,
-                                const int64_t *const_off, const int32_t *const_cnt, int K,
+                                const int64_t *const_off, const int64_t *gout_off,
+                                const int32_t *const_cnt, int K,
                                 float *mse, float *grad, double *gsum, double2 *sums,
                                 SequenceEnd end, cudaStream_t stream) {
   if (n_exprs <= 0) return cudaSuccess;
   tan_finalize_kernel<<<(n_exprs + 7) / 8, 256, 0, stream>>>(
-      partial, gout, n_groups, E, C, exprs, n_exprs, const_off, const_cnt, K, mse, grad, gsum,
-      sums, end);
+      partial, gout, n_groups, C, exprs, n_exprs, const_off, gout_off, const_cnt, K, mse, grad,
+      gsum, sums, end);
   return cudaGetLastError();
 }
 
