@@ -164,7 +164,9 @@ typedef struct sr_stats {
   double host_compile_time_ms;  /* token validation + bytecode compilation    */
   double eval_kernel_time_ms;   /* main interpreter kernel only               */
   int64_t node_evals;           /* sum(tokens) * num_dps (original expressions) */
-  int64_t node_evals_executed;  /* node-evals actually computed (cache skips some) */
+  int64_t node_evals_executed;  /* node-evals actually computed: cached and shared
+                                   subtrees, equal expressions and subtrees of
+                                   constants are not evaluated again          */
   int32_t kernel_launches;      /* launches of this library's kernels         */
   int32_t cache_slots_used;
   int32_t dpt;                  /* launch shape used                          */
@@ -172,7 +174,7 @@ typedef struct sr_stats {
   int32_t blocks;
   int32_t work_items;
   /* Declared work of one launch of the main kernel (roofline model: operator
-   * counts per datapoint summed over expressions, times num_dps). */
+   * counts per datapoint summed over the programs it runs, times num_dps). */
   double declared_sfu_ops;
   double declared_fp32_ops;
   /* Bytes copied host->device / device->host by the call. */

@@ -103,7 +103,7 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
   ps.n_const.assign(static_cast<size_t>(E), 0);
   ps.smax = 0;
   ps.n_instr = 0;
-  ps.n_tokens = 0;
+  ps.n_tokens = ps.n_executed = 0;
   ps.sfu_per_dp = ps.fp32_per_dp = 0.0;
   ps.n_derived = 0;
   // About 20 ns a token, and tens of microseconds to wake the workers: chunks
@@ -139,8 +139,6 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
         if (r == x && share->mark(static_cast<int>(x), marks.data())) h = marks.data();
         if (r != x) {
           info.n_tokens = len;
-          sr::declared_work(tok + off[x], len, &info.sfu_ops, &info.fp32_ops);
-          info.fp32_ops += 3.0;
           continue;
         }
       }
@@ -156,10 +154,6 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
         c.st = s;
         c.bad = x;
         return;
-      }
-      if (share) {  // the declared work is that of the whole expression
-        sr::declared_work(tok + off[x], len, &info.sfu_ops, &info.fp32_ops);
-        info.fp32_ops += 3.0;
       }
       for (const sr::FoldRef &f : refs) {
         const int64_t t0 = off[x] + f.tok;
@@ -223,6 +217,7 @@ sr_status compile_set(sr_context *ctx, int E, const int32_t *tok, const double *
     ps.n_const[static_cast<size_t>(x)] = in.n_const;
     ps.smax = std::max(ps.smax, in.need);
     ps.n_tokens += in.n_tokens;
+    ps.n_executed += in.n_executed;
     ps.sfu_per_dp += in.sfu_ops;
     ps.fp32_per_dp += in.fp32_ops;
     if (share) {
@@ -356,8 +351,9 @@ static sr_status prepare_batched(sr_context *ctx, const sr_population *pop, bool
     st = prepare_programs(ctx, pop, &sh);
   }
   SR_TRY(st);
+  const int64_t row_tokens = ctx->main.n_derived > 0 ? ctx->rows.n_executed : 0;
   ctx->prep_stats.node_evals = ctx->main.n_tokens * ctx->N;
-  ctx->prep_stats.node_evals_executed = ctx->prep_stats.node_evals;
+  ctx->prep_stats.node_evals_executed = (ctx->main.n_executed + row_tokens) * ctx->N;
   return SR_OK;
 }
 
@@ -1381,14 +1377,14 @@ sr_status prepare_cached(sr_context *ctx, const sr_population *pop, uint32_t fla
   // Skeletons (reference mark_cached_subtrees_from_state + skeleton rewrite,
   // cl_gpu_eval.cu:294-329, 433-459).
   ctx->hints.resize(static_cast<size_t>(T));
-  const int64_t removed = sr::mark_cached_subtrees(E, pop->tokens, pop->values, pop->offsets,
-                                                   ctx->cache, threads, ctx->hints.data());
+  sr::mark_cached_subtrees(E, pop->tokens, pop->values, pop->offsets, ctx->cache, threads,
+                           ctx->hints.data());
   SR_TRY(compile_set(ctx, E, pop->tokens, pop->values, pop->offsets, ctx->hints.data(), ctx->main,
                      nullptr, true));
   ctx->prep_stats.host_compile_time_ms = now_ms() - tc0;
   SR_TRY(prepare_main_shape(ctx, false, false));
   ctx->prep_stats.node_evals = T * ctx->N;
-  ctx->prep_stats.node_evals_executed = (T - removed + static_cast<int64_t>(sub_tok.size())) * ctx->N;
+  ctx->prep_stats.node_evals_executed = (ctx->main.n_executed + ctx->sub.n_executed) * ctx->N;
   return SR_OK;
 }
 

@@ -500,7 +500,7 @@ sr_status prepare_grad(sr_context *ctx, const sr_population *pop, bool recompute
                                      cudaMemcpyHostToDevice, s));
   }
   ctx->prep_stats.node_evals = ps.n_tokens * ctx->N;
-  ctx->prep_stats.node_evals_executed = ctx->prep_stats.node_evals;
+  ctx->prep_stats.node_evals_executed = ps.n_executed * ctx->N;
   return SR_OK;
 }
 

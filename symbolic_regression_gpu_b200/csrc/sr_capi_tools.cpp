@@ -216,7 +216,7 @@ static sr_status prepare_device_population(sr_context *ctx, const int32_t *token
   const size_t n_code = static_cast<size_t>(E) * (static_cast<size_t>(stride) + 1) + 1;
   SR_TRY_CUDA(ctx, ps.layout_device(n_code, static_cast<size_t>(E)));
   SR_TRY_CUDA(ctx, ps.layout_host(0, static_cast<size_t>(E)));  // the group table only
-  const size_t n_summary = 8 + 2 * static_cast<size_t>(E);
+  const size_t n_summary = sr::kCompileSummary + 2 * static_cast<size_t>(E);
   SR_TRY_CUDA(ctx, ctx->evo_summary.ensure(n_summary));
   SR_TRY_CUDA(ctx, ctx->h_evo_summary.ensure(n_summary));
   SR_TRY_CUDA(ctx, ctx->mse.ensure(static_cast<size_t>(E) + 1));
@@ -238,6 +238,7 @@ static sr_status prepare_device_population(sr_context *ctx, const int32_t *token
   int64_t n_tok = 0, n_ins = 0;
   std::memcpy(&n_tok, sm + 2, sizeof n_tok);
   std::memcpy(&n_ins, sm + 4, sizeof n_ins);
+  std::memcpy(&ps.n_executed, sm + 8, sizeof ps.n_executed);
   ps.smax = sm[0];
   ps.n_tokens = n_tok;
   ps.n_instr = n_ins;
@@ -249,8 +250,9 @@ static sr_status prepare_device_population(sr_context *ctx, const int32_t *token
   ps.cost.resize(static_cast<size_t>(E));
   for (int x = 0; x < E; ++x) {
     ps.h_off.p[x] = static_cast<int64_t>(x) * (stride + 1);
-    ps.h_len.p[x] = sm[8 + 2 * x];
-    std::memcpy(&ps.cost[static_cast<size_t>(x)], sm + 9 + 2 * x, sizeof(float));
+    const int32_t *of_x = sm + sr::kCompileSummary + 2 * static_cast<int64_t>(x);
+    ps.h_len.p[x] = of_x[0];
+    std::memcpy(&ps.cost[static_cast<size_t>(x)], of_x + 1, sizeof(float));
   }
   ps.n_const.assign(static_cast<size_t>(E), 0);
   ps.sfu_per_dp = 0.0;
@@ -261,7 +263,7 @@ static sr_status prepare_device_population(sr_context *ctx, const int32_t *token
   // context has one, else the profile's default.
   SR_TRY(prepare_main_shape(ctx, false, true));
   ctx->prep_stats.node_evals = n_tok * ctx->N;
-  ctx->prep_stats.node_evals_executed = ctx->prep_stats.node_evals;
+  ctx->prep_stats.node_evals_executed = ps.n_executed * ctx->N;
   ctx->mode = sr::Mode::kBatched;
   return SR_OK;
 }

@@ -171,7 +171,8 @@ struct ProgramSet {
   int64_t n_instr_protected = 0;  // instructions whose opcode kOpsProtected dispatches inline
   bool cache_refs = false;        // some instruction reads a cached subtree
   int64_t n_tokens = 0;      // tokens represented (skeleton-equivalent)
-  double sfu_per_dp = 0.0;   // declared work, summed over expressions
+  int64_t n_executed = 0;    // tokens the programs evaluate at every datapoint
+  double sfu_per_dp = 0.0;   // declared work of the programs, summed over expressions
   double fp32_per_dp = 0.0;
   int n_listed = 0;    // distinct expressions: the ones in the group table
   bool shared = false; // row holds each expression's representative
@@ -369,7 +370,7 @@ struct sr_context {
   sr::DevBuf<int32_t> evo_idx;     // [E]
   sr::DevBuf<int32_t> evo_order;   // [E]
   sr::DevBuf<float> evo_fit;       // [E] fitness in rank order
-  sr::DevBuf<int32_t> evo_summary; // [8 + 2E] see launch_compile_device
+  sr::DevBuf<int32_t> evo_summary; // [kCompileSummary + 2E] see launch_compile_device
   sr::PinnedBuf<int32_t> h_evo_summary;
 
   // timing

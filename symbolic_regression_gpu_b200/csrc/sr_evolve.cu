@@ -562,21 +562,26 @@ __global__ void compile_kernel(const int32_t *__restrict__ tok, const float *__r
     return;
   }
   code_len[i] = count;
-  int prot = 0;
+  int prot = 0, nodes = 0;
   float cost = 6.0f;  // the host compiler's model: its group table is built from these
   for (int k = 0; k < count; ++k) {
     const uint32_t w = with_dispatch(code[base + k].w);
     code[base + k].w = w;
     prot += in_protected_profile(instr_op(w)) ? 1 : 0;
     cost += instr_cost(w);
+    const uint32_t bk = instr_b_kind(w);  // the operator and its leaves
+    nodes += (instr_op(w) != 0) + (instr_load(w) ? 1 : 0) + (bk != kBNone && bk != kBS);
   }
-  summary[8 + 2 * i] = count;
-  summary[9 + 2 * i] = __float_as_int(cost);
+  int32_t *mine = summary + kCompileSummary + 2 * static_cast<int64_t>(i);
+  mine[0] = count;
+  mine[1] = __float_as_int(cost);
   if (prot) atomicAdd(&summary[6], prot);
   atomicMax(&summary[0], need);
   atomicAdd(reinterpret_cast<unsigned long long *>(summary + 2), static_cast<unsigned long long>(n));
   atomicAdd(reinterpret_cast<unsigned long long *>(summary + 4),
             static_cast<unsigned long long>(count));
+  atomicAdd(reinterpret_cast<unsigned long long *>(summary + 8),
+            static_cast<unsigned long long>(nodes));
 }
 
 inline unsigned grid_for(int n, int block) { return static_cast<unsigned>((n + block - 1) / block); }
@@ -630,7 +635,7 @@ cudaError_t launch_compile_device(const int32_t *tok, const float *val, const in
                                   int E, int stride, int num_vars, Instr *code,
                                   int64_t *code_off, int32_t *code_len, int32_t *summary,
                                   cudaStream_t s) {
-  cudaError_t err = cudaMemsetAsync(summary, 0, 8 * sizeof(int32_t), s);
+  cudaError_t err = cudaMemsetAsync(summary, 0, kCompileSummary * sizeof(int32_t), s);
   if (err != cudaSuccess || E <= 0) return err;
   compile_kernel<<<grid_for(E, 64), 64, 0, s>>>(tok, val, len, E, stride, num_vars, code,
                                                 code_off, code_len, summary);

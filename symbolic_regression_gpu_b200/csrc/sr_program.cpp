@@ -232,18 +232,6 @@ const OpTables &op_tables() {
 
 }  // namespace
 
-void declared_work(const int32_t *tok, int len, double *sfu, double *fp32) {
-  const OpTables &tab = op_tables();
-  float s = 0.f, f = 0.f;
-  for (int i = 0; i < len; ++i)
-    if (tok[i] > 0) {
-      s += tab.sfu[tok[i] & 63];
-      f += tab.fp32[tok[i] & 63];
-    }
-  *sfu = s;
-  *fp32 = f;
-}
-
 sr_status compile_expression(const int32_t *tok, const double *val, int len,
                              int num_vars, const int32_t *hints,
                              std::vector<Instr> &out, ExprInfo &info,
@@ -373,6 +361,7 @@ sr_status compile_expression(const int32_t *tok, const double *val, int len,
   }
   const int root = stk[0];
   info.n_const = static_cast<int>(n_const);
+  info.n_executed = n_nodes;
   info.need = nodes[root].need;
   if (info.need > kMaxSpillSlots) {
     if (err) *err = "expression needs " + std::to_string(info.need) +

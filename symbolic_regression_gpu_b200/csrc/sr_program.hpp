@@ -13,6 +13,7 @@ namespace sr {
 // Result of compiling one expression.
 struct ExprInfo {
   int32_t n_tokens = 0;   // tokens of the original expression
+  int32_t n_executed = 0; // of which the program evaluates (a collapsed subtree is one)
   int32_t n_instr = 0;    // bytecode instructions
   int32_t need = 0;       // spill slots used
   int32_t n_const = 0;    // SR_TOK_CONST tokens (adjoint numbering)
@@ -52,9 +53,6 @@ sr_status compile_expression(const int32_t *tok, const double *val, int len,
 // SFU / FP32 operation counts), used for the roofline; not CUDA's
 // implementation.
 void declared_op_work(int tok, double *sfu, double *fp32);
-
-// The same for a whole token run.
-void declared_work(const int32_t *tok, int len, double *sfu, double *fp32);
 
 // Modelled relative device cost of one operator per datapoint (used only to
 // balance warps; calibrated by hand against instruction counts).
