@@ -1,12 +1,15 @@
 // sr_parallel.hpp — host-side parallel passes: a fork-join helper for one-off
 // passes, and a pool of waiting workers for the passes of every call.
 #pragma once
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
 #include <condition_variable>
 #include <cstdint>
 #include <exception>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <system_error>
 #include <thread>
@@ -43,12 +46,19 @@ class WorkerPool {
   WorkerPool(const WorkerPool &) = delete;
   WorkerPool &operator=(const WorkerPool &) = delete;
   ~WorkerPool() {
+    if (!workers_.empty() && getpid() != owner_) {
+      // A forked process holds a copy without the threads: joining them, or
+      // destroying what they sleep on, would wait for ever.
+      new std::vector<std::thread>(std::move(workers_));
+      wake_.release();
+      return;
+    }
     {
       std::lock_guard<std::mutex> lock(m_);
       stop_ = true;
       generation_.fetch_add(1);
     }
-    wake_.notify_all();
+    wake_->notify_all();
     for (auto &t : workers_) t.join();
   }
 
@@ -73,7 +83,7 @@ class WorkerPool {
       std::lock_guard<std::mutex> lock(m_);
       generation_.fetch_add(1);
     }
-    if (sleepers_.load() > 0) wake_.notify_all();
+    if (sleepers_.load() > 0) wake_->notify_all();
     work();
     // Every chunk done, then no worker left inside the pass: the next one may
     // change its description.
@@ -93,6 +103,7 @@ class WorkerPool {
       std::this_thread::yield();
   }
   void grow(int want) {
+    if (workers_.empty()) owner_ = getpid();
     while (static_cast<int>(workers_.size()) < want) {
       try {
         workers_.emplace_back([this] { loop(); });
@@ -118,7 +129,7 @@ class WorkerPool {
       if (generation_.load() == seen) {
         std::unique_lock<std::mutex> lock(m_);
         sleepers_.fetch_add(1);
-        wake_.wait(lock, [&] { return generation_.load() != seen; });
+        wake_->wait(lock, [&] { return generation_.load() != seen; });
         sleepers_.fetch_sub(1);
       }
       seen = generation_.load();
@@ -132,8 +143,9 @@ class WorkerPool {
   }
 
   std::mutex m_;
-  std::condition_variable wake_;
+  std::unique_ptr<std::condition_variable> wake_{new std::condition_variable};
   std::vector<std::thread> workers_;
+  pid_t owner_ = 0;  // the process that started them
   const std::function<void(int)> *fn_ = nullptr;
   int chunks_ = 0;
   std::atomic<int> next_{0}, pending_{0}, inside_{0}, sleepers_{0};
