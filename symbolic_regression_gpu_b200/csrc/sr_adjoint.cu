@@ -3,7 +3,7 @@
 // (No reference counterpart: the reference evaluates MSE only.)
 //
 //   adj_kernel<GTAPE>       fused forward + backward per tile.  Same work
-//                           decomposition as interp_kernel (a producer thread
+//                           decomposition as interp_kernel (a producer warp
 //                           streaming X spans into shared memory, warps
 //                           claiming expressions of a group).  Per tile a warp
 //                           (1) runs the program forward; each instruction's

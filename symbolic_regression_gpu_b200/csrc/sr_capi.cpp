@@ -263,11 +263,11 @@ static sr_status upload_folds(sr_context *ctx) {
 // in global scratch, 46.9).  A bounded part of the device's memory too.
 static int derived_row_limit(const sr_context *ctx, int slots) {
   const int fit = (ctx->max_smem - 9 * 1024 - slots * 31 * 1024) / 4096;
-  int r = std::min(24, fit - (ctx->V + 1));
+  int r = std::min(sr::kMaxDerivedRows, fit - (ctx->V + 1));
   const double row = static_cast<double>(ctx->ldx) * sizeof(float);
   const double room = std::min(1073741824.0, static_cast<double>(ctx->device_memory) / 16.0);
   r = std::min(r, static_cast<int>(room / row));
-  return r < 4 ? 0 : std::min(r, sr::kMaxDerivedRows);
+  return r < 4 ? 0 : r;
 }
 
 // Whether finding shared work pays.  The search and the two more kernels cost
@@ -810,8 +810,7 @@ sr_status prepare_main_shape(sr_context *ctx, bool allow_tune, bool on_device) {
     const bool have = it != ctx->tuned.end();
     int wide = 8;
     if (prot) {
-      const int s_smem = std::min(std::max(ps.smax, 0),
-                                  ps.n_derived > 0 ? 2 : sr::smem_spill_slots(8));
+      const int s_smem = std::min(std::max(ps.smax, 0), sr::smem_spill_slots(8));
       const int W = sr::kMaxInterpWarps;
       if (sr::interp_smem_bytes(8, W, ctx->V + ps.n_derived, s_smem, 32 * 8 * 2, W * 4, false) <=
           static_cast<size_t>(ctx->max_smem))

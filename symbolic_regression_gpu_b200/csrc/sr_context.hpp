@@ -280,9 +280,9 @@ struct GradSet {
   PinnedBuf<float> h_consts;
   PinnedBuf<int32_t> h_groups;
   std::vector<AdjClass> classes;
-  // Forward-mode launches, their mask words ([instructions + 1], aligned with
-  // the code) and span-group sums; the expression lists (tangent sets first,
-  // then the reverse-mode expressions) that the finalize kernels walk.
+  // Forward-mode launches and their span-group sums; the expression lists
+  // (tangent sets first, then the reverse-mode expressions by class, each in the
+  // order of its group table) that the finalize kernels walk.
   std::vector<TanSet> tsets;
   DevBuf<double2> tan_partial;
   DevBuf<double> tan_gout;

@@ -939,7 +939,7 @@ struct SpanPart {
   int32_t e;    // expression
 };
 
-// Per-item accumulator of one expression (producer thread only): the span
+// Per-item accumulator of one expression (producer warp only): the span
 // sums added in span order as a double-double (hi + lo, Knuth's two-sum), so
 // that the result does not depend on how many spans an item covers.
 struct GroupAcc {

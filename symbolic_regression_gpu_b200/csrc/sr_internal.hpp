@@ -215,13 +215,14 @@ constexpr uint32_t kFoldA = 1u << 30, kFoldB = 1u << 31;
 //
 // Work decomposition: expressions are sorted by modelled cost (descending)
 // and cut into groups of G; the datapoint axis is cut into spans of `span`
-// datapoints.  A work item is (span, group); items are numbered span-major
-// and handed out by an atomic counter to persistent blocks.  A block's
-// producer thread copies the item's X span (all V+1 rows) into one of two
-// shared-memory buffers with the bulk-copy engine; the block's evaluating
-// warps claim the group's expressions one at a time from a shared counter and
-// run each over the whole span, tile by tile (32*DPT datapoints per tile).
-// Warps never wait for each other inside an item.
+// datapoints, consecutive spans into span groups.  A work item is (span group,
+// group), numbered group-major; a persistent block takes the item of its own
+// index first and the others from an atomic counter.  Its producer warp copies
+// the item's spans, one after the other, into one of two shared-memory buffers
+// with the bulk-copy engine (all V+1 rows of X, and the derived ones); the
+// block's evaluating warps claim the group's expressions one at a time from a
+// shared counter and run each over the whole span, tile by tile (32*DPT
+// datapoints per tile).  Warps never wait for each other inside an item.
 struct EvalArgs {
   const float *X;        // [(V+1)][ldx], y in row V
   int64_t ldx;           // row stride (floats), multiple of 4096
@@ -232,7 +233,7 @@ struct EvalArgs {
   const int32_t *group_expr; // [n_groups * G] expression index or -1 (tail): gradient launches
   const GroupRec *groups;    // [n_groups * G] the same with its program: interpreter launches
   double2 *partial;      // [n_span_groups][E] x 2 (MSE launches; see span_per_item)
-  int32_t *work_counter; // zeroed before each launch
+  int32_t *work_counter; // zero when the launch starts
   int32_t *error;        // device error word
   const float *cache;    // subtree cache [slot][ldc] (cached-subtree operands)
   int64_t ldc;

@@ -23,7 +23,7 @@
 //
 // The interpreter evaluates two datapoints at once with the paired FP32
 // instructions of sm_100 (fma.rn.f32x2 and friends: sincos_parts2,
-// sr_log_nonneg2); each half is the same correctly rounded operation as the
+// sr_log_normal2); each half is the same correctly rounded operation as the
 // scalar form, so both forms give identical results.
 //
 // Their accuracy is measured on every float argument against the correctly
@@ -287,33 +287,7 @@ __device__ __forceinline__ float sr_log_nonneg(float a) {
   return (a == 0.0f) ? __int_as_float(0xff800000) : (a < INFINITY ? r : a);
 }
 
-// sr_log_nonneg of two arguments, the polynomial in paired operations.
-__device__ __forceinline__ float2 sr_log_nonneg2(float a0, float a1) {
-  const bool sub0 = a0 < 1.17549435e-38f, sub1 = a1 < 1.17549435e-38f;
-  const float as0 = sub0 ? __fmul_rn(a0, 8388608.0f) : a0;
-  const float as1 = sub1 ? __fmul_rn(a1, 8388608.0f) : a1;
-  const int ia0 = __float_as_int(as0), ia1 = __float_as_int(as1);
-  const int e0 = (ia0 - 0x3f3504f3) >> 23, e1 = (ia1 - 0x3f3504f3) >> 23;
-  const float2 m = make_float2(__int_as_float(ia0 - (e0 << 23)), __int_as_float(ia1 - (e1 << 23)));
-  const float2 f = __fadd2_rn(m, f2(-1.0f));
-  const float2 ef = make_float2(static_cast<float>(sub0 ? e0 - 23 : e0),
-                                static_cast<float>(sub1 ? e1 - 23 : e1));
-  float2 p = __ffma2_rn(f2(kR7), f, f2(kR6));
-  p = __ffma2_rn(p, f, f2(kR5));
-  p = __ffma2_rn(p, f, f2(kR4));
-  p = __ffma2_rn(p, f, f2(kR3));
-  p = __ffma2_rn(p, f, f2(kR2));
-  p = __ffma2_rn(p, f, f2(kR1));
-  p = __ffma2_rn(p, f, f2(kR0));
-  p = __ffma2_rn(p, f, f2(-0.5f));
-  const float2 y = __ffma2_rn(__fmul2_rn(f, f), p, f);
-  const float2 r = __ffma2_rn(ef, f2(kLn2Hi), __ffma2_rn(ef, f2(kLn2Lo), y));
-  return make_float2(
-      (a0 == 0.0f) ? __int_as_float(0xff800000) : (a0 < INFINITY ? r.x : a0),
-      (a1 == 0.0f) ? __int_as_float(0xff800000) : (a1 < INFINITY ? r.y : a1));
-}
-
-// The same for two positive normal arguments: no scaling, no special cases
+// sr_log_nonneg of two positive normal arguments: no scaling, no special cases
 // (the exponent becomes a float by adding it to the low bits of 1.5 * 2^23).
 __device__ __forceinline__ float2 sr_log_normal2(float a0, float a1) {
   const int ia0 = __float_as_int(a0), ia1 = __float_as_int(a1);

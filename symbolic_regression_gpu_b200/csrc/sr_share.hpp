@@ -28,7 +28,7 @@ namespace sr {
 constexpr int32_t kHintFold = -3;      // root of a subtree of constants
 constexpr int32_t kHintRow0 = -16;     // root of derived row r: kHintRow0 - r
 
-constexpr int kMaxDerivedRows = 64;
+constexpr int kMaxDerivedRows = 24;
 constexpr int kMaxSharedTokens = 64;   // largest subtree folded or made a row
 
 // Marks the maximal subtrees of constants of one expression (operators over
