@@ -363,7 +363,8 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, MINB) tan_kernel(const TanArg
 // through the tangent kernel's own operators and zero rule (the rows of these
 // constants would hold the same products at the subtree's root), and the
 // partials met on the way.  A subtree's work is that of a few datapoints; the
-// launch over all of them is latency-bound (5 us).
+// launch over all of them is latency-bound: one thread's chain of operators, once per
+// constant (91 us from cold caches for 4,096 trees with 1 to 8 constants).
 constexpr int kMaxFoldDepth = 40;  // values waiting in a subtree of 64 tokens
 __global__ void __launch_bounds__(64)
     fold_grad_kernel(const GradFold *__restrict__ items, const uint2 *__restrict__ tokens, int n,
